@@ -201,13 +201,18 @@ const char* layer_fault(const lfm25_stack_model& model, const lfm25_stack_layer&
     return nullptr;
 }
 
-// y[m, n] = x[m, k] w[n, k]^T: tensor cores for bf16 shapes with 16-byte rows, plain f32 arithmetic otherwise.
+// y[m, n] = x[m, k] w[n, k]^T: tensor cores for shapes with 16-byte rows, plain f32 arithmetic otherwise.
 int32_t linear(lfm25_stack_executor* self, const lfm25_stack_linear& site, const void* x, void* y, size_t rows) {
     if (self->type == Activation::kBf16 && site.k % 8 == 0 && site.n % 8 == 0) {
         lfm25_slice x_slice = {const_cast<void*>(x), rows * site.k};
         lfm25_slice w_slice = {const_cast<void*>(site.weight), site.n * site.k};
         lfm25_slice y_slice = {y, rows * site.n};
         return lfm25_blaslt_linear_bf16(self->blaslt, x_slice, w_slice, y_slice, rows, site.n, site.k);
+    }
+    if (self->type == Activation::kF32 && lfm25::linear_f32_supports(x, site.weight, rows, site.n, site.k)) {
+        STACK_CUDA(lfm25::launch_linear_f32(self->blaslt->stream, x, site.weight, y, rows, site.n, site.k),
+                   "linear launch failed");
+        return LFM25_OK;
     }
     STACK_CUDA(lfm25::launch_linear_simt(self->blaslt->stream, self->type, x, site.weight, y, rows, site.n, site.k),
                "linear launch failed");

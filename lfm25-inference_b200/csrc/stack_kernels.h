@@ -103,8 +103,12 @@ cudaError_t launch_argmax_rows(cudaStream_t stream, Activation type, const void*
 cudaError_t launch_export_logits(cudaStream_t stream, Activation type, const void* logits, size_t pitch, float* out,
                                  size_t rows, size_t vocab, float softcap);
 
-// y[m, n] = sum_k x[m, k] w[n, k] with plain 32-bit multiply-adds: the matrix product of the f32 activation type and
-// of bf16 shapes that the tensor-core paths cannot take.
+// y[m, n] = sum_k x[m, k] w[n, k] for f32 activations with exact products and f32 sums on the tensor cores; rows of x and w
+// in whole 16-byte pieces (`supports`).
+bool linear_f32_supports(const void* x, const void* weight, size_t m, size_t n, size_t k);
+cudaError_t launch_linear_f32(cudaStream_t stream, const void* x, const void* weight, void* y, size_t m, size_t n, size_t k);
+
+// The same with plain 32-bit multiply-adds: shapes of either activation type that the tensor-core paths cannot take.
 cudaError_t launch_linear_simt(cudaStream_t stream, Activation type, const void* x, const void* weight, void* y,
                                size_t m, size_t n, size_t k);
 

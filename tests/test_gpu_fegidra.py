@@ -32,6 +32,15 @@ def check_layer(config, seed, device, dtype, portions, rank=5, change=None):
     assert error.max() <= {"float32": 5e-6, "bfloat16": 2e-2}[dtype], (int(error.argmax()), float(error.max()))
 
 
+def check_layer_rows(config, seed, device, portions, change):
+    """check_layer in f32 with every token against its own size."""
+    tensors = cases.random_tensors(config, seed)
+    change(tensors)
+    got, want = run_layer(config, tensors, device, "float32", portions)
+    error = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert error.max() <= 5e-6, (int(error.argmax()), float(error.max()))
+
+
 # ------------------------------------------------------------------------------------------------ mechanisms alone
 
 ATTENTION_SHAPES = [   # heads, kv_heads, dim, vdim, rot_dims, chunk
@@ -89,6 +98,24 @@ def test_feed_forward(device, dtype, width, ff):
     def only_feed_forward(tensors):
         tensors["l0.mix.o"][:] = 0.0
     check_layer(config, 17, device, dtype, [9, 2, 1], change=only_feed_forward)
+
+
+@pytest.mark.parametrize("width,ff", [(1024, 2048), (64, 136), (256, 1000), (52, 40)])
+def test_f32_products(device, width, ff):
+    """Row counts around the tiles of 16, 32 and 64 rows; sums long enough to be shared by a cluster, sizes that end inside
+    a round of 32 and inside a tile of 128 columns, one without 16-byte rows.  Products are exact and sums f32, so the
+    bound is that of the f32 type (2-norm per row; a serial f32 sum of 2048 products stays below 2e-6)."""
+    config = cases.config_of([cases.delta_layer(1, 16, ff=ff)], width=width)
+    check_layer(config, 29, device, "float32", [1, 15, 16, 17, 32, 33, 64, 65])
+
+
+def test_f32_products_of_large_and_tiny_values(device):
+    """Values over the whole range of exponents beside one another: nothing of x is lost when it is taken apart."""
+    config = cases.config_of([cases.delta_layer(1, 16, ff=64)], width=128)
+
+    def spread(tensors):
+        tensors["embed"] *= 2.0 ** np.random.default_rng(5).integers(-60, 60, tensors["embed"].shape[0])[:, None]
+    check_layer_rows(config, 31, device, [70], spread)
 
 
 @pytest.mark.parametrize("dtype", TYPES)
