@@ -460,72 +460,178 @@ context_order_kernel(const uint32_t* __restrict__ positions, uint32_t num_tokens
 // short_conv_segmented_lfm2_bf16 (kernels/short_conv.cu:100-143) without its loop over the tokens of a segment:
 // the "state" it carries is just the gated inputs g = b * x of the two previous tokens, kept unrounded inside a
 // segment, so y[t] = c[t] * (w0 g[t-2] + w1 g[t-1] + w2 g[t]) can be evaluated per token, operation for operation.
-// One CTA per token.  Only a segment's first two tokens need the stored state and only its first token's CTA
-// touches it: that CTA produces y for offsets 0 and 1 and then stores the new state (the gated inputs of the
-// segment's last two tokens, rounded to bf16), so no CTA reads a state another one writes.
+// A CTA takes kConvTile consecutive tokens, whose segments its warps look up side by side (32 segments per pass), and a
+// thread VEC channels of all of them with every load of the tile in flight at once.  Only a segment's first two tokens
+// need the stored state and only the thread that has its first token touches it: it produces y for offsets 0 and 1 and
+// then stores the new state (the gated inputs of the segment's last two tokens, rounded to bf16), so no thread reads a
+// state another one writes.
+// Bound by HBM (8 bytes per channel and token), in short steps by the look-up and one round of loads.  2048 channels, a CTA
+// per token with single loads against this: 8 x 512 tokens 36 -> 22 us, 31 single tokens + 201 14.4 -> 7.0 us (there the
+// look-up, one segment after another, took longer than the work).
+constexpr uint32_t kConvTile = 4;      // more leaves too few threads per SM for the registers, fewer re-reads more
+
+// VEC (8 or 1) consecutive bf16 values as loaded
+template <int VEC>
+struct RawBf16;
+template <>
+struct RawBf16<8> {
+    uint4 raw;
+    __device__ __forceinline__ void load(const __nv_bfloat16* source) { raw = *reinterpret_cast<const uint4*>(source); }
+    __device__ __forceinline__ float operator[](int i) const {       // bf16 -> f32 is a shift
+        const uint32_t word = i < 2 ? raw.x : (i < 4 ? raw.y : (i < 6 ? raw.z : raw.w));
+        return __uint_as_float(i % 2 == 0 ? word << 16 : word & 0xffff0000u);
+    }
+};
+template <>
+struct RawBf16<1> {
+    __nv_bfloat16 raw;
+    __device__ __forceinline__ void load(const __nv_bfloat16* source) { raw = *source; }
+    __device__ __forceinline__ float operator[](int) const { return __bfloat162float(raw); }
+};
+
+template <int VEC>
 __global__ void __launch_bounds__(kRowThreads)
-short_conv_segmented_kernel(const __nv_bfloat16* __restrict__ projected, const __nv_bfloat16* __restrict__ weight,
-                            __nv_bfloat16* __restrict__ states, const uint32_t* __restrict__ segment_offsets,
-                            const uint32_t* __restrict__ segment_slots, __nv_bfloat16* __restrict__ output,
+short_conv_segmented_kernel(const __nv_bfloat16* projected, const __nv_bfloat16* weight, __nv_bfloat16* states,
+                            const uint32_t* segment_offsets, const uint32_t* segment_slots, __nv_bfloat16* output,
                             size_t num_tokens, size_t num_segments, size_t hidden, size_t num_request_slots) {
+    // (no __restrict__: what the compiler takes for constant memory may be read above pdl_wait())
+    __shared__ uint32_t segment_begin[kConvTile], segment_end[kConvTile], segment_slot[kConvTile];
     pdl_launch_dependents();
     pdl_wait();
-    const size_t token = blockIdx.x;
-    if (token >= num_tokens) {
-        return;
-    }
-    size_t begin = 0;
-    size_t end = 0;
-    size_t slot = num_request_slots;
-    for (size_t segment = 0; segment < num_segments; ++segment) {
-        const size_t first = segment_offsets[segment];
-        const size_t last = segment_offsets[segment + 1];
-        if (token >= first && token < last) {
-            begin = first;
-            end = last < num_tokens ? last : num_tokens;
-            slot = segment_slots[segment];
-            break;
-        }
-    }
-    if (slot >= num_request_slots) {
-        return;   // not in any segment, or a slot beyond the state table: the reference skips the segment
-    }
-    const size_t offset = token - begin;
-    if (offset == 1) {
-        return;   // produced by the CTA of the segment's first token
-    }
-    const size_t row = hidden * 3;
-    for (size_t channel = threadIdx.x; channel < hidden; channel += blockDim.x) {
-        const float w0 = __bfloat162float(weight[channel * 3]);
-        const float w1 = __bfloat162float(weight[channel * 3 + 1]);
-        const float w2 = __bfloat162float(weight[channel * 3 + 2]);
-        auto gated_at = [&](size_t at) {
-            return __bfloat162float(projected[at * row + channel]) * __bfloat162float(projected[at * row + 2 * hidden + channel]);
-        };
-        auto gate_at = [&](size_t at) { return __bfloat162float(projected[at * row + hidden + channel]); };
-        if (offset >= 2) {
-            const float convolved = w0 * gated_at(token - 2) + w1 * gated_at(token - 1) + w2 * gated_at(token);
-            output[token * hidden + channel] = __float2bfloat16_rn(gate_at(token) * convolved);
-            continue;
-        }
-        __nv_bfloat162* state = reinterpret_cast<__nv_bfloat162*>(states) + slot * hidden + channel;
-        const float2 previous = __bfloat1622float2(*state);
-        const float g0 = gated_at(token);
-        output[token * hidden + channel] = __float2bfloat16_rn(gate_at(token) * (w0 * previous.x + w1 * previous.y + w2 * g0));
-        float state0 = previous.y;
-        float state1 = g0;
-        if (token + 1 < end) {
-            const float g1 = gated_at(token + 1);
-            output[(token + 1) * hidden + channel] =
-                __float2bfloat16_rn(gate_at(token + 1) * (w0 * previous.y + w1 * g0 + w2 * g1));
-            state0 = g0;
-            state1 = g1;
-            if (token + 2 < end) {
-                state0 = gated_at(end - 2);
-                state1 = gated_at(end - 1);
+    const size_t first = static_cast<size_t>(blockIdx.x) * kConvTile;
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    if (warp < kConvTile) {
+        // the first segment that holds the token; none, or a slot beyond the state table: the reference skips the token
+        const size_t token = first + warp;
+        if (lane == 0) segment_slot[warp] = 0xffffffffu;
+        __syncwarp();
+        for (size_t base = 0; token < num_tokens && base < num_segments; base += 32) {
+            const size_t segment = base + lane;
+            size_t begin = 0, end = 0;
+            if (segment < num_segments) {
+                begin = segment_offsets[segment];
+                end = segment_offsets[segment + 1];
+            }
+            const uint32_t owners = __ballot_sync(0xffffffffu, token >= begin && token < end);
+            if (owners != 0) {
+                if (lane == static_cast<uint32_t>(__ffs(static_cast<int>(owners)) - 1)) {
+                    const uint32_t slot = segment_slots[segment];
+                    segment_begin[warp] = static_cast<uint32_t>(begin);
+                    segment_end[warp] = static_cast<uint32_t>(end < num_tokens ? end : num_tokens);
+                    segment_slot[warp] = slot < num_request_slots ? slot : 0xffffffffu;
+                }
+                break;
             }
         }
-        *state = __floats2bfloat162_rn(state0, state1);
+    }
+    __syncthreads();
+    const size_t row = hidden * 3;
+    for (size_t channel = static_cast<size_t>(threadIdx.x) * VEC; channel < hidden;
+         channel += static_cast<size_t>(blockDim.x) * VEC) {
+        float w[3][VEC];
+        {
+            __align__(16) __nv_bfloat16 taps[3 * VEC];
+            if constexpr (VEC == 8) {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    reinterpret_cast<uint4*>(taps)[i] = reinterpret_cast<const uint4*>(weight + channel * 3)[i];
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) taps[i] = weight[channel * 3 + i];
+            }
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) {
+#pragma unroll
+                for (int tap = 0; tap < 3; ++tap) w[tap][v] = __bfloat162float(taps[3 * v + tap]);
+            }
+        }
+        // entry j is token first - 2 + j; what a token of the tile reads of the two before it is of its own segment
+        RawBf16<VEC> b[kConvTile + 2], x[kConvTile + 2], c[kConvTile];
+#pragma unroll
+        for (uint32_t j = 0; j < kConvTile + 2; ++j) {
+            const size_t token = first + j - 2;
+            const bool live = segment_slot[j < 2 ? 0 : j - 2] != 0xffffffffu &&
+                              (j >= 2 || first + j >= segment_begin[0] + size_t(2));
+            if (live) {
+                b[j].load(projected + token * row + channel);
+                x[j].load(projected + token * row + 2 * hidden + channel);
+                if (j >= 2) c[j < 2 ? 0 : j - 2].load(projected + token * row + hidden + channel);
+            }
+        }
+        struct Values {
+            float at[VEC];
+        };
+        auto gated = [&](const RawBf16<VEC>& b_raw, const RawBf16<VEC>& x_raw) {
+            Values g;
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) g.at[v] = b_raw[v] * x_raw[v];
+            return g;
+        };
+        auto gated_at = [&](size_t token) {
+            RawBf16<VEC> b_raw, x_raw;
+            b_raw.load(projected + token * row + channel);
+            x_raw.load(projected + token * row + 2 * hidden + channel);
+            return gated(b_raw, x_raw);
+        };
+        auto produce = [&](size_t token, const RawBf16<VEC>& c_raw, const Values& g2, const Values& g1, const Values& g0) {
+            float out[VEC];
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) {
+                const float convolved = w[0][v] * g2.at[v] + w[1][v] * g1.at[v] + w[2][v] * g0.at[v];
+                out[v] = c_raw[v] * convolved;
+            }
+            __nv_bfloat16* target = output + token * hidden + channel;
+            if constexpr (VEC == 8) {
+                *reinterpret_cast<uint4*>(target) = make_uint4(pack_bf16x2(out[0], out[1]), pack_bf16x2(out[2], out[3]),
+                                                               pack_bf16x2(out[4], out[5]), pack_bf16x2(out[6], out[7]));
+            } else {
+                *target = __float2bfloat16_rn(out[0]);
+            }
+        };
+#pragma unroll
+        for (uint32_t i = 0; i < kConvTile; ++i) {
+            const size_t token = first + i;
+            const uint32_t slot = segment_slot[i];
+            if (slot == 0xffffffffu) {
+                continue;              // tokens beyond the step have none either
+            }
+            const size_t begin = segment_begin[i], end = segment_end[i];
+            if (token == begin + 1) {
+                continue;              // produced beside the segment's first token
+            }
+            if (token != begin) {
+                produce(token, c[i], gated(b[i], x[i]), gated(b[i + 1], x[i + 1]), gated(b[i + 2], x[i + 2]));
+                continue;
+            }
+            __nv_bfloat162* state = reinterpret_cast<__nv_bfloat162*>(states) + static_cast<size_t>(slot) * hidden + channel;
+            Values older, newer;
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) {
+                const float2 previous = __bfloat1622float2(state[v]);
+                older.at[v] = previous.x;
+                newer.at[v] = previous.y;
+            }
+            const Values g0 = gated(b[i + 2], x[i + 2]);
+            produce(token, c[i], older, newer, g0);
+            older = newer;
+            newer = g0;
+            if (token + 1 < end) {
+                RawBf16<VEC> next_c;
+                next_c.load(projected + (token + 1) * row + hidden + channel);
+                const Values g1 = gated_at(token + 1);
+                produce(token + 1, next_c, older, newer, g1);
+                older = g0;
+                newer = g1;
+                if (token + 2 < end) {
+                    older = gated_at(end - 2);
+                    newer = gated_at(end - 1);
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) state[v] = __floats2bfloat162_rn(older.at[v], newer.at[v]);
+        }
     }
 }
 
@@ -611,7 +717,12 @@ cudaError_t launch_short_conv_segmented(cudaStream_t stream, const void* project
                                         const uint32_t* segment_offsets, const uint32_t* segment_slots, void* output,
                                         size_t num_tokens, size_t num_segments, size_t hidden,
                                         size_t num_request_slots) {
-    return launch_kernel(short_conv_segmented_kernel, static_cast<unsigned int>(num_tokens), kRowThreads, 0, stream, 1,
+    // eight channels in 16-byte pieces: three taps of bf16 per channel, two values of state
+    const bool vector = hidden % 8 == 0 && ((reinterpret_cast<uintptr_t>(projected) | reinterpret_cast<uintptr_t>(weight) |
+                                               reinterpret_cast<uintptr_t>(states) | reinterpret_cast<uintptr_t>(output)) & 15) == 0;
+    const size_t blocks = (num_tokens + kConvTile - 1) / kConvTile;
+    return launch_kernel(vector ? short_conv_segmented_kernel<8> : short_conv_segmented_kernel<1>,
+                         static_cast<unsigned int>(blocks), kRowThreads, 0, stream, 1,
                          static_cast<const __nv_bfloat16*>(projected), static_cast<const __nv_bfloat16*>(weight),
                          static_cast<__nv_bfloat16*>(states), segment_offsets, segment_slots,
                          static_cast<__nv_bfloat16*>(output), num_tokens, num_segments, hidden, num_request_slots);

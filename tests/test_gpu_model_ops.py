@@ -96,6 +96,26 @@ def test_short_conv_segmented(device):
     assert np.array_equal(bits_of(states), want_states)
 
 
+@pytest.mark.parametrize("hidden", [100, 264, 2048])
+def test_short_conv_segmented_tiles(device, hidden):
+    """Segments that begin and end at every place of a tile of four tokens, more of them than one look-up pass covers, with
+    and without 16-byte channels; bit-exact against the oracle."""
+    rng = np.random.default_rng(hidden)
+    chunks = np.array([1] * 33 + [2, 3, 4, 5, 6, 7, 8, 9, 1, 2, 13, 1])
+    offsets = np.concatenate([[0], np.cumsum(chunks)]).astype(np.uint32)
+    slots = rng.permutation(len(chunks) + 1).astype(np.uint32)[:len(chunks)]     # one of them may be beyond the table
+    projected = workloads.bf16_normal(rng, (int(chunks.sum()), 3 * hidden))
+    weight, stored = workloads.bf16_normal(rng, (hidden, 3), std=0.5), workloads.bf16_normal(rng, (len(chunks), hidden, 2))
+    want_states = stored.copy()
+    want = oracle.short_conv_segmented_bf16(projected, weight, want_states, offsets, slots)
+    states = to_bf16(stored, device)
+    output = torch.zeros((projected.shape[0], hidden), dtype=torch.bfloat16, device=device)
+    ops.short_conv_segmented_lfm2_bf16_into(to_bf16(projected, device), to_bf16(weight, device), states,
+                                            to_u32(offsets, device), to_u32(slots, device), output)
+    assert np.array_equal(bits_of(output), want)
+    assert np.array_equal(bits_of(states), want_states)
+
+
 def test_gather_rows(device):
     rng = np.random.default_rng(9)
     values = workloads.bf16_normal(rng, (11, 2048))
