@@ -80,3 +80,21 @@ def test_silu_mul(device, rows, width):
         ref_codes = torch.zeros_like(codes)
         refkernels.silu_mul_packed_bf16_to_e4m3(packed, ref_codes, 9.75)
         assert torch.equal(hidden, ref_hidden) and torch.equal(codes, ref_codes)
+
+
+@pytest.mark.parametrize("rows,width", [(1184, 8192), (1183, 8200), (300, 8184), (3, 2056)])
+def test_silu_mul_rows_of_several_vectors(device, rows, width):
+    """Either side of the row count from which a thread takes four vectors, rows that end inside a thread's vectors: the
+    rows of a large launch equal those of launches of one row."""
+    packed = to_bf16(workloads.bf16_normal(np.random.default_rng(width), (rows, 2 * width), std=2.0), device)
+    hidden, alone = (torch.zeros((rows, width), dtype=torch.bfloat16, device=device) for _ in range(2))
+    codes, codes_alone = (torch.zeros((rows, width), dtype=torch.uint8, device=device) for _ in range(2))
+    ops.silu_mul_packed_bf16_into(packed, hidden)
+    ops.silu_mul_packed_bf16_to_e4m3_into(packed, codes, 9.75)
+    for row in (0, rows // 2, rows - 1):
+        ops.silu_mul_packed_bf16_into(packed[row:row + 1], alone[row:row + 1])
+        ops.silu_mul_packed_bf16_to_e4m3_into(packed[row:row + 1], codes_alone[row:row + 1], 9.75)
+        assert torch.equal(hidden[row], alone[row]) and torch.equal(codes[row], codes_alone[row])
+    gate, up = packed.double().split(width, 1)
+    want = torch.nn.functional.silu(gate) * up
+    assert float((hidden.double() - want).norm() / want.norm()) < 2 ** -8       # one bf16 rounding: at most 2^-9 each
