@@ -6,7 +6,7 @@
 //
 // A column of S (one value channel) never meets another one, so a CTA takes the columns of one head of one sequence and
 // keeps them in registers over the whole segment: the state is read from and written to memory once per step however
-// long the segment is.  Four kernels:
+// long the segment is.  Few long segments are split along the sequence instead (delta_split.cu).  Four kernels:
 //   decode    one token per sequence: every load is issued up front, then three barriers
 //   chunk     bf16 segments, heads up to 64: tiles of 16 tokens as matrix products on the tensor cores
 //   prompt    bf16 segments, larger heads: half of the warps prepare a tile of 16 tokens (decays with one small tensor-core product,
@@ -17,11 +17,12 @@
 // rounds like the scalar one).
 #include <math.h>
 
+#include <algorithm>
 #include <type_traits>
 
+#include "delta_rule.h"
 #include "launch.h"
 #include "options.h"
-#include "stack_common.cuh"
 
 namespace lfm25 {
 
@@ -56,27 +57,6 @@ __device__ __forceinline__ Pair mul_pair(Pair a, Pair b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(out) : "l"(a), "l"(b));
     return out;
 }
-
-constexpr float kUnitEps = 1e-6f;
-constexpr float kDecayScale = 0.60653065971263342f;    // exp(-1/2)
-
-template <typename T>
-struct DeltaArgs {
-    StackSegments segments;
-    uint32_t heads, dim, rank;
-    const T* projected;
-    size_t pitch;
-    const __nv_bfloat16* decay_up;
-    const __nv_bfloat16* decay_base;
-    const __nv_bfloat16* removal_bias;
-    const __nv_bfloat16* norm;
-    StackRecord record;
-    float* raw;
-    T* out;
-    size_t out_pitch;
-    float eps;
-    uint32_t splits;         // CTAs per head, each with COLUMNS value channels
-};
 
 constexpr uint32_t kTileTokens = 16;
 // per token in shared memory: r, w, -(a * u), u, k over the padded key channels, then v over them as well
@@ -557,11 +537,6 @@ __device__ __forceinline__ void copy_async_wait() {
 __device__ __forceinline__ void named_barrier(uint32_t id, uint32_t threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
-
-// The prompt kernel's decays and rates: the fast f32 exponential and division, a few units in the last place from the
-// correctly rounded ones.
-__device__ __forceinline__ float fast_sigmoid(float z) { return __fdividef(1.0f, 1.0f + __expf(-z)); }
-__device__ __forceinline__ float fast_tanh(float z) { return 1.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * z)); }
 
 constexpr uint32_t kPromptTokens = 16;       // tokens per tile = rows of one MMA tile
 constexpr uint32_t kRawStages = 4;           // being finished, in the recurrence, being prepared, arriving
@@ -1080,96 +1055,6 @@ struct ChunkLayout {
     }
 };
 
-// D(16x8) += A(16x8, tf32) * B(8x8, tf32), f32 accumulation
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const float (&a)[4], const float (&b)[2]) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-        "{%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
-          "r"(__float_as_uint(b[0])), "r"(__float_as_uint(b[1])));
-}
-
-// An operand fragment as high + low: the high part is what TF32 keeps of the value (10 mantissa bits), the low part the
-// rest, of which TF32 keeps another 10.
-template <int N>
-struct SplitFragment {
-    float high[N], low[N];
-    __device__ __forceinline__ void set(int index, float value) {
-        high[index] = __uint_as_float(__float_as_uint(value) & 0xffffe000u);
-        low[index] = value - high[index];
-    }
-};
-using FragmentA = SplitFragment<4>;
-using FragmentB = SplitFragment<2>;
-
-__device__ __forceinline__ void mma_split(float (&d)[4], const FragmentA& a, const FragmentB& b) {
-    mma_tf32(d, a.low, b.high);
-    mma_tf32(d, a.high, b.low);
-    mma_tf32(d, a.high, b.high);
-}
-// B is exact in TF32
-__device__ __forceinline__ void mma_split(float (&d)[4], const FragmentA& a, const float (&b)[2]) {
-    mma_tf32(d, a.low, b);
-    mma_tf32(d, a.high, b);
-}
-// The same for two accumulators, whose products alternate so that none waits for the one before it.
-__device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA& a, const FragmentB& b0, const FragmentB& b1) {
-    mma_tf32(d[0], a.low, b0.high);
-    mma_tf32(d[1], a.low, b1.high);
-    mma_tf32(d[0], a.high, b0.low);
-    mma_tf32(d[1], a.high, b1.low);
-    mma_tf32(d[0], a.high, b0.high);
-    mma_tf32(d[1], a.high, b1.high);
-}
-__device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA& a, const float (&b0)[2], const float (&b1)[2]) {
-    mma_tf32(d[0], a.low, b0);
-    mma_tf32(d[1], a.low, b1);
-    mma_tf32(d[0], a.high, b0);
-    mma_tf32(d[1], a.high, b1);
-}
-
-// rows `source[row * stride + column]` of a 16 x 8 operand
-__device__ __forceinline__ FragmentA load_a(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentA out;
-    const float* at = source + (lane >> 2) * stride + (lane & 3);
-    out.set(0, at[0]);
-    out.set(1, at[8 * stride]);
-    out.set(2, at[4]);
-    out.set(3, at[8 * stride + 4]);
-    return out;
-}
-// the same operand stored transposed: `source[column * stride + row]`
-__device__ __forceinline__ FragmentA load_a_transposed(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentA out;
-    const float* at = source + (lane & 3) * stride + (lane >> 2);
-    out.set(0, at[0]);
-    out.set(1, at[8]);
-    out.set(2, at[4 * stride]);
-    out.set(3, at[4 * stride + 8]);
-    return out;
-}
-// an 8 x 8 operand B[k][n] stored as `source[k * stride + n]`, or transposed as `source[n * stride + k]`
-__device__ __forceinline__ FragmentB load_b(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB out;
-    const float* at = source + (lane & 3) * stride + (lane >> 2);
-    out.set(0, at[0]);
-    out.set(1, at[4 * stride]);
-    return out;
-}
-__device__ __forceinline__ FragmentB load_b_transposed(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB out;
-    const float* at = source + (lane >> 2) * stride + (lane & 3);
-    out.set(0, at[0]);
-    out.set(1, at[4]);
-    return out;
-}
-// a 16 x 8 result to `target[row * stride + column]`
-__device__ __forceinline__ void store_c(float* target, uint32_t stride, uint32_t lane, const float (&c)[4]) {
-    float* at = target + (lane >> 2) * stride + (lane & 3) * 2;
-    *reinterpret_cast<float2*>(at) = make_float2(c[0], c[1]);
-    *reinterpret_cast<float2*>(at + 8 * stride) = make_float2(c[2], c[3]);
-}
-
 constexpr uint32_t kChunkThreads = 512;           // four groups of four warps
 static_assert(kChunkThreads == 8 * kChunkDim, "eight threads per channel stage W2");
 
@@ -1306,11 +1191,11 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
                 float from_state[2][2][4] = {};        // [U, R][8 columns]
 #pragma unroll
                 for (uint32_t k = 0; k < DP / 8; ++k) {
-                    const FragmentB b0 = load_b(state + k * 8 * kColumnStride, kColumnStride, lane);
-                    const FragmentB b1 = load_b(state + k * 8 * kColumnStride + 8, kColumnStride, lane);
+                    const FragmentB<> b0 = load_b(state + k * 8 * kColumnStride, kColumnStride, lane);
+                    const FragmentB<> b1 = load_b(state + k * 8 * kColumnStride + 8, kColumnStride, lane);
 #pragma unroll
                     for (uint32_t m = 0; m < 2; ++m) {
-                        const FragmentA a = load_a(operands + m * kOperandR + k * 8, kRowStride, lane);
+                        const FragmentA<> a = load_a(operands + m * kOperandR + k * 8, kRowStride, lane);
                         mma_split(from_state[m], a, b0, b1);
                     }
                 }
@@ -1331,7 +1216,7 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
                 // right-hand side, then Y
 #pragma unroll
                 for (uint32_t k = 0; k < 2; ++k) {
-                    const FragmentA a = load_a(triangles + 1 * kTriangle + k * 8, kTriangleStride, lane);
+                    const FragmentA<> a = load_a(triangles + 1 * kTriangle + k * 8, kTriangleStride, lane);
                     mma_split(from_state[0], a, v[k][0], v[k][1]);
                 }
                 store_c(columns, kColumnStride, lane, from_state[0][0]);
@@ -1340,7 +1225,7 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
                 float solved[2][4] = {};
 #pragma unroll
                 for (uint32_t k = 0; k < 2; ++k) {
-                    const FragmentA a = load_a(triangles + k * 8, kTriangleStride, lane);
+                    const FragmentA<> a = load_a(triangles + k * 8, kTriangleStride, lane);
                     mma_split(solved, a, load_b(columns + k * 8 * kColumnStride, kColumnStride, lane),
                               load_b(columns + k * 8 * kColumnStride + 8, kColumnStride, lane));
                 }
@@ -1348,7 +1233,7 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
                 store_c(columns, kColumnStride, lane, solved[0]);
                 store_c(columns + 8, kColumnStride, lane, solved[1]);
                 __syncwarp();
-                FragmentB y[2][2];
+                FragmentB<> y[2][2];
 #pragma unroll
                 for (uint32_t k = 0; k < 2; ++k) {
 #pragma unroll
@@ -1359,8 +1244,8 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
                 // O
 #pragma unroll
                 for (uint32_t k = 0; k < 2; ++k) {
-                    const FragmentA with_y = load_a(triangles + 2 * kTriangle + k * 8, kTriangleStride, lane);
-                    const FragmentA with_v = load_a(triangles + 3 * kTriangle + k * 8, kTriangleStride, lane);
+                    const FragmentA<> with_y = load_a(triangles + 2 * kTriangle + k * 8, kTriangleStride, lane);
+                    const FragmentA<> with_v = load_a(triangles + 3 * kTriangle + k * 8, kTriangleStride, lane);
                     mma_split(from_state[1], with_v, v[k][0], v[k][1]);
                     mma_split(from_state[1], with_y, y[k][0], y[k][1]);
                 }
@@ -1373,8 +1258,8 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
 #pragma unroll
                     for (uint32_t k = 0; k < 2; ++k) {
                         const uint32_t at = k * 8 * kTransposedStride + m * 16;
-                        const FragmentA with_v = load_a_transposed(operands + kOperandK + at, kTransposedStride, lane);
-                        const FragmentA with_y = load_a_transposed(operands + kOperandB + at, kTransposedStride, lane);
+                        const FragmentA<> with_v = load_a_transposed(operands + kOperandK + at, kTransposedStride, lane);
+                        const FragmentA<> with_y = load_a_transposed(operands + kOperandB + at, kTransposedStride, lane);
                         mma_split(accumulator[m], with_v, v[k][0], v[k][1]);
                         mma_split(accumulator[m], with_y, y[k][0], y[k][1]);
                     }
@@ -1583,7 +1468,7 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
                 float product[2][4] = {};
 #pragma unroll
                 for (uint32_t k = 0; k < DP / 8; ++k) {
-                    const FragmentA a = load_a(rows + k * 8, kRowStride, lane);
+                    const FragmentA<> a = load_a(rows + k * 8, kRowStride, lane);
                     mma_split(product, a, load_b_transposed(against + k * 8, kTransposedStride, lane),
                               load_b_transposed(against + 8 * kTransposedStride + k * 8, kTransposedStride, lane));
                 }
@@ -1673,6 +1558,31 @@ cudaError_t launch_chunk(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& ar
                          kChunkThreads, shared, stream, 1, args);
 }
 
+// Where prompts are split along the sequence (delta_split.cu): it does about twice the arithmetic of the kernels that carry
+// one head of one segment in a CTA, 0.16 us per head and 64 tokens over the whole chip against 12 us (bf16, four tiles) or
+// 64 us (f32, token by token) in a CTA, so it pays while those leave most SMs idle and a prompt is long enough for its
+// three launches.  Measured in whole steps of a 16-layer model with 32 heads, split against not: one prompt of 250 tokens
+// 1960 against 1929 us, 500: 2489 / 2869, 4000: 12316 / 15837; two prompts of 500: 3523 / 3544; eight of 250: 6099 / 5388.
+// In f32 with 16 heads: one prompt of 64 tokens 1187 / 1220 us, 250: 2508 / 3631; eight of 100: 4266 / 4294.
+template <typename T>
+constexpr size_t split_heads() { return std::is_same<T, float>::value ? 128 : 80; }
+template <typename T>
+constexpr size_t split_tokens() { return std::is_same<T, float>::value ? 64 : 256; }
+
+// The kernels' 16-byte and pairwise accesses, and scratch for one head at least.
+template <typename T>
+bool split_takes(const DeltaArgs<T>& args, const DeltaRuleLaunch& launch) {
+    const int64_t forced = option(kOptDeltaPrompt);
+    const size_t segments = launch.segments.num_segments;
+    const size_t tokens = launch.segments.num_tokens - launch.decode_tokens;
+    return (forced == 0 || forced == 4) && launch.segments.offsets != nullptr && args.dim <= 64 && args.dim % 8 == 0 &&
+           args.pitch % 8 == 0 && args.out_pitch % 2 == 0 && aligned_to(args.projected, 16) &&
+           aligned_to(args.out, 2 * sizeof(T)) && aligned_to(args.decay_up, 16) && aligned_to(args.decay_base, 4) &&
+           aligned_to(args.removal_bias, 4) && aligned_to(args.norm, 4) && launch.chunks != nullptr &&
+           delta_split_bytes(1, tile_bound(launch.segments, 64)) <= launch.chunk_bytes &&
+           (forced == 4 || (segments * args.heads <= split_heads<T>() && tokens >= split_tokens<T>() * segments));
+}
+
 bool prompt_kernel_takes(const DeltaArgs<__nv_bfloat16>& args) {
     const size_t shared = args.dim <= 64 ? PromptLayout<64>(args.rank).total : PromptLayout<128>(args.rank).total;
     return args.dim % 8 == 0 && args.dim <= 128 && args.rank <= kPromptMaxRank && args.pitch % 8 == 0 &&
@@ -1737,9 +1647,10 @@ cudaError_t launch_typed(cudaStream_t stream, const DeltaRuleLaunch& launch) {
         if (launch.dim <= 64) return launch_decode<T, 64>(stream, args);
         return launch_decode<T, 128>(stream, args);
     }
+    if (split_takes(args, launch)) return launch_delta_split(stream, args, launch.chunks, launch.chunk_bytes);
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
         if (launch.segments.offsets != nullptr && option(kOptDeltaPrompt) != 2 && prompt_kernel_takes(args)) {
-            if (launch.dim <= kChunkDim && ChunkLayout(launch.rank).total <= 227 * 1024 && option(kOptDeltaPrompt) == 0) {
+            if (launch.dim <= kChunkDim && ChunkLayout(launch.rank).total <= 227 * 1024 && option(kOptDeltaPrompt) != 1) {
                 return launch_chunk(stream, args);
             }
             return launch.dim <= 64 ? launch_prompt<64, 4, 128>(stream, args) : launch_prompt<128, 4, 128>(stream, args);
@@ -1756,6 +1667,15 @@ cudaError_t launch_typed(cudaStream_t stream, const DeltaRuleLaunch& launch) {
 
 bool delta_rule_needs_scratch(uint32_t dim) { return dim > 128; }
 
+size_t delta_rule_chunk_bytes(Activation type, uint32_t heads, uint32_t dim, size_t tokens, size_t segments) {
+    const bool f32 = type == Activation::kF32;
+    const size_t shortest = f32 ? split_tokens<float>() : split_tokens<__nv_bfloat16>();
+    const size_t most = std::min(std::min(segments, tokens / shortest),
+                                 (f32 ? split_heads<float>() : split_heads<__nv_bfloat16>()) / heads);
+    if (dim > 64 || dim % 8 != 0 || most == 0) return 0;
+    return std::min(delta_split_bytes(heads, tokens / 64 + most), kDeltaChunkBytes);
+}
+
 cudaError_t launch_delta_rule(cudaStream_t stream, const DeltaRuleLaunch& launch) {
     const auto run = [&](const DeltaRuleLaunch& part) {
         return part.type == Activation::kF32 ? launch_typed<float>(stream, part)
@@ -1765,6 +1685,7 @@ cudaError_t launch_delta_rule(cudaStream_t stream, const DeltaRuleLaunch& launch
         return run(launch);
     }
     DeltaRuleLaunch decodes = launch;
+    decodes.decode_tokens = 0;
     decodes.segments.offsets = nullptr;
     decodes.segments.num_segments = launch.decode_tokens;
     decodes.segments.num_tokens = launch.decode_tokens;

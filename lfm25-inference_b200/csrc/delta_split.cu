@@ -1,0 +1,759 @@
+// The generalised delta rule over prompts, split along the sequence.
+//
+// Over a chunk of 64 tokens, with P_t the product of the decays of its tokens up to t, S_t = diag(P_t) Q_t and
+//     U_t = u_t P_(t-1),   R_t = r_t P_t,   K_t = k_t / P_t,   B_t = -(a_t u_t) / P_t          (per key channel)
+// the update is Q_t = Q_(t-1) + B_t (U_t^T Q_(t-1)) + K_t v_t^T.  With
+//     (I - tril(U B^T, -1)) [W | Z] = [U | tril(U K^T, -1) V]
+// the Q_(t-1)^T U_t of the chunk are W S_0 + Z, so the state behind the chunk and the outputs are linear in the state S_0
+// before it:
+//     S = A S_0 + D,          A = diag(P) (I + B^T W),        D = diag(P) (B^T Z + K^T V)
+//     O = R' S_0 + O',        R' = R + tril(R B^T) W,         O' = tril(R B^T) Z + tril(R K^T) V
+// Everything but S_0 belongs to one chunk alone.  Three kernels:
+//     form     A, D, R', O' of every chunk of every head                        all chunks side by side
+//     carry    S <- A S + D through each segment's chunks, S_0 in the place of D    one product of 64 x 64 x 16 per chunk
+//     finish   O = R' S_0 + O', norm, gate                                      all chunks side by side
+// so only `carry` is serial, in steps of 64 tokens of a single small product.  4096 tokens of 32 heads in bf16: 231 + 49 + 45 us
+// (one CTA per head, tile after tile of 16 tokens: 773 us on 32 SMs); 250 tokens of 16 heads in f32: 80 us for the three
+// (token by token: 253 us).
+//
+// Decays are multiplied up by a scan, never summed as logarithms: P_t and the 1 / P_s that meets it come from the same
+// factors, and both carry a handful of roundings.  A decay is at least exp(-exp(-1/2)), so 1 / P_t stays below 1e17 and a
+// product P_t / P_s keeps its relative accuracy.  All matrix products are TF32 with both operands in two parts (bf16 values
+// of v need no second one), with f32 sums; f32 activations take the product of the low parts too and keep the tensor
+// cores' sums short (a model of 8 layers, 250 tokens, against float64: 0.99e-6; with plain multiply-adds 0.94e-6).
+#include <algorithm>
+
+#include "delta_rule.h"
+#include "launch.h"
+
+namespace lfm25 {
+
+namespace {
+
+constexpr uint32_t kDim = 64;                      // padded head size
+constexpr uint32_t kTokens = 64;
+constexpr uint32_t kPitch = 72;                    // rows of U, R, K, B, V in shared memory
+constexpr uint32_t kLowerPitch = 68;
+constexpr uint32_t kInversePitch = 20;
+constexpr uint32_t kMatrix = kDim * kTokens;       // elements of A, D, R' and O'
+constexpr uint32_t kChunkFloats = 4 * kMatrix;
+constexpr uint32_t kD = kMatrix, kR = 2 * kMatrix, kO = 3 * kMatrix;     // behind A
+constexpr uint32_t kFormThreads = 256;
+constexpr uint32_t kCarryThreads = 128;
+constexpr uint32_t kCarryColumns = 16;
+constexpr uint32_t kCarryPitch = 20;
+constexpr uint32_t kCarryStages = 5;
+constexpr uint32_t kFinishThreads = 128;
+
+// Fragments in which k index c of a 16 x 8 operand stands for column (row of B) 2c, and c + 4 for 2c + 1: the accumulator of
+// one product is then an operand of the next as it is, and operands along a row are read two at a time.
+template <bool NEAREST>
+__device__ __forceinline__ FragmentA<NEAREST> load_a_pairs(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentA<NEAREST> out;
+    const float* at = source + (lane >> 2) * stride + (lane & 3) * 2;
+    const float2 upper = *reinterpret_cast<const float2*>(at), lower = *reinterpret_cast<const float2*>(at + 8 * stride);
+    out.set(0, upper.x);
+    out.set(1, lower.x);
+    out.set(2, upper.y);
+    out.set(3, lower.y);
+    return out;
+}
+template <bool NEAREST>
+__device__ __forceinline__ FragmentA<NEAREST> a_from_c(const float (&c)[4]) {
+    FragmentA<NEAREST> out;
+    out.set(0, c[0]);
+    out.set(1, c[2]);
+    out.set(2, c[1]);
+    out.set(3, c[3]);
+    return out;
+}
+template <bool NEAREST>
+__device__ __forceinline__ FragmentB<NEAREST> load_b_transposed_pairs(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentB<NEAREST> out;
+    const float2 both = *reinterpret_cast<const float2*>(source + (lane >> 2) * stride + (lane & 3) * 2);
+    out.set(0, both.x);
+    out.set(1, both.y);
+    return out;
+}
+template <bool NEAREST>
+__device__ __forceinline__ FragmentB<NEAREST> load_b_pairs(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentB<NEAREST> out;
+    const float* at = source + (lane & 3) * 2 * stride + (lane >> 2);
+    out.set(0, at[0]);
+    out.set(1, at[stride]);
+    return out;
+}
+__device__ __forceinline__ void load_c(const float* source, uint32_t stride, uint32_t lane, float (&c)[4]) {
+    const float* at = source + (lane >> 2) * stride + (lane & 3) * 2;
+    const float2 upper = *reinterpret_cast<const float2*>(at), lower = *reinterpret_cast<const float2*>(at + 8 * stride);
+    c[0] = upper.x;
+    c[1] = upper.y;
+    c[2] = lower.x;
+    c[3] = lower.y;
+}
+
+// d[n] += a * rows for eight column blocks, `rows` bf16 (exact in TF32) or f32; PAIRS: in the order of load_b_pairs
+template <bool PAIRS>
+__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA<false>& a, const __nv_bfloat16* rows,
+                                              uint32_t lane) {
+    const uint32_t first = (PAIRS ? (lane & 3) * 2 : lane & 3) * kPitch + (lane >> 2);
+    const uint32_t second = first + (PAIRS ? 1 : 4) * kPitch;
+#pragma unroll
+    for (uint32_t n = 0; n < 8; n += 2) {
+        const float b0[2] = {__bfloat162float(rows[first + n * 8]), __bfloat162float(rows[second + n * 8])};
+        const float b1[2] = {__bfloat162float(rows[first + n * 8 + 8]), __bfloat162float(rows[second + n * 8 + 8])};
+        mma_tf32(d[n], a.low, b0);
+        mma_tf32(d[n + 1], a.low, b1);
+        mma_tf32(d[n], a.high, b0);
+        mma_tf32(d[n + 1], a.high, b1);
+    }
+}
+template <bool PAIRS, bool NEAREST>
+__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA<NEAREST>& a, const float* rows, uint32_t lane) {
+#pragma unroll
+    for (uint32_t n = 0; n < 8; n += 2) {
+        FragmentB<NEAREST> b[2];
+#pragma unroll
+        for (uint32_t q = 0; q < 2; ++q) {
+            b[q] = PAIRS ? load_b_pairs<NEAREST>(rows + (n + q) * 8, kPitch, lane)
+                         : load_b<NEAREST>(rows + (n + q) * 8, kPitch, lane);
+        }
+        mma_split<NEAREST, 2>(d + n, a, b);
+    }
+}
+
+__device__ __forceinline__ float2 load_pair(const __nv_bfloat16* source) {
+    return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(source));
+}
+__device__ __forceinline__ float2 load_pair(const float* source) { return *reinterpret_cast<const float2*>(source); }
+
+// Element functions: the accuracy that each activation type's other kernels have
+template <typename T>
+__device__ __forceinline__ float sigmoid_of(float z) {
+    return std::is_same<T, float>::value ? sigmoidf(z) : fast_sigmoid(z);
+}
+template <typename T>
+__device__ __forceinline__ float tanh_of(float z) {
+    return std::is_same<T, float>::value ? tanhf(z) : fast_tanh(z);
+}
+template <typename T>
+__device__ __forceinline__ float decay_of(float logit) {
+    const float exponent = -kDecayScale * sigmoid_of<T>(logit);
+    return std::is_same<T, float>::value ? expf(exponent) : __expf(exponent);
+}
+
+template <typename T>
+__device__ __forceinline__ float reciprocal_of(float value) {
+    return std::is_same<T, float>::value ? 1.0f / value : __fdividef(1.0f, value);
+}
+
+template <typename T>
+struct FormShared {
+    float u[kTokens * kPitch];                     // U, then W
+    float r[kTokens * kPitch];
+    float k[kTokens * kPitch];                     // K, then Z
+    float b[kTokens * kPitch];
+    float lower[kTokens * kLowerPitch];            // tril(U B^T, -1), blocks on and below the diagonal
+    float inverse[4][16 * kInversePitch];          // of I - lower on the diagonal blocks
+    float block_decay[4][kDim];                    // products over 16 tokens
+    float squares[2][kTokens];                     // |k|^2 over half of the channels each
+    T v[kTokens * kPitch];
+};
+
+// About 6500 m16n8k8 products per chunk, eight cycles each per SM quarter, keep the tensor pipe 37 % busy; the rest is the
+// latency of the five stages between barriers, which two CTAs per SM hide in part.  Longer loops are not unrolled further:
+// the code then outgrows the instruction cache (251 -> 231 us).
+template <typename T>
+__global__ void __launch_bounds__(kFormThreads, std::is_same<T, float>::value ? 1 : 2)
+delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, float* chunks) {
+    constexpr uint32_t kParts = std::is_same<T, float>::value ? 3 : 2;       // bf16 parts of tanh(z): 24 or 16 bits
+    constexpr bool kNearest = std::is_same<T, float>::value;
+    extern __shared__ __align__(16) unsigned char form_shared[];
+    FormShared<T>& shared = *reinterpret_cast<FormShared<T>*>(form_shared);
+    pdl_launch_dependents();
+    pdl_wait();
+    const SegmentTile tile = locate_tile(args.segments, kTokens, blockIdx.x / head_count);
+    if (tile.count == 0) {
+        return;
+    }
+    const uint32_t head = head0 + blockIdx.x % head_count;
+    const uint32_t dim = args.dim;
+    const size_t width = static_cast<size_t>(args.heads) * dim;
+    const size_t head_base = static_cast<size_t>(head) * dim;
+    const T* projected = args.projected + static_cast<size_t>(tile.first) * args.pitch;
+    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+
+    // ---- V
+    constexpr uint32_t kPiece = 16 / sizeof(T);
+    for (uint32_t item = threadIdx.x; item < kTokens * kDim / kPiece; item += kFormThreads) {
+        const uint32_t token = item / (kDim / kPiece), column = item % (kDim / kPiece) * kPiece;
+        const bool inside = token < tile.count && column < dim;
+        copy_async_16(shared.v + token * kPitch + column,
+                      inside ? projected + token * args.pitch + 2 * width + head_base + column : projected, inside);
+    }
+    copy_async_commit();
+
+    // ---- r, k and the removal's logit: 16 tokens x 32 channels per warp, in the layout of the decay product below
+    const uint32_t block = warp % 4, half = warp / 4;
+    const uint32_t row0 = block * 16 + (lane >> 2), pair = (lane & 3) * 2;
+    float2 r[4][2], k[4][2], removal[4][2];
+#pragma unroll
+    for (uint32_t n = 0; n < 4; ++n) {
+        const uint32_t channel = half * 32 + n * 8 + pair;
+#pragma unroll
+        for (uint32_t i = 0; i < 2; ++i) {
+            const uint32_t token = row0 + i * 8;
+            r[n][i] = k[n][i] = removal[n][i] = make_float2(0.0f, 0.0f);
+            if (token < tile.count && channel < dim) {
+                const T* source = projected + token * args.pitch + head_base + channel;
+                r[n][i] = load_pair(source);
+                k[n][i] = load_pair(source + width);
+                removal[n][i] = load_pair(source + 4 * width);
+            }
+        }
+    }
+    // ---- decay logits W2 tanh(z), 64 columns of z at a time; their operands lie where U and R will
+    float logits[4][4] = {};
+    {
+        __nv_bfloat16* w2 = reinterpret_cast<__nv_bfloat16*>(form_shared);
+        __nv_bfloat16* parts = w2 + kDim * kPitch;
+        static_assert((1 + kParts) * kDim * kPitch * 2 <= 2 * kTokens * kPitch * 4, "inside U and R");
+        const bool vector_rank = args.rank % 8 == 0;
+        for (uint32_t z0 = 0; z0 < args.rank; z0 += 64) {
+            if (z0 > 0) __syncthreads();
+#pragma unroll
+            for (uint32_t step = 0; step < 2; ++step) {
+                const uint32_t item = threadIdx.x + step * kFormThreads;
+                const uint32_t row = item / 8, z = item % 8 * 8;
+                uint4 weight = make_uint4(0, 0, 0, 0);
+                if (row < dim && z0 + z < args.rank) {
+                    const __nv_bfloat16* source = args.decay_up + (head_base + row) * args.rank + z0 + z;
+                    if (vector_rank) {
+                        weight = *reinterpret_cast<const uint4*>(source);
+                    } else {
+                        auto* elements = reinterpret_cast<__nv_bfloat16*>(&weight);
+                        for (uint32_t i = 0; i < 8 && z0 + z + i < args.rank; ++i) elements[i] = source[i];
+                    }
+                }
+                *reinterpret_cast<uint4*>(w2 + row * kPitch + z) = weight;
+                float value[8] = {};
+                if (row < tile.count && z0 + z < args.rank) {
+                    load_values<8>(projected + row * args.pitch + 5 * width + z0 + z, value);
+                }
+                // columns between rank and the end of its last 16 bytes belong to nobody
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) value[i] = z0 + z + i < args.rank ? tanh_of<T>(value[i]) : 0.0f;
+#pragma unroll
+                for (uint32_t part = 0; part < kParts; ++part) {
+                    uint32_t packed[4];
+#pragma unroll
+                    for (uint32_t i = 0; i < 4; ++i) {
+                        packed[i] = pack_bf16x2(value[2 * i], value[2 * i + 1]);
+                        const float2 rounded = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&packed[i]));
+                        value[2 * i] -= rounded.x;
+                        value[2 * i + 1] -= rounded.y;
+                    }
+                    *reinterpret_cast<uint4*>(parts + part * kTokens * kPitch + row * kPitch + z) =
+                        make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (uint32_t z = 0; z < 64; z += 16) {
+                uint32_t b[2][4];
+#pragma unroll
+                for (uint32_t q = 0; q < 2; ++q) {
+                    const uint32_t channel = half * 32 + q * 16 + lane / 16 * 8 + lane % 8;
+                    ldmatrix_x4(smem_u32(w2 + channel * kPitch + z + lane / 8 % 2 * 8), b[q][0], b[q][1], b[q][2], b[q][3]);
+                }
+#pragma unroll
+                for (uint32_t part = 0; part < kParts; ++part) {
+                    uint32_t a[4];
+                    ldmatrix_x4(smem_u32(parts + part * kTokens * kPitch + (block * 16 + lane % 16) * kPitch + z + lane / 16 * 8),
+                                a[0], a[1], a[2], a[3]);
+#pragma unroll
+                    for (uint32_t n = 0; n < 4; ++n) {
+                        mma_bf16_16816(logits[n], a[0], a[1], a[2], a[3], b[n / 2][n % 2 * 2], b[n / 2][n % 2 * 2 + 1]);
+                    }
+                }
+            }
+        }
+    }
+    // ---- products of the decays up to each token: of its block of 16 here, of the blocks before it below
+    float upto[4][4], before[4][4];
+    {
+        float squares[2] = {};
+#pragma unroll
+        for (uint32_t n = 0; n < 4; ++n) {
+            const uint32_t channel = half * 32 + n * 8 + pair;
+            float2 base = make_float2(0.0f, 0.0f);
+            if (channel < dim) base = load_pair(args.decay_base + head_base + channel);
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                upto[n][i] = row0 + (i >> 1) * 8 < tile.count ? decay_of<T>(logits[n][i] + (i & 1 ? base.y : base.x)) : 1.0f;
+            }
+#pragma unroll
+            for (uint32_t delta = 4; delta < 32; delta <<= 1) {
+#pragma unroll
+                for (uint32_t i = 0; i < 4; ++i) {
+                    const float other = __shfl_up_sync(0xffffffffu, upto[n][i], delta);
+                    if (lane >= delta) upto[n][i] *= other;
+                }
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < 2; ++i) {
+                const float first_half = __shfl_sync(0xffffffffu, upto[n][i], 28 + (lane & 3));
+                upto[n][2 + i] *= first_half;
+                const float upper = __shfl_up_sync(0xffffffffu, upto[n][i], 4);
+                const float lower = __shfl_up_sync(0xffffffffu, upto[n][2 + i], 4);
+                before[n][i] = lane < 4 ? 1.0f : upper;
+                before[n][2 + i] = lane < 4 ? first_half : lower;
+            }
+            if (lane >= 28) {
+                *reinterpret_cast<float2*>(&shared.block_decay[block][channel]) = make_float2(upto[n][2], upto[n][3]);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < 2; ++i) squares[i] = fmaf(k[n][i].x, k[n][i].x, fmaf(k[n][i].y, k[n][i].y, squares[i]));
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 2; ++i) {
+            squares[i] += __shfl_xor_sync(0xffffffffu, squares[i], 1);
+            squares[i] += __shfl_xor_sync(0xffffffffu, squares[i], 2);
+            if ((lane & 3) == 0) shared.squares[half][row0 + i * 8] = squares[i];
+        }
+    }
+    __syncthreads();
+
+    // ---- U, R, K, B
+#pragma unroll
+    for (uint32_t n = 0; n < 4; ++n) {
+        const uint32_t channel = half * 32 + n * 8 + pair;
+        float2 earlier = make_float2(1.0f, 1.0f), bias = make_float2(0.0f, 0.0f);
+        for (uint32_t other = 0; other < block; ++other) {
+            const float2 decay = *reinterpret_cast<const float2*>(&shared.block_decay[other][channel]);
+            earlier.x *= decay.x;
+            earlier.y *= decay.y;
+        }
+        if (channel < dim) bias = load_pair(args.removal_bias + head_base + channel);
+#pragma unroll
+        for (uint32_t i = 0; i < 2; ++i) {
+            const uint32_t token = row0 + i * 8;
+            const float square = shared.squares[0][token] + shared.squares[1][token] + kUnitEps;
+            const float unit = std::is_same<T, float>::value ? 1.0f / sqrtf(square) : rsqrtf(square);
+            const float px = upto[n][2 * i] * earlier.x, py = upto[n][2 * i + 1] * earlier.y;
+            const float ix = reciprocal_of<T>(px), iy = reciprocal_of<T>(py);
+            const float ux = k[n][i].x * unit, uy = k[n][i].y * unit;
+            const uint32_t at = token * kPitch + channel;
+            *reinterpret_cast<float2*>(shared.u + at) =
+                make_float2(ux * (before[n][2 * i] * earlier.x), uy * (before[n][2 * i + 1] * earlier.y));
+            *reinterpret_cast<float2*>(shared.r + at) = make_float2(r[n][i].x * px, r[n][i].y * py);
+            *reinterpret_cast<float2*>(shared.k + at) = make_float2(k[n][i].x * ix, k[n][i].y * iy);
+            *reinterpret_cast<float2*>(shared.b + at) = make_float2(-sigmoid_of<T>(removal[n][i].x + bias.x) * ux * ix,
+                                                                    -sigmoid_of<T>(removal[n][i].y + bias.y) * uy * iy);
+        }
+    }
+    copy_async_wait<0>();
+    __syncthreads();
+
+    float* chunk = chunks + static_cast<size_t>(blockIdx.x) * kChunkFloats;
+    // Warps 0..3 take 16 tokens of U each, the others 16 tokens of R, the long rows of one beside the short ones of the other.
+    const bool forward = warp < 4;
+    const uint32_t mine = forward ? warp : 7 - warp;
+    const float* rows = (forward ? shared.u : shared.r) + mine * 16 * kPitch;
+    float with_values[8][4] = {};                  // tril(U K^T, -1) V or tril(R K^T) V
+    float against_b[4][2][4];                      // tril(R B^T), 16 x 16 each
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        if (j > mine) continue;
+        float with_b[2][4] = {}, with_k[2][4] = {};
+#pragma unroll 2
+        for (uint32_t c = 0; c < kDim; c += 8) {
+            const FragmentA<kNearest> a = load_a_pairs<kNearest>(rows + c, kPitch, lane);
+            const uint32_t at = j * 16 * kPitch + c;
+            mma_split(with_b, a, load_b_transposed_pairs<kNearest>(shared.b + at, kPitch, lane),
+                      load_b_transposed_pairs<kNearest>(shared.b + at + 8 * kPitch, kPitch, lane));
+            mma_split(with_k, a, load_b_transposed_pairs<kNearest>(shared.k + at, kPitch, lane),
+                      load_b_transposed_pairs<kNearest>(shared.k + at + 8 * kPitch, kPitch, lane));
+        }
+#pragma unroll
+        for (uint32_t n = 0; n < 2; ++n) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                const uint32_t row = (lane >> 2) + (i >> 1) * 8, column = n * 8 + pair + (i & 1);
+                const bool kept = j < mine || (forward ? column < row : column <= row);   // U meets the state before s = t
+                if (!kept) with_b[n][i] = with_k[n][i] = 0.0f;
+                against_b[j][n][i] = with_b[n][i];
+            }
+            if (forward) store_c(shared.lower + mine * 16 * kLowerPitch + j * 16 + n * 8, kLowerPitch, lane, with_b[n]);
+        }
+#pragma unroll
+        for (uint32_t n = 0; n < 2; ++n) {
+            multiply_rows<true>(with_values, a_from_c<kNearest>(with_k[n]), shared.v + (j * 16 + n * 8) * kPitch, lane);
+        }
+    }
+    float behind[8][4] = {};                       // K^T V, then D: 16 key channels per warp of the first four
+    if (forward) {
+        // column `lane` of the inverse of I - L: x_t = e_t + sum over s < t of L[t][s] x_s
+        __syncwarp();
+        const float* lower = shared.lower + mine * 16 * kLowerPitch + mine * 16;
+        float x[16];
+#pragma unroll
+        for (uint32_t t = 0; t < 16; ++t) {
+            float even = t == lane ? 1.0f : 0.0f, odd = 0.0f;
+#pragma unroll
+            for (uint32_t s = 0; s < t; s += 2) {
+                const float2 both = *reinterpret_cast<const float2*>(lower + t * kLowerPitch + s);
+                even = fmaf(both.x, x[s], even);
+                if (s + 1 < t) odd = fmaf(both.y, x[s + 1], odd);
+            }
+            x[t] = even + odd;
+            if (lane < 16) shared.inverse[mine][t * kInversePitch + lane] = x[t];
+        }
+#pragma unroll 2
+        for (uint32_t t = 0; t < kTokens; t += 8) {
+            multiply_rows<false>(behind, load_a_transposed<kNearest>(shared.k + t * kPitch + mine * 16, kPitch, lane),
+                                   shared.v + t * kPitch, lane);
+        }
+    }
+    __syncthreads();                               // K is free
+    if (forward) {
+#pragma unroll
+        for (uint32_t n = 0; n < 8; ++n) {
+            store_c(shared.k + mine * 16 * kPitch + n * 8, kPitch, lane, with_values[n]);
+        }
+    }
+    __syncthreads();
+
+    // ---- W (first four warps, over U) and Z (the others, over K): 16 columns per warp, 16 rows after 16 rows
+    {
+        float* columns = (forward ? shared.u : shared.k) + warp % 4 * 16;
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            float* target = columns + i * 16 * kPitch;
+            if (i > 0) {
+                float side[2][4];
+                load_c(target, kPitch, lane, side[0]);
+                load_c(target + 8, kPitch, lane, side[1]);
+#pragma unroll
+                for (uint32_t s = 0; s < i * 16; s += 8) {
+                    mma_split(side, load_a<kNearest>(shared.lower + i * 16 * kLowerPitch + s, kLowerPitch, lane),
+                              load_b<kNearest>(columns + s * kPitch, kPitch, lane), load_b<kNearest>(columns + s * kPitch + 8, kPitch, lane));
+                }
+                __syncwarp();
+                store_c(target, kPitch, lane, side[0]);
+                store_c(target + 8, kPitch, lane, side[1]);
+                __syncwarp();
+            }
+            float solved[2][4] = {};
+#pragma unroll
+            for (uint32_t s = 0; s < 16; s += 8) {
+                mma_split(solved, load_a<kNearest>(shared.inverse[i] + s, kInversePitch, lane),
+                          load_b<kNearest>(target + s * kPitch, kPitch, lane), load_b<kNearest>(target + s * kPitch + 8, kPitch, lane));
+            }
+            __syncwarp();
+            store_c(target, kPitch, lane, solved[0]);
+            store_c(target + 8, kPitch, lane, solved[1]);
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+
+    float from_state[8][4] = {};                   // A or R'
+    if (forward) {
+#pragma unroll 1
+        for (uint32_t t = 0; t < kTokens; t += 8) {
+            const FragmentA<kNearest> a = load_a_transposed<kNearest>(shared.b + t * kPitch + mine * 16, kPitch, lane);
+            multiply_rows<false>(from_state, a, shared.u + t * kPitch, lane);
+            multiply_rows<false>(behind, a, shared.k + t * kPitch, lane);
+        }
+        const uint32_t channel = mine * 16 + (lane >> 2);
+        float decay[2] = {1.0f, 1.0f};
+#pragma unroll
+        for (uint32_t other = 0; other < 4; ++other) {
+            decay[0] *= shared.block_decay[other][channel];
+            decay[1] *= shared.block_decay[other][channel + 8];
+        }
+#pragma unroll
+        for (uint32_t n = 0; n < 8; ++n) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                const float one = n * 8 + pair + (i & 1) == channel + (i >> 1) * 8 ? 1.0f : 0.0f;
+                from_state[n][i] = (from_state[n][i] + one) * decay[i >> 1];
+                behind[n][i] *= decay[i >> 1];
+            }
+        }
+    } else {
+#pragma unroll
+        for (uint32_t n = 0; n < 8; ++n) load_c(rows + n * 8, kPitch, lane, from_state[n]);
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            if (j > mine) continue;
+#pragma unroll
+            for (uint32_t n = 0; n < 2; ++n) {
+                const FragmentA<kNearest> a = a_from_c<kNearest>(against_b[j][n]);
+                multiply_rows<true>(from_state, a, shared.u + (j * 16 + n * 8) * kPitch, lane);
+                multiply_rows<true>(with_values, a, shared.k + (j * 16 + n * 8) * kPitch, lane);
+            }
+        }
+    }
+    float4* first = reinterpret_cast<float4*>(chunk + (forward ? 0 : kR)) + mine * 8 * 32 + lane;
+    float4* second = reinterpret_cast<float4*>(chunk + (forward ? kD : kO)) + mine * 8 * 32 + lane;
+#pragma unroll
+    for (uint32_t n = 0; n < 8; ++n) {
+        // A and R' as operands of the next product, D and O' as accumulators
+        first[n * 32] = make_float4(from_state[n][0], from_state[n][2], from_state[n][1], from_state[n][3]);
+        second[n * 32] = forward ? make_float4(behind[n][0], behind[n][1], behind[n][2], behind[n][3])
+                                 : make_float4(with_values[n][0], with_values[n][1], with_values[n][2], with_values[n][3]);
+    }
+}
+
+template <bool NEAREST>
+__device__ __forceinline__ FragmentA<NEAREST> operand_of(const float4& stored) {
+    FragmentA<NEAREST> out;
+    out.set(0, stored.x);
+    out.set(1, stored.y);
+    out.set(2, stored.z);
+    out.set(3, stored.w);
+    return out;
+}
+
+// A CTA carries 16 value columns of one head through one segment; a warp owns 16 key channels of A and D and copies them
+// into its own part of shared memory kCarryStages - 1 chunks ahead.  Bound by the chain load S, multiply, store S, barrier.
+template <typename T>
+__global__ void __launch_bounds__(kCarryThreads)
+delta_carry_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, float* chunks) {
+    constexpr bool kNearest = std::is_same<T, float>::value;
+    extern __shared__ __align__(16) float carry_shared[];
+    float4* stages = reinterpret_cast<float4*>(carry_shared);                     // [stage][10][thread]
+    float* states = carry_shared + kCarryStages * 10 * kCarryThreads * 4;         // [2][channel][kCarryPitch]
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t part = blockIdx.x % (kDim / kCarryColumns);
+    const uint32_t local_head = blockIdx.x / (kDim / kCarryColumns) % head_count;
+    const uint32_t segment = blockIdx.x / (kDim / kCarryColumns) / head_count;
+    const uint32_t head = head0 + local_head;
+    const size_t slot = args.segments.slots[segment];
+    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    auto chunks_of = [&](uint32_t which) {
+        const uint32_t begin = args.segments.offsets[which];
+        uint32_t end = args.segments.offsets[which + 1];
+        end = end < args.segments.num_tokens ? end : static_cast<uint32_t>(args.segments.num_tokens);
+        return end > begin ? (end - begin + kTokens - 1) / kTokens : 0u;
+    };
+    const uint32_t count = chunks_of(segment);
+    if (count == 0 || slot >= args.segments.num_request_slots) {
+        return;
+    }
+    uint32_t before = 0;
+    for (uint32_t other = lane; other < segment; other += 32) before += chunks_of(other);
+    before = __reduce_add_sync(0xffffffffu, before);
+
+    const uint32_t dim = args.dim;
+    float* state_base = reinterpret_cast<float*>(static_cast<unsigned char*>(args.record.base) + slot * args.record.stride +
+                                                 args.record.offset) +
+                        static_cast<size_t>(head) * dim * dim;
+    for (uint32_t item = threadIdx.x; item < kDim * kCarryColumns; item += kCarryThreads) {
+        const uint32_t column = part * kCarryColumns + item / kDim, row = item % kDim;
+        states[row * kCarryPitch + item / kDim] =
+            row < dim && column < dim ? state_base[static_cast<size_t>(column) * dim + row] : 0.0f;
+    }
+    auto chunk_of = [&](uint32_t index) {
+        return chunks + (static_cast<size_t>(before + index) * head_count + local_head) * kChunkFloats;
+    };
+    const uint32_t own = warp * 8 * 32 + lane;               // this lane's pieces of A; those of D start at own_d
+    const uint32_t own_d = own + part * 2 * 32;
+    auto load = [&](uint32_t index) {
+        if (index < count) {
+            const float4* a = reinterpret_cast<const float4*>(chunk_of(index)) + own;
+            const float4* d = reinterpret_cast<const float4*>(chunk_of(index) + kD) + own_d;
+            float4* stage = stages + index % kCarryStages * 10 * kCarryThreads + threadIdx.x;
+#pragma unroll
+            for (uint32_t n = 0; n < 8; ++n) copy_async_16(stage + n * kCarryThreads, a + n * 32, true);
+#pragma unroll
+            for (uint32_t n = 0; n < 2; ++n) copy_async_16(stage + (8 + n) * kCarryThreads, d + n * 32, true);
+        }
+        copy_async_commit();
+    };
+    for (uint32_t index = 0; index + 1 < kCarryStages; ++index) load(index);
+    for (uint32_t index = 0; index < count; ++index) {
+        copy_async_wait<kCarryStages - 2>();                 // a thread reads what it copied itself
+        __syncthreads();
+        load(index + kCarryStages - 1);
+        const float* state = states + index % 2 * kDim * kCarryPitch;
+        const float4* stage = stages + index % kCarryStages * 10 * kCarryThreads + threadIdx.x;
+        float sum[2][4], high_low[2][4] = {}, low_high[2][4] = {};
+#pragma unroll
+        for (uint32_t n = 0; n < 2; ++n) {
+            const float4 d = stage[(8 + n) * kCarryThreads];
+            sum[n][0] = d.x;
+            sum[n][1] = d.y;
+            sum[n][2] = d.z;
+            sum[n][3] = d.w;
+        }
+        float4 kept[2];
+#pragma unroll
+        for (uint32_t c = 0; c < 8; ++c) {
+            const FragmentA<kNearest> a = operand_of<kNearest>(stage[c * kCarryThreads]);
+            const float* rows = state + (c * 8 + (lane & 3) * 2) * kCarryPitch + (lane >> 2);
+#pragma unroll
+            for (uint32_t n = 0; n < 2; ++n) {
+                FragmentB<kNearest> b;
+                const float first = rows[n * 8], second = rows[n * 8 + kCarryPitch];
+                b.set(0, first);
+                b.set(1, second);
+                if (c == 2 * warp) {
+                    kept[n].x = first;
+                    kept[n].y = second;
+                } else if (c == 2 * warp + 1) {
+                    kept[n].z = first;
+                    kept[n].w = second;
+                }
+                if (kNearest) {
+                    mma_split(sum[n], a, b);
+                } else {
+                    mma_tf32(low_high[n], a.low, b.high);
+                    mma_tf32(high_low[n], a.high, b.low);
+                    mma_tf32(sum[n], a.high, b.high);
+                }
+            }
+        }
+        // the state before the chunk, as operands of the outputs' product
+        float4* before_chunk = reinterpret_cast<float4*>(chunk_of(index) + kD) + own_d;
+        float* next = states + (index + 1) % 2 * kDim * kCarryPitch + warp * 16 * kCarryPitch;
+#pragma unroll
+        for (uint32_t n = 0; n < 2; ++n) {
+            before_chunk[n * 32] = kept[n];
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) sum[n][i] += low_high[n][i] + high_low[n][i];
+            store_c(next + n * 8, kCarryPitch, lane, sum[n]);
+        }
+    }
+    __syncthreads();
+    const float* state = states + count % 2 * kDim * kCarryPitch;
+    for (uint32_t item = threadIdx.x; item < kDim * kCarryColumns; item += kCarryThreads) {
+        const uint32_t column = part * kCarryColumns + item / kDim, row = item % kDim;
+        if (row < dim && column < dim) {
+            state_base[static_cast<size_t>(column) * dim + row] = state[row * kCarryPitch + item / kDim];
+        }
+    }
+}
+
+__device__ __forceinline__ void store_pair(__nv_bfloat16* target, float low, float high) {
+    *reinterpret_cast<uint32_t*>(target) = pack_bf16x2(low, high);
+}
+__device__ __forceinline__ void store_pair(float* target, float low, float high) {
+    *reinterpret_cast<float2*>(target) = make_float2(low, high);
+}
+
+// 16 tokens per warp: O = R' S_0 + O', the norm over the head, the gate.  Bound by reading 48 KB per chunk.
+template <typename T>
+__global__ void __launch_bounds__(kFinishThreads)
+delta_finish_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, const float* chunks) {
+    constexpr bool kNearest = std::is_same<T, float>::value;
+    pdl_launch_dependents();
+    pdl_wait();
+    const SegmentTile tile = locate_tile(args.segments, kTokens, blockIdx.x / head_count);
+    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (warp * 16 >= tile.count || args.segments.slots[tile.segment] >= args.segments.num_request_slots) {
+        return;
+    }
+    const size_t head_base = static_cast<size_t>(head0 + blockIdx.x % head_count) * args.dim;
+    const size_t width = static_cast<size_t>(args.heads) * args.dim;
+    const float* chunk = chunks + static_cast<size_t>(blockIdx.x) * kChunkFloats;
+    const float4* operands = reinterpret_cast<const float4*>(chunk + kR) + warp * 8 * 32 + lane;
+    const float4* partial = reinterpret_cast<const float4*>(chunk + kO) + warp * 8 * 32 + lane;
+    const float4* states = reinterpret_cast<const float4*>(chunk + kD) + lane;
+    float out[8][4];
+#pragma unroll
+    for (uint32_t n = 0; n < 8; ++n) {
+        const float4 value = partial[n * 32];
+        out[n][0] = value.x;
+        out[n][1] = value.y;
+        out[n][2] = value.z;
+        out[n][3] = value.w;
+    }
+#pragma unroll
+    for (uint32_t m = 0; m < 4; ++m) {
+        const FragmentA<kNearest> a0 = operand_of<kNearest>(operands[2 * m * 32]), a1 = operand_of<kNearest>(operands[(2 * m + 1) * 32]);
+#pragma unroll
+        for (uint32_t n = 0; n < 8; ++n) {
+            const float4 state = states[(m * 8 + n) * 32];
+            FragmentB<kNearest> b0, b1;
+            b0.set(0, state.x);
+            b0.set(1, state.y);
+            b1.set(0, state.z);
+            b1.set(1, state.w);
+            mma_split(out[n], a0, b0);
+            mma_split(out[n], a1, b1);
+        }
+    }
+#pragma unroll
+    for (uint32_t half = 0; half < 2; ++half) {
+        float squares = 0.0f;
+#pragma unroll
+        for (uint32_t n = 0; n < 8; ++n) {
+            squares = fmaf(out[n][2 * half], out[n][2 * half], fmaf(out[n][2 * half + 1], out[n][2 * half + 1], squares));
+        }
+        squares += __shfl_xor_sync(0xffffffffu, squares, 1);
+        squares += __shfl_xor_sync(0xffffffffu, squares, 2);
+        const float factor = std::is_same<T, float>::value
+                                 ? inverse_rms(squares, args.dim, args.eps)
+                                 : rsqrtf(squares / static_cast<float>(args.dim) + args.eps);
+        const uint32_t token = warp * 16 + (lane >> 2) + half * 8;
+        if (token < tile.count) {
+            const T* gates = args.projected + static_cast<size_t>(tile.first + token) * args.pitch + 3 * width + head_base;
+            T* target = args.out + static_cast<size_t>(tile.first + token) * args.out_pitch + head_base;
+#pragma unroll
+            for (uint32_t n = 0; n < 8; ++n) {
+                const uint32_t channel = n * 8 + (lane & 3) * 2;
+                if (channel < args.dim) {
+                    const float2 gate = load_pair(gates + channel);
+                    const float2 weight = load_pair(args.norm + head_base + channel);
+                    store_pair(target + channel, out[n][2 * half] * factor * weight.x * sigmoid_of<T>(gate.x),
+                               out[n][2 * half + 1] * factor * weight.y * sigmoid_of<T>(gate.y));
+                }
+            }
+        }
+    }
+}
+
+}  // namespace
+
+size_t delta_split_bytes(size_t heads, size_t tiles) { return heads * tiles * kChunkFloats * sizeof(float); }
+
+// Heads are taken in groups whose chunks fit the scratch.
+template <typename T>
+cudaError_t launch_delta_split(cudaStream_t stream, const DeltaArgs<T>& args, float* chunks, size_t chunk_bytes) {
+    const size_t tiles = tile_bound(args.segments, kTokens);
+    const uint32_t most = static_cast<uint32_t>(std::min<size_t>(args.heads, chunk_bytes / delta_split_bytes(1, tiles)));
+    if (most == 0) return cudaErrorInvalidValue;
+    const uint32_t groups = (args.heads + most - 1) / most;
+    const uint32_t group = (args.heads + groups - 1) / groups;
+    const size_t carry_bytes = (kCarryStages * 10 * kCarryThreads * 4 + 2 * kDim * kCarryPitch) * sizeof(float);
+    cudaError_t status = cudaFuncSetAttribute(reinterpret_cast<const void*>(delta_form_kernel<T>),
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(FormShared<T>));
+    if (status == cudaSuccess) {
+        status = cudaFuncSetAttribute(reinterpret_cast<const void*>(delta_carry_kernel<T>),
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(carry_bytes));
+    }
+    for (uint32_t head0 = 0; head0 < args.heads && status == cudaSuccess; head0 += group) {
+        const uint32_t count = std::min(group, args.heads - head0);
+        const unsigned int blocks = static_cast<unsigned int>(tiles * count);
+        status = launch_kernel(delta_form_kernel<T>, blocks, kFormThreads, sizeof(FormShared<T>), stream, 1, args, head0, count,
+                               chunks);
+        if (status == cudaSuccess) {
+            status = launch_kernel(delta_carry_kernel<T>,
+                                   static_cast<unsigned int>(args.segments.num_segments * count * (kDim / kCarryColumns)),
+                                   kCarryThreads, carry_bytes, stream, 1, args, head0, count, chunks);
+        }
+        if (status == cudaSuccess) {
+            status = launch_kernel(delta_finish_kernel<T>, blocks, kFinishThreads, 0, stream, 1, args, head0, count, chunks);
+        }
+    }
+    return status;
+}
+
+template cudaError_t launch_delta_split<float>(cudaStream_t, const DeltaArgs<float>&, float*, size_t);
+template cudaError_t launch_delta_split<__nv_bfloat16>(cudaStream_t, const DeltaArgs<__nv_bfloat16>&, float*, size_t);
+
+}  // namespace lfm25

@@ -43,6 +43,8 @@ struct lfm25_stack_executor {
     void* head_input;          // [R, width]
     void* logits;              // [R, head.n], before a cap
     float* raw;                // [T, widest heads * dim] when a delta rule needs it
+    float* chunks = nullptr;   // of a delta rule split along the sequence
+    size_t chunk_bytes = 0;
     void* compressed;          // [T, widest q_rank]: latent attention's query latent
     void* absorbed;            // [T, widest heads * kv_rank]: queries against latents
     void* weighted;            // [T, widest heads * kv_rank]: weighted latents
@@ -303,6 +305,8 @@ int32_t run_general_delta(lfm25_stack_executor* self, const Step& step, const lf
     delta.norm = layer.head_norm;
     delta.record = {model.records, model.record_bytes, layer.state_offset};
     delta.raw = self->raw;
+    delta.chunks = self->chunks;
+    delta.chunk_bytes = self->chunk_bytes;
     delta.out = self->joined;
     delta.out_pitch = layer.output.k;
     delta.eps = model.norm_eps;
@@ -771,7 +775,7 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
         return lfm25::report_error(LFM25_ERR_INVALID_ARGUMENT, "stack model sizes are inconsistent");
     }
     size_t projection = 0, query = 0, up = 0, joined = 0, raw = 0, compressed = 0, latents = 0, channels = 0, scanned = 0;
-    size_t context_rank = 0, context_keys = 0, context_columns = 0;
+    size_t context_rank = 0, context_keys = 0, context_columns = 0, chunk_bytes = 0;
     const Activation type = static_cast<Activation>(model->activation);
     for (uint32_t index = 0; index < model->num_layers; ++index) {
         const lfm25_stack_layer& layer = model->layers[index];
@@ -788,6 +792,10 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
         if (layer.mixer == LFM25_MIXER_ATTENTION) query = std::max(query, width);
         if (layer.mixer == LFM25_MIXER_GENERAL_DELTA && lfm25::delta_rule_needs_scratch(layer.dim))
             raw = std::max(raw, width);
+        if (layer.mixer == LFM25_MIXER_GENERAL_DELTA) {
+            chunk_bytes = std::max(chunk_bytes, lfm25::delta_rule_chunk_bytes(type, layer.heads, layer.dim, maximum_tokens,
+                                                                              maximum_rows));
+        }
         if (layer.mixer == LFM25_MIXER_LATENT_ATTENTION) {
             const lfm25::LatentAttentionShape shape = {layer.heads, layer.dim, layer.rot_dim, layer.vdim, layer.kv_rank,
                                                        layer.scale};
@@ -850,6 +858,15 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
         *fields[index] = sizes[index] > 0 ? cursor : nullptr;
         cursor += (sizes[index] + 255) & ~static_cast<size_t>(255);
     }
+    if (chunk_bytes > 0) {
+        // without it prompts run tile after tile
+        if (cudaMalloc(reinterpret_cast<void**>(&self->chunks), chunk_bytes) == cudaSuccess) {
+            self->chunk_bytes = chunk_bytes;
+        } else {
+            self->chunks = nullptr;
+            cudaGetLastError();
+        }
+    }
     *out = self;
     return LFM25_OK;
 }
@@ -857,6 +874,7 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
 void lfm25_stack_executor_destroy(lfm25_stack_executor* self) {
     if (self == nullptr) return;
     cudaFree(self->allocation);
+    cudaFree(self->chunks);
     cudaFree(self->exported);
     delete self;
 }

@@ -364,12 +364,18 @@ struct DeltaRuleLaunch {
     const void* norm;              // bf16 [heads * dim]
     StackRecord record;
     float* raw;                    // f32 [T, heads * dim] scratch, needed when delta_rule_needs_scratch(dim)
+    float* chunks;                 // chunk_bytes of scratch, or nullptr: prompts are not split along the sequence
+    size_t chunk_bytes;
     void* out;                     // activations, rows out_pitch apart, heads * dim columns
     size_t out_pitch;
     float eps;
 };
 constexpr uint32_t kDeltaMaxDim = 256;
 bool delta_rule_needs_scratch(uint32_t dim);
+constexpr size_t kDeltaChunkBytes = size_t(256) << 20;
+// Scratch for prompts that are split along the sequence, in steps of up to `tokens` tokens in `segments` segments; more heads
+// than it holds are taken in turns.
+size_t delta_rule_chunk_bytes(Activation type, uint32_t heads, uint32_t dim, size_t tokens, size_t segments);
 cudaError_t launch_delta_rule(cudaStream_t stream, const DeltaRuleLaunch& launch);
 
 }  // namespace lfm25

@@ -90,6 +90,49 @@ def test_delta_rule_prompt_kernels_agree(device, library_option, heads, dim, ran
 
 
 @pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("heads,dim,rank", [(3, 64, 16), (1, 8, 5), (2, 24, 130), (12, 40, 64)])
+def test_delta_rule_split_along_the_sequence(device, library_option, dtype, heads, dim, rank):
+    """Portions that end at, before and behind the edges of 16- and 64-token pieces, strong decays beside weak ones."""
+    library_option("delta_prompt", 4)
+
+    def strong(tensors):
+        tensors["l0.mix.w0"][::2] = 9.0
+    config = cases.config_of([cases.delta_layer(heads, dim, ff=0)])
+    check_layer(config, 17, device, dtype, [64, 63, 2, 65, 128, 17, 1, 200], rank, strong)
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+def test_delta_rule_split_mixed_step(device, library_option, dtype):
+    """Sequences side by side behind single tokens, with more heads than the scratch holds at once, against the kernels that
+    carry a segment in one CTA: f32 arithmetic in both, so bf16 results differ by their last rounding."""
+    import torch
+
+    from lfm25_inference_b200 import model as lfm_model
+    from lfm25_inference_b200 import ops, stack, workloads
+    config = cases.config_of([cases.delta_layer(64, 8, ff=0)])
+    tensors = cases.random_tensors(config, 29, 16)
+    chunks = np.array([1, 1, 70, 64, 129, 65, 80, 3])
+    tokens = np.random.default_rng(5).integers(0, config["vocab"], size=chunks.sum()).astype(np.uint32)
+    results = []
+    for forced in (3, 4):
+        library_option("delta_prompt", forced)
+        with torch.cuda.stream(torch.cuda.Stream(device)):
+            blaslt = ops.BlasLt()
+            layout = workloads.mixed_step_batch(1, np.zeros(len(chunks), np.int64), chunks, 64)
+            model = cases.product_model(config, tensors, device, dtype, 64, len(chunks))
+            executor = stack.StackExecutor(blaslt, model, len(tokens), len(chunks))
+            steps = []
+            for _ in range(2):                     # the second continues from the first one's state
+                executor.forward_ragged(lfm_model.RaggedBatch(device, layout, tokens))
+                steps.append(executor.residual(len(tokens)))
+            results.append(np.concatenate(steps))
+            executor.close()
+            blaslt.close()
+    assert np.isfinite(results[0]).all()
+    assert cases.relative_error(results[1], results[0]).max() < {"float32": 5e-6, "bfloat16": 4e-3}[dtype]
+
+
+@pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("width,ff", [(48, 40), (256, 72), (64, 1000), (50, 30), (96, 9)])
 def test_feed_forward(device, dtype, width, ff):
     """The mixer's output projection is zero: only PolyNorm is left."""
