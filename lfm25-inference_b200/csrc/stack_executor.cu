@@ -55,6 +55,9 @@ struct lfm25_stack_executor {
     uint32_t* token_order;     // [T]: the tokens that attend to latents, longest context first
     void* convolved;           // [T, widest channels] of a state-space mixer
     void* scanned;             // [T, widest heads * vdim]
+    void* factors;             // [widest heads, T]: what the tokens contribute to a state-space recurrence
+    float* pieces;             // states between the pieces of long segments
+    size_t piece_bytes = 0;
     size_t context_capacity = 0;
     const void* last_post = nullptr;   // norm between `update` and the residual stream of the last step
     uint32_t* sampled;         // [R]
@@ -514,6 +517,9 @@ int32_t run_state_space(lfm25_stack_executor* self, const Step& step, const lfm2
     scan.skip = layer.skip;
     scan.record = {model.records, model.record_bytes, layer.state_offset};
     scan.out = self->scanned;
+    scan.factors = self->factors;
+    scan.pieces = self->pieces;
+    scan.piece_bytes = self->piece_bytes;
     STACK_CUDA(lfm25::launch_state_space(stream, scan), "state-space launch failed");
     lfm25::GatedGroupNormLaunch norm;
     norm.type = self->type;
@@ -775,7 +781,7 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
         return lfm25::report_error(LFM25_ERR_INVALID_ARGUMENT, "stack model sizes are inconsistent");
     }
     size_t projection = 0, query = 0, up = 0, joined = 0, raw = 0, compressed = 0, latents = 0, channels = 0, scanned = 0;
-    size_t context_rank = 0, context_keys = 0, context_columns = 0, chunk_bytes = 0;
+    size_t context_rank = 0, context_keys = 0, context_columns = 0, chunk_bytes = 0, factors = 0, pieces = 0;
     const Activation type = static_cast<Activation>(model->activation);
     for (uint32_t index = 0; index < model->num_layers; ++index) {
         const lfm25_stack_layer& layer = model->layers[index];
@@ -811,6 +817,11 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
         if (layer.mixer == LFM25_MIXER_STATE_SPACE) {
             channels = std::max(channels, state_space_channels(layer));
             scanned = std::max(scanned, mixer_columns(layer));
+            if (type == Activation::kBf16) {
+                factors = std::max(factors, lfm25::state_space_factor_bytes(layer.heads, maximum_tokens));
+                pieces = std::max(pieces, lfm25::state_space_piece_bytes(layer.heads, layer.state_size, layer.vdim,
+                                                                         maximum_tokens));
+            }
         }
     }
     lfm25_stack_executor* self = new (std::nothrow) lfm25_stack_executor();
@@ -830,20 +841,21 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
             LFM25_CONTEXT_ROWS;
     }
     self->context_capacity = c;
+    self->piece_bytes = pieces;
     void** fields[] = {reinterpret_cast<void**>(&self->residual[0]), reinterpret_cast<void**>(&self->residual[1]),
                        &self->mixed, &self->normalized, &self->projected, &self->query, &self->up, &self->joined,
                        &self->update, &self->head_input, &self->logits, reinterpret_cast<void**>(&self->raw),
                        reinterpret_cast<void**>(&self->sampled), &self->compressed, &self->absorbed, &self->weighted,
                        &self->context_latents, &self->context_keys, &self->expanded,
                        reinterpret_cast<void**>(&self->context_bases), reinterpret_cast<void**>(&self->token_order),
-                       &self->convolved, &self->scanned};
+                       &self->convolved, &self->scanned, &self->factors, reinterpret_cast<void**>(&self->pieces)};
     const size_t sizes[] = {t * model->width * 4, t * model->width * 4, t * model->width * bytes,
                             t * model->width * bytes, t * projection * bytes, t * query * bytes, t * up * bytes,
                             t * joined * bytes, t * model->width * bytes, r * model->width * bytes,
                             r * model->head.n * bytes, t * raw * 4, r * 4, t * compressed * bytes, t * latents * bytes,
                             t * latents * bytes, c * context_rank * bytes, c * context_keys * bytes,
                             c * context_columns * bytes, (t + 1) * 4, latents > 0 ? t * 4 : 0, t * channels * bytes,
-                            t * scanned * bytes};
+                            t * scanned * bytes, factors, pieces};
     size_t total = 0;
     for (size_t size : sizes) total += (size + 255) & ~static_cast<size_t>(255);
     cudaError_t status = cudaMalloc(&self->allocation, total);

@@ -327,7 +327,12 @@ struct StateSpaceLaunch {
     const void* skip;
     StackRecord record;
     void* out;                     // [T, heads * vdim]
+    void* factors;                 // state_space_factor_bytes() of scratch, for prompts of bf16 activations
+    float* pieces;                 // piece_bytes of scratch, may be nullptr
+    size_t piece_bytes;
 };
+size_t state_space_factor_bytes(size_t heads, size_t tokens);
+size_t state_space_piece_bytes(uint32_t heads, uint32_t size, uint32_t vdim, size_t tokens);
 constexpr uint32_t kStateSpaceMaxSize = 512;
 cudaError_t launch_state_space(cudaStream_t stream, const StateSpaceLaunch& launch);
 

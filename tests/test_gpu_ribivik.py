@@ -107,6 +107,40 @@ def test_state_space_prompt_kernels_agree(device, library_option, shape):
     assert cases.relative_error(results[1], results[0]).max() < 4e-3
 
 
+@pytest.mark.parametrize("shape", [(4, 64, 128, 1, 1, 4), (8, 64, 64, 2, 8, 4), (2, 128, 256, 2, 1, 4), (5, 40, 24, 5, 4, 2)],
+                         ids=lambda shape: "x".join(map(str, shape)))
+def test_state_space_in_pieces(device, library_option, shape):
+    """Sequences long enough to be cut into pieces, behind single tokens and beside short ones, against the token-by-token
+    kernel; decays from next to nothing to next to everything; the second step continues from the first one's state.  Both
+    keep 32 bits, so they differ by rounding of the bf16 output."""
+    import torch
+
+    from lfm25_inference_b200 import model as lfm_model
+    from lfm25_inference_b200 import ops, stack, workloads
+    config = cases.config_of([cases.mamba_layer(*shape)])
+    tensors = cases.random_tensors(config, 89)
+    tensors["l0.mix.A_log"][:] = np.linspace(-6.0, 3.0, shape[0])
+    chunks = np.array([1, 1, 1100, 20, 515, 1024])
+    tokens = np.random.default_rng(5).integers(0, config["vocab"], size=chunks.sum()).astype(np.uint32)
+    results = []
+    for forced in (0, 1):
+        library_option("state_space_prompt", forced)
+        with torch.cuda.stream(torch.cuda.Stream(device)):
+            blaslt = ops.BlasLt()
+            layout = workloads.mixed_step_batch(1, np.zeros(len(chunks), np.int64), chunks, 200)
+            model = cases.product_model(config, tensors, device, "bfloat16", 200, len(chunks))
+            executor = stack.StackExecutor(blaslt, model, len(tokens), len(chunks))
+            steps = []
+            for _ in range(2):
+                executor.forward_ragged(lfm_model.RaggedBatch(device, layout, tokens))
+                steps.append(executor.residual(len(tokens)))
+            results.append(np.concatenate(steps))
+            executor.close()
+            blaslt.close()
+    assert np.isfinite(results[0]).all()
+    assert cases.relative_error(results[1], results[0]).max() < 4e-3
+
+
 def test_latent_attention_kernels_agree(device, library_option):
     """Latents on the tensor cores, keys and values formed from them, and the plain kernel on the same inputs."""
     config = cases.config_of([cases.latent_layer(24, 64, 32, 48, 64, 256, scale=0.3, ff=0)])
