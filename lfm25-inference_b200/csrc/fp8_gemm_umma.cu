@@ -10,8 +10,7 @@
 //            per stage a 128 x 128 B weight tile and the M_pad x 128 B activation tile of the same K block
 //   warp 1   allocates TMEM; one thread issues 4 tcgen05.mma per stage (K = 32 each) into a
 //            128-lane x M_pad-column fp32 accumulator and releases the stage with tcgen05.commit
-//   warp 6   a second issuer with an accumulator of its own: the two take alternate K blocks (one thread issues an
-//            MMA every ~180 cycles whatever its shape, which is 4 KiB of weights, about an SM's share of HBM)
+//   warp 6   a second issuer with an accumulator of its own: the two take alternate K blocks
 //   warps 2-5  epilogue: tcgen05.ld the accumulators (thread = weight row, registers = batch columns), add them,
 //            scale, round to bf16, transpose through shared memory and store 16 bytes per lane
 //
@@ -135,7 +134,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_co
                      const UmmaParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);     // the same value to the compiler's eye as well
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t tile = blockIdx.x / p.splits;
     const uint32_t split = p.splits > 1 ? cluster_rank() : 0;
@@ -216,7 +215,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_co
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             pdl_wait();
             for (uint32_t block = 0; block < ahead; ++block) {
                 tma_load_2d(smem_base + block * stage_bytes + kWeightTileBytes, &x_map, bar_full + 8 * block,
@@ -245,12 +244,14 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const __grid_co
         }
         __syncwarp();   // whole warps reach the CTA barriers below
     } else if (warp == 1 || warp == 6) {
-        // One thread issues a tcgen05.mma every ~180 cycles whatever its shape, i.e. 4 KiB of weights per 180 cycles:
-        // about an SM's share of HBM and no more.  A second issuing warp with an accumulator of its own runs at the
-        // same rate beside it, so the K blocks alternate between the two (the slot count is even: a slot always
-        // belongs to the same issuer, which therefore sees every phase of its barrier).
+        // The issuing lane is elected, so that the compiler keeps the MMAs' operands in uniform registers: picked by its
+        // number it took ~180 cycles per MMA, 4 KiB of weights, which is an SM's share of HBM and no more (decode steps
+        // of 1 and 23 sequences 661 -> 639 and 857 -> 845 us, with 32 of a layer stack 1466 -> 1447).  Barrier waits and
+        // commits still cost a few hundred cycles per K block, so the K blocks alternate between two issuing warps with
+        // an accumulator each (the slot count is even: a slot always belongs to the same issuer, which therefore sees
+        // every phase of its barrier).
         const uint32_t issuer = warp == 1 ? 0u : 1u;
-        if (lane == 0 && issuer < p.issuers) {
+        if (issuer < p.issuers && elect_one()) {
             // instruction descriptor: D = f32, A = B = E4M3 (format 0) or BF16 (format 1), both K-major,
             // N = m_pad, M = 128
             const uint32_t formats = BF16 ? ((1u << 7) | (1u << 10)) : 0u;

@@ -9,12 +9,10 @@
 //     rows) is the M = 128 operand of tcgen05.mma and a tile of `n_tile` weight rows is its N operand.  N of the
 //     instruction is any multiple of 16 up to 256, so the host picks n_tile such that the number of tiles just fills
 //     the SMs (16384 rows in tiles of 112 are 147 CTAs on 148 SMs), which a fixed 128-row weight tile cannot do.
-//   * One thread cannot issue tcgen05.mma fast enough.  Measured on a B200: a thread issues one M = 128 MMA every
-//     ~182 cycles whatever its N (16 .. 256), i.e. N * 32 bytes of weights per 182 cycles -- 39 GB/s per SM at
-//     N = 112, below an SM's share of HBM -- while a second issuing warp runs at the same rate beside it (the
-//     tensor pipe itself takes an N = 256 MMA every ~145 cycles), and every K block costs its issuer another few
-//     hundred cycles for the barrier wait and the commit.  So the K blocks are dealt out round-robin to 2 or 4
-//     issuing warps, each with accumulators of its own in TMEM; the epilogue adds the accumulators.
+//   * One thread cannot issue tcgen05.mma fast enough.  Every K block costs its issuer a few hundred cycles for the
+//     barrier wait and the commit beside its MMAs, so the K blocks are dealt out round-robin to 2 or 4 issuing warps,
+//     each with accumulators of its own in TMEM; the epilogue adds the accumulators.  The issuing lane is elected:
+//     picked by its number it kept the MMAs' operands in per-lane registers and took ~182 cycles per MMA.
 //   * The accumulator has one batch row per lane and one output feature per column: an epilogue thread owns a
 //     batch row and holds consecutive features of it, so it stores 32 contiguous bytes at a time with no
 //     transposition, and SiLU(gate) * up of the packed Gate/Up projection is plain register arithmetic (a tile
@@ -201,7 +199,7 @@ gemm_rows_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const __gr
                       const RowsParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);     // the same value to the compiler's eye as well
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t tile = blockIdx.x / (p.splits * p.slices);
     const uint32_t slice = (blockIdx.x / p.splits) % p.slices;
@@ -291,7 +289,7 @@ gemm_rows_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const __gr
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             pdl_wait();   // the activations are the predecessor's output
             for (uint32_t block = 0; block < ahead; ++block) {
                 if (block != p.drop_block) {
@@ -318,7 +316,7 @@ gemm_rows_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const __gr
         }
     } else if (warp < kFirstEpilogueWarp) {
         const uint32_t issuer = warp - 1;
-        if (lane == 0 && issuer < p.issuers) {
+        if (issuer < p.issuers && elect_one()) {
             // instruction descriptor: D = f32, A = B = E4M3 (format 0) or BF16 (format 1), both K-major,
             // N = n_tile, M = 128
             const uint32_t formats = BF16 ? ((1u << 7) | (1u << 10)) : 0u;

@@ -102,7 +102,7 @@ hybrid_attention_umma_kernel(const __grid_constant__ CUtensorMap query_map, cons
                              const __grid_constant__ CUtensorMap value_map,
                              const __grid_constant__ CUtensorMap current_key_map,
                              const __grid_constant__ CUtensorMap current_value_map, const UmmaAttentionParams p) {
-    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);     // the same value to the compiler's eye as well
     const uint32_t lane = threadIdx.x & 31;
     pdl_launch_dependents();
     pdl_wait();
@@ -203,7 +203,7 @@ hybrid_attention_umma_kernel(const __grid_constant__ CUtensorMap query_map, cons
 
     if (warp == 0) {
         // ------------------------------------------------------------------------------------ producer
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_arrive_expect_tx(bar_q, kQBytes);
             tma_load_3d(q_base, &query_map, bar_q, 0, static_cast<int32_t>(kv_head * kQPerKv),
                         static_cast<int32_t>(tile_begin));
@@ -262,7 +262,7 @@ hybrid_attention_umma_kernel(const __grid_constant__ CUtensorMap query_map, cons
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             // instruction descriptors: D = f32, A = B = bf16, M = 128; QK^T: both K-major, N = keys of the stage;
             // PV: B (the V rows) MN-major, N = 64 dims
             const uint32_t idesc_common = (1u << 4) | (1u << 7) | (1u << 10) | ((kTileRows >> 4) << 24);
