@@ -154,6 +154,14 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tensor_map
         : "memory");
 }
 
+// Brings the same box into the L2 only; nothing waits for it.
+__device__ __forceinline__ void tma_prefetch_2d(const void* tensor_map, int32_t x, int32_t y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(
+                     reinterpret_cast<uint64_t>(tensor_map)),
+                 "r"(x), "r"(y)
+                 : "memory");
+}
+
 // The same load with an L2 eviction-priority hint: a policy from l2_evict_first_policy() marks the lines as the
 // first to be replaced, for data that is read once (a KV stream), so that it does not push reusable lines out.
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {
