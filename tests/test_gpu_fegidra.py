@@ -65,6 +65,37 @@ def test_attention_layer(device, dtype, shape):
     check_layer(config, 11, device, dtype, [75, 2, 1, 50, 1, 1])
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim", [(8, 2, 64), (3, 3, 128), (16, 16, 16)])
+def test_decode_attention_splits_by_context(device, library_option, heads, kv_heads, dim):
+    """Single tokens behind contexts around multiples of the 1024 keys that one CTA takes, short ones beside them, against the
+    general kernel: the weights keep 16 bits in one and 32 in the other."""
+    import torch
+
+    from lfm25_inference_b200 import model as lfm_model
+    from lfm25_inference_b200 import ops, stack, workloads
+    config = cases.config_of([cases.attention_layer(heads, kv_heads, dim, dim, 1 << 20, 8, ff=0)])
+    tensors = cases.random_tensors(config, 31)
+    prefixes = np.array([3, 1022, 1023, 1024, 40, 2047, 2048, 4100, 0])
+    tokens = np.random.default_rng(5).integers(0, config["vocab"], size=len(prefixes)).astype(np.uint32)
+    layout = workloads.mixed_step_batch(1, prefixes, np.ones(len(prefixes), np.int64), 800)
+    results = []
+    for forced in (0, 1):
+        library_option("stack_attention", forced)
+        with torch.cuda.stream(torch.cuda.Stream(device)):
+            blaslt = ops.BlasLt()
+            model = cases.product_model(config, tensors, device, "bfloat16", 800, len(prefixes))
+            for index, cache in enumerate(cache for pair in model.caches for cache in pair):
+                generator = torch.Generator(device=device).manual_seed(index)
+                cache.copy_(torch.randn(cache.shape, generator=generator, device=device).to(cache.dtype))
+            executor = stack.StackExecutor(blaslt, model, len(prefixes))
+            executor.forward_ragged(lfm_model.RaggedBatch(device, layout, tokens))
+            results.append(executor.residual(len(prefixes)))
+            executor.close()
+            blaslt.close()
+    assert np.isfinite(results[0]).all()
+    assert cases.relative_error(results[0], results[1]).max() < 1e-2
+
+
 @pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("heads,dim,rank", [(3, 16, 5), (2, 64, 16), (1, 24, 1), (2, 128, 33), (1, 80, 3), (2, 160, 8),
                                             (1, 256, 64), (1, 10, 7), (2, 128, 700)])
