@@ -183,6 +183,13 @@ def test_f32_products(device, width, ff):
     check_layer(config, 29, device, "float32", [1, 15, 16, 17, 32, 33, 64, 65])
 
 
+@pytest.mark.parametrize("width,ff", [(1024, 2048), (256, 1000)])
+def test_f32_products_of_three_small_tiles(device, width, ff):
+    """Row counts that take three tiles of 32, and the first that takes two of 64; the bound as above."""
+    config = cases.config_of([cases.delta_layer(1, 16, ff=ff)], width=width)
+    check_layer(config, 37, device, "float32", [65, 80, 96, 97])
+
+
 def test_f32_products_of_large_and_tiny_values(device):
     """Values over the whole range of exponents beside one another: nothing of x is lost when it is taken apart."""
     config = cases.config_of([cases.delta_layer(1, 16, ff=64)], width=128)
