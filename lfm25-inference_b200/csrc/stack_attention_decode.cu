@@ -55,17 +55,9 @@ struct Params {
     __nv_bfloat16* out;
     size_t out_pitch;
     unsigned int* status;
-    uint32_t splits;         // CTAs of a cluster
-    uint32_t least_splits;   // of them that work on every token; longer contexts take more (see working_splits)
+    uint32_t splits;
     uint64_t wait_limit;
 };
-
-// CTAs of its cluster that work on a token: one per kPagesPerSplit pages.  The others leave at once.
-constexpr uint32_t kPagesPerSplit = 64;
-__host__ __device__ constexpr uint32_t working_splits(uint32_t pages, uint32_t least, uint32_t most) {
-    const uint32_t wanted = (pages + kPagesPerSplit - 1) / kPagesPerSplit;
-    return wanted < least ? least : (wanted > most ? most : wanted);
-}
 
 template <uint32_t KC, uint32_t VC>
 __global__ void __launch_bounds__(kThreads)
@@ -109,11 +101,7 @@ stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const
     const uint32_t pages = valid ? position / kPageSize - first_page + 1 : 0;
     const uint32_t* table = p.block_tables + (valid ? table_row * p.block_table_stride : 0);
     // this warp's pages: first_page + mine, + stride, ...
-    const uint32_t splits = working_splits(pages, p.least_splits, p.splits);
-    if (split >= splits) {
-        return;        // the barriers of the cluster wait for threads that are still there
-    }
-    const uint32_t stride = kWarps * splits;
+    const uint32_t stride = kWarps * p.splits;
     const uint32_t mine = split * kWarps + warp;
     const uint32_t count = pages > mine ? (pages - mine + stride - 1) / stride : 0;
 
@@ -337,7 +325,7 @@ stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const
             total = fmaf(warp_sums[w * kGroupRows + row], factor, total);
             value = fmaf(partial[(w * kGroupRows + row) * L::kColumns + column], factor, value);
         }
-        if (splits == 1) {
+        if (p.splits == 1) {
             if (!aborted) target[item] = __float2bfloat16_rn(total > 0.0f ? value / total : 0.0f);
         } else {
             result[row * L::kColumns + column] = value;
@@ -347,26 +335,26 @@ stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const
             }
         }
     }
-    if (splits == 1) {
+    if (p.splits == 1) {
         return;
     }
     // ---- splits of the token: every CTA of the cluster finishes a share of the outputs
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
     bool any_abort = false;
-    for (uint32_t rank = 0; rank < splits; ++rank) {
+    for (uint32_t rank = 0; rank < p.splits; ++rank) {
         any_abort = any_abort || *cluster.map_shared_rank(const_cast<uint32_t*>(abort_flag), rank) != 0;
     }
-    for (uint32_t item = threadIdx.x * splits + split; item < group * vdim; item += kThreads * splits) {
+    for (uint32_t item = threadIdx.x * p.splits + split; item < group * vdim; item += kThreads * p.splits) {
         const uint32_t row = item / vdim;
         const uint32_t column = item - row * vdim;
         float best = -INFINITY;
-        for (uint32_t rank = 0; rank < splits; ++rank) {
+        for (uint32_t rank = 0; rank < p.splits; ++rank) {
             best = fmaxf(best, cluster.map_shared_rank(cta_top, rank)[row]);
         }
         const float base = best == -INFINITY ? 0.0f : best;
         float total = 0.0f, value = 0.0f;
-        for (uint32_t rank = 0; rank < splits; ++rank) {
+        for (uint32_t rank = 0; rank < p.splits; ++rank) {
             const float factor = fast_exp2((cluster.map_shared_rank(cta_top, rank)[row] - base) * scale_log2);
             total = fmaf(cluster.map_shared_rank(cta_sum, rank)[row], factor, total);
             value = fmaf(cluster.map_shared_rank(result, rank)[row * L::kColumns + column], factor, value);
@@ -376,26 +364,8 @@ stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const
     cluster.sync();           // nobody leaves while its results are being read
 }
 
-size_t visible_pages(const StackAttentionShape& shape, size_t context) {
-    const size_t visible = shape.chunk != 0 ? std::min<size_t>(context, shape.chunk) : context;
-    return (visible + kPageSize - 1) / kPageSize;
-}
-
-// Where all CTAs are resident at once, the longest context decides when the kernel is done: it is split further, over a
-// cluster of up to eight.  Whole steps with 8 key/value heads: 32 sequences of 128 to 4096 tokens 1433 -> 1385 us, 16 of
-// 100 to 4000 1144 -> 1093; 64 of 200 to 4096 tokens (more CTAs than are resident: those that leave cost more than the
-// split gives) 1918 -> 1989, so not there.  Splitting every token alike costs equal contexts, each CTA with its start and its
-// merge: 32 of 1000 tokens 1220 -> 1258 us.
-uint32_t stack_attention_most_splits(const StackAttentionShape& shape, size_t tokens, size_t context, uint32_t least) {
-    uint32_t most = least;
-    if (tokens * shape.kv_heads * least <= 2 * 148) {
-        while (most < 8 && most * kPagesPerSplit < visible_pages(shape, context)) most *= 2;
-    }
-    return most;
-}
-
 template <uint32_t KC, uint32_t VC>
-cudaError_t launch_sized(cudaStream_t stream, const StackAttentionLaunch& launch, uint32_t least) {
+cudaError_t launch_sized(cudaStream_t stream, const StackAttentionLaunch& launch, uint32_t splits) {
     using L = Layout<KC, VC>;
     CUtensorMap key_map, value_map;
     if (!make_page_map(&key_map, launch, false) || !make_page_map(&value_map, launch, true)) {
@@ -418,9 +388,7 @@ cudaError_t launch_sized(cudaStream_t stream, const StackAttentionLaunch& launch
     params.out = static_cast<__nv_bfloat16*>(launch.out);
     params.out_pitch = launch.out_pitch;
     params.status = launch.status;
-    const uint32_t splits = stack_attention_most_splits(launch.shape, launch.decode_tokens, launch.decode_context, least);
     params.splits = splits;
-    params.least_splits = least;
     params.wait_limit = wait_limit_ns();
     const size_t blocks = launch.decode_tokens * launch.shape.kv_heads * splits;
     return launch_kernel(kernel, static_cast<unsigned int>(blocks), kThreads, L::kSharedBytes, stream, splits, key_map,
@@ -440,7 +408,8 @@ cudaError_t launch_keys(cudaStream_t stream, const StackAttentionLaunch& launch,
 
 // CTAs per token and head over the key axis: enough to fill the machine twice while every warp keeps two pages.
 uint32_t stack_attention_splits(const StackAttentionShape& shape, size_t tokens, size_t context) {
-    const size_t pages = visible_pages(shape, context);
+    const size_t visible = shape.chunk != 0 ? std::min<size_t>(context, shape.chunk) : context;
+    const size_t pages = (visible + kPageSize - 1) / kPageSize;
     uint32_t splits = 1;
     while (splits < 8 && tokens * shape.kv_heads * splits * 2 <= 2 * 148 && pages >= 2 * kWarps * splits * 2) splits *= 2;
     return splits;

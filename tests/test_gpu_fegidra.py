@@ -65,25 +65,28 @@ def test_attention_layer(device, dtype, shape):
     check_layer(config, 11, device, dtype, [75, 2, 1, 50, 1, 1])
 
 
-@pytest.mark.parametrize("heads,kv_heads,dim", [(8, 2, 64), (3, 3, 128), (16, 16, 16)])
-def test_decode_attention_splits_by_context(device, library_option, heads, kv_heads, dim):
-    """Single tokens behind contexts around multiples of the 1024 keys that one CTA takes, short ones beside them, against the
-    general kernel: the weights keep 16 bits in one and 32 in the other."""
+@pytest.mark.parametrize("heads,kv_heads,dim,copies", [(8, 2, 64, 1), (3, 3, 128, 1), (16, 16, 16, 1), (32, 8, 64, 1),
+                                                       (32, 8, 64, 2), (16, 8, 128, 3)])
+def test_decode_attention_long_contexts(device, library_option, heads, kv_heads, dim, copies):
+    """Single tokens behind long and short contexts side by side, around borders of pages and of 1024 keys, in clusters of
+    8, 8, 2, 4, 2 and 1 CTAs per token and head (9 tokens times `copies`), against the general kernel: the weights keep 16
+    bits in one and 32 in the other."""
     import torch
 
     from lfm25_inference_b200 import model as lfm_model
     from lfm25_inference_b200 import ops, stack, workloads
     config = cases.config_of([cases.attention_layer(heads, kv_heads, dim, dim, 1 << 20, 8, ff=0)])
     tensors = cases.random_tensors(config, 31)
-    prefixes = np.array([3, 1022, 1023, 1024, 40, 2047, 2048, 4100, 0])
+    prefixes = np.array([3, 1022, 1023, 1024, 40, 2047, 2048, 4100, 0] * copies)
+    pages = 800 * copies
     tokens = np.random.default_rng(5).integers(0, config["vocab"], size=len(prefixes)).astype(np.uint32)
-    layout = workloads.mixed_step_batch(1, prefixes, np.ones(len(prefixes), np.int64), 800)
+    layout = workloads.mixed_step_batch(1, prefixes, np.ones(len(prefixes), np.int64), pages)
     results = []
     for forced in (0, 1):
         library_option("stack_attention", forced)
         with torch.cuda.stream(torch.cuda.Stream(device)):
             blaslt = ops.BlasLt()
-            model = cases.product_model(config, tensors, device, "bfloat16", 800, len(prefixes))
+            model = cases.product_model(config, tensors, device, "bfloat16", pages, len(prefixes))
             for index, cache in enumerate(cache for pair in model.caches for cache in pair):
                 generator = torch.Generator(device=device).manual_seed(index)
                 cache.copy_(torch.randn(cache.shape, generator=generator, device=device).to(cache.dtype))
