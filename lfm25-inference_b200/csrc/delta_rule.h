@@ -41,64 +41,39 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const float (&a)[4], con
           "r"(__float_as_uint(b[0])), "r"(__float_as_uint(b[1])));
 }
 
-// An operand fragment as high + low.  TF32 keeps 10 mantissa bits and ignores the rest: the high part is what it keeps of the
-// value, the low part the remainder, of which it keeps another 10.  NEAREST: the high part is rounded to nearest, which
-// halves the low one and leaves it either sign; with the product of the low parts for f32 activations.
-template <int N, bool NEAREST = false>
+// An operand fragment as high + low: the high part is what TF32 keeps of the value (10 mantissa bits), the low part the
+// rest, of which TF32 keeps another 10.
+template <int N>
 struct SplitFragment {
     float high[N], low[N];
     __device__ __forceinline__ void set(int index, float value) {
-        if (NEAREST) {
-            high[index] = __uint_as_float((__float_as_uint(value) + 0x1000u) & 0xffffe000u);
-        } else {
-            high[index] = __uint_as_float(__float_as_uint(value) & 0xffffe000u);
-        }
-        low[index] = value - high[index];          // NaN also where the sum above has left its range
+        high[index] = __uint_as_float(__float_as_uint(value) & 0xffffe000u);
+        low[index] = value - high[index];
     }
 };
-template <bool NEAREST = false>
-using FragmentA = SplitFragment<4, NEAREST>;
-template <bool NEAREST = false>
-using FragmentB = SplitFragment<2, NEAREST>;
+using FragmentA = SplitFragment<4>;
+using FragmentB = SplitFragment<2>;
 
-// The tensor cores cut what falls behind the accumulator's last bit; NEAREST: every product of fragments starts from zero
-// and is added up with rounding to nearest.
-template <bool NEAREST, uint32_t COUNT>
-__device__ __forceinline__ void mma_split(float (*d)[4], const FragmentA<NEAREST>& a, const FragmentB<NEAREST> (&b)[COUNT]) {
-    float sums[COUNT][4] = {};
-    float (*target)[4] = NEAREST ? sums : d;
-    if (NEAREST) {
-#pragma unroll
-        for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(target[n], a.low, b[n].low);
-    }
+template <uint32_t COUNT>
+__device__ __forceinline__ void mma_split(float (*d)[4], const FragmentA& a, const FragmentB (&b)[COUNT]) {
     // the accumulators' products alternate so that none waits for the one before it
 #pragma unroll
-    for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(target[n], a.low, b[n].high);
+    for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(d[n], a.low, b[n].high);
 #pragma unroll
-    for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(target[n], a.high, b[n].low);
+    for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(d[n], a.high, b[n].low);
 #pragma unroll
-    for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(target[n], a.high, b[n].high);
-    if (NEAREST) {
-#pragma unroll
-        for (uint32_t n = 0; n < COUNT; ++n) {
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) d[n][i] += sums[n][i];
-        }
-    }
+    for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(d[n], a.high, b[n].high);
 }
-template <bool NEAREST>
-__device__ __forceinline__ void mma_split(float (&d)[4], const FragmentA<NEAREST>& a, const FragmentB<NEAREST>& b) {
-    const FragmentB<NEAREST> one[1] = {b};
-    mma_split<NEAREST, 1>(&d, a, one);
+__device__ __forceinline__ void mma_split(float (&d)[4], const FragmentA& a, const FragmentB& b) {
+    const FragmentB one[1] = {b};
+    mma_split(&d, a, one);
 }
-template <bool NEAREST>
-__device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA<NEAREST>& a, const FragmentB<NEAREST>& b0,
-                                          const FragmentB<NEAREST>& b1) {
-    const FragmentB<NEAREST> both[2] = {b0, b1};
-    mma_split<NEAREST, 2>(d, a, both);
+__device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA& a, const FragmentB& b0, const FragmentB& b1) {
+    const FragmentB both[2] = {b0, b1};
+    mma_split(d, a, both);
 }
 // B is exact in TF32
-__device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA<>& a, const float (&b0)[2], const float (&b1)[2]) {
+__device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA& a, const float (&b0)[2], const float (&b1)[2]) {
     mma_tf32(d[0], a.low, b0);
     mma_tf32(d[1], a.low, b1);
     mma_tf32(d[0], a.high, b0);
@@ -106,9 +81,8 @@ __device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA<>& a
 }
 
 // rows `source[row * stride + column]` of a 16 x 8 operand
-template <bool NEAREST = false>
-__device__ __forceinline__ FragmentA<NEAREST> load_a(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentA<NEAREST> out;
+__device__ __forceinline__ FragmentA load_a(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentA out;
     const float* at = source + (lane >> 2) * stride + (lane & 3);
     out.set(0, at[0]);
     out.set(1, at[8 * stride]);
@@ -117,9 +91,8 @@ __device__ __forceinline__ FragmentA<NEAREST> load_a(const float* source, uint32
     return out;
 }
 // the same operand stored transposed: `source[column * stride + row]`
-template <bool NEAREST = false>
-__device__ __forceinline__ FragmentA<NEAREST> load_a_transposed(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentA<NEAREST> out;
+__device__ __forceinline__ FragmentA load_a_transposed(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentA out;
     const float* at = source + (lane & 3) * stride + (lane >> 2);
     out.set(0, at[0]);
     out.set(1, at[8]);
@@ -128,17 +101,15 @@ __device__ __forceinline__ FragmentA<NEAREST> load_a_transposed(const float* sou
     return out;
 }
 // an 8 x 8 operand B[k][n] stored as `source[k * stride + n]`, or transposed as `source[n * stride + k]`
-template <bool NEAREST = false>
-__device__ __forceinline__ FragmentB<NEAREST> load_b(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB<NEAREST> out;
+__device__ __forceinline__ FragmentB load_b(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentB out;
     const float* at = source + (lane & 3) * stride + (lane >> 2);
     out.set(0, at[0]);
     out.set(1, at[4 * stride]);
     return out;
 }
-template <bool NEAREST = false>
-__device__ __forceinline__ FragmentB<NEAREST> load_b_transposed(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB<NEAREST> out;
+__device__ __forceinline__ FragmentB load_b_transposed(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentB out;
     const float* at = source + (lane >> 2) * stride + (lane & 3);
     out.set(0, at[0]);
     out.set(1, at[4]);
@@ -151,9 +122,8 @@ __device__ __forceinline__ void store_c(float* target, uint32_t stride, uint32_t
     *reinterpret_cast<float2*>(at + 8 * stride) = make_float2(c[2], c[3]);
 }
 
-// The kernels of delta_split.cu: segments whose projections lie in whole 16-byte pieces, heads up to 64.
+// The kernels of delta_split.cu: bf16 segments whose projections lie in whole 16-byte pieces, heads up to 64.
 size_t delta_split_bytes(size_t heads, size_t tiles);
-template <typename T>
-cudaError_t launch_delta_split(cudaStream_t stream, const DeltaArgs<T>& args, float* chunks, size_t chunk_bytes);
+cudaError_t launch_delta_split(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& args, float* chunks, size_t chunk_bytes);
 
 }  // namespace lfm25

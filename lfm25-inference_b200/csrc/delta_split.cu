@@ -1,4 +1,4 @@
-// The generalised delta rule over prompts, split along the sequence.
+// The generalised delta rule over bf16 prompts, split along the sequence.
 //
 // Over a chunk of 64 tokens, with P_t the product of the decays of its tokens up to t, S_t = diag(P_t) Q_t and
 //     U_t = u_t P_(t-1),   R_t = r_t P_t,   K_t = k_t / P_t,   B_t = -(a_t u_t) / P_t          (per key channel)
@@ -12,15 +12,15 @@
 //     form     A, D, R', O' of every chunk of every head                        all chunks side by side
 //     carry    S <- A S + D through each segment's chunks, S_0 in the place of D    one product of 64 x 64 x 16 per chunk
 //     finish   O = R' S_0 + O', norm, gate                                      all chunks side by side
-// so only `carry` is serial, in steps of 64 tokens of a single small product.  4096 tokens of 32 heads in bf16: 231 + 49 + 45 us
-// (one CTA per head, tile after tile of 16 tokens: 773 us on 32 SMs); 250 tokens of 16 heads in f32: 80 us for the three
-// (token by token: 253 us).
+// so only `carry` is serial, in steps of 64 tokens of a single small product.  4096 tokens of 32 heads: 231 + 49 + 45 us
+// (one CTA per head, tile after tile of 16 tokens: 773 us on 32 SMs).
 //
 // Decays are multiplied up by a scan, never summed as logarithms: P_t and the 1 / P_s that meets it come from the same
 // factors, and both carry a handful of roundings.  A decay is at least exp(-exp(-1/2)), so 1 / P_t stays below 1e17 and a
 // product P_t / P_s keeps its relative accuracy.  All matrix products are TF32 with both operands in two parts (bf16 values
-// of v need no second one), with f32 sums; f32 activations take the product of the low parts too and keep the tensor
-// cores' sums short (a model of 8 layers, 250 tokens, against float64: 0.99e-6; with plain multiply-adds 0.94e-6).
+// of v need no second one), with f32 sums.  Not for f32 activations: the decays' products, their reciprocals and the parts
+// each round once more than the token-by-token recurrence does (250 tokens of 16 heads, state against float64: 1.44e-7
+// with the best form of the products, 0.76e-7 token by token).
 #include <algorithm>
 
 #include "delta_rule.h"
@@ -47,9 +47,8 @@ constexpr uint32_t kFinishThreads = 128;
 
 // Fragments in which k index c of a 16 x 8 operand stands for column (row of B) 2c, and c + 4 for 2c + 1: the accumulator of
 // one product is then an operand of the next as it is, and operands along a row are read two at a time.
-template <bool NEAREST>
-__device__ __forceinline__ FragmentA<NEAREST> load_a_pairs(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentA<NEAREST> out;
+__device__ __forceinline__ FragmentA load_a_pairs(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentA out;
     const float* at = source + (lane >> 2) * stride + (lane & 3) * 2;
     const float2 upper = *reinterpret_cast<const float2*>(at), lower = *reinterpret_cast<const float2*>(at + 8 * stride);
     out.set(0, upper.x);
@@ -58,26 +57,23 @@ __device__ __forceinline__ FragmentA<NEAREST> load_a_pairs(const float* source, 
     out.set(3, lower.y);
     return out;
 }
-template <bool NEAREST>
-__device__ __forceinline__ FragmentA<NEAREST> a_from_c(const float (&c)[4]) {
-    FragmentA<NEAREST> out;
+__device__ __forceinline__ FragmentA a_from_c(const float (&c)[4]) {
+    FragmentA out;
     out.set(0, c[0]);
     out.set(1, c[2]);
     out.set(2, c[1]);
     out.set(3, c[3]);
     return out;
 }
-template <bool NEAREST>
-__device__ __forceinline__ FragmentB<NEAREST> load_b_transposed_pairs(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB<NEAREST> out;
+__device__ __forceinline__ FragmentB load_b_transposed_pairs(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentB out;
     const float2 both = *reinterpret_cast<const float2*>(source + (lane >> 2) * stride + (lane & 3) * 2);
     out.set(0, both.x);
     out.set(1, both.y);
     return out;
 }
-template <bool NEAREST>
-__device__ __forceinline__ FragmentB<NEAREST> load_b_pairs(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB<NEAREST> out;
+__device__ __forceinline__ FragmentB load_b_pairs(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentB out;
     const float* at = source + (lane & 3) * 2 * stride + (lane >> 2);
     out.set(0, at[0]);
     out.set(1, at[stride]);
@@ -94,7 +90,7 @@ __device__ __forceinline__ void load_c(const float* source, uint32_t stride, uin
 
 // d[n] += a * rows for eight column blocks, `rows` bf16 (exact in TF32) or f32; PAIRS: in the order of load_b_pairs
 template <bool PAIRS>
-__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA<false>& a, const __nv_bfloat16* rows,
+__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA& a, const __nv_bfloat16* rows,
                                               uint32_t lane) {
     const uint32_t first = (PAIRS ? (lane & 3) * 2 : lane & 3) * kPitch + (lane >> 2);
     const uint32_t second = first + (PAIRS ? 1 : 4) * kPitch;
@@ -108,46 +104,26 @@ __device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA<
         mma_tf32(d[n + 1], a.high, b1);
     }
 }
-template <bool PAIRS, bool NEAREST>
-__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA<NEAREST>& a, const float* rows, uint32_t lane) {
+template <bool PAIRS>
+__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA& a, const float* rows, uint32_t lane) {
 #pragma unroll
     for (uint32_t n = 0; n < 8; n += 2) {
-        FragmentB<NEAREST> b[2];
+        FragmentB b[2];
 #pragma unroll
         for (uint32_t q = 0; q < 2; ++q) {
-            b[q] = PAIRS ? load_b_pairs<NEAREST>(rows + (n + q) * 8, kPitch, lane)
-                         : load_b<NEAREST>(rows + (n + q) * 8, kPitch, lane);
+            b[q] = PAIRS ? load_b_pairs(rows + (n + q) * 8, kPitch, lane)
+                         : load_b(rows + (n + q) * 8, kPitch, lane);
         }
-        mma_split<NEAREST, 2>(d + n, a, b);
+        mma_split(d + n, a, b);
     }
 }
 
 __device__ __forceinline__ float2 load_pair(const __nv_bfloat16* source) {
     return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(source));
 }
-__device__ __forceinline__ float2 load_pair(const float* source) { return *reinterpret_cast<const float2*>(source); }
 
-// Element functions: the accuracy that each activation type's other kernels have
-template <typename T>
-__device__ __forceinline__ float sigmoid_of(float z) {
-    return std::is_same<T, float>::value ? sigmoidf(z) : fast_sigmoid(z);
-}
-template <typename T>
-__device__ __forceinline__ float tanh_of(float z) {
-    return std::is_same<T, float>::value ? tanhf(z) : fast_tanh(z);
-}
-template <typename T>
-__device__ __forceinline__ float decay_of(float logit) {
-    const float exponent = -kDecayScale * sigmoid_of<T>(logit);
-    return std::is_same<T, float>::value ? expf(exponent) : __expf(exponent);
-}
+__device__ __forceinline__ float decay_of(float logit) { return __expf(-kDecayScale * fast_sigmoid(logit)); }
 
-template <typename T>
-__device__ __forceinline__ float reciprocal_of(float value) {
-    return std::is_same<T, float>::value ? 1.0f / value : __fdividef(1.0f, value);
-}
-
-template <typename T>
 struct FormShared {
     float u[kTokens * kPitch];                     // U, then W
     float r[kTokens * kPitch];
@@ -157,19 +133,17 @@ struct FormShared {
     float inverse[4][16 * kInversePitch];          // of I - lower on the diagonal blocks
     float block_decay[4][kDim];                    // products over 16 tokens
     float squares[2][kTokens];                     // |k|^2 over half of the channels each
-    T v[kTokens * kPitch];
+    __nv_bfloat16 v[kTokens * kPitch];
 };
 
 // About 6500 m16n8k8 products per chunk, eight cycles each per SM quarter, keep the tensor pipe 37 % busy; the rest is the
 // latency of the five stages between barriers, which two CTAs per SM hide in part.  Longer loops are not unrolled further:
 // the code then outgrows the instruction cache (251 -> 231 us).
-template <typename T>
-__global__ void __launch_bounds__(kFormThreads, std::is_same<T, float>::value ? 1 : 2)
-delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, float* chunks) {
-    constexpr uint32_t kParts = std::is_same<T, float>::value ? 3 : 2;       // bf16 parts of tanh(z): 24 or 16 bits
-    constexpr bool kNearest = std::is_same<T, float>::value;
+__global__ void __launch_bounds__(kFormThreads, 2)
+delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t head_count, float* chunks) {
+    constexpr uint32_t kParts = 2;                 // bf16 parts of tanh(z): 16 bits
     extern __shared__ __align__(16) unsigned char form_shared[];
-    FormShared<T>& shared = *reinterpret_cast<FormShared<T>*>(form_shared);
+    FormShared& shared = *reinterpret_cast<FormShared*>(form_shared);
     pdl_launch_dependents();
     pdl_wait();
     const SegmentTile tile = locate_tile(args.segments, kTokens, blockIdx.x / head_count);
@@ -180,11 +154,11 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
     const uint32_t dim = args.dim;
     const size_t width = static_cast<size_t>(args.heads) * dim;
     const size_t head_base = static_cast<size_t>(head) * dim;
-    const T* projected = args.projected + static_cast<size_t>(tile.first) * args.pitch;
+    const __nv_bfloat16* projected = args.projected + static_cast<size_t>(tile.first) * args.pitch;
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 
     // ---- V
-    constexpr uint32_t kPiece = 16 / sizeof(T);
+    constexpr uint32_t kPiece = 8;                 // elements of 16 bytes
     for (uint32_t item = threadIdx.x; item < kTokens * kDim / kPiece; item += kFormThreads) {
         const uint32_t token = item / (kDim / kPiece), column = item % (kDim / kPiece) * kPiece;
         const bool inside = token < tile.count && column < dim;
@@ -205,7 +179,7 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
             const uint32_t token = row0 + i * 8;
             r[n][i] = k[n][i] = removal[n][i] = make_float2(0.0f, 0.0f);
             if (token < tile.count && channel < dim) {
-                const T* source = projected + token * args.pitch + head_base + channel;
+                const __nv_bfloat16* source = projected + token * args.pitch + head_base + channel;
                 r[n][i] = load_pair(source);
                 k[n][i] = load_pair(source + width);
                 removal[n][i] = load_pair(source + 4 * width);
@@ -242,7 +216,7 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
                 }
                 // columns between rank and the end of its last 16 bytes belong to nobody
 #pragma unroll
-                for (uint32_t i = 0; i < 8; ++i) value[i] = z0 + z + i < args.rank ? tanh_of<T>(value[i]) : 0.0f;
+                for (uint32_t i = 0; i < 8; ++i) value[i] = z0 + z + i < args.rank ? fast_tanh(value[i]) : 0.0f;
 #pragma unroll
                 for (uint32_t part = 0; part < kParts; ++part) {
                     uint32_t packed[4];
@@ -290,7 +264,7 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
             if (channel < dim) base = load_pair(args.decay_base + head_base + channel);
 #pragma unroll
             for (uint32_t i = 0; i < 4; ++i) {
-                upto[n][i] = row0 + (i >> 1) * 8 < tile.count ? decay_of<T>(logits[n][i] + (i & 1 ? base.y : base.x)) : 1.0f;
+                upto[n][i] = row0 + (i >> 1) * 8 < tile.count ? decay_of(logits[n][i] + (i & 1 ? base.y : base.x)) : 1.0f;
             }
 #pragma unroll
             for (uint32_t delta = 4; delta < 32; delta <<= 1) {
@@ -339,17 +313,17 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
         for (uint32_t i = 0; i < 2; ++i) {
             const uint32_t token = row0 + i * 8;
             const float square = shared.squares[0][token] + shared.squares[1][token] + kUnitEps;
-            const float unit = std::is_same<T, float>::value ? 1.0f / sqrtf(square) : rsqrtf(square);
+            const float unit = rsqrtf(square);
             const float px = upto[n][2 * i] * earlier.x, py = upto[n][2 * i + 1] * earlier.y;
-            const float ix = reciprocal_of<T>(px), iy = reciprocal_of<T>(py);
+            const float ix = __fdividef(1.0f, px), iy = __fdividef(1.0f, py);
             const float ux = k[n][i].x * unit, uy = k[n][i].y * unit;
             const uint32_t at = token * kPitch + channel;
             *reinterpret_cast<float2*>(shared.u + at) =
                 make_float2(ux * (before[n][2 * i] * earlier.x), uy * (before[n][2 * i + 1] * earlier.y));
             *reinterpret_cast<float2*>(shared.r + at) = make_float2(r[n][i].x * px, r[n][i].y * py);
             *reinterpret_cast<float2*>(shared.k + at) = make_float2(k[n][i].x * ix, k[n][i].y * iy);
-            *reinterpret_cast<float2*>(shared.b + at) = make_float2(-sigmoid_of<T>(removal[n][i].x + bias.x) * ux * ix,
-                                                                    -sigmoid_of<T>(removal[n][i].y + bias.y) * uy * iy);
+            *reinterpret_cast<float2*>(shared.b + at) = make_float2(-fast_sigmoid(removal[n][i].x + bias.x) * ux * ix,
+                                                                    -fast_sigmoid(removal[n][i].y + bias.y) * uy * iy);
         }
     }
     copy_async_wait<0>();
@@ -368,12 +342,12 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
         float with_b[2][4] = {}, with_k[2][4] = {};
 #pragma unroll 2
         for (uint32_t c = 0; c < kDim; c += 8) {
-            const FragmentA<kNearest> a = load_a_pairs<kNearest>(rows + c, kPitch, lane);
+            const FragmentA a = load_a_pairs(rows + c, kPitch, lane);
             const uint32_t at = j * 16 * kPitch + c;
-            mma_split(with_b, a, load_b_transposed_pairs<kNearest>(shared.b + at, kPitch, lane),
-                      load_b_transposed_pairs<kNearest>(shared.b + at + 8 * kPitch, kPitch, lane));
-            mma_split(with_k, a, load_b_transposed_pairs<kNearest>(shared.k + at, kPitch, lane),
-                      load_b_transposed_pairs<kNearest>(shared.k + at + 8 * kPitch, kPitch, lane));
+            mma_split(with_b, a, load_b_transposed_pairs(shared.b + at, kPitch, lane),
+                      load_b_transposed_pairs(shared.b + at + 8 * kPitch, kPitch, lane));
+            mma_split(with_k, a, load_b_transposed_pairs(shared.k + at, kPitch, lane),
+                      load_b_transposed_pairs(shared.k + at + 8 * kPitch, kPitch, lane));
         }
 #pragma unroll
         for (uint32_t n = 0; n < 2; ++n) {
@@ -388,7 +362,7 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
         }
 #pragma unroll
         for (uint32_t n = 0; n < 2; ++n) {
-            multiply_rows<true>(with_values, a_from_c<kNearest>(with_k[n]), shared.v + (j * 16 + n * 8) * kPitch, lane);
+            multiply_rows<true>(with_values, a_from_c(with_k[n]), shared.v + (j * 16 + n * 8) * kPitch, lane);
         }
     }
     float behind[8][4] = {};                       // K^T V, then D: 16 key channels per warp of the first four
@@ -411,7 +385,7 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
         }
 #pragma unroll 2
         for (uint32_t t = 0; t < kTokens; t += 8) {
-            multiply_rows<false>(behind, load_a_transposed<kNearest>(shared.k + t * kPitch + mine * 16, kPitch, lane),
+            multiply_rows<false>(behind, load_a_transposed(shared.k + t * kPitch + mine * 16, kPitch, lane),
                                    shared.v + t * kPitch, lane);
         }
     }
@@ -436,8 +410,8 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
                 load_c(target + 8, kPitch, lane, side[1]);
 #pragma unroll
                 for (uint32_t s = 0; s < i * 16; s += 8) {
-                    mma_split(side, load_a<kNearest>(shared.lower + i * 16 * kLowerPitch + s, kLowerPitch, lane),
-                              load_b<kNearest>(columns + s * kPitch, kPitch, lane), load_b<kNearest>(columns + s * kPitch + 8, kPitch, lane));
+                    mma_split(side, load_a(shared.lower + i * 16 * kLowerPitch + s, kLowerPitch, lane),
+                              load_b(columns + s * kPitch, kPitch, lane), load_b(columns + s * kPitch + 8, kPitch, lane));
                 }
                 __syncwarp();
                 store_c(target, kPitch, lane, side[0]);
@@ -447,8 +421,8 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
             float solved[2][4] = {};
 #pragma unroll
             for (uint32_t s = 0; s < 16; s += 8) {
-                mma_split(solved, load_a<kNearest>(shared.inverse[i] + s, kInversePitch, lane),
-                          load_b<kNearest>(target + s * kPitch, kPitch, lane), load_b<kNearest>(target + s * kPitch + 8, kPitch, lane));
+                mma_split(solved, load_a(shared.inverse[i] + s, kInversePitch, lane),
+                          load_b(target + s * kPitch, kPitch, lane), load_b(target + s * kPitch + 8, kPitch, lane));
             }
             __syncwarp();
             store_c(target, kPitch, lane, solved[0]);
@@ -462,7 +436,7 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
     if (forward) {
 #pragma unroll 1
         for (uint32_t t = 0; t < kTokens; t += 8) {
-            const FragmentA<kNearest> a = load_a_transposed<kNearest>(shared.b + t * kPitch + mine * 16, kPitch, lane);
+            const FragmentA a = load_a_transposed(shared.b + t * kPitch + mine * 16, kPitch, lane);
             multiply_rows<false>(from_state, a, shared.u + t * kPitch, lane);
             multiply_rows<false>(behind, a, shared.k + t * kPitch, lane);
         }
@@ -490,7 +464,7 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
             if (j > mine) continue;
 #pragma unroll
             for (uint32_t n = 0; n < 2; ++n) {
-                const FragmentA<kNearest> a = a_from_c<kNearest>(against_b[j][n]);
+                const FragmentA a = a_from_c(against_b[j][n]);
                 multiply_rows<true>(from_state, a, shared.u + (j * 16 + n * 8) * kPitch, lane);
                 multiply_rows<true>(with_values, a, shared.k + (j * 16 + n * 8) * kPitch, lane);
             }
@@ -507,9 +481,8 @@ delta_form_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, 
     }
 }
 
-template <bool NEAREST>
-__device__ __forceinline__ FragmentA<NEAREST> operand_of(const float4& stored) {
-    FragmentA<NEAREST> out;
+__device__ __forceinline__ FragmentA operand_of(const float4& stored) {
+    FragmentA out;
     out.set(0, stored.x);
     out.set(1, stored.y);
     out.set(2, stored.z);
@@ -519,10 +492,8 @@ __device__ __forceinline__ FragmentA<NEAREST> operand_of(const float4& stored) {
 
 // A CTA carries 16 value columns of one head through one segment; a warp owns 16 key channels of A and D and copies them
 // into its own part of shared memory kCarryStages - 1 chunks ahead.  Bound by the chain load S, multiply, store S, barrier.
-template <typename T>
 __global__ void __launch_bounds__(kCarryThreads)
-delta_carry_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, float* chunks) {
-    constexpr bool kNearest = std::is_same<T, float>::value;
+delta_carry_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t head_count, float* chunks) {
     extern __shared__ __align__(16) float carry_shared[];
     float4* stages = reinterpret_cast<float4*>(carry_shared);                     // [stage][10][thread]
     float* states = carry_shared + kCarryStages * 10 * kCarryThreads * 4;         // [2][channel][kCarryPitch]
@@ -593,11 +564,11 @@ delta_carry_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count,
         float4 kept[2];
 #pragma unroll
         for (uint32_t c = 0; c < 8; ++c) {
-            const FragmentA<kNearest> a = operand_of<kNearest>(stage[c * kCarryThreads]);
+            const FragmentA a = operand_of(stage[c * kCarryThreads]);
             const float* rows = state + (c * 8 + (lane & 3) * 2) * kCarryPitch + (lane >> 2);
 #pragma unroll
             for (uint32_t n = 0; n < 2; ++n) {
-                FragmentB<kNearest> b;
+                FragmentB b;
                 const float first = rows[n * 8], second = rows[n * 8 + kCarryPitch];
                 b.set(0, first);
                 b.set(1, second);
@@ -608,13 +579,9 @@ delta_carry_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count,
                     kept[n].z = first;
                     kept[n].w = second;
                 }
-                if (kNearest) {
-                    mma_split(sum[n], a, b);
-                } else {
-                    mma_tf32(low_high[n], a.low, b.high);
-                    mma_tf32(high_low[n], a.high, b.low);
-                    mma_tf32(sum[n], a.high, b.high);
-                }
+                mma_tf32(low_high[n], a.low, b.high);
+                mma_tf32(high_low[n], a.high, b.low);
+                mma_tf32(sum[n], a.high, b.high);
             }
         }
         // the state before the chunk, as operands of the outputs' product
@@ -641,15 +608,10 @@ delta_carry_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count,
 __device__ __forceinline__ void store_pair(__nv_bfloat16* target, float low, float high) {
     *reinterpret_cast<uint32_t*>(target) = pack_bf16x2(low, high);
 }
-__device__ __forceinline__ void store_pair(float* target, float low, float high) {
-    *reinterpret_cast<float2*>(target) = make_float2(low, high);
-}
 
 // 16 tokens per warp: O = R' S_0 + O', the norm over the head, the gate.  Bound by reading 48 KB per chunk.
-template <typename T>
 __global__ void __launch_bounds__(kFinishThreads)
-delta_finish_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count, const float* chunks) {
-    constexpr bool kNearest = std::is_same<T, float>::value;
+delta_finish_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t head_count, const float* chunks) {
     pdl_launch_dependents();
     pdl_wait();
     const SegmentTile tile = locate_tile(args.segments, kTokens, blockIdx.x / head_count);
@@ -674,11 +636,11 @@ delta_finish_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count
     }
 #pragma unroll
     for (uint32_t m = 0; m < 4; ++m) {
-        const FragmentA<kNearest> a0 = operand_of<kNearest>(operands[2 * m * 32]), a1 = operand_of<kNearest>(operands[(2 * m + 1) * 32]);
+        const FragmentA a0 = operand_of(operands[2 * m * 32]), a1 = operand_of(operands[(2 * m + 1) * 32]);
 #pragma unroll
         for (uint32_t n = 0; n < 8; ++n) {
             const float4 state = states[(m * 8 + n) * 32];
-            FragmentB<kNearest> b0, b1;
+            FragmentB b0, b1;
             b0.set(0, state.x);
             b0.set(1, state.y);
             b1.set(0, state.z);
@@ -696,21 +658,19 @@ delta_finish_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count
         }
         squares += __shfl_xor_sync(0xffffffffu, squares, 1);
         squares += __shfl_xor_sync(0xffffffffu, squares, 2);
-        const float factor = std::is_same<T, float>::value
-                                 ? inverse_rms(squares, args.dim, args.eps)
-                                 : rsqrtf(squares / static_cast<float>(args.dim) + args.eps);
+        const float factor = rsqrtf(squares / static_cast<float>(args.dim) + args.eps);
         const uint32_t token = warp * 16 + (lane >> 2) + half * 8;
         if (token < tile.count) {
-            const T* gates = args.projected + static_cast<size_t>(tile.first + token) * args.pitch + 3 * width + head_base;
-            T* target = args.out + static_cast<size_t>(tile.first + token) * args.out_pitch + head_base;
+            const __nv_bfloat16* gates = args.projected + static_cast<size_t>(tile.first + token) * args.pitch + 3 * width + head_base;
+            __nv_bfloat16* target = args.out + static_cast<size_t>(tile.first + token) * args.out_pitch + head_base;
 #pragma unroll
             for (uint32_t n = 0; n < 8; ++n) {
                 const uint32_t channel = n * 8 + (lane & 3) * 2;
                 if (channel < args.dim) {
                     const float2 gate = load_pair(gates + channel);
                     const float2 weight = load_pair(args.norm + head_base + channel);
-                    store_pair(target + channel, out[n][2 * half] * factor * weight.x * sigmoid_of<T>(gate.x),
-                               out[n][2 * half + 1] * factor * weight.y * sigmoid_of<T>(gate.y));
+                    store_pair(target + channel, out[n][2 * half] * factor * weight.x * fast_sigmoid(gate.x),
+                               out[n][2 * half + 1] * factor * weight.y * fast_sigmoid(gate.y));
                 }
             }
         }
@@ -722,38 +682,34 @@ delta_finish_kernel(const DeltaArgs<T> args, uint32_t head0, uint32_t head_count
 size_t delta_split_bytes(size_t heads, size_t tiles) { return heads * tiles * kChunkFloats * sizeof(float); }
 
 // Heads are taken in groups whose chunks fit the scratch.
-template <typename T>
-cudaError_t launch_delta_split(cudaStream_t stream, const DeltaArgs<T>& args, float* chunks, size_t chunk_bytes) {
+cudaError_t launch_delta_split(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& args, float* chunks, size_t chunk_bytes) {
     const size_t tiles = tile_bound(args.segments, kTokens);
     const uint32_t most = static_cast<uint32_t>(std::min<size_t>(args.heads, chunk_bytes / delta_split_bytes(1, tiles)));
     if (most == 0) return cudaErrorInvalidValue;
     const uint32_t groups = (args.heads + most - 1) / most;
     const uint32_t group = (args.heads + groups - 1) / groups;
     const size_t carry_bytes = (kCarryStages * 10 * kCarryThreads * 4 + 2 * kDim * kCarryPitch) * sizeof(float);
-    cudaError_t status = cudaFuncSetAttribute(reinterpret_cast<const void*>(delta_form_kernel<T>),
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(FormShared<T>));
+    cudaError_t status = cudaFuncSetAttribute(reinterpret_cast<const void*>(delta_form_kernel),
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(FormShared));
     if (status == cudaSuccess) {
-        status = cudaFuncSetAttribute(reinterpret_cast<const void*>(delta_carry_kernel<T>),
+        status = cudaFuncSetAttribute(reinterpret_cast<const void*>(delta_carry_kernel),
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(carry_bytes));
     }
     for (uint32_t head0 = 0; head0 < args.heads && status == cudaSuccess; head0 += group) {
         const uint32_t count = std::min(group, args.heads - head0);
         const unsigned int blocks = static_cast<unsigned int>(tiles * count);
-        status = launch_kernel(delta_form_kernel<T>, blocks, kFormThreads, sizeof(FormShared<T>), stream, 1, args, head0, count,
+        status = launch_kernel(delta_form_kernel, blocks, kFormThreads, sizeof(FormShared), stream, 1, args, head0, count,
                                chunks);
         if (status == cudaSuccess) {
-            status = launch_kernel(delta_carry_kernel<T>,
+            status = launch_kernel(delta_carry_kernel,
                                    static_cast<unsigned int>(args.segments.num_segments * count * (kDim / kCarryColumns)),
                                    kCarryThreads, carry_bytes, stream, 1, args, head0, count, chunks);
         }
         if (status == cudaSuccess) {
-            status = launch_kernel(delta_finish_kernel<T>, blocks, kFinishThreads, 0, stream, 1, args, head0, count, chunks);
+            status = launch_kernel(delta_finish_kernel, blocks, kFinishThreads, 0, stream, 1, args, head0, count, chunks);
         }
     }
     return status;
 }
-
-template cudaError_t launch_delta_split<float>(cudaStream_t, const DeltaArgs<float>&, float*, size_t);
-template cudaError_t launch_delta_split<__nv_bfloat16>(cudaStream_t, const DeltaArgs<__nv_bfloat16>&, float*, size_t);
 
 }  // namespace lfm25

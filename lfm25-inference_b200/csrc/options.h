@@ -18,10 +18,10 @@
 //   hybrid_attention     0 auto | 1 umma | 2 mma               0         kernel of the mixed-step attention
 //   stack_attention      0 auto | 1 scalar                     0         attention of layer-stack models: the tensor-core kernels
 //                                                                        where they take the shape, or always the scalar one
-//   delta_prompt         0 auto | 1 scan | 2 general           0         delta rule over segments: tensor-core chunks where they
-//                        | 3 carried | 4 split                           take the type and head size, the token-by-token prompt
-//                                                                        kernel, or the general kernel; 3 and 4: chunks, never
-//                                                                        or always split along the sequence
+//   delta_prompt         0 auto | 1 scan | 2 general           0         delta rule over bf16 segments: tensor-core chunks where they
+//                        | 3 carried | 4 split                           take the head size, the token-by-token prompt kernel, or
+//                                                                        the general kernel; 3 and 4: chunks, never or always
+//                                                                        split along the sequence (f32: the general kernel)
 //   state_space_prompt   0 auto | 1 scan                       0         state-space recurrence over bf16 segments: tensor-core
 //                                                                        chunks where they take the sizes, or the
 //                                                                        token-by-token kernel

@@ -126,7 +126,8 @@ def test_delta_rule_prompt_kernels_agree(device, library_option, heads, dim, ran
 @pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("heads,dim,rank", [(3, 64, 16), (1, 8, 5), (2, 24, 130), (12, 40, 64)])
 def test_delta_rule_split_along_the_sequence(device, library_option, dtype, heads, dim, rank):
-    """Portions that end at, before and behind the edges of 16- and 64-token pieces, strong decays beside weak ones."""
+    """Portions that end at, before and behind the edges of 16- and 64-token pieces, strong decays beside weak ones (f32, which
+    is never split: the same through the general kernel)."""
     library_option("delta_prompt", 4)
 
     def strong(tensors):
@@ -135,35 +136,54 @@ def test_delta_rule_split_along_the_sequence(device, library_option, dtype, head
     check_layer(config, 17, device, dtype, [64, 63, 2, 65, 128, 17, 1, 200], rank, strong)
 
 
-@pytest.mark.parametrize("dtype", TYPES)
-def test_delta_rule_split_mixed_step(device, library_option, dtype):
-    """Sequences side by side behind single tokens, with more heads than the scratch holds at once, against the kernels that
-    carry a segment in one CTA: f32 arithmetic in both, so bf16 results differ by their last rounding."""
+def delta_steps(config, tensors, device, dtype, chunks, forced, library_option):
+    """Residual streams and recurrent states of two steps over the same tokens, the second from the first one's state."""
     import torch
 
     from lfm25_inference_b200 import model as lfm_model
     from lfm25_inference_b200 import ops, stack, workloads
+    library_option("delta_prompt", forced)
+    tokens = np.random.default_rng(5).integers(0, config["vocab"], size=chunks.sum()).astype(np.uint32)
+    with torch.cuda.stream(torch.cuda.Stream(device)):
+        blaslt = ops.BlasLt()
+        layout = workloads.mixed_step_batch(1, np.zeros(len(chunks), np.int64), chunks, 100)
+        model = cases.product_model(config, tensors, device, dtype, 100, len(chunks))
+        executor = stack.StackExecutor(blaslt, model, len(tokens), len(chunks))
+        steps = []
+        for _ in range(2):
+            executor.forward_ragged(lfm_model.RaggedBatch(device, layout, tokens))
+            steps.append(executor.residual(len(tokens)))
+        executor.close()
+        blaslt.close()
+        mixer, offset = config["layers"][0]["mixer"], model.struct.layers[0].state_offset
+        records = model.records.view(len(chunks), -1).cpu().numpy()
+        states = np.ascontiguousarray(records[:, offset:offset + 4 * mixer["heads"] * mixer["dim"] ** 2]).view(np.float32)
+    return np.concatenate(steps), states
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+def test_delta_rule_split_mixed_step(device, library_option, dtype):
+    """Sequences side by side behind single tokens, with more heads than the scratch holds at once, against the kernels that
+    carry a segment in one CTA: f32 arithmetic in both, so bf16 results differ by their last rounding."""
     config = cases.config_of([cases.delta_layer(64, 8, ff=0)])
     tensors = cases.random_tensors(config, 29, 16)
     chunks = np.array([1, 1, 70, 64, 129, 65, 80, 3])
-    tokens = np.random.default_rng(5).integers(0, config["vocab"], size=chunks.sum()).astype(np.uint32)
-    results = []
-    for forced in (3, 4):
-        library_option("delta_prompt", forced)
-        with torch.cuda.stream(torch.cuda.Stream(device)):
-            blaslt = ops.BlasLt()
-            layout = workloads.mixed_step_batch(1, np.zeros(len(chunks), np.int64), chunks, 64)
-            model = cases.product_model(config, tensors, device, dtype, 64, len(chunks))
-            executor = stack.StackExecutor(blaslt, model, len(tokens), len(chunks))
-            steps = []
-            for _ in range(2):                     # the second continues from the first one's state
-                executor.forward_ragged(lfm_model.RaggedBatch(device, layout, tokens))
-                steps.append(executor.residual(len(tokens)))
-            results.append(np.concatenate(steps))
-            executor.close()
-            blaslt.close()
-    assert np.isfinite(results[0]).all()
-    assert cases.relative_error(results[1], results[0]).max() < {"float32": 5e-6, "bfloat16": 4e-3}[dtype]
+    results = [delta_steps(config, tensors, device, dtype, chunks, forced, library_option) for forced in (3, 4)]
+    assert np.isfinite(results[0][0]).all()
+    assert cases.relative_error(results[1][0], results[0][0]).max() < {"float32": 5e-6, "bfloat16": 4e-3}[dtype]
+    # the routes' rounding differs where there are two
+    assert np.array_equal(results[1][1], results[0][1]) == (dtype == "float32")
+
+
+@pytest.mark.parametrize("chunks", [[250], [64, 1, 64], [1500]])
+def test_delta_rule_f32_prompts_token_by_token(device, library_option, chunks):
+    """f32 activations keep plain f32 multiply-adds however few and long the prompts are: the general kernel's bits."""
+    config = cases.config_of([cases.delta_layer(3, 64, ff=0)])
+    tensors = cases.random_tensors(config, 29, 16)
+    results = [delta_steps(config, tensors, device, "float32", np.array(sorted(chunks)), forced, library_option)
+               for forced in (0, 2)]
+    for got, want in zip(*results):
+        assert np.array_equal(got, want)
 
 
 @pytest.mark.parametrize("dtype", TYPES)
