@@ -1191,11 +1191,11 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
                 float from_state[2][2][4] = {};        // [U, R][8 columns]
 #pragma unroll
                 for (uint32_t k = 0; k < DP / 8; ++k) {
-                    const FragmentB b0 = load_b(state + k * 8 * kColumnStride, kColumnStride, lane);
-                    const FragmentB b1 = load_b(state + k * 8 * kColumnStride + 8, kColumnStride, lane);
+                    const FragmentB<> b0 = load_b(state + k * 8 * kColumnStride, kColumnStride, lane);
+                    const FragmentB<> b1 = load_b(state + k * 8 * kColumnStride + 8, kColumnStride, lane);
 #pragma unroll
                     for (uint32_t m = 0; m < 2; ++m) {
-                        const FragmentA a = load_a(operands + m * kOperandR + k * 8, kRowStride, lane);
+                        const FragmentA<> a = load_a(operands + m * kOperandR + k * 8, kRowStride, lane);
                         mma_split(from_state[m], a, b0, b1);
                     }
                 }
@@ -1216,7 +1216,7 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
                 // right-hand side, then Y
 #pragma unroll
                 for (uint32_t k = 0; k < 2; ++k) {
-                    const FragmentA a = load_a(triangles + 1 * kTriangle + k * 8, kTriangleStride, lane);
+                    const FragmentA<> a = load_a(triangles + 1 * kTriangle + k * 8, kTriangleStride, lane);
                     mma_split(from_state[0], a, v[k][0], v[k][1]);
                 }
                 store_c(columns, kColumnStride, lane, from_state[0][0]);
@@ -1225,7 +1225,7 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
                 float solved[2][4] = {};
 #pragma unroll
                 for (uint32_t k = 0; k < 2; ++k) {
-                    const FragmentA a = load_a(triangles + k * 8, kTriangleStride, lane);
+                    const FragmentA<> a = load_a(triangles + k * 8, kTriangleStride, lane);
                     mma_split(solved, a, load_b(columns + k * 8 * kColumnStride, kColumnStride, lane),
                               load_b(columns + k * 8 * kColumnStride + 8, kColumnStride, lane));
                 }
@@ -1233,7 +1233,7 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
                 store_c(columns, kColumnStride, lane, solved[0]);
                 store_c(columns + 8, kColumnStride, lane, solved[1]);
                 __syncwarp();
-                FragmentB y[2][2];
+                FragmentB<> y[2][2];
 #pragma unroll
                 for (uint32_t k = 0; k < 2; ++k) {
 #pragma unroll
@@ -1244,8 +1244,8 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
                 // O
 #pragma unroll
                 for (uint32_t k = 0; k < 2; ++k) {
-                    const FragmentA with_y = load_a(triangles + 2 * kTriangle + k * 8, kTriangleStride, lane);
-                    const FragmentA with_v = load_a(triangles + 3 * kTriangle + k * 8, kTriangleStride, lane);
+                    const FragmentA<> with_y = load_a(triangles + 2 * kTriangle + k * 8, kTriangleStride, lane);
+                    const FragmentA<> with_v = load_a(triangles + 3 * kTriangle + k * 8, kTriangleStride, lane);
                     mma_split(from_state[1], with_v, v[k][0], v[k][1]);
                     mma_split(from_state[1], with_y, y[k][0], y[k][1]);
                 }
@@ -1258,8 +1258,8 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
 #pragma unroll
                     for (uint32_t k = 0; k < 2; ++k) {
                         const uint32_t at = k * 8 * kTransposedStride + m * 16;
-                        const FragmentA with_v = load_a_transposed(operands + kOperandK + at, kTransposedStride, lane);
-                        const FragmentA with_y = load_a_transposed(operands + kOperandB + at, kTransposedStride, lane);
+                        const FragmentA<> with_v = load_a_transposed(operands + kOperandK + at, kTransposedStride, lane);
+                        const FragmentA<> with_y = load_a_transposed(operands + kOperandB + at, kTransposedStride, lane);
                         mma_split(accumulator[m], with_v, v[k][0], v[k][1]);
                         mma_split(accumulator[m], with_y, y[k][0], y[k][1]);
                     }
@@ -1468,7 +1468,7 @@ delta_chunk_kernel(const DeltaArgs<__nv_bfloat16> args) {
                 float product[2][4] = {};
 #pragma unroll
                 for (uint32_t k = 0; k < DP / 8; ++k) {
-                    const FragmentA a = load_a(rows + k * 8, kRowStride, lane);
+                    const FragmentA<> a = load_a(rows + k * 8, kRowStride, lane);
                     mma_split(product, a, load_b_transposed(against + k * 8, kTransposedStride, lane),
                               load_b_transposed(against + 8 * kTransposedStride + k * 8, kTransposedStride, lane));
                 }
@@ -1558,6 +1558,14 @@ cudaError_t launch_chunk(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& ar
                          kChunkThreads, shared, stream, 1, args);
 }
 
+bool prompt_kernel_takes(const DeltaArgs<__nv_bfloat16>& args) {
+    const size_t shared = args.dim <= 64 ? PromptLayout<64>(args.rank).total : PromptLayout<128>(args.rank).total;
+    return args.dim % 8 == 0 && args.dim <= 128 && args.rank <= kPromptMaxRank && args.pitch % 8 == 0 &&
+           args.out_pitch % 2 == 0 && aligned_to(args.projected, 16) && aligned_to(args.out, 4) &&
+           aligned_to(args.decay_up, 16) &&
+           shared <= 227 * 1024;
+}
+
 // Where bf16 prompts are split along the sequence (delta_split.cu): it does about twice the arithmetic of the kernels that
 // carry one head of one segment in a CTA, 0.16 us per head and 64 tokens over the whole chip against 12 us (four tiles) in a
 // CTA, so it pays while those leave most SMs idle and a prompt is long enough for its three launches.  Measured in whole steps of a 16-layer model with 32 heads, split against not: one prompt of 250 tokens
@@ -1565,25 +1573,14 @@ cudaError_t launch_chunk(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& ar
 constexpr size_t kSplitHeads = 80;
 constexpr size_t kSplitTokens = 256;
 
-// The kernels' 16-byte and pairwise accesses, and scratch for one head at least.
+// The kernels' pairwise accesses, and scratch for one head at least (beside what the chunk kernel needs).
 bool split_takes(const DeltaArgs<__nv_bfloat16>& args, const DeltaRuleLaunch& launch) {
     const int64_t forced = option(kOptDeltaPrompt);
     const size_t segments = launch.segments.num_segments;
     const size_t tokens = launch.segments.num_tokens - launch.decode_tokens;
-    return (forced == 0 || forced == 4) && launch.segments.offsets != nullptr && args.dim <= 64 && args.dim % 8 == 0 &&
-           args.pitch % 8 == 0 && args.out_pitch % 2 == 0 && aligned_to(args.projected, 16) && aligned_to(args.out, 4) &&
-           aligned_to(args.decay_up, 16) && aligned_to(args.decay_base, 4) && aligned_to(args.removal_bias, 4) &&
-           aligned_to(args.norm, 4) && launch.chunks != nullptr &&
-           delta_split_bytes(1, tile_bound(launch.segments, 64)) <= launch.chunk_bytes &&
-           (forced == 4 || (segments * args.heads <= kSplitHeads && tokens >= kSplitTokens * segments));
-}
-
-bool prompt_kernel_takes(const DeltaArgs<__nv_bfloat16>& args) {
-    const size_t shared = args.dim <= 64 ? PromptLayout<64>(args.rank).total : PromptLayout<128>(args.rank).total;
-    return args.dim % 8 == 0 && args.dim <= 128 && args.rank <= kPromptMaxRank && args.pitch % 8 == 0 &&
-           args.out_pitch % 2 == 0 && aligned_to(args.projected, 16) && aligned_to(args.out, 4) &&
-           aligned_to(args.decay_up, 16) &&
-           shared <= 227 * 1024;
+    return (forced == 4 || (forced == 0 && segments * args.heads <= kSplitHeads && tokens >= kSplitTokens * segments)) &&
+           aligned_to(args.decay_base, 4) && aligned_to(args.removal_bias, 4) && aligned_to(args.norm, 4) &&
+           launch.chunks != nullptr && delta_split_bytes(1, tile_bound(launch.segments, 64)) <= launch.chunk_bytes;
 }
 
 template <typename T, uint32_t DP, uint32_t LANES, uint32_t COLUMNS>
@@ -1643,9 +1640,10 @@ cudaError_t launch_typed(cudaStream_t stream, const DeltaRuleLaunch& launch) {
         return launch_decode<T, 128>(stream, args);
     }
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-        if (split_takes(args, launch)) return launch_delta_split(stream, args, launch.chunks, launch.chunk_bytes);
         if (launch.segments.offsets != nullptr && option(kOptDeltaPrompt) != 2 && prompt_kernel_takes(args)) {
             if (launch.dim <= kChunkDim && ChunkLayout(launch.rank).total <= 227 * 1024 && option(kOptDeltaPrompt) != 1) {
+                // the kernels for larger ranks keep more bits than the split ones
+                if (split_takes(args, launch)) return launch_delta_split(stream, args, launch.chunks, launch.chunk_bytes);
                 return launch_chunk(stream, args);
             }
             return launch.dim <= 64 ? launch_prompt<64, 4, 128>(stream, args) : launch_prompt<128, 4, 128>(stream, args);
@@ -1664,7 +1662,7 @@ bool delta_rule_needs_scratch(uint32_t dim) { return dim > 128; }
 
 size_t delta_rule_chunk_bytes(Activation type, uint32_t heads, uint32_t dim, size_t tokens, size_t segments) {
     const size_t most = std::min(std::min(segments, tokens / kSplitTokens), kSplitHeads / heads);
-    if (type != Activation::kBf16 || dim > 64 || dim % 8 != 0 || most == 0) return 0;
+    if (type != Activation::kBf16 || dim > kChunkDim || dim % 8 != 0 || most == 0) return 0;
     return std::min(delta_split_bytes(heads, tokens / 64 + most), kDeltaChunkBytes);
 }
 

@@ -41,39 +41,56 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const float (&a)[4], con
           "r"(__float_as_uint(b[0])), "r"(__float_as_uint(b[1])));
 }
 
-// An operand fragment as high + low: the high part is what TF32 keeps of the value (10 mantissa bits), the low part the
-// rest, of which TF32 keeps another 10.
-template <int N>
+// An operand fragment as high + low.  TF32 keeps 10 mantissa bits and ignores the rest: the high part is what it keeps of the
+// value, the low part the remainder, of which it keeps another 10.  NEAREST: the high part is rounded to nearest, which
+// halves the low one and leaves it either sign, so that what the products leave out has no direction.
+template <int N, bool NEAREST = false>
 struct SplitFragment {
     float high[N], low[N];
     __device__ __forceinline__ void set(int index, float value) {
-        high[index] = __uint_as_float(__float_as_uint(value) & 0xffffe000u);
+        high[index] = __uint_as_float((__float_as_uint(value) + (NEAREST ? 0x1000u : 0u)) & 0xffffe000u);
         low[index] = value - high[index];
     }
 };
-using FragmentA = SplitFragment<4>;
-using FragmentB = SplitFragment<2>;
+template <bool NEAREST = false>
+using FragmentA = SplitFragment<4, NEAREST>;
+template <bool NEAREST = false>
+using FragmentB = SplitFragment<2, NEAREST>;
 
-template <uint32_t COUNT>
-__device__ __forceinline__ void mma_split(float (*d)[4], const FragmentA& a, const FragmentB (&b)[COUNT]) {
+// The tensor cores cut what falls behind the accumulator's last bit.  NEAREST: every product of fragments starts from zero
+// and is added up with rounding to nearest.
+template <bool NEAREST, uint32_t COUNT>
+__device__ __forceinline__ void mma_split(float (*d)[4], const FragmentA<NEAREST>& a, const FragmentB<NEAREST> (&b)[COUNT]) {
+    float sums[COUNT][4] = {};
+    float (*target)[4] = NEAREST ? sums : d;
     // the accumulators' products alternate so that none waits for the one before it
 #pragma unroll
-    for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(d[n], a.low, b[n].high);
+    for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(target[n], a.low, b[n].high);
 #pragma unroll
-    for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(d[n], a.high, b[n].low);
+    for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(target[n], a.high, b[n].low);
 #pragma unroll
-    for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(d[n], a.high, b[n].high);
+    for (uint32_t n = 0; n < COUNT; ++n) mma_tf32(target[n], a.high, b[n].high);
+    if (NEAREST) {
+#pragma unroll
+        for (uint32_t n = 0; n < COUNT; ++n) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) d[n][i] += sums[n][i];
+        }
+    }
 }
-__device__ __forceinline__ void mma_split(float (&d)[4], const FragmentA& a, const FragmentB& b) {
-    const FragmentB one[1] = {b};
-    mma_split(&d, a, one);
+template <bool NEAREST>
+__device__ __forceinline__ void mma_split(float (&d)[4], const FragmentA<NEAREST>& a, const FragmentB<NEAREST>& b) {
+    const FragmentB<NEAREST> one[1] = {b};
+    mma_split<NEAREST, 1>(&d, a, one);
 }
-__device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA& a, const FragmentB& b0, const FragmentB& b1) {
-    const FragmentB both[2] = {b0, b1};
-    mma_split(d, a, both);
+template <bool NEAREST>
+__device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA<NEAREST>& a, const FragmentB<NEAREST>& b0,
+                                          const FragmentB<NEAREST>& b1) {
+    const FragmentB<NEAREST> both[2] = {b0, b1};
+    mma_split<NEAREST, 2>(d, a, both);
 }
 // B is exact in TF32
-__device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA& a, const float (&b0)[2], const float (&b1)[2]) {
+__device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA<>& a, const float (&b0)[2], const float (&b1)[2]) {
     mma_tf32(d[0], a.low, b0);
     mma_tf32(d[1], a.low, b1);
     mma_tf32(d[0], a.high, b0);
@@ -81,8 +98,9 @@ __device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA& a, 
 }
 
 // rows `source[row * stride + column]` of a 16 x 8 operand
-__device__ __forceinline__ FragmentA load_a(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentA out;
+template <bool NEAREST = false>
+__device__ __forceinline__ FragmentA<NEAREST> load_a(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentA<NEAREST> out;
     const float* at = source + (lane >> 2) * stride + (lane & 3);
     out.set(0, at[0]);
     out.set(1, at[8 * stride]);
@@ -91,8 +109,9 @@ __device__ __forceinline__ FragmentA load_a(const float* source, uint32_t stride
     return out;
 }
 // the same operand stored transposed: `source[column * stride + row]`
-__device__ __forceinline__ FragmentA load_a_transposed(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentA out;
+template <bool NEAREST = false>
+__device__ __forceinline__ FragmentA<NEAREST> load_a_transposed(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentA<NEAREST> out;
     const float* at = source + (lane & 3) * stride + (lane >> 2);
     out.set(0, at[0]);
     out.set(1, at[8]);
@@ -101,15 +120,17 @@ __device__ __forceinline__ FragmentA load_a_transposed(const float* source, uint
     return out;
 }
 // an 8 x 8 operand B[k][n] stored as `source[k * stride + n]`, or transposed as `source[n * stride + k]`
-__device__ __forceinline__ FragmentB load_b(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB out;
+template <bool NEAREST = false>
+__device__ __forceinline__ FragmentB<NEAREST> load_b(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentB<NEAREST> out;
     const float* at = source + (lane & 3) * stride + (lane >> 2);
     out.set(0, at[0]);
     out.set(1, at[4 * stride]);
     return out;
 }
-__device__ __forceinline__ FragmentB load_b_transposed(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB out;
+template <bool NEAREST = false>
+__device__ __forceinline__ FragmentB<NEAREST> load_b_transposed(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentB<NEAREST> out;
     const float* at = source + (lane >> 2) * stride + (lane & 3);
     out.set(0, at[0]);
     out.set(1, at[4]);
@@ -124,6 +145,7 @@ __device__ __forceinline__ void store_c(float* target, uint32_t stride, uint32_t
 
 // The kernels of delta_split.cu: bf16 segments whose projections lie in whole 16-byte pieces, heads up to 64.
 size_t delta_split_bytes(size_t heads, size_t tiles);
-cudaError_t launch_delta_split(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& args, float* chunks, size_t chunk_bytes);
+cudaError_t launch_delta_split(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& args, float* chunks,
+                               size_t chunk_bytes);
 
 }  // namespace lfm25

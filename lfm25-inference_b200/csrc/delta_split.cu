@@ -6,21 +6,27 @@
 //     (I - tril(U B^T, -1)) [W | Z] = [U | tril(U K^T, -1) V]
 // the Q_(t-1)^T U_t of the chunk are W S_0 + Z, so the state behind the chunk and the outputs are linear in the state S_0
 // before it:
-//     S = A S_0 + D,          A = diag(P) (I + B^T W),        D = diag(P) (B^T Z + K^T V)
+//     S = diag(P) S_0 + A S_0 + D,        A = diag(P) B^T W,        D = diag(P) (B^T Z + K^T V)
 //     O = R' S_0 + O',        R' = R + tril(R B^T) W,         O' = tril(R B^T) Z + tril(R K^T) V
 // Everything but S_0 belongs to one chunk alone.  Three kernels:
-//     form     A, D, R', O' of every chunk of every head                        all chunks side by side
-//     carry    S <- A S + D through each segment's chunks, S_0 in the place of D    one product of 64 x 64 x 16 per chunk
+//     form     P, A, D, R', O' of every chunk of every head                     all chunks side by side
+//     carry    S through each segment's chunks, S_0 in the place of D           one product of 64 x 64 x 16 per chunk
 //     finish   O = R' S_0 + O', norm, gate                                      all chunks side by side
-// so only `carry` is serial, in steps of 64 tokens of a single small product.  4096 tokens of 32 heads: 231 + 49 + 45 us
-// (one CTA per head, tile after tile of 16 tokens: 773 us on 32 SMs).
+// so only `carry` is serial, in steps of 64 tokens of a single small product.  4096 tokens of 32 heads: 418 us for the three
+// (one CTA per head, tile after tile of 16 tokens: 769 us on 32 SMs).
 //
 // Decays are multiplied up by a scan, never summed as logarithms: P_t and the 1 / P_s that meets it come from the same
 // factors, and both carry a handful of roundings.  A decay is at least exp(-exp(-1/2)), so 1 / P_t stays below 1e17 and a
-// product P_t / P_s keeps its relative accuracy.  All matrix products are TF32 with both operands in two parts (bf16 values
-// of v need no second one), with f32 sums.  Not for f32 activations: the decays' products, their reciprocals and the parts
-// each round once more than the token-by-token recurrence does (250 tokens of 16 heads, state against float64: 1.44e-7
-// with the best form of the products, 0.76e-7 token by token).
+// product P_t / P_s keeps its relative accuracy.
+//
+// All matrix products are TF32 with both operands in two parts (bf16 values of v need no second one) and f32 sums.  What
+// reaches the state is held to no larger an error than the carrying kernel has: parts rounded to nearest, short sums that are
+// added up outside the tensor cores, decays rounded without a direction (decay_of), the state's own part diag(P) S_0 as f32
+// multiply-adds.  State against float64 (2-norm; 300 to 4096 tokens, heads of 64, decay logits around 0, spread around -2,
+// around -6): 1.5e-7, 2.2e-7, 2.9e-7; the carrying kernel 4.1e-7, 7.4e-7, 1.7e-6.  With plain parts and sums inside the tensor
+// cores it was 9e-7, 1.6e-6, 2.0e-6 in 338 us instead of 418.  The outputs' own product ends in their bf16 rounding and needs
+// none of this.  Not for f32 activations: the decays' products, their reciprocals and the parts each round once more than the
+// token-by-token recurrence does (250 tokens of 16 heads: 1.44e-7 at best, 0.76e-7 token by token).
 #include <algorithm>
 
 #include "delta_rule.h"
@@ -35,9 +41,9 @@ constexpr uint32_t kTokens = 64;
 constexpr uint32_t kPitch = 72;                    // rows of U, R, K, B, V in shared memory
 constexpr uint32_t kLowerPitch = 68;
 constexpr uint32_t kInversePitch = 20;
-constexpr uint32_t kMatrix = kDim * kTokens;       // elements of A, D, R' and O'
-constexpr uint32_t kChunkFloats = 4 * kMatrix;
-constexpr uint32_t kD = kMatrix, kR = 2 * kMatrix, kO = 3 * kMatrix;     // behind A
+constexpr uint32_t kMatrix = kDim * kTokens;       // elements of A, D, R' and O'; P behind them
+constexpr uint32_t kChunkFloats = 4 * kMatrix + kDim;
+constexpr uint32_t kD = kMatrix, kR = 2 * kMatrix, kO = 3 * kMatrix, kP = 4 * kMatrix;     // behind A
 constexpr uint32_t kFormThreads = 256;
 constexpr uint32_t kCarryThreads = 128;
 constexpr uint32_t kCarryColumns = 16;
@@ -47,8 +53,9 @@ constexpr uint32_t kFinishThreads = 128;
 
 // Fragments in which k index c of a 16 x 8 operand stands for column (row of B) 2c, and c + 4 for 2c + 1: the accumulator of
 // one product is then an operand of the next as it is, and operands along a row are read two at a time.
-__device__ __forceinline__ FragmentA load_a_pairs(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentA out;
+template <bool NEAREST>
+__device__ __forceinline__ FragmentA<NEAREST> load_a_pairs(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentA<NEAREST> out;
     const float* at = source + (lane >> 2) * stride + (lane & 3) * 2;
     const float2 upper = *reinterpret_cast<const float2*>(at), lower = *reinterpret_cast<const float2*>(at + 8 * stride);
     out.set(0, upper.x);
@@ -57,23 +64,26 @@ __device__ __forceinline__ FragmentA load_a_pairs(const float* source, uint32_t 
     out.set(3, lower.y);
     return out;
 }
-__device__ __forceinline__ FragmentA a_from_c(const float (&c)[4]) {
-    FragmentA out;
+template <bool NEAREST>
+__device__ __forceinline__ FragmentA<NEAREST> a_from_c(const float (&c)[4]) {
+    FragmentA<NEAREST> out;
     out.set(0, c[0]);
     out.set(1, c[2]);
     out.set(2, c[1]);
     out.set(3, c[3]);
     return out;
 }
-__device__ __forceinline__ FragmentB load_b_transposed_pairs(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB out;
+template <bool NEAREST>
+__device__ __forceinline__ FragmentB<NEAREST> load_b_transposed_pairs(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentB<NEAREST> out;
     const float2 both = *reinterpret_cast<const float2*>(source + (lane >> 2) * stride + (lane & 3) * 2);
     out.set(0, both.x);
     out.set(1, both.y);
     return out;
 }
-__device__ __forceinline__ FragmentB load_b_pairs(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB out;
+template <bool NEAREST>
+__device__ __forceinline__ FragmentB<NEAREST> load_b_pairs(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentB<NEAREST> out;
     const float* at = source + (lane & 3) * 2 * stride + (lane >> 2);
     out.set(0, at[0]);
     out.set(1, at[stride]);
@@ -89,8 +99,8 @@ __device__ __forceinline__ void load_c(const float* source, uint32_t stride, uin
 }
 
 // d[n] += a * rows for eight column blocks, `rows` bf16 (exact in TF32) or f32; PAIRS: in the order of load_b_pairs
-template <bool PAIRS>
-__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA& a, const __nv_bfloat16* rows,
+template <bool PAIRS, bool NEAREST>
+__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA<NEAREST>& a, const __nv_bfloat16* rows,
                                               uint32_t lane) {
     const uint32_t first = (PAIRS ? (lane & 3) * 2 : lane & 3) * kPitch + (lane >> 2);
     const uint32_t second = first + (PAIRS ? 1 : 4) * kPitch;
@@ -98,23 +108,32 @@ __device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA&
     for (uint32_t n = 0; n < 8; n += 2) {
         const float b0[2] = {__bfloat162float(rows[first + n * 8]), __bfloat162float(rows[second + n * 8])};
         const float b1[2] = {__bfloat162float(rows[first + n * 8 + 8]), __bfloat162float(rows[second + n * 8 + 8])};
-        mma_tf32(d[n], a.low, b0);
-        mma_tf32(d[n + 1], a.low, b1);
-        mma_tf32(d[n], a.high, b0);
-        mma_tf32(d[n + 1], a.high, b1);
+        float sums[2][4] = {};
+        float (*target)[4] = NEAREST ? sums : d + n;
+        mma_tf32(target[0], a.low, b0);
+        mma_tf32(target[1], a.low, b1);
+        mma_tf32(target[0], a.high, b0);
+        mma_tf32(target[1], a.high, b1);
+        if (NEAREST) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                d[n][i] += sums[0][i];
+                d[n + 1][i] += sums[1][i];
+            }
+        }
     }
 }
-template <bool PAIRS>
-__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA& a, const float* rows, uint32_t lane) {
+template <bool PAIRS, bool NEAREST>
+__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA<NEAREST>& a, const float* rows, uint32_t lane) {
 #pragma unroll
     for (uint32_t n = 0; n < 8; n += 2) {
-        FragmentB b[2];
+        FragmentB<NEAREST> b[2];
 #pragma unroll
         for (uint32_t q = 0; q < 2; ++q) {
-            b[q] = PAIRS ? load_b_pairs(rows + (n + q) * 8, kPitch, lane)
-                         : load_b(rows + (n + q) * 8, kPitch, lane);
+            b[q] = PAIRS ? load_b_pairs<NEAREST>(rows + (n + q) * 8, kPitch, lane)
+                         : load_b<NEAREST>(rows + (n + q) * 8, kPitch, lane);
         }
-        mma_split(d + n, a, b);
+        mma_split<NEAREST, 2>(d + n, a, b);
     }
 }
 
@@ -122,7 +141,9 @@ __device__ __forceinline__ float2 load_pair(const __nv_bfloat16* source) {
     return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(source));
 }
 
-__device__ __forceinline__ float decay_of(float logit) { return __expf(-kDecayScale * fast_sigmoid(logit)); }
+// 1 - (1 - exp(x)): close to 1, where a rounding to the same side in every token would add up over a long memory, the sum is
+// rounded to nearest
+__device__ __forceinline__ float decay_of(float logit) { return 1.0f + expm1f(-kDecayScale * sigmoidf(logit)); }
 
 struct FormShared {
     float u[kTokens * kPitch];                     // U, then W
@@ -136,12 +157,12 @@ struct FormShared {
     __nv_bfloat16 v[kTokens * kPitch];
 };
 
-// About 6500 m16n8k8 products per chunk, eight cycles each per SM quarter, keep the tensor pipe 37 % busy; the rest is the
-// latency of the five stages between barriers, which two CTAs per SM hide in part.  Longer loops are not unrolled further:
-// the code then outgrows the instruction cache (251 -> 231 us).
+// About 6500 m16n8k8 products per chunk, eight cycles each per SM quarter, beside cutting their operands and adding up their
+// sums; the rest is the latency of the five stages between barriers, which two CTAs per SM hide in part.  Longer loops are
+// not unrolled further: the code then outgrows the instruction cache.
 __global__ void __launch_bounds__(kFormThreads, 2)
 delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t head_count, float* chunks) {
-    constexpr uint32_t kParts = 2;                 // bf16 parts of tanh(z): 16 bits
+    constexpr uint32_t kParts = 3;                 // bf16 parts of tanh(z)
     extern __shared__ __align__(16) unsigned char form_shared[];
     FormShared& shared = *reinterpret_cast<FormShared*>(form_shared);
     pdl_launch_dependents();
@@ -342,12 +363,12 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
         float with_b[2][4] = {}, with_k[2][4] = {};
 #pragma unroll 2
         for (uint32_t c = 0; c < kDim; c += 8) {
-            const FragmentA a = load_a_pairs(rows + c, kPitch, lane);
+            const FragmentA<true> a = load_a_pairs<true>(rows + c, kPitch, lane);
             const uint32_t at = j * 16 * kPitch + c;
-            mma_split(with_b, a, load_b_transposed_pairs(shared.b + at, kPitch, lane),
-                      load_b_transposed_pairs(shared.b + at + 8 * kPitch, kPitch, lane));
-            mma_split(with_k, a, load_b_transposed_pairs(shared.k + at, kPitch, lane),
-                      load_b_transposed_pairs(shared.k + at + 8 * kPitch, kPitch, lane));
+            mma_split(with_b, a, load_b_transposed_pairs<true>(shared.b + at, kPitch, lane),
+                      load_b_transposed_pairs<true>(shared.b + at + 8 * kPitch, kPitch, lane));
+            mma_split(with_k, a, load_b_transposed_pairs<true>(shared.k + at, kPitch, lane),
+                      load_b_transposed_pairs<true>(shared.k + at + 8 * kPitch, kPitch, lane));
         }
 #pragma unroll
         for (uint32_t n = 0; n < 2; ++n) {
@@ -362,7 +383,7 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
         }
 #pragma unroll
         for (uint32_t n = 0; n < 2; ++n) {
-            multiply_rows<true>(with_values, a_from_c(with_k[n]), shared.v + (j * 16 + n * 8) * kPitch, lane);
+            multiply_rows<true>(with_values, a_from_c<true>(with_k[n]), shared.v + (j * 16 + n * 8) * kPitch, lane);
         }
     }
     float behind[8][4] = {};                       // K^T V, then D: 16 key channels per warp of the first four
@@ -385,7 +406,7 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
         }
 #pragma unroll 2
         for (uint32_t t = 0; t < kTokens; t += 8) {
-            multiply_rows<false>(behind, load_a_transposed(shared.k + t * kPitch + mine * 16, kPitch, lane),
+            multiply_rows<false>(behind, load_a_transposed<true>(shared.k + t * kPitch + mine * 16, kPitch, lane),
                                    shared.v + t * kPitch, lane);
         }
     }
@@ -410,8 +431,8 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
                 load_c(target + 8, kPitch, lane, side[1]);
 #pragma unroll
                 for (uint32_t s = 0; s < i * 16; s += 8) {
-                    mma_split(side, load_a(shared.lower + i * 16 * kLowerPitch + s, kLowerPitch, lane),
-                              load_b(columns + s * kPitch, kPitch, lane), load_b(columns + s * kPitch + 8, kPitch, lane));
+                    mma_split(side, load_a<true>(shared.lower + i * 16 * kLowerPitch + s, kLowerPitch, lane),
+                              load_b<true>(columns + s * kPitch, kPitch, lane), load_b<true>(columns + s * kPitch + 8, kPitch, lane));
                 }
                 __syncwarp();
                 store_c(target, kPitch, lane, side[0]);
@@ -421,8 +442,8 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
             float solved[2][4] = {};
 #pragma unroll
             for (uint32_t s = 0; s < 16; s += 8) {
-                mma_split(solved, load_a(shared.inverse[i] + s, kInversePitch, lane),
-                          load_b(target + s * kPitch, kPitch, lane), load_b(target + s * kPitch + 8, kPitch, lane));
+                mma_split(solved, load_a<true>(shared.inverse[i] + s, kInversePitch, lane),
+                          load_b<true>(target + s * kPitch, kPitch, lane), load_b<true>(target + s * kPitch + 8, kPitch, lane));
             }
             __syncwarp();
             store_c(target, kPitch, lane, solved[0]);
@@ -436,7 +457,7 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
     if (forward) {
 #pragma unroll 1
         for (uint32_t t = 0; t < kTokens; t += 8) {
-            const FragmentA a = load_a_transposed(shared.b + t * kPitch + mine * 16, kPitch, lane);
+            const FragmentA<true> a = load_a_transposed<true>(shared.b + t * kPitch + mine * 16, kPitch, lane);
             multiply_rows<false>(from_state, a, shared.u + t * kPitch, lane);
             multiply_rows<false>(behind, a, shared.k + t * kPitch, lane);
         }
@@ -447,12 +468,15 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
             decay[0] *= shared.block_decay[other][channel];
             decay[1] *= shared.block_decay[other][channel + 8];
         }
+        if ((lane & 3) == 0) {
+            chunk[kP + channel] = decay[0];
+            chunk[kP + channel + 8] = decay[1];
+        }
 #pragma unroll
         for (uint32_t n = 0; n < 8; ++n) {
 #pragma unroll
             for (uint32_t i = 0; i < 4; ++i) {
-                const float one = n * 8 + pair + (i & 1) == channel + (i >> 1) * 8 ? 1.0f : 0.0f;
-                from_state[n][i] = (from_state[n][i] + one) * decay[i >> 1];
+                from_state[n][i] *= decay[i >> 1];
                 behind[n][i] *= decay[i >> 1];
             }
         }
@@ -464,7 +488,7 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
             if (j > mine) continue;
 #pragma unroll
             for (uint32_t n = 0; n < 2; ++n) {
-                const FragmentA a = a_from_c(against_b[j][n]);
+                const FragmentA<true> a = a_from_c<true>(against_b[j][n]);
                 multiply_rows<true>(from_state, a, shared.u + (j * 16 + n * 8) * kPitch, lane);
                 multiply_rows<true>(with_values, a, shared.k + (j * 16 + n * 8) * kPitch, lane);
             }
@@ -481,8 +505,9 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
     }
 }
 
-__device__ __forceinline__ FragmentA operand_of(const float4& stored) {
-    FragmentA out;
+template <bool NEAREST>
+__device__ __forceinline__ FragmentA<NEAREST> operand_of(const float4& stored) {
+    FragmentA<NEAREST> out;
     out.set(0, stored.x);
     out.set(1, stored.y);
     out.set(2, stored.z);
@@ -497,6 +522,7 @@ delta_carry_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t
     extern __shared__ __align__(16) float carry_shared[];
     float4* stages = reinterpret_cast<float4*>(carry_shared);                     // [stage][10][thread]
     float* states = carry_shared + kCarryStages * 10 * kCarryThreads * 4;         // [2][channel][kCarryPitch]
+    float* decays = states + 2 * kDim * kCarryPitch;                              // [stage][channel]
     pdl_launch_dependents();
     pdl_wait();
     const uint32_t part = blockIdx.x % (kDim / kCarryColumns);
@@ -542,17 +568,21 @@ delta_carry_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t
             for (uint32_t n = 0; n < 8; ++n) copy_async_16(stage + n * kCarryThreads, a + n * 32, true);
 #pragma unroll
             for (uint32_t n = 0; n < 2; ++n) copy_async_16(stage + (8 + n) * kCarryThreads, d + n * 32, true);
+            if (threadIdx.x < kDim / 4) {
+                copy_async_16(decays + index % kCarryStages * kDim + threadIdx.x * 4, chunk_of(index) + kP + threadIdx.x * 4,
+                              true);
+            }
         }
         copy_async_commit();
     };
     for (uint32_t index = 0; index + 1 < kCarryStages; ++index) load(index);
     for (uint32_t index = 0; index < count; ++index) {
-        copy_async_wait<kCarryStages - 2>();                 // a thread reads what it copied itself
+        copy_async_wait<kCarryStages - 2>();                 // a thread reads A and D that it copied itself
         __syncthreads();
         load(index + kCarryStages - 1);
         const float* state = states + index % 2 * kDim * kCarryPitch;
         const float4* stage = stages + index % kCarryStages * 10 * kCarryThreads + threadIdx.x;
-        float sum[2][4], high_low[2][4] = {}, low_high[2][4] = {};
+        float sum[2][4];
 #pragma unroll
         for (uint32_t n = 0; n < 2; ++n) {
             const float4 d = stage[(8 + n) * kCarryThreads];
@@ -560,15 +590,20 @@ delta_carry_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t
             sum[n][1] = d.y;
             sum[n][2] = d.z;
             sum[n][3] = d.w;
+            const float* decay = decays + index % kCarryStages * kDim + warp * 16 + (lane >> 2);
+            float held[4];
+            load_c(state + warp * 16 * kCarryPitch + n * 8, kCarryPitch, lane, held);
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) sum[n][i] = fmaf(decay[i >> 1 << 3], held[i], sum[n][i]);
         }
         float4 kept[2];
 #pragma unroll
         for (uint32_t c = 0; c < 8; ++c) {
-            const FragmentA a = operand_of(stage[c * kCarryThreads]);
+            const FragmentA<true> a = operand_of<true>(stage[c * kCarryThreads]);
             const float* rows = state + (c * 8 + (lane & 3) * 2) * kCarryPitch + (lane >> 2);
 #pragma unroll
             for (uint32_t n = 0; n < 2; ++n) {
-                FragmentB b;
+                FragmentB<true> b;
                 const float first = rows[n * 8], second = rows[n * 8 + kCarryPitch];
                 b.set(0, first);
                 b.set(1, second);
@@ -579,9 +614,7 @@ delta_carry_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t
                     kept[n].z = first;
                     kept[n].w = second;
                 }
-                mma_tf32(low_high[n], a.low, b.high);
-                mma_tf32(high_low[n], a.high, b.low);
-                mma_tf32(sum[n], a.high, b.high);
+                mma_split(sum[n], a, b);
             }
         }
         // the state before the chunk, as operands of the outputs' product
@@ -590,8 +623,6 @@ delta_carry_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t
 #pragma unroll
         for (uint32_t n = 0; n < 2; ++n) {
             before_chunk[n * 32] = kept[n];
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) sum[n][i] += low_high[n][i] + high_low[n][i];
             store_c(next + n * 8, kCarryPitch, lane, sum[n]);
         }
     }
@@ -636,11 +667,11 @@ delta_finish_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_
     }
 #pragma unroll
     for (uint32_t m = 0; m < 4; ++m) {
-        const FragmentA a0 = operand_of(operands[2 * m * 32]), a1 = operand_of(operands[(2 * m + 1) * 32]);
+        const FragmentA<> a0 = operand_of<false>(operands[2 * m * 32]), a1 = operand_of<false>(operands[(2 * m + 1) * 32]);
 #pragma unroll
         for (uint32_t n = 0; n < 8; ++n) {
             const float4 state = states[(m * 8 + n) * 32];
-            FragmentB b0, b1;
+            FragmentB<> b0, b1;
             b0.set(0, state.x);
             b0.set(1, state.y);
             b1.set(0, state.z);
@@ -682,13 +713,14 @@ delta_finish_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_
 size_t delta_split_bytes(size_t heads, size_t tiles) { return heads * tiles * kChunkFloats * sizeof(float); }
 
 // Heads are taken in groups whose chunks fit the scratch.
-cudaError_t launch_delta_split(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& args, float* chunks, size_t chunk_bytes) {
+cudaError_t launch_delta_split(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& args, float* chunks,
+                               size_t chunk_bytes) {
     const size_t tiles = tile_bound(args.segments, kTokens);
     const uint32_t most = static_cast<uint32_t>(std::min<size_t>(args.heads, chunk_bytes / delta_split_bytes(1, tiles)));
     if (most == 0) return cudaErrorInvalidValue;
     const uint32_t groups = (args.heads + most - 1) / most;
     const uint32_t group = (args.heads + groups - 1) / groups;
-    const size_t carry_bytes = (kCarryStages * 10 * kCarryThreads * 4 + 2 * kDim * kCarryPitch) * sizeof(float);
+    const size_t carry_bytes = (kCarryStages * (10 * kCarryThreads * 4 + kDim) + 2 * kDim * kCarryPitch) * sizeof(float);
     cudaError_t status = cudaFuncSetAttribute(reinterpret_cast<const void*>(delta_form_kernel),
                                               cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(FormShared));
     if (status == cudaSuccess) {

@@ -175,6 +175,37 @@ def test_delta_rule_split_mixed_step(device, library_option, dtype):
     assert np.array_equal(results[1][1], results[0][1]) == (dtype == "float32")
 
 
+@pytest.mark.parametrize("heads,dim,level", [(2, 64, -2.0), (3, 40, 0.0), (1, 64, -6.0)])
+def test_delta_rule_split_state(device, library_option, heads, dim, level):
+    """The state that the split kernels leave against float64 from the same inputs.  Embeddings of +-1, no convolution and one-hot
+    projections hand the kernels values that are known exactly: their own norm weight, with a sign.  An element of the state
+    is a sum of products of about eight f32 roundings each (decays, reciprocals, scale and removal of the key, operands,
+    sums) of at most 2^-24, and the sums' own: 2^-21."""
+    rank = 16
+    size = heads * dim
+    width = 5 * size + rank
+    config = cases.config_of([cases.delta_layer(heads, dim, ff=0)], width=width, eps=1e-12)
+    tensors = cases.random_tensors(config, 43, rank)
+    rng = np.random.default_rng(47)
+    tensors["embed"] = rng.choice([-1.0, 1.0], size=tensors["embed"].shape)
+    tensors["l0.norm1"] = cases.bf16_values(rng.standard_normal(width))
+    tensors["l0.canon1"] = np.zeros_like(tensors["l0.canon1"])
+    for index, name in enumerate(("r", "k", "v", "g", "a")):
+        tensors["l0.mix." + name] = np.eye(width)[index * size:(index + 1) * size]
+    tensors["l0.mix.w1"] = np.eye(width)[5 * size:]
+    tensors["l0.mix.w0"] = cases.bf16_values(level + 0.5 * rng.standard_normal(size))
+    chunks = np.array([330])
+    _, states = delta_steps(config, tensors, device, "bfloat16", chunks, 4, library_option)
+    tokens = np.random.default_rng(5).integers(0, config["vocab"], size=chunks.sum()).astype(np.uint32)
+    model = cases.oracle_model(config, tensors)
+    held = model.new_state()
+    for _ in range(2):
+        model.forward(tokens, held)
+    want = held["layers"][0]["state"].transpose(0, 2, 1)       # the record holds [value, key]
+    got = states.reshape(want.shape).astype(np.float64)
+    assert np.linalg.norm(got - want) <= 2.0 ** -21 * np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("chunks", [[250], [64, 1, 64], [1500]])
 def test_delta_rule_f32_prompts_token_by_token(device, library_option, chunks):
     """f32 activations keep plain f32 multiply-adds however few and long the prompts are: the general kernel's bits."""
