@@ -1566,21 +1566,27 @@ bool prompt_kernel_takes(const DeltaArgs<__nv_bfloat16>& args) {
            shared <= 227 * 1024;
 }
 
-// Where bf16 prompts are split along the sequence (delta_split.cu): it does about twice the arithmetic of the kernels that
-// carry one head of one segment in a CTA, 0.16 us per head and 64 tokens over the whole chip against 12 us (four tiles) in a
-// CTA, so it pays while those leave most SMs idle and a prompt is long enough for its three launches.  Measured in whole steps of a 16-layer model with 32 heads, split against not: one prompt of 250 tokens
-// 1960 against 1929 us, 500: 2489 / 2869, 4000: 12316 / 15837; two prompts of 500: 3523 / 3544; eight of 250: 6099 / 5388.
-constexpr size_t kSplitHeads = 80;
-constexpr size_t kSplitTokens = 256;
+// Where prompts are split along the sequence (delta_split.cu) instead of carried by one CTA per segment and head: it does about
+// twice the arithmetic and takes three launches, so it pays while the carrying CTAs leave most SMs idle and a prompt is
+// long.  The lengths are on the device, so the line is drawn for segments of equal length, where the longest one does not
+// help.  Inside steps of whole models, segments x heads (of 64 dimensions): what a layer gains in us at tokens a segment
+//     16: 256 1, 320 10, 1000 114, 4000 495        32: 320 0, 400 9 to 11, 600 8, 1000 70, 4096 292
+//     48: 400 -29, 512 -13, 720 21, 2000 67        64: 400 -25, 1000 -20 to 1, 2000 -36 to 38
+constexpr size_t kSplitMostHeads = 48;             // of all segments
+constexpr size_t split_shortest(size_t heads) { return heads <= 16 ? 320 : (heads <= 32 ? 400 : 720); }
+
+bool split_pays(const DeltaRuleLaunch& launch) {
+    const size_t segments = launch.segments.num_segments, heads = segments * launch.heads;
+    const size_t tokens = launch.segments.num_tokens - launch.decode_tokens;
+    return heads <= kSplitMostHeads && tokens >= split_shortest(heads) * segments;
+}
 
 // The kernels' pairwise accesses, and scratch for one head at least (beside what the chunk kernel needs).
 bool split_takes(const DeltaArgs<__nv_bfloat16>& args, const DeltaRuleLaunch& launch) {
     const int64_t forced = option(kOptDeltaPrompt);
-    const size_t segments = launch.segments.num_segments;
-    const size_t tokens = launch.segments.num_tokens - launch.decode_tokens;
-    return (forced == 4 || (forced == 0 && segments * args.heads <= kSplitHeads && tokens >= kSplitTokens * segments)) &&
-           aligned_to(args.decay_base, 4) && aligned_to(args.removal_bias, 4) && aligned_to(args.norm, 4) &&
-           launch.chunks != nullptr && delta_split_bytes(1, tile_bound(launch.segments, 64)) <= launch.chunk_bytes;
+    return (forced == 4 || (forced == 0 && split_pays(launch))) && aligned_to(args.decay_base, 4) &&
+           aligned_to(args.removal_bias, 4) && aligned_to(args.norm, 4) && launch.chunks != nullptr &&
+           delta_split_bytes(1, tile_bound(launch.segments, 64)) <= launch.chunk_bytes;
 }
 
 template <typename T, uint32_t DP, uint32_t LANES, uint32_t COLUMNS>
@@ -1661,7 +1667,7 @@ cudaError_t launch_typed(cudaStream_t stream, const DeltaRuleLaunch& launch) {
 bool delta_rule_needs_scratch(uint32_t dim) { return dim > 128; }
 
 size_t delta_rule_chunk_bytes(Activation type, uint32_t heads, uint32_t dim, size_t tokens, size_t segments) {
-    const size_t most = std::min(std::min(segments, tokens / kSplitTokens), kSplitHeads / heads);
+    const size_t most = std::min(std::min(segments, tokens / split_shortest(heads)), kSplitMostHeads / heads);
     if (type != Activation::kBf16 || dim > kChunkDim || dim % 8 != 0 || most == 0) return 0;
     return std::min(delta_split_bytes(heads, tokens / 64 + most), kDeltaChunkBytes);
 }

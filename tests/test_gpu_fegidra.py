@@ -146,8 +146,8 @@ def delta_steps(config, tensors, device, dtype, chunks, forced, library_option):
     tokens = np.random.default_rng(5).integers(0, config["vocab"], size=chunks.sum()).astype(np.uint32)
     with torch.cuda.stream(torch.cuda.Stream(device)):
         blaslt = ops.BlasLt()
-        layout = workloads.mixed_step_batch(1, np.zeros(len(chunks), np.int64), chunks, 100)
-        model = cases.product_model(config, tensors, device, dtype, 100, len(chunks))
+        layout = workloads.mixed_step_batch(1, np.zeros(len(chunks), np.int64), chunks, 200)
+        model = cases.product_model(config, tensors, device, dtype, 200, len(chunks))
         executor = stack.StackExecutor(blaslt, model, len(tokens), len(chunks))
         steps = []
         for _ in range(2):
@@ -165,9 +165,9 @@ def delta_steps(config, tensors, device, dtype, chunks, forced, library_option):
 def test_delta_rule_split_mixed_step(device, library_option, dtype):
     """Sequences side by side behind single tokens, with more heads than the scratch holds at once, against the kernels that
     carry a segment in one CTA: f32 arithmetic in both, so bf16 results differ by their last rounding."""
-    config = cases.config_of([cases.delta_layer(64, 8, ff=0)])
+    config = cases.config_of([cases.delta_layer(16, 8, ff=0)])
     tensors = cases.random_tensors(config, 29, 16)
-    chunks = np.array([1, 1, 70, 64, 129, 65, 80, 3])
+    chunks = np.array([1, 1, 70, 64, 129, 65, 80, 3])      # scratch for one prompt of that many tokens: 16 heads x 7 tiles of 12
     results = [delta_steps(config, tensors, device, dtype, chunks, forced, library_option) for forced in (3, 4)]
     assert np.isfinite(results[0][0]).all()
     assert cases.relative_error(results[1][0], results[0][0]).max() < {"float32": 5e-6, "bfloat16": 4e-3}[dtype]
@@ -204,6 +204,18 @@ def test_delta_rule_split_state(device, library_option, heads, dim, level):
     want = held["layers"][0]["state"].transpose(0, 2, 1)       # the record holds [value, key]
     got = states.reshape(want.shape).astype(np.float64)
     assert np.linalg.norm(got - want) <= 2.0 ** -21 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("heads,chunks,split", [(16, [300] * 4, False), (16, [320], True), (16, [319], False),
+                                                (16, [400, 400], True), (16, [399, 400], False), (12, [720] * 4, True),
+                                                (12, [719, 720, 720, 720], False), (33, [720], True), (49, [1600], False),
+                                                (32, [1000, 1000], False)])
+def test_delta_rule_split_where_it_pays(device, library_option, heads, chunks, split):
+    """Either side of the line between the kernels that carry a segment and those that split it: the former's bits or not."""
+    config = cases.config_of([cases.delta_layer(heads, 8, ff=0)])
+    tensors = cases.random_tensors(config, 37, 16)
+    results = [delta_steps(config, tensors, device, "bfloat16", np.array(chunks), forced, library_option) for forced in (0, 3)]
+    assert np.array_equal(results[0][1], results[1][1]) != split
 
 
 @pytest.mark.parametrize("chunks", [[250], [64, 1, 64], [1500]])
