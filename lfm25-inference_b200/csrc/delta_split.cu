@@ -518,7 +518,7 @@ __device__ __forceinline__ FragmentA<NEAREST> operand_of(const float4& stored) {
 // A CTA carries 16 value columns of one head through one segment; a warp owns 16 key channels of A and D and copies them
 // into its own part of shared memory kCarryStages - 1 chunks ahead.  Bound by the chain load S, multiply, store S, barrier.
 __global__ void __launch_bounds__(kCarryThreads)
-delta_carry_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t head_count, float* chunks) {
+delta_carry_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t head_count, uint32_t tiles, float* chunks) {
     extern __shared__ __align__(16) float carry_shared[];
     float4* stages = reinterpret_cast<float4*>(carry_shared);                     // [stage][10][thread]
     float* states = carry_shared + kCarryStages * 10 * kCarryThreads * 4;         // [2][channel][kCarryPitch]
@@ -544,6 +544,11 @@ delta_carry_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t
     uint32_t before = 0;
     for (uint32_t other = lane; other < segment; other += 32) before += chunks_of(other);
     before = __reduce_add_sync(0xffffffffu, before);
+    // Offsets that go back name more chunks than the step's tokens have, and the scratch holds `tiles` of them: a segment
+    // that reaches beyond is left out, here and by the outputs.
+    if (before + count > tiles) {
+        return;
+    }
 
     const uint32_t dim = args.dim;
     float* state_base = reinterpret_cast<float*>(static_cast<unsigned char*>(args.record.base) + slot * args.record.stride +
@@ -647,7 +652,8 @@ delta_finish_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_
     pdl_wait();
     const SegmentTile tile = locate_tile(args.segments, kTokens, blockIdx.x / head_count);
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    if (warp * 16 >= tile.count || args.segments.slots[tile.segment] >= args.segments.num_request_slots) {
+    if (warp * 16 >= tile.count || args.segments.slots[tile.segment] >= args.segments.num_request_slots ||
+        segment_end_tile(tile, kTokens, blockIdx.x / head_count) > gridDim.x / head_count) {
         return;
     }
     const size_t head_base = static_cast<size_t>(head0 + blockIdx.x % head_count) * args.dim;
@@ -735,7 +741,7 @@ cudaError_t launch_delta_split(cudaStream_t stream, const DeltaArgs<__nv_bfloat1
         if (status == cudaSuccess) {
             status = launch_kernel(delta_carry_kernel,
                                    static_cast<unsigned int>(args.segments.num_segments * count * (kDim / kCarryColumns)),
-                                   kCarryThreads, carry_bytes, stream, 1, args, head0, count, chunks);
+                                   kCarryThreads, carry_bytes, stream, 1, args, head0, count, tiles, chunks);
         }
         if (status == cudaSuccess) {
             status = launch_kernel(delta_finish_kernel, blocks, kFinishThreads, 0, stream, 1, args, head0, count, chunks);

@@ -174,7 +174,13 @@ __device__ __forceinline__ SegmentTile locate_tile(const StackSegments& segments
     return tile;
 }
 
-// Upper bound of the number of tiles locate_tile() can return work for.
+// The number of tiles of `rows` tokens up to the end of the segment that `tile`, the one at `index`, belongs to.  More than
+// tile_bound() where offsets go back: scratch that is addressed by tile does not reach that far.
+__device__ __forceinline__ uint32_t segment_end_tile(const SegmentTile& tile, uint32_t rows, uint32_t index) {
+    return index - (tile.first - tile.begin) / rows + (tile.end - tile.begin + rows - 1) / rows;
+}
+
+// Upper bound of the number of tiles locate_tile() can return work for, as long as the segments do not overlap.
 inline size_t tile_bound(const StackSegments& segments, size_t rows) {
     if (segments.offsets == nullptr) {
         return segments.num_tokens;

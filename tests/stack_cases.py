@@ -65,6 +65,34 @@ def residual_in_portions(make_model, device, tokens, portions) -> np.ndarray:
     return np.concatenate(got)
 
 
+def states_of_step(make_model, device, vocab, chunks, offsets, state_floats):
+    """One step over as many tokens and segments as `chunks`, with `offsets` in the place of its segment offsets on the
+    device.  Every slot's state (`state_floats` values of the first layer) is 0.5 before it.  Residual stream and the
+    segments' states."""
+    import torch
+
+    from lfm25_inference_b200 import model as lfm_model
+    from lfm25_inference_b200 import ops, stack, workloads
+    chunks = np.asarray(chunks)
+    tokens = np.random.default_rng(5).integers(0, vocab, size=chunks.sum()).astype(np.uint32)
+    pages = int(((chunks + 15) // 16).sum())
+    with torch.cuda.stream(torch.cuda.Stream(device)):
+        blaslt = ops.BlasLt()
+        layout = workloads.mixed_step_batch(1, np.zeros(len(chunks), np.int64), chunks, pages, shuffle_slots=False)
+        model = make_model(pages, len(chunks))
+        offset = model.struct.layers[0].state_offset
+        states = model.records.view(len(chunks), -1)[:, offset:offset + 4 * state_floats].view(torch.float32)
+        states.fill_(0.5)
+        executor = stack.StackExecutor(blaslt, model, len(tokens), len(chunks))
+        batch = lfm_model.RaggedBatch(device, layout, tokens)
+        batch.segment_offsets.copy_(torch.tensor(offsets, dtype=torch.int32))
+        executor.forward_ragged(batch)
+        residual = executor.residual(len(tokens))
+        executor.close()
+        blaslt.close()
+        return residual, states.cpu().numpy()
+
+
 def feed(engine, vocab, request, tokens, portions):
     """Feeds `tokens` of one request in portions of the given sizes; every token's logits."""
     rows, at = [], 0

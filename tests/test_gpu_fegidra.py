@@ -218,6 +218,24 @@ def test_delta_rule_split_where_it_pays(device, library_option, heads, chunks, s
     assert np.array_equal(results[0][1], results[1][1]) != split
 
 
+def test_delta_rule_split_offsets_that_go_back(device, library_option):
+    """Offsets that go back name more chunks than the scratch has room for: the segment that reaches beyond is left out and
+    keeps its state, the others have the state and outputs of a step without it."""
+    library_option("delta_prompt", 4)
+    heads, dim, count = 2, 24, 768
+    config = cases.config_of([cases.delta_layer(heads, dim, ff=0)])
+    tensors = cases.random_tensors(config, 53, 16)
+
+    def states(chunks, offsets):
+        return stack_cases.states_of_step(
+            lambda pages, slots: cases.product_model(config, tensors, device, "bfloat16", pages, slots), device,
+            config["vocab"], chunks, offsets, heads * dim * dim)
+    residual, got = states([count - 2, 1, 1], [0, count, 0, count])
+    want_residual, want = states([count], [0, count])
+    assert np.array_equal(got[0], want[0]) and (got[1:] == 0.5).all()
+    assert np.array_equal(residual, want_residual)
+
+
 @pytest.mark.parametrize("chunks", [[250], [64, 1, 64], [1500]])
 def test_delta_rule_f32_prompts_token_by_token(device, library_option, chunks):
     """f32 activations keep plain f32 multiply-adds however few and long the prompts are: the general kernel's bits."""
