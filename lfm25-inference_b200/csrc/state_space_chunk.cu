@@ -145,6 +145,8 @@ state_space_chunk_kernel(const StateSpaceArgs<__nv_bfloat16> args, const PieceAr
         end = tile.first + tile.count;
         piece = (tile.first - tile.begin) / pieces.tokens;
         last_piece = (tile.end - tile.begin - 1) / pieces.tokens;
+        // offsets that go back name more pieces than there is room for: a segment that reaches beyond is left out
+        if (segment_end_tile(tile, pieces.tokens, index) > gridDim.x / column_blocks / args.heads) return;
         if (PASS == Pass::kContribute && piece == last_piece) return;
     }
     const size_t slot = args.segments.slots[segment];

@@ -141,6 +141,23 @@ def test_state_space_in_pieces(device, library_option, shape):
     assert cases.relative_error(results[1], results[0]).max() < 4e-3
 
 
+def test_state_space_pieces_with_offsets_that_go_back(device):
+    """Offsets that go back name more pieces than there is room for: the segment that reaches beyond is left out and keeps its
+    state, the others have the state and outputs of a step without it (in other pieces: other rounding of f32)."""
+    heads, vdim, size, count = 2, 64, 64, 4096
+    config = cases.config_of([cases.mamba_layer(heads, vdim, size, 1, 1, 4)])
+    tensors = cases.random_tensors(config, 97)
+
+    def states(chunks, offsets):
+        return stack_cases.states_of_step(
+            lambda pages, slots: cases.product_model(config, tensors, device, "bfloat16", pages, slots), device,
+            config["vocab"], chunks, offsets, heads * size * vdim)
+    residual, got = states([count - 2, 1, 1], [0, count, 0, count])
+    want_residual, want = states([count], [0, count])
+    assert np.linalg.norm(got[0] - want[0]) <= 2e-5 * np.linalg.norm(want[0]) and (got[1:] == 0.5).all()
+    assert cases.relative_error(residual, want_residual).max() < 4e-3
+
+
 def test_latent_attention_kernels_agree(device, library_option):
     """Latents on the tensor cores, keys and values formed from them, and the plain kernel on the same inputs."""
     config = cases.config_of([cases.latent_layer(24, 64, 32, 48, 64, 256, scale=0.3, ff=0)])
