@@ -1650,6 +1650,7 @@ cudaError_t launch_typed(cudaStream_t stream, const DeltaRuleLaunch& launch) {
             if (launch.dim <= kChunkDim && ChunkLayout(launch.rank).total <= 227 * 1024 && option(kOptDeltaPrompt) != 1) {
                 // the kernels for larger ranks keep more bits than the split ones
                 if (split_takes(args, launch)) return launch_delta_split(stream, args, launch.chunks, launch.chunk_bytes);
+                if (option(kOptDeltaPrompt) == 4) return cudaErrorInvalidValue;       // no scratch for what was asked for
                 return launch_chunk(stream, args);
             }
             return launch.dim <= 64 ? launch_prompt<64, 4, 128>(stream, args) : launch_prompt<128, 4, 128>(stream, args);

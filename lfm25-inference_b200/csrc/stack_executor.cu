@@ -43,7 +43,7 @@ struct lfm25_stack_executor {
     void* head_input;          // [R, width]
     void* logits;              // [R, head.n], before a cap
     float* raw;                // [T, widest heads * dim] when a delta rule needs it
-    float* chunks = nullptr;   // of a delta rule split along the sequence
+    float* chunks;             // of a delta rule split along the sequence
     size_t chunk_bytes = 0;
     void* compressed;          // [T, widest q_rank]: latent attention's query latent
     void* absorbed;            // [T, widest heads * kv_rank]: queries against latents
@@ -842,20 +842,22 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
     }
     self->context_capacity = c;
     self->piece_bytes = pieces;
+    self->chunk_bytes = chunk_bytes;
     void** fields[] = {reinterpret_cast<void**>(&self->residual[0]), reinterpret_cast<void**>(&self->residual[1]),
                        &self->mixed, &self->normalized, &self->projected, &self->query, &self->up, &self->joined,
                        &self->update, &self->head_input, &self->logits, reinterpret_cast<void**>(&self->raw),
                        reinterpret_cast<void**>(&self->sampled), &self->compressed, &self->absorbed, &self->weighted,
                        &self->context_latents, &self->context_keys, &self->expanded,
                        reinterpret_cast<void**>(&self->context_bases), reinterpret_cast<void**>(&self->token_order),
-                       &self->convolved, &self->scanned, &self->factors, reinterpret_cast<void**>(&self->pieces)};
+                       &self->convolved, &self->scanned, &self->factors, reinterpret_cast<void**>(&self->pieces),
+                       reinterpret_cast<void**>(&self->chunks)};
     const size_t sizes[] = {t * model->width * 4, t * model->width * 4, t * model->width * bytes,
                             t * model->width * bytes, t * projection * bytes, t * query * bytes, t * up * bytes,
                             t * joined * bytes, t * model->width * bytes, r * model->width * bytes,
                             r * model->head.n * bytes, t * raw * 4, r * 4, t * compressed * bytes, t * latents * bytes,
                             t * latents * bytes, c * context_rank * bytes, c * context_keys * bytes,
                             c * context_columns * bytes, (t + 1) * 4, latents > 0 ? t * 4 : 0, t * channels * bytes,
-                            t * scanned * bytes, factors, pieces};
+                            t * scanned * bytes, factors, pieces, chunk_bytes};
     size_t total = 0;
     for (size_t size : sizes) total += (size + 255) & ~static_cast<size_t>(255);
     cudaError_t status = cudaMalloc(&self->allocation, total);
@@ -870,15 +872,6 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
         *fields[index] = sizes[index] > 0 ? cursor : nullptr;
         cursor += (sizes[index] + 255) & ~static_cast<size_t>(255);
     }
-    if (chunk_bytes > 0) {
-        // without it prompts run tile after tile
-        if (cudaMalloc(reinterpret_cast<void**>(&self->chunks), chunk_bytes) == cudaSuccess) {
-            self->chunk_bytes = chunk_bytes;
-        } else {
-            self->chunks = nullptr;
-            cudaGetLastError();
-        }
-    }
     *out = self;
     return LFM25_OK;
 }
@@ -886,7 +879,6 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
 void lfm25_stack_executor_destroy(lfm25_stack_executor* self) {
     if (self == nullptr) return;
     cudaFree(self->allocation);
-    cudaFree(self->chunks);
     cudaFree(self->exported);
     delete self;
 }

@@ -206,6 +206,13 @@ def test_delta_rule_split_state(device, library_option, heads, dim, level):
     assert np.linalg.norm(got - want) <= 2.0 ** -21 * np.linalg.norm(want)
 
 
+def test_delta_rule_split_without_scratch(device, library_option):
+    """Asked for by the option, the split kernels run or the step fails: an executor for 200 tokens has no scratch for them."""
+    config = cases.config_of([cases.delta_layer(2, 8, ff=0)])
+    with pytest.raises(RuntimeError, match="delta rule launch failed"):
+        delta_steps(config, cases.random_tensors(config, 29, 16), device, "bfloat16", np.array([200]), 4, library_option)
+
+
 @pytest.mark.parametrize("heads,chunks,split", [(16, [300] * 4, False), (16, [320], True), (16, [319], False),
                                                 (16, [400, 400], True), (16, [399, 400], False), (12, [720] * 4, True),
                                                 (12, [719, 720, 720, 720], False), (33, [720], True), (49, [1600], False),
