@@ -282,7 +282,8 @@ def test_f32_products_of_three_small_tiles(device, width, ff):
 
 
 def test_f32_products_of_large_and_tiny_values(device):
-    """Values over the whole range of exponents beside one another: nothing of x is lost when it is taken apart."""
+    """Residual rows of every size beside one another in a tile of the products (test_gpu_linear_f32.py has the products of
+    such values themselves: here a norm stands in front of them)."""
     config = cases.config_of([cases.delta_layer(1, 16, ff=64)], width=128)
 
     def spread(tensors):
