@@ -9,12 +9,12 @@
 // long the segment is.  Few long bf16 segments are split along the sequence instead (delta_split.cu).  Four kernels:
 //   decode    one token per sequence: every load is issued up front, then three barriers
 //   chunk     bf16 segments, heads up to 64: tiles of 16 tokens as matrix products on the tensor cores
-//   prompt    bf16 segments, larger heads: half of the warps prepare a tile of 16 tokens (decays with one small tensor-core product,
-//             removal rates, unit scales) and finish the previous one (norm, gate), the others run the recurrence over
-//             the tile between them; projections arrive through cp.async two tiles ahead
+//   prompt    bf16 segments, larger heads: half of the warps prepare a tile of 16 tokens (decays with one small tensor-core
+//             product, removal rates, unit scales) and finish the previous one (norm, gate), the others run the recurrence
+//             over the tile between them; projections arrive through cp.async two tiles ahead
 //   general   any activation type and head size
-// Outside the chunk kernel (see there) all arithmetic on the state is f32 multiply-adds, two-wide where the sm_100 packed instructions take it (each half
-// rounds like the scalar one).
+// Outside the chunk kernel (see there) and delta_split.cu all arithmetic on the state is f32 multiply-adds, two-wide where the
+// sm_100 packed instructions take it (each half rounds like the scalar one).
 #include <math.h>
 
 #include <algorithm>

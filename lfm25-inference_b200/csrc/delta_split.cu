@@ -2,7 +2,8 @@
 //
 // Over a chunk of 64 tokens, with P_t the product of the decays of its tokens up to t, S_t = diag(P_t) Q_t and
 //     U_t = u_t P_(t-1),   R_t = r_t P_t,   K_t = k_t / P_t,   B_t = -(a_t u_t) / P_t          (per key channel)
-// the update is Q_t = Q_(t-1) + B_t (U_t^T Q_(t-1)) + K_t v_t^T.  With
+// the update is Q_t = Q_(t-1) + B_t (U_t^T Q_(t-1)) + K_t v_t^T: the chunked form of the delta rule (Yang et al. 2024, after
+// Bischof and Van Loan's WY form of products of rank-one updates), here with a decay per key channel.  With
 //     (I - tril(U B^T, -1)) [W | Z] = [U | tril(U K^T, -1) V]
 // the Q_(t-1)^T U_t of the chunk are W S_0 + Z, so the state behind the chunk and the outputs are linear in the state S_0
 // before it:
@@ -432,7 +433,8 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
 #pragma unroll
                 for (uint32_t s = 0; s < i * 16; s += 8) {
                     mma_split(side, load_a<true>(shared.lower + i * 16 * kLowerPitch + s, kLowerPitch, lane),
-                              load_b<true>(columns + s * kPitch, kPitch, lane), load_b<true>(columns + s * kPitch + 8, kPitch, lane));
+                              load_b<true>(columns + s * kPitch, kPitch, lane),
+                              load_b<true>(columns + s * kPitch + 8, kPitch, lane));
                 }
                 __syncwarp();
                 store_c(target, kPitch, lane, side[0]);
@@ -443,7 +445,8 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
 #pragma unroll
             for (uint32_t s = 0; s < 16; s += 8) {
                 mma_split(solved, load_a<true>(shared.inverse[i] + s, kInversePitch, lane),
-                          load_b<true>(target + s * kPitch, kPitch, lane), load_b<true>(target + s * kPitch + 8, kPitch, lane));
+                          load_b<true>(target + s * kPitch, kPitch, lane),
+                          load_b<true>(target + s * kPitch + 8, kPitch, lane));
             }
             __syncwarp();
             store_c(target, kPitch, lane, solved[0]);
@@ -698,8 +701,9 @@ delta_finish_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_
         const float factor = rsqrtf(squares / static_cast<float>(args.dim) + args.eps);
         const uint32_t token = warp * 16 + (lane >> 2) + half * 8;
         if (token < tile.count) {
-            const __nv_bfloat16* gates = args.projected + static_cast<size_t>(tile.first + token) * args.pitch + 3 * width + head_base;
-            __nv_bfloat16* target = args.out + static_cast<size_t>(tile.first + token) * args.out_pitch + head_base;
+            const size_t row = tile.first + token;
+            const __nv_bfloat16* gates = args.projected + row * args.pitch + 3 * width + head_base;
+            __nv_bfloat16* target = args.out + row * args.out_pitch + head_base;
 #pragma unroll
             for (uint32_t n = 0; n < 8; ++n) {
                 const uint32_t channel = n * 8 + (lane & 3) * 2;

@@ -718,8 +718,9 @@ cudaError_t launch_short_conv_segmented(cudaStream_t stream, const void* project
                                         size_t num_tokens, size_t num_segments, size_t hidden,
                                         size_t num_request_slots) {
     // eight channels in 16-byte pieces: three taps of bf16 per channel, two values of state
-    const bool vector = hidden % 8 == 0 && ((reinterpret_cast<uintptr_t>(projected) | reinterpret_cast<uintptr_t>(weight) |
-                                               reinterpret_cast<uintptr_t>(states) | reinterpret_cast<uintptr_t>(output)) & 15) == 0;
+    const uintptr_t addresses = reinterpret_cast<uintptr_t>(projected) | reinterpret_cast<uintptr_t>(weight) |
+                                reinterpret_cast<uintptr_t>(states) | reinterpret_cast<uintptr_t>(output);
+    const bool vector = hidden % 8 == 0 && addresses % 16 == 0;
     const size_t blocks = (num_tokens + kConvTile - 1) / kConvTile;
     return launch_kernel(vector ? short_conv_segmented_kernel<8> : short_conv_segmented_kernel<1>,
                          static_cast<unsigned int>(blocks), kRowThreads, 0, stream, 1,

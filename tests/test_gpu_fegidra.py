@@ -206,6 +206,23 @@ def test_delta_rule_split_state(device, library_option, heads, dim, level):
     assert np.linalg.norm(got - want) <= 2.0 ** -21 * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("count", [40, 250])
+def test_delta_rule_f32_nan_stays_behind(device, count):
+    """A token whose values are no numbers leaves those in front of it in an f32 prompt as they are."""
+    config = cases.config_of([cases.delta_layer(2, 16, ff=0)])
+    tensors = cases.random_tensors(config, 59)
+    tokens = np.random.default_rng(5).integers(0, config["vocab"] - 1, size=count).astype(np.uint32)
+    bad = count - 7
+    rows = []
+    for value in (0.0, np.nan):
+        tensors["embed"][-1] = value
+        tokens[bad] = config["vocab"] - 1
+        rows.append(stack_cases.residual_in_portions(
+            lambda pages, slots: cases.product_model(config, tensors, device, "float32", pages, slots), device, tokens, [count]))
+    assert np.isnan(rows[1][bad:]).any(axis=1).all()
+    assert np.isfinite(rows[1][:bad]).all() and np.array_equal(rows[0][:bad], rows[1][:bad])
+
+
 def test_delta_rule_split_without_scratch(device, library_option):
     """Asked for by the option, the split kernels run or the step fails: an executor for 200 tokens has no scratch for them."""
     config = cases.config_of([cases.delta_layer(2, 8, ff=0)])
