@@ -54,9 +54,8 @@ constexpr uint32_t kFinishThreads = 128;
 
 // Fragments in which k index c of a 16 x 8 operand stands for column (row of B) 2c, and c + 4 for 2c + 1: the accumulator of
 // one product is then an operand of the next as it is, and operands along a row are read two at a time.
-template <bool NEAREST>
-__device__ __forceinline__ FragmentA<NEAREST> load_a_pairs(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentA<NEAREST> out;
+__device__ __forceinline__ FragmentA<true> load_a_pairs(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentA<true> out;
     const float* at = source + (lane >> 2) * stride + (lane & 3) * 2;
     const float2 upper = *reinterpret_cast<const float2*>(at), lower = *reinterpret_cast<const float2*>(at + 8 * stride);
     out.set(0, upper.x);
@@ -65,26 +64,23 @@ __device__ __forceinline__ FragmentA<NEAREST> load_a_pairs(const float* source, 
     out.set(3, lower.y);
     return out;
 }
-template <bool NEAREST>
-__device__ __forceinline__ FragmentA<NEAREST> a_from_c(const float (&c)[4]) {
-    FragmentA<NEAREST> out;
+__device__ __forceinline__ FragmentA<true> a_from_c(const float (&c)[4]) {
+    FragmentA<true> out;
     out.set(0, c[0]);
     out.set(1, c[2]);
     out.set(2, c[1]);
     out.set(3, c[3]);
     return out;
 }
-template <bool NEAREST>
-__device__ __forceinline__ FragmentB<NEAREST> load_b_transposed_pairs(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB<NEAREST> out;
+__device__ __forceinline__ FragmentB<true> load_b_transposed_pairs(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentB<true> out;
     const float2 both = *reinterpret_cast<const float2*>(source + (lane >> 2) * stride + (lane & 3) * 2);
     out.set(0, both.x);
     out.set(1, both.y);
     return out;
 }
-template <bool NEAREST>
-__device__ __forceinline__ FragmentB<NEAREST> load_b_pairs(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB<NEAREST> out;
+__device__ __forceinline__ FragmentB<true> load_b_pairs(const float* source, uint32_t stride, uint32_t lane) {
+    FragmentB<true> out;
     const float* at = source + (lane & 3) * 2 * stride + (lane >> 2);
     out.set(0, at[0]);
     out.set(1, at[stride]);
@@ -100,8 +96,8 @@ __device__ __forceinline__ void load_c(const float* source, uint32_t stride, uin
 }
 
 // d[n] += a * rows for eight column blocks, `rows` bf16 (exact in TF32) or f32; PAIRS: in the order of load_b_pairs
-template <bool PAIRS, bool NEAREST>
-__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA<NEAREST>& a, const __nv_bfloat16* rows,
+template <bool PAIRS>
+__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA<true>& a, const __nv_bfloat16* rows,
                                               uint32_t lane) {
     const uint32_t first = (PAIRS ? (lane & 3) * 2 : lane & 3) * kPitch + (lane >> 2);
     const uint32_t second = first + (PAIRS ? 1 : 4) * kPitch;
@@ -110,31 +106,28 @@ __device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA<
         const float b0[2] = {__bfloat162float(rows[first + n * 8]), __bfloat162float(rows[second + n * 8])};
         const float b1[2] = {__bfloat162float(rows[first + n * 8 + 8]), __bfloat162float(rows[second + n * 8 + 8])};
         float sums[2][4] = {};
-        float (*target)[4] = NEAREST ? sums : d + n;
-        mma_tf32(target[0], a.low, b0);
-        mma_tf32(target[1], a.low, b1);
-        mma_tf32(target[0], a.high, b0);
-        mma_tf32(target[1], a.high, b1);
-        if (NEAREST) {
+        mma_tf32(sums[0], a.low, b0);
+        mma_tf32(sums[1], a.low, b1);
+        mma_tf32(sums[0], a.high, b0);
+        mma_tf32(sums[1], a.high, b1);
 #pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) {
-                d[n][i] += sums[0][i];
-                d[n + 1][i] += sums[1][i];
-            }
+        for (uint32_t i = 0; i < 4; ++i) {
+            d[n][i] += sums[0][i];
+            d[n + 1][i] += sums[1][i];
         }
     }
 }
-template <bool PAIRS, bool NEAREST>
-__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA<NEAREST>& a, const float* rows, uint32_t lane) {
+template <bool PAIRS>
+__device__ __forceinline__ void multiply_rows(float (&d)[8][4], const FragmentA<true>& a, const float* rows, uint32_t lane) {
 #pragma unroll
     for (uint32_t n = 0; n < 8; n += 2) {
-        FragmentB<NEAREST> b[2];
+        FragmentB<true> b[2];
 #pragma unroll
         for (uint32_t q = 0; q < 2; ++q) {
-            b[q] = PAIRS ? load_b_pairs<NEAREST>(rows + (n + q) * 8, kPitch, lane)
-                         : load_b<NEAREST>(rows + (n + q) * 8, kPitch, lane);
+            b[q] = PAIRS ? load_b_pairs(rows + (n + q) * 8, kPitch, lane)
+                         : load_b<true>(rows + (n + q) * 8, kPitch, lane);
         }
-        mma_split<NEAREST, 2>(d + n, a, b);
+        mma_split<true, 2>(d + n, a, b);
     }
 }
 
@@ -364,12 +357,12 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
         float with_b[2][4] = {}, with_k[2][4] = {};
 #pragma unroll 2
         for (uint32_t c = 0; c < kDim; c += 8) {
-            const FragmentA<true> a = load_a_pairs<true>(rows + c, kPitch, lane);
+            const FragmentA<true> a = load_a_pairs(rows + c, kPitch, lane);
             const uint32_t at = j * 16 * kPitch + c;
-            mma_split(with_b, a, load_b_transposed_pairs<true>(shared.b + at, kPitch, lane),
-                      load_b_transposed_pairs<true>(shared.b + at + 8 * kPitch, kPitch, lane));
-            mma_split(with_k, a, load_b_transposed_pairs<true>(shared.k + at, kPitch, lane),
-                      load_b_transposed_pairs<true>(shared.k + at + 8 * kPitch, kPitch, lane));
+            mma_split(with_b, a, load_b_transposed_pairs(shared.b + at, kPitch, lane),
+                      load_b_transposed_pairs(shared.b + at + 8 * kPitch, kPitch, lane));
+            mma_split(with_k, a, load_b_transposed_pairs(shared.k + at, kPitch, lane),
+                      load_b_transposed_pairs(shared.k + at + 8 * kPitch, kPitch, lane));
         }
 #pragma unroll
         for (uint32_t n = 0; n < 2; ++n) {
@@ -384,7 +377,7 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
         }
 #pragma unroll
         for (uint32_t n = 0; n < 2; ++n) {
-            multiply_rows<true>(with_values, a_from_c<true>(with_k[n]), shared.v + (j * 16 + n * 8) * kPitch, lane);
+            multiply_rows<true>(with_values, a_from_c(with_k[n]), shared.v + (j * 16 + n * 8) * kPitch, lane);
         }
     }
     float behind[8][4] = {};                       // K^T V, then D: 16 key channels per warp of the first four
@@ -491,7 +484,7 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
             if (j > mine) continue;
 #pragma unroll
             for (uint32_t n = 0; n < 2; ++n) {
-                const FragmentA<true> a = a_from_c<true>(against_b[j][n]);
+                const FragmentA<true> a = a_from_c(against_b[j][n]);
                 multiply_rows<true>(from_state, a, shared.u + (j * 16 + n * 8) * kPitch, lane);
                 multiply_rows<true>(with_values, a, shared.k + (j * 16 + n * 8) * kPitch, lane);
             }
