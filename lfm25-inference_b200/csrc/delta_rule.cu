@@ -12,7 +12,7 @@
 //   prompt    bf16 segments, larger heads: half of the warps prepare a tile of 16 tokens (decays with one small tensor-core
 //             product, removal rates, unit scales) and finish the previous one (norm, gate), the others run the recurrence
 //             over the tile between them; projections arrive through cp.async two tiles ahead
-//   general   any activation type and head size
+//   general   one token per sequence, head sizes and ranks beyond the decode kernel
 // Outside the chunk kernel (see there) and delta_split.cu all arithmetic on the state is f32 multiply-adds, two-wide where the
 // sm_100 packed instructions take it (each half rounds like the scalar one).
 #include <math.h>
@@ -28,48 +28,12 @@ namespace lfm25 {
 
 namespace {
 
-using Pair = unsigned long long;     // two f32 values
-
-__device__ __forceinline__ Pair pair_of(float low, float high) {
-    Pair out;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(out) : "f"(low), "f"(high));
-    return out;
-}
-__device__ __forceinline__ float pair_sum(Pair value) {
-    float low, high;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(low), "=f"(high) : "l"(value));
-    return low + high;
-}
-__device__ __forceinline__ float low_of(Pair value) { return __uint_as_float(static_cast<uint32_t>(value)); }
-__device__ __forceinline__ float high_of(Pair value) { return __uint_as_float(static_cast<uint32_t>(value >> 32)); }
-__device__ __forceinline__ Pair fma_pair(Pair a, Pair b, Pair c) {
-    Pair out;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(out) : "l"(a), "l"(b), "l"(c));
-    return out;
-}
-__device__ __forceinline__ Pair add_pair(Pair a, Pair b) {
-    Pair out;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(out) : "l"(a), "l"(b));
-    return out;
-}
-__device__ __forceinline__ Pair mul_pair(Pair a, Pair b) {
-    Pair out;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(out) : "l"(a), "l"(b));
-    return out;
-}
-
-constexpr uint32_t kTileTokens = 16;
 // per token in shared memory: r, w, -(a * u), u, k over the padded key channels, then v over them as well
 constexpr uint32_t kVectors = 6;
 
-inline uint32_t padded_rank(uint32_t rank) { return (rank + 3) / 4 * 4; }
-
 template <uint32_t DP>
-size_t delta_shared_bytes(uint32_t tokens, uint32_t rank, bool staged) {
-    const size_t padded = padded_rank(rank);
-    size_t floats = static_cast<size_t>(tokens) * (kVectors + 1) * DP + tokens * padded + 2 * tokens;
-    floats = (floats + 3) / 4 * 4;
-    return floats * sizeof(float) + (staged ? padded * DP * sizeof(__nv_bfloat16) : 0);
+size_t delta_shared_bytes(uint32_t rank) {
+    return ((kVectors + 1) * DP + (rank + 3) / 4 * 4 + 4) * sizeof(float);
 }
 
 // What one token's projections turn into for one key channel.
@@ -92,15 +56,13 @@ __device__ __forceinline__ Prepared prepare(const DeltaArgs<T>& args, const T* r
 
 // ------------------------------------------------------------------------------------------------ general kernel
 
-// LANES threads a column.  Everything a token contributes is prepared for a tile of tokens in shared memory (all in f32)
-// and then consumed token by token: per token a thread forms its share of u^T S, LANES threads add theirs up, and the
-// same pass over its rows updates S and accumulates r^T S.
-// TOKENS: tokens per tile (1 = decode steps).  STAGED: the head's rows of W2 sit in shared memory.
-template <typename T, uint32_t DP, uint32_t LANES, uint32_t COLUMNS, uint32_t TOKENS, bool STAGED>
+// One token per sequence, for head sizes and ranks beyond the decode kernel.  LANES threads a column: what the token
+// contributes is prepared in shared memory (all in f32), then a thread forms its share of u^T S, LANES threads add theirs up,
+// and the same pass over its rows updates S and accumulates r^T S.
+template <typename T, uint32_t DP, uint32_t LANES, uint32_t COLUMNS>
 __global__ void __launch_bounds__(LANES * COLUMNS)
 delta_rule_kernel(const DeltaArgs<T> args) {
     constexpr uint32_t kThreads = LANES * COLUMNS;
-    constexpr uint32_t kWarps = kThreads / 32;
     constexpr uint32_t kRows = DP / LANES;              // key channels per thread, in groups of four
     constexpr uint32_t kGroups = kRows / 4;
     static_assert(kRows % 4 == 0, "four consecutive key channels per access");
@@ -108,25 +70,16 @@ delta_rule_kernel(const DeltaArgs<T> args) {
     pdl_wait();
     extern __shared__ __align__(16) float shared[];
     const uint32_t dim = args.dim;
-    const uint32_t padded_z = (args.rank + 3) / 4 * 4;
-    float* vectors = shared;                                          // [TOKENS][kVectors][DP]
-    float* produced = vectors + TOKENS * kVectors * DP;               // [TOKENS][DP]
-    float* z_values = produced + TOKENS * DP;                         // [TOKENS][padded_z], tanh applied
-    float* unit_scale = z_values + TOKENS * padded_z;                 // [TOKENS]
-    __nv_bfloat162* w2 = reinterpret_cast<__nv_bfloat162*>(
-        shared + (TOKENS * ((kVectors + 1) * DP + padded_z + 2) + 3) / 4 * 4);   // [padded_z / 2][DP]
+    float* vectors = shared;                                          // [kVectors][DP]
+    float* produced = vectors + kVectors * DP;                        // [DP]
+    float* unit_scale = produced + DP;                                // [1], padded to four
+    float* z_values = unit_scale + 4;                                 // [rank], tanh applied
 
     const uint32_t split = blockIdx.x % args.splits;
     const uint32_t head = blockIdx.x / args.splits % args.heads;
-    const uint32_t segment = blockIdx.x / args.splits / args.heads;
-    uint32_t begin = segment, end = segment + 1;
-    if (args.segments.offsets != nullptr) {
-        begin = args.segments.offsets[segment];
-        end = args.segments.offsets[segment + 1];
-        end = end < args.segments.num_tokens ? end : static_cast<uint32_t>(args.segments.num_tokens);
-    }
-    const size_t slot = args.segments.slots[segment];
-    if (begin >= end || slot >= args.segments.num_request_slots) {
+    const size_t token = blockIdx.x / args.splits / args.heads;
+    const size_t slot = args.segments.slots[token];
+    if (slot >= args.segments.num_request_slots) {
         return;
     }
     const uint32_t lane = threadIdx.x % LANES;
@@ -157,169 +110,103 @@ delta_rule_kernel(const DeltaArgs<T> args) {
         state[2 * g] = pair_of(value.x, value.y);
         state[2 * g + 1] = pair_of(value.z, value.w);
     }
-    if (STAGED) {
-        for (uint32_t item = threadIdx.x; item < padded_z / 2 * DP; item += kThreads) {
-            const uint32_t channel = item % DP;
-            const uint32_t z = item / DP * 2;
-            const __nv_bfloat16 zero = __float2bfloat16_rn(0.0f);
-            const __nv_bfloat16* source = args.decay_up + (head_base + channel) * args.rank;
-            w2[item] = __halves2bfloat162(channel < dim && z < args.rank ? source[z] : zero,
-                                          channel < dim && z + 1 < args.rank ? source[z + 1] : zero);
-        }
-    }
 
     const uint32_t warp = threadIdx.x / 32;
     const uint32_t warp_lane = threadIdx.x % 32;
-    for (uint32_t tile = begin; tile < end; tile += TOKENS) {
-        const uint32_t tokens = end - tile < TOKENS ? end - tile : TOKENS;
-        for (uint32_t t = warp; t < tokens; t += kWarps) {
-            const T* row = args.projected + static_cast<size_t>(tile + t) * args.pitch;
-            float sum = 0.0f;
-            for (uint32_t channel = warp_lane; channel < dim; channel += 32) {
-                const float value = to_float<T>(row[width + head_base + channel]);
-                sum = fmaf(value, value, sum);
-            }
-            sum = warp_sum(sum);
-            if (warp_lane == 0) unit_scale[t] = 1.0f / sqrtf(sum + kUnitEps);
+    const T* row = args.projected + token * args.pitch;
+    if (warp == 0) {
+        float sum = 0.0f;
+        for (uint32_t channel = warp_lane; channel < dim; channel += 32) {
+            const float value = to_float<T>(row[width + head_base + channel]);
+            sum = fmaf(value, value, sum);
         }
-        for (uint32_t item = threadIdx.x; item < tokens * padded_z; item += kThreads) {
-            const uint32_t t = item / padded_z;
-            const uint32_t z = item % padded_z;
-            z_values[item] = z < args.rank ? tanhf(to_float<T>(args.projected[static_cast<size_t>(tile + t) * args.pitch +
-                                                                             5 * width + z]))
-                                           : 0.0f;
+        sum = warp_sum(sum);
+        if (warp_lane == 0) *unit_scale = 1.0f / sqrtf(sum + kUnitEps);
+    }
+    for (uint32_t z = threadIdx.x; z < args.rank; z += kThreads) z_values[z] = tanhf(to_float<T>(row[5 * width + z]));
+    __syncthreads();
+    for (uint32_t channel = threadIdx.x; channel < DP; channel += kThreads) {
+        Prepared p = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        if (channel < dim) {
+            const __nv_bfloat16* source = args.decay_up + (head_base + channel) * args.rank;
+            float logit = 0.0f;
+            for (uint32_t z = 0; z < args.rank; ++z) logit = fmaf(__bfloat162float(source[z]), z_values[z], logit);
+            p = prepare<T>(args, row, width, head_base + channel, logit, *unit_scale);
         }
-        __syncthreads();
-        // one key channel and every (kThreads / DP)-th group of four tokens per thread, so that a W2 value serves four
-        constexpr uint32_t kShared = TOKENS < 4 ? TOKENS : 4;
-        constexpr uint32_t kStride = kThreads >= DP ? kThreads / DP : 1;
-        for (uint32_t channel = threadIdx.x % DP; channel < DP; channel += kThreads >= DP ? DP : kThreads) {
-            for (uint32_t t0 = threadIdx.x / DP * kShared; t0 < tokens; t0 += kStride * kShared) {
-                float logit[kShared];
-#pragma unroll
-                for (uint32_t i = 0; i < kShared; ++i) logit[i] = 0.0f;
-                if (channel < dim) {
-                    if (STAGED) {
-                        for (uint32_t z = 0; z < padded_z; z += 4) {
-                            const float2 low = __bfloat1622float2(w2[z / 2 * DP + channel]);
-                            const float2 high = __bfloat1622float2(w2[(z / 2 + 1) * DP + channel]);
-#pragma unroll
-                            for (uint32_t i = 0; i < kShared; ++i) {
-                                const float4 value =
-                                    *reinterpret_cast<const float4*>(z_values + (t0 + i) * padded_z + z);
-                                logit[i] = fmaf(low.x, value.x, logit[i]);
-                                logit[i] = fmaf(low.y, value.y, logit[i]);
-                                logit[i] = fmaf(high.x, value.z, logit[i]);
-                                logit[i] = fmaf(high.y, value.w, logit[i]);
-                            }
-                        }
-                    } else {
-                        const __nv_bfloat16* source = args.decay_up + (head_base + channel) * args.rank;
-                        for (uint32_t z = 0; z < args.rank; ++z) {
-                            const float weight = __bfloat162float(source[z]);
-#pragma unroll
-                            for (uint32_t i = 0; i < kShared; ++i) {
-                                logit[i] = fmaf(weight, z_values[(t0 + i) * padded_z + z], logit[i]);
-                            }
-                        }
-                    }
-                }
-#pragma unroll
-                for (uint32_t i = 0; i < kShared; ++i) {
-                    const uint32_t t = t0 + i;
-                    if (t >= tokens) break;
-                    Prepared p = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-                    if (channel < dim) {
-                        p = prepare<T>(args, args.projected + static_cast<size_t>(tile + t) * args.pitch, width,
-                                       head_base + channel, logit[i], unit_scale[t]);
-                    }
-                    float* target = vectors + t * kVectors * DP + channel;
-                    target[0 * DP] = p.r;
-                    target[1 * DP] = p.w;
-                    target[2 * DP] = p.removal;
-                    target[3 * DP] = p.u;
-                    target[4 * DP] = p.k;
-                    target[5 * DP] = p.v;
-                }
-            }
-        }
-        __syncthreads();
+        float* target = vectors + channel;
+        target[0 * DP] = p.r;
+        target[1 * DP] = p.w;
+        target[2 * DP] = p.removal;
+        target[3 * DP] = p.u;
+        target[4 * DP] = p.k;
+        target[5 * DP] = p.v;
+    }
+    __syncthreads();
 
-        for (uint32_t t = 0; t < tokens; ++t) {
-            const float* token = vectors + t * kVectors * DP;
-            const float value = token[5 * DP + (column < DP ? column : 0)];
-            Pair dot0 = 0, dot1 = 0;                                // bit pattern of (0.0f, 0.0f)
+    const float value = vectors[5 * DP + (column < DP ? column : 0)];
+    Pair dot0 = 0, dot1 = 0;                                    // bit pattern of (0.0f, 0.0f)
 #pragma unroll
-            for (uint32_t g = 0; g < kGroups; ++g) {
-                const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(token + 3 * DP + (g * LANES + lane) * 4);
-                dot0 = fma_pair(u.x, state[2 * g], dot0);
-                dot1 = fma_pair(u.y, state[2 * g + 1], dot1);
-            }
-            float dot = pair_sum(dot0) + pair_sum(dot1);
+    for (uint32_t g = 0; g < kGroups; ++g) {
+        const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(vectors + 3 * DP + (g * LANES + lane) * 4);
+        dot0 = fma_pair(u.x, state[2 * g], dot0);
+        dot1 = fma_pair(u.y, state[2 * g + 1], dot1);
+    }
+    float dot = pair_sum(dot0) + pair_sum(dot1);
 #pragma unroll
-            for (uint32_t delta = 1; delta < LANES; delta <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, delta);
-            const Pair recalled = pair_of(dot, dot);
-            const Pair values = pair_of(value, value);
-            Pair sum0 = 0, sum1 = 0;
+    for (uint32_t delta = 1; delta < LANES; delta <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, delta);
+    const Pair recalled = pair_of(dot, dot);
+    const Pair values = pair_of(value, value);
+    Pair sum0 = 0, sum1 = 0;
 #pragma unroll
-            for (uint32_t g = 0; g < kGroups; ++g) {
-                const uint32_t row = (g * LANES + lane) * 4;
-                const ulonglong2 r = *reinterpret_cast<const ulonglong2*>(token + row);
-                const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(token + 1 * DP + row);
-                const ulonglong2 removal = *reinterpret_cast<const ulonglong2*>(token + 2 * DP + row);
-                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(token + 4 * DP + row);
-                state[2 * g] = fma_pair(k.x, values, fma_pair(removal.x, recalled, mul_pair(w.x, state[2 * g])));
-                state[2 * g + 1] =
-                    fma_pair(k.y, values, fma_pair(removal.y, recalled, mul_pair(w.y, state[2 * g + 1])));
-                sum0 = fma_pair(r.x, state[2 * g], sum0);
-                sum1 = fma_pair(r.y, state[2 * g + 1], sum1);
-            }
-            float result = pair_sum(sum0) + pair_sum(sum1);
+    for (uint32_t g = 0; g < kGroups; ++g) {
+        const float* at = vectors + (g * LANES + lane) * 4;
+        const ulonglong2 r = *reinterpret_cast<const ulonglong2*>(at);
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(at + 1 * DP);
+        const ulonglong2 removal = *reinterpret_cast<const ulonglong2*>(at + 2 * DP);
+        const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(at + 4 * DP);
+        state[2 * g] = fma_pair(k.x, values, fma_pair(removal.x, recalled, mul_pair(w.x, state[2 * g])));
+        state[2 * g + 1] = fma_pair(k.y, values, fma_pair(removal.y, recalled, mul_pair(w.y, state[2 * g + 1])));
+        sum0 = fma_pair(r.x, state[2 * g], sum0);
+        sum1 = fma_pair(r.y, state[2 * g + 1], sum1);
+    }
+    float result = pair_sum(sum0) + pair_sum(sum1);
 #pragma unroll
-            for (uint32_t delta = 1; delta < LANES; delta <<= 1) result += __shfl_xor_sync(0xffffffffu, result, delta);
-            if (lane == 0 && live) {
-                if (args.raw != nullptr) {
-                    args.raw[static_cast<size_t>(tile + t) * width + head_base + column] = result;
-                } else {
-                    produced[t * DP + column] = result;
-                }
-            }
+    for (uint32_t delta = 1; delta < LANES; delta <<= 1) result += __shfl_xor_sync(0xffffffffu, result, delta);
+    if (lane == 0 && live) {
+        if (args.raw != nullptr) {
+            args.raw[token * width + head_base + column] = result;
+        } else {
+            produced[column] = result;
         }
-        __syncthreads();
-        if (args.raw == nullptr) {
-            for (uint32_t t = warp; t < tokens; t += kWarps) {
-                const size_t token = tile + t;
-                const T* gate = args.projected + token * args.pitch + 3 * width + head_base;
-                float sum = 0.0f;
-                for (uint32_t channel = warp_lane; channel < dim; channel += 32) {
-                    sum = fmaf(produced[t * DP + channel], produced[t * DP + channel], sum);
-                }
-                const float scale = inverse_rms(warp_sum(sum), dim, args.eps);
-                for (uint32_t channel = warp_lane; channel < dim; channel += 32) {
-                    const float normalised =
-                        produced[t * DP + channel] * scale * __bfloat162float(args.norm[head_base + channel]);
-                    args.out[token * args.out_pitch + head_base + channel] =
-                        from_float<T>(normalised * sigmoidf(to_float<T>(gate[channel])));
-                }
-            }
+    }
+    __syncthreads();
+    if (args.raw == nullptr && warp == 0) {
+        const T* gate = row + 3 * width + head_base;
+        float sum = 0.0f;
+        for (uint32_t channel = warp_lane; channel < dim; channel += 32) {
+            sum = fmaf(produced[channel], produced[channel], sum);
         }
-        // the next tile's first barrier lies behind writes to unit_scale and z_values only, which nobody reads now
+        const float scale = inverse_rms(warp_sum(sum), dim, args.eps);
+        for (uint32_t channel = warp_lane; channel < dim; channel += 32) {
+            const float normalised = produced[channel] * scale * __bfloat162float(args.norm[head_base + channel]);
+            args.out[token * args.out_pitch + head_base + channel] =
+                from_float<T>(normalised * sigmoidf(to_float<T>(gate[channel])));
+        }
     }
 
 #pragma unroll
     for (uint32_t g = 0; g < kGroups; ++g) {
-        const uint32_t row = (g * LANES + lane) * 4;
-        if (live && row < dim) {
-            float4 value;
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(value.x), "=f"(value.y) : "l"(state[2 * g]));
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(value.z), "=f"(value.w) : "l"(state[2 * g + 1]));
+        const uint32_t at = (g * LANES + lane) * 4;
+        if (live && at < dim) {
+            const float4 held = {low_of(state[2 * g]), high_of(state[2 * g]), low_of(state[2 * g + 1]),
+                                 high_of(state[2 * g + 1])};
             if (vector_state) {
-                *reinterpret_cast<float4*>(state_column + row) = value;
+                *reinterpret_cast<float4*>(state_column + at) = held;
             } else {
-                state_column[row] = value.x;
-                if (row + 1 < dim) state_column[row + 1] = value.y;
-                if (row + 2 < dim) state_column[row + 2] = value.z;
-                if (row + 3 < dim) state_column[row + 3] = value.w;
+                state_column[at] = held.x;
+                if (at + 1 < dim) state_column[at + 1] = held.y;
+                if (at + 2 < dim) state_column[at + 2] = held.z;
+                if (at + 3 < dim) state_column[at + 3] = held.w;
             }
         }
     }
@@ -1592,15 +1479,8 @@ bool split_takes(const DeltaArgs<__nv_bfloat16>& args, const DeltaRuleLaunch& la
 template <typename T, uint32_t DP, uint32_t LANES, uint32_t COLUMNS>
 cudaError_t launch_sized(cudaStream_t stream, DeltaArgs<T> args) {
     args.splits = (args.dim + COLUMNS - 1) / COLUMNS;
-    const bool single = args.segments.offsets == nullptr;
-    const size_t staged_bytes = delta_shared_bytes<DP>(kTileTokens, args.rank, true);
-    const bool staged = !single && staged_bytes <= 160 * 1024;
-    const size_t shared = single ? delta_shared_bytes<DP>(1, args.rank, false)
-                                 : (staged ? staged_bytes : delta_shared_bytes<DP>(kTileTokens, args.rank, false));
-    void (*kernel)(const DeltaArgs<T>) =
-        single ? delta_rule_kernel<T, DP, LANES, COLUMNS, 1, false>
-               : (staged ? delta_rule_kernel<T, DP, LANES, COLUMNS, kTileTokens, true>
-                         : delta_rule_kernel<T, DP, LANES, COLUMNS, kTileTokens, false>);
+    const size_t shared = delta_shared_bytes<DP>(args.rank);
+    void (*kernel)(const DeltaArgs<T>) = delta_rule_kernel<T, DP, LANES, COLUMNS>;
     if (shared > 227 * 1024) {
         return cudaErrorInvalidValue;
     }
@@ -1656,6 +1536,7 @@ cudaError_t launch_typed(cudaStream_t stream, const DeltaRuleLaunch& launch) {
             return launch.dim <= 64 ? launch_prompt<64, 4, 128>(stream, args) : launch_prompt<128, 4, 128>(stream, args);
         }
     }
+    if (launch.segments.offsets != nullptr) return launch_delta_scan(stream, args, launch.vectors, launch.vector_bytes);
     if (launch.dim <= 32) return launch_sized<T, 32, 4, 32>(stream, args);
     if (launch.dim <= 64) return launch_sized<T, 64, 4, 64>(stream, args);
     if (launch.dim <= 128) return launch_sized<T, 128, 4, 128>(stream, args);
@@ -1666,6 +1547,13 @@ cudaError_t launch_typed(cudaStream_t stream, const DeltaRuleLaunch& launch) {
 }  // namespace
 
 bool delta_rule_needs_scratch(uint32_t dim) { return dim > 128; }
+
+size_t delta_rule_vector_bytes(Activation type, uint32_t heads, uint32_t dim, uint32_t rank, size_t pitch, size_t out_pitch,
+                               size_t tokens) {
+    const bool others = type == Activation::kBf16 && dim % 8 == 0 && dim <= 128 && rank <= kPromptMaxRank && pitch % 8 == 0 &&
+                        out_pitch % 2 == 0;      // kernels of their own, see prompt_kernel_takes()
+    return delta_scan_bytes(others ? 1 : heads, dim, tokens);
+}
 
 size_t delta_rule_chunk_bytes(Activation type, uint32_t heads, uint32_t dim, size_t tokens, size_t segments) {
     const size_t most = std::min(std::min(segments, tokens / split_shortest(heads)), kSplitMostHeads / heads);

@@ -27,6 +27,36 @@ struct DeltaArgs {
     uint32_t splits;         // CTAs per head, each with COLUMNS value channels
 };
 
+using Pair = unsigned long long;     // two f32 values
+
+__device__ __forceinline__ Pair pair_of(float low, float high) {
+    Pair out;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(out) : "f"(low), "f"(high));
+    return out;
+}
+__device__ __forceinline__ float pair_sum(Pair value) {
+    float low, high;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(low), "=f"(high) : "l"(value));
+    return low + high;
+}
+__device__ __forceinline__ float low_of(Pair value) { return __uint_as_float(static_cast<uint32_t>(value)); }
+__device__ __forceinline__ float high_of(Pair value) { return __uint_as_float(static_cast<uint32_t>(value >> 32)); }
+__device__ __forceinline__ Pair fma_pair(Pair a, Pair b, Pair c) {
+    Pair out;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(out) : "l"(a), "l"(b), "l"(c));
+    return out;
+}
+__device__ __forceinline__ Pair add_pair(Pair a, Pair b) {
+    Pair out;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(out) : "l"(a), "l"(b));
+    return out;
+}
+__device__ __forceinline__ Pair mul_pair(Pair a, Pair b) {
+    Pair out;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(out) : "l"(a), "l"(b));
+    return out;
+}
+
 // Decays and rates: the fast f32 exponential and division, a few units in the last place from the
 // correctly rounded ones.
 __device__ __forceinline__ float fast_sigmoid(float z) { return __fdividef(1.0f, 1.0f + __expf(-z)); }
@@ -142,6 +172,12 @@ __device__ __forceinline__ void store_c(float* target, uint32_t stride, uint32_t
     *reinterpret_cast<float2*>(at) = make_float2(c[0], c[1]);
     *reinterpret_cast<float2*>(at + 8 * stride) = make_float2(c[2], c[3]);
 }
+
+// The kernels of delta_scan.cu: segments of any length in plain f32 arithmetic.  Scratch for `heads` heads of a step of `tokens`
+// tokens: all of them, or as many as a bound allows, which are then taken in turns.
+size_t delta_scan_bytes(size_t heads, uint32_t dim, size_t tokens);
+template <typename T>
+cudaError_t launch_delta_scan(cudaStream_t stream, const DeltaArgs<T>& args, float* scratch, size_t scratch_bytes);
 
 // The kernels of delta_split.cu: bf16 segments whose projections lie in whole 16-byte pieces, heads up to 64.
 size_t delta_split_bytes(size_t heads, size_t tiles);

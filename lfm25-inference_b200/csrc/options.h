@@ -20,8 +20,8 @@
 //                                                                        where they take the shape, or always the scalar one
 //   delta_prompt         0 auto | 1 scan | 2 general           0         delta rule over bf16 segments: tensor-core chunks where they
 //                        | 3 carried | 4 split                           take the head size, the token-by-token prompt kernel, or
-//                                                                        the general kernel; 3 and 4: chunks, never or always
-//                                                                        split along the sequence (f32: the general kernel;
+//                                                                        the f32 kernels of every type; 3 and 4: chunks, never or
+//                                                                        always split along the sequence (f32: the f32 kernels;
 //                                                                        4 fails where an executor has no scratch for it)
 //   state_space_prompt   0 auto | 1 scan                       0         state-space recurrence over bf16 segments: tensor-core
 //                                                                        chunks where they take the sizes, or the

@@ -45,6 +45,8 @@ struct lfm25_stack_executor {
     float* raw;                // [T, widest heads * dim] when a delta rule needs it
     float* chunks;             // of a delta rule split along the sequence
     size_t chunk_bytes = 0;
+    float* vectors;            // of a delta rule that runs token by token in f32
+    size_t vector_bytes = 0;
     void* compressed;          // [T, widest q_rank]: latent attention's query latent
     void* absorbed;            // [T, widest heads * kv_rank]: queries against latents
     void* weighted;            // [T, widest heads * kv_rank]: weighted latents
@@ -310,6 +312,8 @@ int32_t run_general_delta(lfm25_stack_executor* self, const Step& step, const lf
     delta.raw = self->raw;
     delta.chunks = self->chunks;
     delta.chunk_bytes = self->chunk_bytes;
+    delta.vectors = self->vectors;
+    delta.vector_bytes = self->vector_bytes;
     delta.out = self->joined;
     delta.out_pitch = layer.output.k;
     delta.eps = model.norm_eps;
@@ -781,7 +785,7 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
         return lfm25::report_error(LFM25_ERR_INVALID_ARGUMENT, "stack model sizes are inconsistent");
     }
     size_t projection = 0, query = 0, up = 0, joined = 0, raw = 0, compressed = 0, latents = 0, channels = 0, scanned = 0;
-    size_t context_rank = 0, context_keys = 0, context_columns = 0, chunk_bytes = 0, factors = 0, pieces = 0;
+    size_t context_rank = 0, context_keys = 0, context_columns = 0, chunk_bytes = 0, vector_bytes = 0, factors = 0, pieces = 0;
     const Activation type = static_cast<Activation>(model->activation);
     for (uint32_t index = 0; index < model->num_layers; ++index) {
         const lfm25_stack_layer& layer = model->layers[index];
@@ -801,6 +805,9 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
         if (layer.mixer == LFM25_MIXER_GENERAL_DELTA) {
             chunk_bytes = std::max(chunk_bytes, lfm25::delta_rule_chunk_bytes(type, layer.heads, layer.dim, maximum_tokens,
                                                                               maximum_rows));
+            vector_bytes = std::max(vector_bytes, lfm25::delta_rule_vector_bytes(type, layer.heads, layer.dim, layer.rank,
+                                                                                 layer.projection.n, layer.output.k,
+                                                                                 maximum_tokens));
         }
         if (layer.mixer == LFM25_MIXER_LATENT_ATTENTION) {
             const lfm25::LatentAttentionShape shape = {layer.heads, layer.dim, layer.rot_dim, layer.vdim, layer.kv_rank,
@@ -843,6 +850,7 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
     self->context_capacity = c;
     self->piece_bytes = pieces;
     self->chunk_bytes = chunk_bytes;
+    self->vector_bytes = vector_bytes;
     void** fields[] = {reinterpret_cast<void**>(&self->residual[0]), reinterpret_cast<void**>(&self->residual[1]),
                        &self->mixed, &self->normalized, &self->projected, &self->query, &self->up, &self->joined,
                        &self->update, &self->head_input, &self->logits, reinterpret_cast<void**>(&self->raw),
@@ -850,14 +858,14 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
                        &self->context_latents, &self->context_keys, &self->expanded,
                        reinterpret_cast<void**>(&self->context_bases), reinterpret_cast<void**>(&self->token_order),
                        &self->convolved, &self->scanned, &self->factors, reinterpret_cast<void**>(&self->pieces),
-                       reinterpret_cast<void**>(&self->chunks)};
+                       reinterpret_cast<void**>(&self->chunks), reinterpret_cast<void**>(&self->vectors)};
     const size_t sizes[] = {t * model->width * 4, t * model->width * 4, t * model->width * bytes,
                             t * model->width * bytes, t * projection * bytes, t * query * bytes, t * up * bytes,
                             t * joined * bytes, t * model->width * bytes, r * model->width * bytes,
                             r * model->head.n * bytes, t * raw * 4, r * 4, t * compressed * bytes, t * latents * bytes,
                             t * latents * bytes, c * context_rank * bytes, c * context_keys * bytes,
                             c * context_columns * bytes, (t + 1) * 4, latents > 0 ? t * 4 : 0, t * channels * bytes,
-                            t * scanned * bytes, factors, pieces, chunk_bytes};
+                            t * scanned * bytes, factors, pieces, chunk_bytes, vector_bytes};
     size_t total = 0;
     for (size_t size : sizes) total += (size + 255) & ~static_cast<size_t>(255);
     cudaError_t status = cudaMalloc(&self->allocation, total);

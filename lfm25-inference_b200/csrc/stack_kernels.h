@@ -371,6 +371,8 @@ struct DeltaRuleLaunch {
     float* raw;                    // f32 [T, heads * dim] scratch, needed when delta_rule_needs_scratch(dim)
     float* chunks;                 // chunk_bytes of scratch, or nullptr: prompts are not split along the sequence
     size_t chunk_bytes;
+    float* vectors;                // vector_bytes of scratch, needed by prompts that run token by token in f32
+    size_t vector_bytes;
     void* out;                     // activations, rows out_pitch apart, heads * dim columns
     size_t out_pitch;
     float eps;
@@ -381,6 +383,10 @@ constexpr size_t kDeltaChunkBytes = size_t(256) << 20;
 // Scratch for prompts that are split along the sequence, in steps of up to `tokens` tokens in `segments` segments; more heads
 // than it holds are taken in turns.
 size_t delta_rule_chunk_bytes(Activation type, uint32_t heads, uint32_t dim, size_t tokens, size_t segments);
+// Scratch for prompts that run token by token in f32, in steps of up to `tokens` tokens: every head of the shapes that always
+// do, one head (heads are taken in turns) of those with faster kernels.
+size_t delta_rule_vector_bytes(Activation type, uint32_t heads, uint32_t dim, uint32_t rank, size_t pitch, size_t out_pitch,
+                               size_t tokens);
 cudaError_t launch_delta_rule(cudaStream_t stream, const DeltaRuleLaunch& launch);
 
 }  // namespace lfm25

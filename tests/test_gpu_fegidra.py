@@ -107,6 +107,16 @@ def test_delta_rule_layer(device, dtype, heads, dim, rank):
     check_layer(config, 13, device, dtype, [37, 2, 1, 16, 1, 5], rank)
 
 
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("heads,dim,rank", [(1, 8, 3), (2, 64, 72), (3, 36, 64), (1, 72, 8), (2, 136, 65)])
+def test_delta_rule_token_by_token(device, library_option, dtype, heads, dim, rank):
+    """The f32 kernels for prompts at the edges of their tiles of 16 and 8 tokens and of 8 and 16 value columns; bf16 models take
+    them by the option, with scratch for one head at a time."""
+    library_option("delta_prompt", 2)
+    config = cases.config_of([cases.delta_layer(heads, dim, ff=0)])
+    check_layer(config, 19, device, dtype, [1, 1, 15, 16, 17, 2, 7, 8, 9, 33], rank)
+
+
 @pytest.mark.parametrize("heads,dim,rank", [(3, 16, 5), (2, 64, 16), (1, 24, 1), (2, 48, 70), (1, 128, 40), (2, 64, 250)])
 def test_delta_rule_prompt_kernels_agree(device, library_option, heads, dim, rank):
     """The tensor-core chunks, the token-by-token prompt kernel and the general kernel on the same bf16 inputs: all keep
