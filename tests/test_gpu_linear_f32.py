@@ -81,3 +81,20 @@ def test_values_that_are_no_finite_numbers(device, m, k, n):
     assert np.array_equal(np.isinf(got), infinite) and np.array_equal(got[infinite], want[infinite].astype(np.float32))
     finite = np.isfinite(want)
     assert finite.any() and np.allclose(got[finite], want[finite], rtol=0, atol=1e-5 * np.sqrt(k))
+
+
+@pytest.mark.parametrize("m,k,n", [(31, 64, 127), (32, 72, 128), (64, 192, 129), (65, 128, 1), (96, 328, 300), (97, 520, 24),
+                                   (400, 2056, 700), (3, 2048, 1100)])
+def test_edges_of_tiles(device, m, k, n):
+    """Tiles of 32, 64 and 96 rows by 128 columns, whole and cut; odd and even numbers of 64-wide blocks of k, the last one cut;
+    sums in one CTA and in clusters.  The bound of test_sums with 64 products in a short sum: a rounding (2^-24) for each of
+    them, for every pair of them and in a cluster's sum, and 2^-20 for what the tensor core cuts on the way: it adds four times
+    16 products, each time cutting less than 2^-22 of the largest term or partial sum for each of up to 17 terms' alignment
+    and the result, so less than 4 * 2^-22 of the products' sizes where it cuts terms that are aligned to their largest."""
+    rng = np.random.default_rng(m * k + n)
+    weight = rng.standard_normal((n, k)).astype(np.float32).view(np.uint32) & 0xFFFF0000
+    weight = weight.view(np.float32).astype(np.float64)
+    for x in (spread(rng, (m, k)), rng.standard_normal((m, k)).astype(np.float32)):
+        error = np.abs(product(device, x, weight) - x.astype(np.float64) @ weight.T)
+        bound = (k / 64 + k / 128 + 10) * 2.0 ** -24 + 2.0 ** -20 + k / 8 * 2.0 ** -30
+        assert (error <= bound * (np.abs(x).astype(np.float64) @ np.abs(weight).T)).all()
