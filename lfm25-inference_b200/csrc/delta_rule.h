@@ -173,6 +173,12 @@ __device__ __forceinline__ void store_c(float* target, uint32_t stride, uint32_t
     *reinterpret_cast<float2*>(at + 8 * stride) = make_float2(c[2], c[3]);
 }
 
+// The kernel of delta_chunk.cu: bf16 segments whose projections lie in whole 16-byte pieces, heads up to kDeltaChunkDim and ranks
+// up to what its shared memory holds.
+constexpr uint32_t kDeltaChunkDim = 64;
+bool delta_chunk_takes(uint32_t dim, uint32_t rank);
+cudaError_t launch_delta_chunk(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& args);
+
 // The kernels of delta_scan.cu: segments of any length in plain f32 arithmetic.  Scratch for `heads` heads of a step of `tokens`
 // tokens: all of them, or as many as a bound allows, which are then taken in turns.
 size_t delta_scan_bytes(size_t heads, uint32_t dim, size_t tokens);
