@@ -215,6 +215,150 @@ bool merge_in_kernel_preferred(size_t tokens, size_t splits) {
     return false;
 }
 
+constexpr size_t kPackedWidth = kQueryWidth + 2 * kKvWidth;
+
+// Query, key and value of an attention layer.  One GEMM when their BF16 matrices are adjacent in memory (q | k | v rows of one
+// [3072, 2048] allocation): the outputs then sit side by side in `wide`, [tokens, 3072], and *packed is set; the one-kernel
+// attention and the QK-norm + RoPE + append kernel both take token strides.
+int32_t project_qkv(lfm25_decode_executor* self, const lfm25_layer& layer, size_t tokens, bool use_fp8, bool* packed) {
+    const uint16_t* query_weight = static_cast<const uint16_t*>(layer.query.bf16);
+    *packed = query_weight != nullptr && !(use_fp8 && (layer.query.fp8.data || layer.key.fp8.data || layer.value.fp8.data)) &&
+              layer.key.bf16 == query_weight + kQueryWidth * kHidden &&
+              layer.value.bf16 == query_weight + (kQueryWidth + kKvWidth) * kHidden && layer.query.k == kHidden &&
+              layer.key.k == kHidden && layer.value.k == kHidden;
+    if (*packed) {
+        lfm25_linear_weights all = layer.query;
+        all.n = kPackedWidth;
+        return linear_decode(self, all, self->normalized, self->wide, tokens, false);
+    }
+    LFM25_TRY(linear_decode(self, layer.query, self->normalized, self->query, tokens, use_fp8));
+    LFM25_TRY(linear_decode(self, layer.key, self->normalized, self->key, tokens, use_fp8));
+    return linear_decode(self, layer.value, self->normalized, self->value, tokens, use_fp8);
+}
+
+// QK-norm, RoPE and the paged append.  A packed projection is read in place; the rotated query goes to the dense array that
+// attention reads.
+int32_t append_qkv(lfm25_decode_executor* self, const lfm25_qk_postprocess_launch& post, bool packed) {
+    RegionTimer timer(self, LFM25_REGION_APPEND);
+    if (!packed) return lfm25_qk_norm_rope_kv_write_decode(self->blaslt->stream, &post);
+    const uint16_t* packed_rows = static_cast<const uint16_t*>(self->wide);
+    lfm25::QkPostprocessArgs strided;
+    strided.query = packed_rows;
+    strided.query_out = self->query;
+    strided.query_token_stride = kPackedWidth;
+    strided.kv_token_stride = kPackedWidth;
+    strided.key = packed_rows + kQueryWidth;
+    strided.value = packed_rows + kQueryWidth + kKvWidth;
+    strided.query_norm = post.query_norm.ptr;
+    strided.key_norm = post.key_norm.ptr;
+    strided.inv_freq = static_cast<const float*>(post.inv_freq.ptr);
+    strided.position_ids = static_cast<const uint32_t*>(post.position_ids.ptr);
+    strided.slot_mapping = static_cast<const int64_t*>(post.slot_mapping.ptr);
+    strided.key_cache = post.key_cache.ptr;
+    strided.value_cache = post.value_cache.ptr;
+    strided.num_tokens = post.num_tokens;
+    strided.num_pages = post.num_pages;
+    strided.eps = post.eps;
+    const cudaError_t status = lfm25::launch_qk_norm_rope_kv_write_decode(self->blaslt->stream, strided);
+    return status == cudaSuccess ? LFM25_OK : cuda_failure(status, "QK postprocess launch failed");
+}
+
+// Gate/Up, SiLU(gate) * up and Down of a layer, from `normalized` (and, with gate_up_fp8, its codes in fp8_input) to
+// `operator_output`.
+int32_t feed_forward(lfm25_decode_executor* self, const lfm25_layer& layer, size_t tokens, bool use_fp8, bool gate_up_fp8) {
+    cudaStream_t stream = self->blaslt->stream;
+    // An FP8 Gate/Up whose shape the tensor-core kernel takes runs with SiLU(gate) * up in its epilogue: the
+    // packed projection is never written, and the activation arrives as the Down site's E4M3 codes or as bf16.
+    const bool fuse_gate = lfm25::option(lfm25::kOptFusedSilu) != 0;
+    const bool down_fp8 = use_fp8 && layer.down.fp8.data != nullptr;
+    bool gate_fused = false;
+    if (fuse_gate && gate_up_fp8 && layer.gate_up.n == 2 * kFfn && (down_fp8 || layer.down.bf16 != nullptr)) {
+        RegionTimer timer(self, LFM25_REGION_FP8_LINEAR);
+        lfm25_fp8_linear_config config;
+        config.m = tokens;
+        config.n = 2 * kFfn;
+        config.k = kHidden;
+        config.scale_mode = LFM25_FP8_SCALE_TENSORWIDE;
+        config.output_scale = layer.gate_up.fp8.activation_dequantize * layer.gate_up.fp8.weight_dequantize;
+        // the codes of the normalised rows are in fp8_input; the activation's codes go to `activated` (the Down
+        // GEMM reads them from there), the bf16 activation too
+        const int32_t rc = lfm25_blaslt_linear_fp8_silu_mul(
+            self->blaslt, slice_of(self->fp8_input, tokens * kHidden),
+            slice_of(layer.gate_up.fp8.data, 2 * kFfn * kHidden),
+            slice_of(self->activated, down_fp8 ? tokens * kFfn * 2 : tokens * kFfn), &config,
+            down_fp8 ? layer.down.fp8.activation_quantize : 1.0f, down_fp8 ? 1u : 0u);
+        if (rc == LFM25_OK) {
+            gate_fused = true;
+        } else if (rc != LFM25_ERR_UNSUPPORTED) {
+            return rc;
+        }
+    }
+    if (!gate_fused && fuse_gate && !gate_up_fp8 && layer.gate_up.bf16 != nullptr && layer.gate_up.n == 2 * kFfn &&
+        layer.gate_up.k == kHidden && (down_fp8 || layer.down.bf16 != nullptr) &&
+        lfm25::option(lfm25::kOptFusedSiluBf16) != 0) {
+        // the same fusion for a Gate/Up site that stays in BF16 (batch-major tcgen05 kernel)
+        RegionTimer timer(self, LFM25_REGION_BF16_LINEAR);
+        const int32_t rc = lfm25_blaslt_linear_bf16_silu_mul(
+            self->blaslt, slice_of(self->normalized, tokens * kHidden), slice_of(layer.gate_up.bf16, 2 * kFfn * kHidden),
+            slice_of(self->activated, down_fp8 ? tokens * kFfn * 2 : tokens * kFfn), tokens, 2 * kFfn, kHidden,
+            down_fp8 ? layer.down.fp8.activation_quantize : 1.0f, down_fp8 ? 1u : 0u);
+        if (rc == LFM25_OK) {
+            gate_fused = true;
+        } else if (rc != LFM25_ERR_UNSUPPORTED) {
+            return rc;
+        }
+    }
+    if (gate_fused) {
+        if (down_fp8) {
+            RegionTimer timer(self, LFM25_REGION_FP8_LINEAR);
+            lfm25_fp8_linear_config config;
+            config.m = tokens;
+            config.n = kHidden;
+            config.k = kFfn;
+            config.scale_mode = LFM25_FP8_SCALE_TENSORWIDE;
+            config.output_scale = layer.down.fp8.activation_dequantize * layer.down.fp8.weight_dequantize;
+            LFM25_TRY(lfm25_blaslt_linear_fp8_scaled(self->blaslt, slice_of(self->activated, tokens * kFfn),
+                                                     slice_of(layer.down.fp8.data, kHidden * kFfn),
+                                                     slice_of(self->operator_output, tokens * kHidden), &config));
+        } else {
+            RegionTimer timer(self, LFM25_REGION_BF16_LINEAR);
+            LFM25_TRY(lfm25_blaslt_linear_bf16(self->blaslt, slice_of(self->activated, tokens * kFfn),
+                                               slice_of(layer.down.bf16, kHidden * kFfn),
+                                               slice_of(self->operator_output, tokens * kHidden), tokens, kHidden,
+                                               kFfn));
+        }
+    } else {
+    LFM25_TRY(linear_decode(self, layer.gate_up, self->normalized, self->wide, tokens, use_fp8, gate_up_fp8));
+    if (use_fp8 && layer.down.fp8.data != nullptr) {
+        RegionTimer timer(self, LFM25_REGION_FP8_LINEAR);
+        LFM25_TRY(lfm25_silu_mul_packed_bf16_to_e4m3(stream, slice_of(self->wide, tokens * 2 * kFfn),
+                                                     slice_of(self->fp8_input, self->maximum_tokens * kFfn),
+                                                     tokens, kFfn, layer.down.fp8.activation_quantize));
+        lfm25_fp8_linear_config config;
+        config.m = tokens;
+        config.n = kHidden;
+        config.k = kFfn;
+        config.scale_mode = LFM25_FP8_SCALE_TENSORWIDE;
+        config.output_scale = layer.down.fp8.activation_dequantize * layer.down.fp8.weight_dequantize;
+        LFM25_TRY(lfm25_blaslt_linear_fp8_scaled(self->blaslt, slice_of(self->fp8_input, tokens * kFfn),
+                                                 slice_of(layer.down.fp8.data, kHidden * kFfn),
+                                                 slice_of(self->operator_output, tokens * kHidden), &config));
+    } else {
+        RegionTimer timer(self, LFM25_REGION_BF16_LINEAR);
+        LFM25_TRY(lfm25_silu_mul_packed_bf16(stream, slice_of(self->wide, tokens * 2 * kFfn),
+                                             slice_of(self->activated, tokens * kFfn), tokens, kFfn));
+        if (layer.down.bf16 == nullptr) {
+            return lfm25::report_error(LFM25_ERR_NULL_POINTER, "Down site has no BF16 weights resident");
+        }
+        LFM25_TRY(lfm25_blaslt_linear_bf16(self->blaslt, slice_of(self->activated, tokens * kFfn),
+                                           slice_of(layer.down.bf16, kHidden * kFfn),
+                                           slice_of(self->operator_output, tokens * kHidden), tokens, kHidden,
+                                           kFfn));
+    }
+    }
+    return LFM25_OK;
+}
+
 int32_t forward(lfm25_decode_executor* self, const lfm25_model* model, const lfm25_decode_batch* batch, bool use_fp8,
                 bool advance) {
     cudaStream_t stream = self->blaslt->stream;
@@ -252,25 +396,8 @@ int32_t forward(lfm25_decode_executor* self, const lfm25_model* model, const lfm
             const int64_t route = lfm25::option(lfm25::kOptFusedAppend);
             const bool fused_append =
                 route == 2 ? lfm25_decode_one_kernel_preferred(16, batch->max_context_tokens, tokens) != 0 : route != 0;
-            // One GEMM for the three projections when their BF16 matrices are adjacent in memory (q | k | v rows of
-            // one [3072, 2048] allocation): the outputs then sit side by side in `wide`, [tokens, 3072]; the one-kernel
-            // attention and the QK-norm + RoPE + append kernel both take token strides.
-            const uint16_t* query_weight = static_cast<const uint16_t*>(layer.query.bf16);
-            const bool packed_qkv = query_weight != nullptr &&
-                                    !(use_fp8 && (layer.query.fp8.data || layer.key.fp8.data || layer.value.fp8.data)) &&
-                                    layer.key.bf16 == query_weight + kQueryWidth * kHidden &&
-                                    layer.value.bf16 == query_weight + (kQueryWidth + kKvWidth) * kHidden &&
-                                    layer.query.k == kHidden && layer.key.k == kHidden && layer.value.k == kHidden;
-            constexpr size_t kPackedWidth = kQueryWidth + 2 * kKvWidth;
-            if (packed_qkv) {
-                lfm25_linear_weights packed = layer.query;
-                packed.n = kPackedWidth;
-                LFM25_TRY(linear_decode(self, packed, self->normalized, self->wide, tokens, false));
-            } else {
-                LFM25_TRY(linear_decode(self, layer.query, self->normalized, self->query, tokens, use_fp8));
-                LFM25_TRY(linear_decode(self, layer.key, self->normalized, self->key, tokens, use_fp8));
-                LFM25_TRY(linear_decode(self, layer.value, self->normalized, self->value, tokens, use_fp8));
-            }
+            bool packed_qkv = false;
+            LFM25_TRY(project_qkv(self, layer, tokens, use_fp8, &packed_qkv));
             const size_t cache_elements = model->num_pages * 8 * 16 * 64;
             lfm25_qk_postprocess_launch post;
             post.page_size = 16;
@@ -332,33 +459,7 @@ int32_t forward(lfm25_decode_executor* self, const lfm25_model* model, const lfm
                 }
                 LFM25_TRY(lfm25_fused_ragged_paged_attention_decode_lfm2_bf16(stream, &fused));
             } else {
-            if (packed_qkv) {
-                // the packed projection is read in place; the rotated query goes to the dense array attention reads
-                RegionTimer timer(self, LFM25_REGION_APPEND);
-                const uint16_t* packed_rows = static_cast<const uint16_t*>(self->wide);
-                lfm25::QkPostprocessArgs strided;
-                strided.query = packed_rows;
-                strided.query_out = self->query;
-                strided.query_token_stride = kPackedWidth;
-                strided.kv_token_stride = kPackedWidth;
-                strided.key = packed_rows + kQueryWidth;
-                strided.value = packed_rows + kQueryWidth + kKvWidth;
-                strided.query_norm = layer.query_norm;
-                strided.key_norm = layer.key_norm;
-                strided.inv_freq = static_cast<const float*>(model->inv_freq);
-                strided.position_ids = static_cast<const uint32_t*>(batch->positions);
-                strided.slot_mapping = static_cast<const int64_t*>(batch->physical_slots);
-                strided.key_cache = layer.key_cache;
-                strided.value_cache = layer.value_cache;
-                strided.num_tokens = tokens;
-                strided.num_pages = model->num_pages;
-                strided.eps = model->norm_eps;
-                const cudaError_t status = lfm25::launch_qk_norm_rope_kv_write_decode(stream, strided);
-                if (status != cudaSuccess) return cuda_failure(status, "QK postprocess launch failed");
-            } else {
-                RegionTimer timer(self, LFM25_REGION_APPEND);
-                LFM25_TRY(lfm25_qk_norm_rope_kv_write_decode(stream, &post));
-            }
+            LFM25_TRY(append_qkv(self, post, packed_qkv));
             {
             RegionTimer attention_timer(self, LFM25_REGION_ATTENTION);
             lfm25_splitk_ragged_attention_launch attention;
@@ -412,95 +513,7 @@ int32_t forward(lfm25_decode_executor* self, const lfm25_model* model, const lfm
         }
         if (status != cudaSuccess) return cuda_failure(status, "residual_rms_norm launch failed");
 
-        // An FP8 Gate/Up whose shape the tensor-core kernel takes runs with SiLU(gate) * up in its epilogue: the
-        // packed projection is never written, and the activation arrives as the Down site's E4M3 codes or as bf16.
-        const bool fuse_gate = lfm25::option(lfm25::kOptFusedSilu) != 0;
-        const bool down_fp8 = use_fp8 && layer.down.fp8.data != nullptr;
-        bool gate_fused = false;
-        if (fuse_gate && gate_up_fp8 && layer.gate_up.n == 2 * kFfn && (down_fp8 || layer.down.bf16 != nullptr)) {
-            RegionTimer timer(self, LFM25_REGION_FP8_LINEAR);
-            lfm25_fp8_linear_config config;
-            config.m = tokens;
-            config.n = 2 * kFfn;
-            config.k = kHidden;
-            config.scale_mode = LFM25_FP8_SCALE_TENSORWIDE;
-            config.output_scale = layer.gate_up.fp8.activation_dequantize * layer.gate_up.fp8.weight_dequantize;
-            // the codes of the normalised rows are in fp8_input; the activation's codes go to `activated` (the Down
-            // GEMM reads them from there), the bf16 activation too
-            const int32_t rc = lfm25_blaslt_linear_fp8_silu_mul(
-                self->blaslt, slice_of(self->fp8_input, tokens * kHidden),
-                slice_of(layer.gate_up.fp8.data, 2 * kFfn * kHidden),
-                slice_of(self->activated, down_fp8 ? tokens * kFfn * 2 : tokens * kFfn), &config,
-                down_fp8 ? layer.down.fp8.activation_quantize : 1.0f, down_fp8 ? 1u : 0u);
-            if (rc == LFM25_OK) {
-                gate_fused = true;
-            } else if (rc != LFM25_ERR_UNSUPPORTED) {
-                return rc;
-            }
-        }
-        if (!gate_fused && fuse_gate && !gate_up_fp8 && layer.gate_up.bf16 != nullptr && layer.gate_up.n == 2 * kFfn &&
-            layer.gate_up.k == kHidden && (down_fp8 || layer.down.bf16 != nullptr) &&
-            lfm25::option(lfm25::kOptFusedSiluBf16) != 0) {
-            // the same fusion for a Gate/Up site that stays in BF16 (batch-major tcgen05 kernel)
-            RegionTimer timer(self, LFM25_REGION_BF16_LINEAR);
-            const int32_t rc = lfm25_blaslt_linear_bf16_silu_mul(
-                self->blaslt, slice_of(self->normalized, tokens * kHidden), slice_of(layer.gate_up.bf16, 2 * kFfn * kHidden),
-                slice_of(self->activated, down_fp8 ? tokens * kFfn * 2 : tokens * kFfn), tokens, 2 * kFfn, kHidden,
-                down_fp8 ? layer.down.fp8.activation_quantize : 1.0f, down_fp8 ? 1u : 0u);
-            if (rc == LFM25_OK) {
-                gate_fused = true;
-            } else if (rc != LFM25_ERR_UNSUPPORTED) {
-                return rc;
-            }
-        }
-        if (gate_fused) {
-            if (down_fp8) {
-                RegionTimer timer(self, LFM25_REGION_FP8_LINEAR);
-                lfm25_fp8_linear_config config;
-                config.m = tokens;
-                config.n = kHidden;
-                config.k = kFfn;
-                config.scale_mode = LFM25_FP8_SCALE_TENSORWIDE;
-                config.output_scale = layer.down.fp8.activation_dequantize * layer.down.fp8.weight_dequantize;
-                LFM25_TRY(lfm25_blaslt_linear_fp8_scaled(self->blaslt, slice_of(self->activated, tokens * kFfn),
-                                                         slice_of(layer.down.fp8.data, kHidden * kFfn),
-                                                         slice_of(self->operator_output, tokens * kHidden), &config));
-            } else {
-                RegionTimer timer(self, LFM25_REGION_BF16_LINEAR);
-                LFM25_TRY(lfm25_blaslt_linear_bf16(self->blaslt, slice_of(self->activated, tokens * kFfn),
-                                                   slice_of(layer.down.bf16, kHidden * kFfn),
-                                                   slice_of(self->operator_output, tokens * kHidden), tokens, kHidden,
-                                                   kFfn));
-            }
-        } else {
-        LFM25_TRY(linear_decode(self, layer.gate_up, self->normalized, self->wide, tokens, use_fp8, gate_up_fp8));
-        if (use_fp8 && layer.down.fp8.data != nullptr) {
-            RegionTimer timer(self, LFM25_REGION_FP8_LINEAR);
-            LFM25_TRY(lfm25_silu_mul_packed_bf16_to_e4m3(stream, slice_of(self->wide, tokens * 2 * kFfn),
-                                                         slice_of(self->fp8_input, self->maximum_tokens * kFfn),
-                                                         tokens, kFfn, layer.down.fp8.activation_quantize));
-            lfm25_fp8_linear_config config;
-            config.m = tokens;
-            config.n = kHidden;
-            config.k = kFfn;
-            config.scale_mode = LFM25_FP8_SCALE_TENSORWIDE;
-            config.output_scale = layer.down.fp8.activation_dequantize * layer.down.fp8.weight_dequantize;
-            LFM25_TRY(lfm25_blaslt_linear_fp8_scaled(self->blaslt, slice_of(self->fp8_input, tokens * kFfn),
-                                                     slice_of(layer.down.fp8.data, kHidden * kFfn),
-                                                     slice_of(self->operator_output, tokens * kHidden), &config));
-        } else {
-            RegionTimer timer(self, LFM25_REGION_BF16_LINEAR);
-            LFM25_TRY(lfm25_silu_mul_packed_bf16(stream, slice_of(self->wide, tokens * 2 * kFfn),
-                                                 slice_of(self->activated, tokens * kFfn), tokens, kFfn));
-            if (layer.down.bf16 == nullptr) {
-                return lfm25::report_error(LFM25_ERR_NULL_POINTER, "Down site has no BF16 weights resident");
-            }
-            LFM25_TRY(lfm25_blaslt_linear_bf16(self->blaslt, slice_of(self->activated, tokens * kFfn),
-                                               slice_of(layer.down.bf16, kHidden * kFfn),
-                                               slice_of(self->operator_output, tokens * kHidden), tokens, kHidden,
-                                               kFfn));
-        }
-        }
+        LFM25_TRY(feed_forward(self, layer, tokens, use_fp8, gate_up_fp8));
 
         const bool last_layer = index + 1 == model->num_layers;
         const void* next_norm = last_layer ? model->final_norm : model->layers[index + 1].operator_norm;
@@ -584,9 +597,8 @@ int32_t forward_ragged(lfm25_decode_executor* self, const lfm25_model* model, co
             LFM25_TRY(linear_decode(self, layer.conv_output, self->post_operator, self->operator_output, tokens,
                                     use_fp8));
         } else {
-            LFM25_TRY(linear_decode(self, layer.query, self->normalized, self->query, tokens, use_fp8));
-            LFM25_TRY(linear_decode(self, layer.key, self->normalized, self->key, tokens, use_fp8));
-            LFM25_TRY(linear_decode(self, layer.value, self->normalized, self->value, tokens, use_fp8));
+            bool packed_qkv = false;
+            LFM25_TRY(project_qkv(self, layer, tokens, use_fp8, &packed_qkv));
             const size_t cache_elements = model->num_pages * 8 * 16 * 64;
             lfm25_qk_postprocess_launch post;
             post.page_size = 16;
@@ -603,10 +615,7 @@ int32_t forward_ragged(lfm25_decode_executor* self, const lfm25_model* model, co
             post.num_tokens = tokens;
             post.num_pages = model->num_pages;
             post.eps = model->norm_eps;
-            {
-                RegionTimer timer(self, LFM25_REGION_APPEND);
-                LFM25_TRY(lfm25_qk_norm_rope_kv_write_decode(stream, &post));
-            }
+            LFM25_TRY(append_qkv(self, post, packed_qkv));
             const size_t decode_tokens = batch->num_decode_segments;
             const lfm25_slice tables_slice =
                 slice_of(batch->block_tables, batch->block_table_stride * batch->block_table_rows);
@@ -689,33 +698,7 @@ int32_t forward_ragged(lfm25_decode_executor* self, const lfm25_model* model, co
                 gate_up_fp8 ? layer.gate_up.fp8.activation_quantize : 1.0f);
         }
         if (status != cudaSuccess) return cuda_failure(status, "residual_rms_norm launch failed");
-        LFM25_TRY(linear_decode(self, layer.gate_up, self->normalized, self->wide, tokens, use_fp8, gate_up_fp8));
-        if (use_fp8 && layer.down.fp8.data != nullptr) {
-            RegionTimer timer(self, LFM25_REGION_FP8_LINEAR);
-            LFM25_TRY(lfm25_silu_mul_packed_bf16_to_e4m3(stream, slice_of(self->wide, tokens * 2 * kFfn),
-                                                         slice_of(self->fp8_input, self->maximum_tokens * kFfn),
-                                                         tokens, kFfn, layer.down.fp8.activation_quantize));
-            lfm25_fp8_linear_config config;
-            config.m = tokens;
-            config.n = kHidden;
-            config.k = kFfn;
-            config.scale_mode = LFM25_FP8_SCALE_TENSORWIDE;
-            config.output_scale = layer.down.fp8.activation_dequantize * layer.down.fp8.weight_dequantize;
-            LFM25_TRY(lfm25_blaslt_linear_fp8_scaled(self->blaslt, slice_of(self->fp8_input, tokens * kFfn),
-                                                     slice_of(layer.down.fp8.data, kHidden * kFfn),
-                                                     slice_of(self->operator_output, tokens * kHidden), &config));
-        } else {
-            RegionTimer timer(self, LFM25_REGION_BF16_LINEAR);
-            LFM25_TRY(lfm25_silu_mul_packed_bf16(stream, slice_of(self->wide, tokens * 2 * kFfn),
-                                                 slice_of(self->activated, tokens * kFfn), tokens, kFfn));
-            if (layer.down.bf16 == nullptr) {
-                return lfm25::report_error(LFM25_ERR_NULL_POINTER, "Down site has no BF16 weights resident");
-            }
-            LFM25_TRY(lfm25_blaslt_linear_bf16(self->blaslt, slice_of(self->activated, tokens * kFfn),
-                                               slice_of(layer.down.bf16, kHidden * kFfn),
-                                               slice_of(self->operator_output, tokens * kHidden), tokens, kHidden,
-                                               kFfn));
-        }
+        LFM25_TRY(feed_forward(self, layer, tokens, use_fp8, gate_up_fp8));
         const bool last_layer = index + 1 == model->num_layers;
         const void* next_norm = last_layer ? model->final_norm : model->layers[index + 1].operator_norm;
         {
