@@ -237,6 +237,27 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float out;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(out) : "f"(a), "f"(b), "f"(c));
+    return out;
+}
+
+// Two f32 values at a time, each rounded as by itself: the packed instructions of sm_100 halve what the issue slots see.
+__device__ __forceinline__ float2 add_two(float2 a, float2 b) {
+    float2 out;
+    asm("{\n.reg .b64 x, y;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nadd.rn.f32x2 x, x, y;\nmov.b64 {%0, %1}, x;\n}"
+        : "=f"(out.x), "=f"(out.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return out;
+}
+__device__ __forceinline__ float2 fma_two(float2 a, float b, float c) {      // a * b + c, b and c for both
+    float2 out;
+    asm("{\n.reg .b64 x, y, z;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %4};\nmov.b64 z, {%5, %5};\nfma.rn.f32x2 x, x, y, z;\n"
+        "mov.b64 {%0, %1}, x;\n}"
+        : "=f"(out.x), "=f"(out.y) : "f"(a.x), "f"(a.y), "f"(b), "f"(c));
+    return out;
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float low, float high) {
     const __nv_bfloat162 pair = __floats2bfloat162_rn(low, high);
     return *reinterpret_cast<const uint32_t*>(&pair);
