@@ -1,11 +1,17 @@
 // Decode attention of the layer stack for bf16 activations: one query token per sequence, any grouping of up to 16
 // query heads per key/value head, query/key and value sizes up to 256, an optional chunk mask.
 //
-// One CTA per token, key/value head and split of the visible pages; its four warps take pages in turn, each through a
+// One CTA per token, key/value head and split of the visible pages; its warps take pages in turn, each through a
 // ring of its own that TMA fills (one box of 64 dimensions x 16 keys per copy, 128-byte swizzle).  A page is 16 keys of
-// one head: S = Q K^T and O += P V are mma.sync tiles whose 16 rows are the query heads of the group.  The weights enter
-// the second product as a sum of two bf16 values (16 significant bits); maximum, sum and accumulators are f32.  The four
-// warps merge through shared memory, the splits of a token through the distributed shared memory of their cluster.
+// one head, the rows of S^T = K Q^T and the contracted index of O^T += V^T P^T, mma.sync tiles whose 8 columns are the query
+// heads of the group (two tiles beyond 8): with the heads as rows a group of four left three quarters of them empty.  The
+// weights turn from rows into columns by movmatrix and enter the second product as a sum of two bf16 values (16 significant
+// bits); maximum, sum and accumulators are f32.  The warps merge through shared memory, the splits of a token through the
+// distributed shared memory of their cluster.
+//
+// Bound by the latency of a page in a warp until the memory's rate is reached.  32 tokens, 32 query heads on 8 key/value heads of
+// 64, us with four warps and the heads as rows, and now: contexts of 128 to 4096 48.4 / 31.3 (the longest decides), all 4096
+// 57.1 / 46.2 (5.8 TB/s), all 1100 19.0 / 11.7; 24 tokens of 100 to 4000 on 2 heads of 128 21.5 / 16.8.
 #include <cooperative_groups.h>
 #include <math.h>
 
@@ -22,15 +28,19 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr uint32_t kWarps = 4;
-constexpr uint32_t kThreads = kWarps * 32;
 constexpr uint32_t kBoxBytes = kPageSize * 128;   // 16 keys x 64 dimensions
 constexpr uint32_t kGroupRows = 16;
 
 template <uint32_t KC, uint32_t VC>
 struct Layout {
+    // Many warps with short rings, taken two pages at a time: 96 KiB of ring, two CTAs per SM.  32 tokens of 128 to 4096 keys,
+    // 8 key/value heads of 64, by (warps, stages, pages at a time): (4, 4, 1) 53 us, (4, 6, 3) 42, (6, 4, 2) 37, (8, 3, 3) 34,
+    // (12, 2, 2) 31.
+    static constexpr uint32_t kWarps = KC + VC <= 2 ? 12 : (KC + VC <= 4 ? 6 : 4);
+    static constexpr uint32_t kThreads = kWarps * 32;
     static constexpr uint32_t kStageBytes = (KC + VC) * kBoxBytes;
-    static constexpr uint32_t kStages = KC + VC <= 2 ? 4 : (KC + VC <= 4 ? 3 : 2);
+    static constexpr uint32_t kStages = 2;
+    static constexpr uint32_t kPages = KC + VC <= 4 ? 2 : 1;        // that a warp takes at a time
     static constexpr uint32_t kRingBytes = kWarps * kStages * kStageBytes;
     static constexpr uint32_t kColumns = 64 * VC;
     // the warps' partial results reuse the ring once every page has been consumed
@@ -59,11 +69,19 @@ struct Params {
     uint64_t wait_limit;
 };
 
-template <uint32_t KC, uint32_t VC>
-__global__ void __launch_bounds__(kThreads)
+// The 8 x 8 matrix of 16-bit values that a warp holds, row g of it in the lanes 4 g .. 4 g + 3, with rows and columns swapped.
+__device__ __forceinline__ uint32_t transposed_8x8(uint32_t pair) {
+    uint32_t out;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(out) : "r"(pair));
+    return out;
+}
+
+template <uint32_t KC, uint32_t VC, uint32_t TILES>
+__global__ void __launch_bounds__(Layout<KC, VC>::kThreads)
 stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const __grid_constant__ CUtensorMap value_map,
                               const Params p) {
     using L = Layout<KC, VC>;
+    constexpr uint32_t kWarps = L::kWarps, kThreads = L::kThreads;
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31;
     extern __shared__ uint8_t decode_smem[];
@@ -141,54 +159,78 @@ stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const
     uint32_t issued = 0;
     for (; issued < L::kStages && issued < count; ++issued) issue(issued);
 
-    // query fragments: row = head of the group, times nothing (the scale is applied to the f32 scores)
-    const uint32_t row0 = lane >> 2;
+    // query fragments: column = head of the group, times nothing (the scale is applied to the f32 scores)
+    const uint32_t g = lane >> 2;
     const uint32_t pair = (lane & 3) * 2;
-    uint32_t query[KC * 4][4];
+    uint32_t query[KC * 4][TILES][2];
     const __nv_bfloat16* query_rows = p.query + (token * p.shape.heads + static_cast<size_t>(kv_head) * group) * p.shape.dim;
 #pragma unroll
     for (uint32_t ks = 0; ks < KC * 4; ++ks) {
 #pragma unroll
-        for (uint32_t part = 0; part < 4; ++part) {
-            const uint32_t row = row0 + (part & 1) * 8;
-            const uint32_t dim = ks * 16 + pair + (part >> 1) * 8;
-            query[ks][part] = row < group && dim < p.shape.dim
-                                  ? *reinterpret_cast<const uint32_t*>(query_rows + row * p.shape.dim + dim)
-                                  : 0u;
+        for (uint32_t tile = 0; tile < TILES; ++tile) {
+#pragma unroll
+            for (uint32_t part = 0; part < 2; ++part) {
+                const uint32_t head = tile * 8 + g;
+                const uint32_t dim = ks * 16 + pair + part * 8;
+                query[ks][tile][part] = head < group && dim < p.shape.dim
+                                            ? *reinterpret_cast<const uint32_t*>(query_rows + head * p.shape.dim + dim)
+                                            : 0u;
+            }
         }
     }
 
-    float out[VC * 8][4];
+    // [16 value dimensions][8 heads]: dimensions g and g + 8, heads 2 (lane % 4) and the next
+    float out[VC * 4][TILES][4];
 #pragma unroll
-    for (uint32_t n = 0; n < VC * 8; ++n) {
+    for (uint32_t m = 0; m < VC * 4; ++m) {
 #pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) out[n][i] = 0.0f;
+        for (uint32_t tile = 0; tile < TILES; ++tile) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) out[m][tile][i] = 0.0f;
+        }
     }
-    float top[2] = {-INFINITY, -INFINITY};
-    float sum[2] = {0.0f, 0.0f};
+    float top[TILES][2], sum[TILES][2];              // of the lane's two heads; a sum covers its own keys
+#pragma unroll
+    for (uint32_t tile = 0; tile < TILES; ++tile) {
+        top[tile][0] = top[tile][1] = -INFINITY;
+        sum[tile][0] = sum[tile][1] = 0.0f;
+    }
     const float scale_log2 = p.shape.scale * kLog2e;
     bool ok = true;
     uint32_t waited = 0;
-    for (uint32_t index = 0; index < count; ++index) {
-        const uint32_t stage = index % L::kStages;
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar + 8 * stage, (index / L::kStages) & 1, p.wait_limit))) {
-            ok = false;
-            break;
-        }
-        waited = index + 1;
-        const uint32_t key_base = ring + stage * L::kStageBytes;
-        const uint32_t value_base = key_base + KC * kBoxBytes;
-        const uint32_t page_first = (first_page + mine + index * stride) * kPageSize;
-        if (usable >> stage & 1u) {
-            float scores[2][4] = {};
+    for (uint32_t index = 0; index < count; index += L::kPages) {
+        // keys g and g + 8 of a page, the lane's two heads
+        float scores[L::kPages][TILES][4];
+        bool there[L::kPages];
+#pragma unroll
+        for (uint32_t j = 0; j < L::kPages; ++j) {
+            const uint32_t stage = (index + j) % L::kStages;
+            there[j] = index + j < count;
+            if (there[j]) {
+                ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(bar + 8 * stage, ((index + j) / L::kStages) & 1, p.wait_limit));
+                if (!ok) break;
+                waited = index + j + 1;
+                there[j] = usable >> stage & 1u;
+            }
+#pragma unroll
+            for (uint32_t tile = 0; tile < TILES; ++tile) {
+#pragma unroll
+                for (uint32_t i = 0; i < 4; ++i) scores[j][tile][i] = there[j] ? 0.0f : -INFINITY;
+            }
+            if (!there[j]) continue;
+            const uint32_t key_base = ring + stage * L::kStageBytes;
+            const uint32_t value_base = key_base + KC * kBoxBytes;
+            const uint32_t page_first = (first_page + mine + (index + j) * stride) * kPageSize;
 #pragma unroll
             for (uint32_t ks = 0; ks < KC * 4; ++ks) {
-                const uint32_t key = (lane >> 4) * 8 + (lane & 7);
-                const uint32_t part = (ks & 3) * 2 + (lane >> 3 & 1);
-                uint32_t b0, b1, b2, b3;
-                ldmatrix_x4(key_base + (ks >> 2) * kBoxBytes + key * 128 + ((part ^ (key & 7)) << 4), b0, b1, b2, b3);
-                mma_bf16_16816(scores[0], query[ks][0], query[ks][1], query[ks][2], query[ks][3], b0, b1);
-                mma_bf16_16816(scores[1], query[ks][0], query[ks][1], query[ks][2], query[ks][3], b2, b3);
+                const uint32_t key = lane & 15;
+                const uint32_t part = (ks & 3) * 2 + (lane >> 4);
+                uint32_t a0, a1, a2, a3;
+                ldmatrix_x4(key_base + (ks >> 2) * kBoxBytes + key * 128 + ((part ^ (key & 7)) << 4), a0, a1, a2, a3);
+#pragma unroll
+                for (uint32_t tile = 0; tile < TILES; ++tile) {
+                    mma_bf16_16816(scores[j][tile], a0, a1, a2, a3, query[ks][tile][0], query[ks][tile][1]);
+                }
             }
             const bool whole = page_first >= first && page_first + kPageSize - 1 <= position;
             if (!whole) {
@@ -206,73 +248,96 @@ stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const
                     __syncwarp();
                 }
 #pragma unroll
-                for (uint32_t n = 0; n < 2; ++n) {
+                for (uint32_t i = 0; i < 4; ++i) {
+                    const uint32_t key = page_first + g + (i >> 1) * 8;
+                    if (key < first || key > position) {
 #pragma unroll
-                    for (uint32_t i = 0; i < 4; ++i) {
-                        const uint32_t key = page_first + n * 8 + pair + (i & 1);
-                        if (key < first || key > position) scores[n][i] = -INFINITY;
+                        for (uint32_t tile = 0; tile < TILES; ++tile) scores[j][tile][i] = -INFINITY;
                     }
                 }
             }
-            float rescale[2];
+        }
+        if (!ok) break;
+        float rescale[TILES][2];
+        uint32_t high[L::kPages][TILES][2], low[L::kPages][TILES][2];        // [8 keys], turned into columns
+        bool same = true;
 #pragma unroll
-            for (uint32_t r = 0; r < 2; ++r) {
-                float best = fmaxf(fmaxf(scores[0][2 * r], scores[0][2 * r + 1]),
-                                   fmaxf(scores[1][2 * r], scores[1][2 * r + 1]));
-                best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, 1));
-                best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, 2));
-                const float now = fmaxf(top[r], best);
+        for (uint32_t tile = 0; tile < TILES; ++tile) {
+            float best[2];
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+                best[h] = fmaxf(scores[0][tile][h], scores[0][tile][2 + h]);
+#pragma unroll
+                for (uint32_t j = 1; j < L::kPages; ++j) best[h] = max3(best[h], scores[j][tile][h], scores[j][tile][2 + h]);
+            }
+#pragma unroll
+            for (uint32_t delta = 4; delta < 32; delta <<= 1) {
+#pragma unroll
+                for (uint32_t h = 0; h < 2; ++h) best[h] = fmaxf(best[h], __shfl_xor_sync(0xffffffffu, best[h], delta));
+            }
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+                const float now = fmaxf(top[tile][h], best[h]);
                 const float base = now == -INFINITY ? 0.0f : now;
-                rescale[r] = fast_exp2((top[r] - base) * scale_log2);
+                rescale[tile][h] = fast_exp2((top[tile][h] - base) * scale_log2);
                 const float offset = -base * scale_log2;
                 float total = 0.0f;
 #pragma unroll
-                for (uint32_t n = 0; n < 2; ++n) {
-#pragma unroll
-                    for (uint32_t i = 0; i < 2; ++i) {
-                        const float weight = fast_exp2(fmaf(scores[n][2 * r + i], scale_log2, offset));
-                        scores[n][2 * r + i] = weight;
-                        total += weight;
-                    }
+                for (uint32_t j = 0; j < L::kPages; ++j) {
+                    scores[j][tile][h] = fast_exp2(fmaf(scores[j][tile][h], scale_log2, offset));
+                    scores[j][tile][2 + h] = fast_exp2(fmaf(scores[j][tile][2 + h], scale_log2, offset));
+                    total += scores[j][tile][h] + scores[j][tile][2 + h];
                 }
-                sum[r] = fmaf(sum[r], rescale[r], total);
-                top[r] = now;
+                sum[tile][h] = fmaf(sum[tile][h], rescale[tile][h], total);
+                top[tile][h] = now;
+                same = same && rescale[tile][h] == 1.0f;
             }
-            if (!__all_sync(0xffffffffu, rescale[0] == 1.0f && rescale[1] == 1.0f)) {
 #pragma unroll
-                for (uint32_t n = 0; n < VC * 8; ++n) {
-                    out[n][0] *= rescale[0];
-                    out[n][1] *= rescale[0];
-                    out[n][2] *= rescale[1];
-                    out[n][3] *= rescale[1];
+            for (uint32_t j = 0; j < L::kPages; ++j) {
+#pragma unroll
+                for (uint32_t part = 0; part < 2; ++part) {
+                    const float a = scores[j][tile][2 * part], b = scores[j][tile][2 * part + 1];
+                    const uint32_t both = pack_bf16x2(a, b);
+                    const float2 rounded = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&both));
+                    high[j][tile][part] = transposed_8x8(both);
+                    low[j][tile][part] = transposed_8x8(pack_bf16x2(a - rounded.x, b - rounded.y));
                 }
             }
-            uint32_t high[4], low[4];
+        }
+        if (!__all_sync(0xffffffffu, same)) {
 #pragma unroll
-            for (uint32_t part = 0; part < 4; ++part) {
-                const float a = scores[part >> 1][(part & 1) * 2];
-                const float b = scores[part >> 1][(part & 1) * 2 + 1];
-                high[part] = pack_bf16x2(a, b);
-                const float2 rounded = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&high[part]));
-                low[part] = pack_bf16x2(a - rounded.x, b - rounded.y);
+            for (uint32_t m = 0; m < VC * 4; ++m) {
+#pragma unroll
+                for (uint32_t tile = 0; tile < TILES; ++tile) {
+#pragma unroll
+                    for (uint32_t i = 0; i < 4; ++i) out[m][tile][i] *= rescale[tile][i & 1];
+                }
             }
+        }
 #pragma unroll
-            for (uint32_t n = 0; n < VC * 4; ++n) {     // 16 value dimensions at a time
-                const uint32_t key = (lane >> 3 & 1) * 8 + (lane & 7);
-                const uint32_t part = (n & 3) * 2 + (lane >> 4);
-                uint32_t b0, b1, b2, b3;
-                ldmatrix_x4_trans(value_base + (n >> 2) * kBoxBytes + key * 128 + ((part ^ (key & 7)) << 4), b0, b1, b2,
-                                  b3);
-                mma_bf16_16816(out[2 * n], high[0], high[1], high[2], high[3], b0, b1);
-                mma_bf16_16816(out[2 * n + 1], high[0], high[1], high[2], high[3], b2, b3);
-                mma_bf16_16816(out[2 * n], low[0], low[1], low[2], low[3], b0, b1);
-                mma_bf16_16816(out[2 * n + 1], low[0], low[1], low[2], low[3], b2, b3);
+        for (uint32_t j = 0; j < L::kPages; ++j) {
+            if (!there[j]) continue;
+            const uint32_t value_base = ring + (index + j) % L::kStages * L::kStageBytes + KC * kBoxBytes;
+#pragma unroll
+            for (uint32_t m = 0; m < VC * 4; ++m) {     // 16 value dimensions at a time
+                const uint32_t key = (lane >> 4) * 8 + (lane & 7);
+                const uint32_t part = (m & 3) * 2 + (lane >> 3 & 1);
+                uint32_t a0, a1, a2, a3;
+                ldmatrix_x4_trans(value_base + (m >> 2) * kBoxBytes + key * 128 + ((part ^ (key & 7)) << 4), a0, a1, a2, a3);
+#pragma unroll
+                for (uint32_t tile = 0; tile < TILES; ++tile) {
+                    mma_bf16_16816(out[m][tile], a0, a1, a2, a3, high[j][tile][0], high[j][tile][1]);
+                    mma_bf16_16816(out[m][tile], a0, a1, a2, a3, low[j][tile][0], low[j][tile][1]);
+                }
             }
         }
         __syncwarp();
-        if (issued < count) {
-            issue(issued);
-            ++issued;
+#pragma unroll
+        for (uint32_t j = 0; j < L::kPages; ++j) {
+            if (issued < count) {
+                issue(issued);
+                ++issued;
+            }
         }
     }
     if (!ok) {
@@ -287,23 +352,32 @@ stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const
 
     // ---- warps of the CTA
 #pragma unroll
-    for (uint32_t r = 0; r < 2; ++r) {
-        sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
-        sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
+    for (uint32_t tile = 0; tile < TILES; ++tile) {
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+#pragma unroll
+            for (uint32_t delta = 4; delta < 32; delta <<= 1) {
+                sum[tile][h] += __shfl_xor_sync(0xffffffffu, sum[tile][h], delta);
+            }
+        }
     }
     __syncthreads();          // every ring is drained
 #pragma unroll
-    for (uint32_t r = 0; r < 2; ++r) {
-        const uint32_t row = row0 + r * 8;
-        if (row < group) {
-            if ((lane & 3) == 0) {
-                warp_top[warp * kGroupRows + row] = top[r];
-                warp_sums[warp * kGroupRows + row] = sum[r];
-            }
-            float* target = partial + (warp * kGroupRows + row) * L::kColumns + pair;
+    for (uint32_t tile = 0; tile < TILES; ++tile) {
 #pragma unroll
-            for (uint32_t n = 0; n < VC * 8; ++n) {
-                *reinterpret_cast<float2*>(target + n * 8) = make_float2(out[n][2 * r], out[n][2 * r + 1]);
+        for (uint32_t h = 0; h < 2; ++h) {
+            const uint32_t row = tile * 8 + pair + h;
+            if (row < group) {
+                if (g == 0) {
+                    warp_top[warp * kGroupRows + row] = top[tile][h];
+                    warp_sums[warp * kGroupRows + row] = sum[tile][h];
+                }
+                float* target = partial + (warp * kGroupRows + row) * L::kColumns + g;
+#pragma unroll
+                for (uint32_t m = 0; m < VC * 4; ++m) {
+                    target[m * 16] = out[m][tile][h];
+                    target[m * 16 + 8] = out[m][tile][2 + h];
+                }
             }
         }
     }
@@ -364,14 +438,14 @@ stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const
     cluster.sync();           // nobody leaves while its results are being read
 }
 
-template <uint32_t KC, uint32_t VC>
-cudaError_t launch_sized(cudaStream_t stream, const StackAttentionLaunch& launch, uint32_t splits) {
+template <uint32_t KC, uint32_t VC, uint32_t TILES>
+cudaError_t launch_tiles(cudaStream_t stream, const StackAttentionLaunch& launch, uint32_t splits) {
     using L = Layout<KC, VC>;
     CUtensorMap key_map, value_map;
     if (!make_page_map(&key_map, launch, false) || !make_page_map(&value_map, launch, true)) {
         return cudaErrorInvalidValue;
     }
-    const auto kernel = stack_attention_decode_kernel<KC, VC>;
+    const auto kernel = stack_attention_decode_kernel<KC, VC, TILES>;
     const cudaError_t status = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                     static_cast<int>(L::kSharedBytes));
@@ -391,8 +465,14 @@ cudaError_t launch_sized(cudaStream_t stream, const StackAttentionLaunch& launch
     params.splits = splits;
     params.wait_limit = wait_limit_ns();
     const size_t blocks = launch.decode_tokens * launch.shape.kv_heads * splits;
-    return launch_kernel(kernel, static_cast<unsigned int>(blocks), kThreads, L::kSharedBytes, stream, splits, key_map,
+    return launch_kernel(kernel, static_cast<unsigned int>(blocks), L::kThreads, L::kSharedBytes, stream, splits, key_map,
                          value_map, params);
+}
+
+template <uint32_t KC, uint32_t VC>
+cudaError_t launch_sized(cudaStream_t stream, const StackAttentionLaunch& launch, uint32_t splits) {
+    return launch.shape.heads / launch.shape.kv_heads <= 8 ? launch_tiles<KC, VC, 1>(stream, launch, splits)
+                                                           : launch_tiles<KC, VC, 2>(stream, launch, splits);
 }
 
 template <uint32_t KC>
@@ -406,12 +486,12 @@ cudaError_t launch_keys(cudaStream_t stream, const StackAttentionLaunch& launch,
 
 }  // namespace
 
-// CTAs per token and head over the key axis: enough to fill the machine twice while every warp keeps two pages.
+// CTAs per token and head over the key axis: enough to fill the machine twice while a CTA keeps eight pages.
 uint32_t stack_attention_splits(const StackAttentionShape& shape, size_t tokens, size_t context) {
     const size_t visible = shape.chunk != 0 ? std::min<size_t>(context, shape.chunk) : context;
     const size_t pages = (visible + kPageSize - 1) / kPageSize;
     uint32_t splits = 1;
-    while (splits < 8 && tokens * shape.kv_heads * splits * 2 <= 2 * 148 && pages >= 2 * kWarps * splits * 2) splits *= 2;
+    while (splits < 8 && tokens * shape.kv_heads * splits * 2 <= 2 * 148 && pages >= 16 * splits) splits *= 2;
     return splits;
 }
 

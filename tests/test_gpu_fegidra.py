@@ -99,6 +99,14 @@ def test_decode_attention_long_contexts(device, library_option, heads, kv_heads,
     assert cases.relative_error(results[0], results[1]).max() < 1e-2
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim,copies", [(8, 1, 64, 1), (9, 1, 64, 1), (16, 1, 64, 2), (24, 2, 128, 1), (16, 1, 72, 1),
+                                                       (6, 2, 136, 1), (13, 1, 256, 1)])
+def test_decode_attention_groups(device, library_option, heads, kv_heads, dim, copies):
+    """The same with groups of eight heads and less, which are one tile of columns, and beyond, with heads of one to four
+    pieces of 64: every number of warps, pages at a time and tiles of the decode kernel."""
+    test_decode_attention_long_contexts(device, library_option, heads, kv_heads, dim, copies)
+
+
 @pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("heads,dim,rank", [(3, 16, 5), (2, 64, 16), (1, 24, 1), (2, 128, 33), (1, 80, 3), (2, 160, 8),
                                             (1, 256, 64), (1, 10, 7), (2, 128, 700)])
