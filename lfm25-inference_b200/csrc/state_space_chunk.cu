@@ -4,8 +4,10 @@
 // With a_t = exp(-rate dt_t), A_t = a_1 ... a_t inside a chunk of 64 tokens and S the state before it,
 //     y_t = A_t S^T C_t + sum_{s <= t} (A_t / A_s) dt_s (C_t . B_s) x_s + skip x_t
 //     S  <- A_64 S + sum_s (A_64 / A_s) dt_s B_s x_s^T
-// A CTA owns one segment, one head and 64 columns of its state, and walks the segment chunk by chunk: the state stays in
-// f32 accumulators (its product B^T x is added there), C B^T and C S share the loads of C.  x, B and C are bf16 already;
+// A CTA owns one segment, one head and 64 columns of its state, and walks the segment chunk by chunk.  Four warps carry 16
+// columns of the state each, transposed, in f32 accumulators: these are operands of C S as they are, and x^T B is added to
+// them.  Four more warps copy the next chunk and form the triangle of weights from C B^T, which does not wait for the state,
+// and leave it in the order of the operands.  The two sides meet twice per chunk.  x, B and C are bf16 already;
 // everything that the recurrence multiplies them with -- the decays, the triangle of weights, the state itself -- enters
 // the tensor core as a sum of two bf16 values (16 significant bits).  The logarithms of the A_t are summed in double and
 // kept as two floats, so that the ratio of two neighbours behind a long decay is exact; one kernel forms them for all heads of
@@ -16,10 +18,12 @@
 // of the pieces before it.  Only the order of the f32 sums over the state changes; state against float64 (4096 tokens, 64 heads
 // with 128 rows; rates from 2^-9 to 20, 1, 0.02): 5.0e-6, 2.5e-6, 3.3e-6, from end to end 6.7e-6, 2.5e-6, 3.3e-6.
 //
-// Bound by the latency of a chunk's stages (tensor pipe 33 % busy with two CTAs per SM), so the shapes in use have strides
-// known to the compiler (45 instead of 60 us for 8 x 512 tokens of 32 heads with 64 state rows, where the index arithmetic
-// was a fifth of the instructions).  One segment of 4096 tokens, 64 heads with 128 state rows: 6 us factors, 35 us
-// contributions, 133 us pieces; one CTA per head from end to end: 502 us on 64 SMs.
+// Bound by the tensor cores' legacy products where two CTAs share an SM (336 of 16x8x16 per chunk and SM quarter each, eight
+// cycles apiece, of 7300 cycles that two chunks take), and by the chain C S, outputs, x^T B of one warp elsewhere (5400 cycles a
+// chunk).  Shapes in use have strides known to the compiler.  One segment of 4096 tokens, 64 heads with 128 state rows: 6 us
+// factors, 30 us contributions, 89 us pieces; one CTA per head from end to end: 295 us on 64 SMs.  8 x 512 tokens of 32 heads
+// with 64 state rows: 30 us.  With all eight warps on one stage after another and the state and weighted x between them in shared
+// memory it was 35 + 133 us, 301 and 45 us.
 #include <algorithm>
 #include <type_traits>
 
@@ -35,7 +39,6 @@ constexpr uint32_t kTokens = 64;
 constexpr uint32_t kColumns = 64;
 constexpr uint32_t kPad = 8;                            // elements behind each row: conflict-free ldmatrix
 constexpr uint32_t kColumnPitch = kColumns + kPad;
-constexpr size_t kSharedLimit = 227 * 1024;
 
 // What a token contributes to a head: log2 A_t as high + low, dt_t, (A_64 / A_t) dt_t
 struct __align__(16) TokenFactors {
@@ -48,14 +51,14 @@ enum class Pass {
     kPieces,        // every piece: outputs, the state behind the last one
 };
 
-// Bytes of one buffer of a chunk's B, C and x
-__host__ __device__ constexpr size_t chunk_bytes(uint32_t padded) {
-    return (2 * kTokens * (padded + kPad) + kTokens * kColumnPitch) * 2;
+// Bytes of one buffer of a chunk's B, C (where there are outputs) and x
+__host__ __device__ constexpr size_t chunk_bytes(uint32_t padded, bool outputs) {
+    return ((outputs ? 2 : 1) * kTokens * (padded + kPad) + kTokens * kColumnPitch) * 2;
 }
-constexpr size_t shared_bytes(uint32_t padded, uint32_t buffers, bool outputs) {
-    // state (where there are outputs) and weighted x, both as two bf16 parts
-    return buffers * chunk_bytes(padded) + 2 * ((outputs ? padded : 0) + kTokens) * kColumnPitch * 2 +
-           2 * kTokens * sizeof(TokenFactors);
+constexpr uint32_t kBlocks = 10;                        // 16 x 16 blocks on and below the diagonal of a chunk's weights
+constexpr size_t kWeightBytes = kBlocks * 2 * 32 * 16;  // in two bf16 parts, as operands
+constexpr size_t shared_bytes(uint32_t padded, bool outputs) {
+    return 2 * (chunk_bytes(padded, outputs) + (outputs ? kWeightBytes : 0) + kTokens * sizeof(TokenFactors));
 }
 
 __device__ __forceinline__ void split_pair(float a, float b, uint32_t& high, uint32_t& low) {
@@ -111,23 +114,33 @@ struct PieceArgs {
     uint32_t tokens;               // per piece, a multiple of 64
 };
 
-// UNITS: units of 16 state rows x 32 columns per warp (8 warps).  FULL: the state has exactly that many rows, so that all
-// strides are constants and the loops over them unroll.
+constexpr uint32_t kRoleThreads = kThreads / 2;
+enum : uint32_t { kFullBarrier = 1, kFreeBarrier = 3, kLoadedBarrier = 5 };      // the first two: one per buffer
+
+__device__ __forceinline__ void barrier_sync(uint32_t id, uint32_t threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void barrier_arrive(uint32_t id, uint32_t threads) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Warps 0..3 own the state, warps 4..7 load and weigh.  168 and 88 registers a thread: with 160 and 96 the state's warps spill
+// (8 x 512 tokens 31.9 instead of 30.0 us), 176 and 80 are no faster.
+// UNITS: 64 state rows each.  FULL: the state has exactly that many rows, so that all strides are constants and the loops over
+// them unroll.
 template <int UNITS, Pass PASS, bool FULL>
 __global__ void __launch_bounds__(kThreads, UNITS <= 2 ? 2 : 1)
 state_space_chunk_kernel(const StateSpaceArgs<__nv_bfloat16> args, const PieceArgs pieces, uint32_t column_blocks,
-                         uint32_t padded_rows, uint32_t buffers) {
+                         uint32_t padded_rows) {
+    constexpr uint32_t kTiles = 8 * UNITS;             // of eight state rows
     const uint32_t padded = FULL ? 64 * UNITS : padded_rows;
     extern __shared__ __align__(16) unsigned char chunk_smem[];
     const uint32_t pitch = padded + kPad;
     __nv_bfloat16* tiles = reinterpret_cast<__nv_bfloat16*>(chunk_smem);
-    const uint32_t tile_elements = static_cast<uint32_t>(chunk_bytes(padded) / 2);
-    __nv_bfloat16* state_high = tiles + buffers * tile_elements;        // [padded][columns]
-    __nv_bfloat16* state_low = state_high + padded * kColumnPitch;
-    __nv_bfloat16* input_high =                                         // [tokens][columns]
-        PASS == Pass::kContribute ? state_high : state_low + padded * kColumnPitch;
-    __nv_bfloat16* input_low = input_high + kTokens * kColumnPitch;
-    TokenFactors* factor_tiles = reinterpret_cast<TokenFactors*>(input_low + kTokens * kColumnPitch);   // [2][tokens]
+    const uint32_t tile_elements = static_cast<uint32_t>(chunk_bytes(padded, PASS != Pass::kContribute) / 2);
+    uint4* weights = reinterpret_cast<uint4*>(tiles + 2 * tile_elements);        // [2][block][part][lane]
+    TokenFactors* factor_tiles =                                                 // [2][tokens]
+        reinterpret_cast<TokenFactors*>(weights + (PASS == Pass::kContribute ? 0 : 2 * kBlocks * 2 * 32));
     pdl_launch_dependents();
     pdl_wait();
 
@@ -155,245 +168,316 @@ state_space_chunk_kernel(const StateSpaceArgs<__nv_bfloat16> args, const PieceAr
     if (slot >= args.segments.num_request_slots) {
         return;
     }
-    const uint32_t group = head / (args.heads / args.groups);
     const size_t inner = static_cast<size_t>(args.heads) * args.vdim;
     const uint32_t column0 = block * kColumns;
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t row0 = lane >> 2;
     const uint32_t pair = (lane & 3) * 2;
-    const float skip = __bfloat162float(args.skip[head]);
-    // state between pieces of piece `other` of this segment
-    auto state_between = [&](uint32_t other) {
-        return pieces.states +
-               ((static_cast<size_t>(index - piece + other) * args.heads + head) * column_blocks + block) * args.size * kColumns;
-    };
-    auto decay_between = [&](uint32_t other) -> float& {
-        return pieces.decays[static_cast<size_t>(index - piece + other) * args.heads + head];
+    const auto inputs_of = [&](uint32_t buffer) { return tiles + buffer * tile_elements; };      // B, then C, then x
+    const auto columns_of = [&](uint32_t buffer) {
+        return inputs_of(buffer) + (PASS == Pass::kContribute ? 1 : 2) * kTokens * pitch;
     };
 
-    auto load_chunk = [&](uint32_t first, uint32_t buffer) {
-        __nv_bfloat16* b = tiles + buffer * tile_elements;
-        __nv_bfloat16* c = b + kTokens * pitch;
-        __nv_bfloat16* x = c + kTokens * pitch;
-        const uint32_t vectors = padded / 8;
-        for (uint32_t item = threadIdx.x; item < kTokens * vectors; item += kThreads) {
-            const uint32_t row = item / vectors, n = item % vectors * 8;
-            const bool inside = first + row < end && (FULL || n < args.size);
-            const __nv_bfloat16* source = args.mixed;
-            if (inside) source += static_cast<size_t>(first + row) * args.mixed_pitch + inner + group * args.size + n;
-            copy_async_16(b + row * pitch + n, source, inside);
-            if (PASS != Pass::kContribute) {
-                copy_async_16(c + row * pitch + n, source + (inside ? args.groups * args.size : 0), inside);
-            }
-        }
-        for (uint32_t item = threadIdx.x; item < kTokens * kColumns / 8; item += kThreads) {
-            const uint32_t row = item / (kColumns / 8), v = item % (kColumns / 8) * 8;
-            const bool inside = first + row < end && column0 + v < args.vdim;
-            copy_async_16(x + row * kColumnPitch + v,
-                       args.mixed + (inside ? static_cast<size_t>(first + row) * args.mixed_pitch + head * args.vdim +
-                                                  column0 + v
-                                            : 0),
-                       inside);
-        }
-        if (threadIdx.x < kTokens) {
-            // tokens behind the end weigh nothing (their x is zero), and their decays are the last token's
-            const uint32_t token = first + threadIdx.x < end ? first + threadIdx.x : end - 1;
-            copy_async_16(factor_tiles + (first - begin) / kTokens % 2 * kTokens + threadIdx.x,
-                          pieces.factors + static_cast<size_t>(head) * args.segments.num_tokens + token, true);
-        }
-        copy_async_commit();
-    };
-
-    float* state = state_of(args, slot, head);
-    float held[UNITS][4][4];
-    // calls `visit` with the address of each pair of state values that this thread holds, as rows `row_pitch` apart
-    auto each_pair = [&](float* base, size_t row_pitch, auto&& visit) {
+    if (warp >= kRoleThreads / 32) {
+        // ---- copies, and the weights of each chunk's inputs in its outputs: at most three blocks of 16 x 16 per warp
+        if constexpr (UNITS <= 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+        const uint32_t thread = threadIdx.x - kRoleThreads;
+        const uint32_t weigher = warp - kRoleThreads / 32;
+        const uint32_t group = head / (args.heads / args.groups);
+        // eight threads per row, 16 rows at a time; behind the end and beyond the state's size zeros
+        const uint32_t row = thread / 8, vector = thread % 8 * 8;
+        const __nv_bfloat16* source = args.mixed + static_cast<size_t>(begin + row) * args.mixed_pitch;
+        const size_t first_row = static_cast<size_t>(inner) + group * args.size, second_row = args.groups * args.size;
+        const bool column_inside = column0 + vector < args.vdim;
+        const size_t column = column_inside ? head * args.vdim + column0 + vector : 0;
+        const TokenFactors* source_factors = pieces.factors + static_cast<size_t>(head) * args.segments.num_tokens;
+        const auto load_chunk = [&](uint32_t first, uint32_t buffer) {
+            __nv_bfloat16* b = inputs_of(buffer) + row * pitch + vector;
+            __nv_bfloat16* c = b + kTokens * pitch;
+            __nv_bfloat16* x = columns_of(buffer) + row * kColumnPitch + vector;
 #pragma unroll
-        for (int unit = 0; unit < UNITS; ++unit) {
-            const uint32_t part = warp + 8 * unit;
-            const uint32_t n = part / 2 * 16 + row0;
+            for (uint32_t i = 0; i < kTokens; i += 16) {
+                const bool inside = first + row + i < end;
+                const __nv_bfloat16* at = inside ? source + i * args.mixed_pitch : args.mixed;
 #pragma unroll
-            for (uint32_t tile = 0; tile < 4; ++tile) {
-                const uint32_t v = part % 2 * 32 + tile * 8 + pair;
-#pragma unroll
-                for (uint32_t half = 0; half < 2; ++half) {
-                    if (n + half * 8 < args.size && column0 + v < args.vdim) {
-                        visit(reinterpret_cast<float2*>(base + static_cast<size_t>(n + half * 8) * row_pitch + v),
-                              held[unit][tile][2 * half], held[unit][tile][2 * half + 1]);
+                for (uint32_t n = 0; n < 64 * UNITS; n += 64) {
+                    if (!FULL && n + vector >= padded) continue;
+                    const bool filled = inside && (FULL || n + vector < args.size);
+                    const __nv_bfloat16* from = filled ? at + first_row + n + vector : args.mixed;
+                    copy_async_16(b + i * pitch + n, from, filled);
+                    if (PASS != Pass::kContribute) {
+                        copy_async_16(c + i * pitch + n, filled ? from + second_row : args.mixed, filled);
                     }
                 }
+                copy_async_16(x + i * kColumnPitch, at + (inside ? column : 0), inside && column_inside);
+            }
+            if (thread < kTokens) {
+                // tokens behind the end weigh nothing (their x is zero), and their decays are the last token's
+                const uint32_t token = first + thread < end ? first + thread : end - 1;
+                copy_async_16(factor_tiles + buffer * kTokens + thread, source_factors + token, true);
+            }
+            copy_async_commit();
+            source += kTokens * args.mixed_pitch;
+        };
+        if (begin < end) load_chunk(begin, 0);
+        uint32_t buffer = 0;
+        for (uint32_t first = begin; first < end; first += kTokens, buffer ^= 1) {
+            copy_async_wait<0>();
+            if (PASS != Pass::kContribute) {
+                barrier_sync(kLoadedBarrier, kRoleThreads);
+                const __nv_bfloat16* b = inputs_of(buffer);
+                const __nv_bfloat16* c = b + kTokens * pitch;
+                const TokenFactors* factors = factor_tiles + buffer * kTokens;
+                // blocks (kRow, kFirst) to (kRow, kLast)
+                const auto weigh = [&](auto row_index, auto first_index, auto last_index) {
+                    constexpr uint32_t kRow = decltype(row_index)::value, kFirst = decltype(first_index)::value;
+                    constexpr uint32_t kCount = decltype(last_index)::value + 1 - kFirst;
+                    float products[2 * kCount][4] = {};
+#pragma unroll 4
+                    for (uint32_t k = 0; k < padded; k += 16) {
+                        uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
+                        ldmatrix_x4(smem_u32(c + (kRow * 16 + (lane & 15)) * pitch + k + (lane >> 4) * 8), a0, a1, a2, a3);
+#pragma unroll
+                        for (uint32_t j = 0; j < kCount; ++j) {
+                            ldmatrix_x4(smem_u32(b + ((kFirst + j) * 16 + (lane >> 4) * 8 + (lane & 7)) * pitch + k +
+                                                 (lane >> 3 & 1) * 8),
+                                        b0, b1, b2, b3);
+                            mma_bf16_16816(products[2 * j], a0, a1, a2, a3, b0, b1);
+                            mma_bf16_16816(products[2 * j + 1], a0, a1, a2, a3, b2, b3);
+                        }
+                    }
+                    const float log_high[2] = {factors[kRow * 16 + row0].log_high, factors[kRow * 16 + row0 + 8].log_high};
+                    const float log_low[2] = {factors[kRow * 16 + row0].log_low, factors[kRow * 16 + row0 + 8].log_low};
+                    uint4* target = weights + ((buffer * kBlocks + kRow * (kRow + 1) / 2 + kFirst) * 2) * 32 + lane;
+#pragma unroll
+                    for (uint32_t j = 0; j < kCount; ++j) {
+                        uint32_t high[4], low[4];
+#pragma unroll
+                        for (uint32_t part = 0; part < 2; ++part) {            // 8 tokens s each
+                            const uint32_t s = part * 8 + pair;
+                            const TokenFactors* at = factors + (kFirst + j) * 16 + s;
+                            const TokenFactors from[2] = {at[0], at[1]};
+#pragma unroll
+                            for (uint32_t half = 0; half < 2; ++half) {
+                                float value[2];
+#pragma unroll
+                                for (uint32_t i = 0; i < 2; ++i) {
+                                    const float weight = fast_exp2((log_high[half] - from[i].log_high) +
+                                                                   (log_low[half] - from[i].log_low)) * from[i].step;
+                                    value[i] = kFirst + j != kRow || s + i <= row0 + half * 8
+                                                   ? products[2 * j + part][2 * half + i] * weight
+                                                   : 0.0f;
+                                }
+                                split_pair(value[0], value[1], high[2 * part + half], low[2 * part + half]);
+                            }
+                        }
+                        target[j * 64] = make_uint4(high[0], high[1], high[2], high[3]);
+                        target[j * 64 + 32] = make_uint4(low[0], low[1], low[2], low[3]);
+                    }
+                };
+                const std::integral_constant<uint32_t, 0> zero;
+                const std::integral_constant<uint32_t, 1> one;
+                const std::integral_constant<uint32_t, 2> two;
+                const std::integral_constant<uint32_t, 3> three;
+                if (weigher == 0) {
+                    weigh(zero, zero, zero);
+                    weigh(three, zero, zero);
+                } else if (weigher == 1) {
+                    weigh(one, zero, one);
+                } else if (weigher == 2) {
+                    weigh(two, zero, two);
+                } else {
+                    weigh(three, one, three);
+                }
+            }
+            barrier_arrive(kFullBarrier + buffer, kThreads);
+            if (first + kTokens < end) {
+                if (first != begin) barrier_sync(kFreeBarrier + (buffer ^ 1), kThreads);
+                load_chunk(first + kTokens, buffer ^ 1);
+            }
+        }
+        return;
+    }
+
+    // ---- the state, transposed: 16 columns and all rows per warp
+    if constexpr (UNITS <= 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
+    const float skip = __bfloat162float(args.skip[head]);
+    float* state = state_of(args, slot, head);
+    float held[kTiles][4];
+    const uint32_t own = warp * 16;                    // first column
+    // calls `visit` with the address in the record and the value
+    const auto each_value = [&](auto&& visit) {
+#pragma unroll
+        for (uint32_t tile = 0; tile < kTiles; ++tile) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                const uint32_t n = tile * 8 + pair + (i & 1), v = column0 + own + row0 + (i >> 1) * 8;
+                if (n < args.size && v < args.vdim) visit(state + static_cast<size_t>(n) * args.vdim + v, held[tile][i]);
             }
         }
     };
-    const auto read = [](const float2* at, float& x, float& y) {
-        const float2 value = *at;
-        x = value.x;
-        y = value.y;
-    };
-    const auto write = [](float2* at, float x, float y) { *at = make_float2(x, y); };
+    const auto read = [](const float* at, float& x) { x = *at; };
+    const auto write = [](float* at, float x) { *at = x; };
+    // state between pieces of piece `other` of this segment, in the order of the registers: [warp][tile][lane][4]
+    const auto each_between = [&](uint32_t other, auto&& visit) {
+        float4* base = reinterpret_cast<float4*>(
+                           pieces.states + ((static_cast<size_t>(index - piece + other) * args.heads + head) * column_blocks +
+                                            block) * args.size * kColumns) +
+                       warp * (args.size / 8) * 32 + lane;
 #pragma unroll
-    for (int unit = 0; unit < UNITS; ++unit) {
-#pragma unroll
-        for (uint32_t tile = 0; tile < 4; ++tile) {
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) held[unit][tile][i] = 0.0f;
+        for (uint32_t tile = 0; tile < kTiles; ++tile) {
+            if (tile * 8 < args.size) visit(base + tile * 32, held[tile]);
         }
+    };
+    const auto read_between = [](const float4* at, float (&x)[4]) {
+        const float4 value = *at;
+        x[0] = value.x;
+        x[1] = value.y;
+        x[2] = value.z;
+        x[3] = value.w;
+    };
+    const auto write_between = [](float4* at, const float (&x)[4]) { *at = make_float4(x[0], x[1], x[2], x[3]); };
+    const auto decay_between = [&](uint32_t other) -> float& {
+        return pieces.decays[static_cast<size_t>(index - piece + other) * args.heads + head];
+    };
+#pragma unroll
+    for (uint32_t tile = 0; tile < kTiles; ++tile) {
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) held[tile][i] = 0.0f;
     }
-    if (begin < end) load_chunk(begin, 0);
-    float total_log = 0.0f;                        // of this piece's decay
+    float total_log = 0.0f;                            // of this piece's decay
     if (PASS == Pass::kWhole || last_piece == 0) {
-        each_pair(state + column0, args.vdim, read);
+        each_value(read);
     } else if (PASS == Pass::kContribute) {
         // the first piece takes the state before the segment along and leaves a copy where the last piece's would be:
         // the record is overwritten by whichever CTA of the second pass comes to its end
         if (piece == 0) {
-            each_pair(state + column0, args.vdim, read);
-            each_pair(state_between(last_piece), kColumns, write);
+            each_value(read);
+            each_between(last_piece, write_between);
         }
     } else if (piece == 0) {
-        each_pair(state_between(last_piece), kColumns, read);
+        each_between(last_piece, read_between);
     } else {
-        each_pair(state_between(0), kColumns, read);
+        each_between(0, read_between);
         for (uint32_t other = 1; other < piece; ++other) {
             const float decay = fast_exp2(decay_between(other));
-            each_pair(state_between(other), kColumns, [decay](const float2* at, float& x, float& y) {
-                const float2 value = *at;
-                x = fmaf(x, decay, value.x);
-                y = fmaf(y, decay, value.y);
+            each_between(other, [decay](const float4* at, float (&x)[4]) {
+                const float4 value = *at;
+                x[0] = fmaf(x[0], decay, value.x);
+                x[1] = fmaf(x[1], decay, value.y);
+                x[2] = fmaf(x[2], decay, value.z);
+                x[3] = fmaf(x[3], decay, value.w);
             });
         }
     }
+    const uint32_t columns_left = column0 + own + pair < args.vdim ? args.vdim - column0 - own - pair : 0;
+    __nv_bfloat16* target = args.out + (static_cast<size_t>(begin) + row0) * inner + head * args.vdim + column0 + own + pair;
     uint32_t buffer = 0;
-    for (uint32_t first = begin; first < end; first += kTokens) {
-        copy_async_wait<0>();
-        __syncthreads();
-        if (buffers == 2 && first + kTokens < end) load_chunk(first + kTokens, buffer ^ 1);
-        const __nv_bfloat16* b = tiles + buffer * tile_elements;
+    for (uint32_t first = begin; first < end; first += kTokens, buffer ^= 1) {
+        barrier_sync(kFullBarrier + buffer, kThreads);
+        const __nv_bfloat16* b = inputs_of(buffer);
         const __nv_bfloat16* c = b + kTokens * pitch;
-        const __nv_bfloat16* x = c + kTokens * pitch;
-        const TokenFactors* factors = factor_tiles + (first - begin) / kTokens % 2 * kTokens;
-        // ---- the state and the weighted inputs as two bf16 parts each
-#pragma unroll
-        for (int unit = 0; unit < UNITS; ++unit) {
-            const uint32_t part = warp + 8 * unit;
-            if (PASS != Pass::kContribute && part / 2 * 16 < padded) {
-#pragma unroll
-                for (uint32_t tile = 0; tile < 4; ++tile) {
-#pragma unroll
-                    for (uint32_t half = 0; half < 2; ++half) {
-                        uint32_t high, low;
-                        split_pair(held[unit][tile][2 * half], held[unit][tile][2 * half + 1], high, low);
-                        const uint32_t row = part / 2 * 16 + row0 + half * 8;
-                        const uint32_t at = row * kColumnPitch + part % 2 * 32 + tile * 8 + pair;
-                        *reinterpret_cast<uint32_t*>(state_high + at) = high;
-                        *reinterpret_cast<uint32_t*>(state_low + at) = low;
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (uint32_t item = threadIdx.x; item < kTokens * kColumns / 8; item += kThreads) {
-            const uint32_t row = item / (kColumns / 8), v = item % (kColumns / 8) * 8;
-            float value[8];
-            load_values<8>(x + row * kColumnPitch + v, value);
-            const float weight = factors[row].into_state;
-            uint32_t high[4], low[4];
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) split_pair(value[2 * i] * weight, value[2 * i + 1] * weight, high[i], low[i]);
-            *reinterpret_cast<uint4*>(input_high + row * kColumnPitch + v) = make_uint4(high[0], high[1], high[2], high[3]);
-            *reinterpret_cast<uint4*>(input_low + row * kColumnPitch + v) = make_uint4(low[0], low[1], low[2], low[3]);
-        }
-        __syncthreads();
-
-        // ---- outputs: 16 tokens x 32 columns per warp
+        const __nv_bfloat16* x = columns_of(buffer) + own;
+        const TokenFactors* factors = factor_tiles + buffer * kTokens;
         if (PASS != Pass::kContribute) {
-            const uint32_t tile_row = warp & 3;
-            const uint32_t half_column = (warp >> 2) * 32;
-            float products[8][4] = {}, carried[4][4] = {};
-#pragma unroll 2
-            for (uint32_t k = 0; k < padded; k += 16) {
-                uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
-                ldmatrix_x4(smem_u32(c + (tile_row * 16 + (lane & 15)) * pitch + k + (lane >> 4) * 8), a0, a1, a2, a3);
+            // ---- from the state: its accumulators are operands as they are
+            float carried[4][2][4] = {};
+            uint32_t tokens[2][4][4];                  // C of 16 state rows, and of the next ones
+            const auto load_tokens = [&](uint32_t q) {
 #pragma unroll
-                for (uint32_t j = 0; j < 4; ++j) {
-                    if (j <= tile_row) {
-                        ldmatrix_x4(smem_u32(b + (j * 16 + (lane >> 4) * 8 + (lane & 7)) * pitch + k + (lane >> 3 & 1) * 8),
-                                    b0, b1, b2, b3);
-                        mma_bf16_16816(products[2 * j], a0, a1, a2, a3, b0, b1);
-                        mma_bf16_16816(products[2 * j + 1], a0, a1, a2, a3, b2, b3);
-                    }
+                for (uint32_t row_tile = 0; row_tile < 4; ++row_tile) {
+                    uint32_t(&a)[4] = tokens[q % 2][row_tile];
+                    ldmatrix_x4(smem_u32(c + (row_tile * 16 + (lane & 15)) * pitch + q * 16 + (lane >> 4) * 8), a[0], a[1], a[2],
+                                a[3]);
                 }
+            };
+            load_tokens(0);
 #pragma unroll
-                for (uint32_t q = 0; q < 2; ++q) {
-                    const uint32_t at = (k + (lane >> 3 & 1) * 8 + (lane & 7)) * kColumnPitch + half_column + q * 16 +
-                                        (lane >> 4) * 8;
-                    ldmatrix_x4_trans(smem_u32(state_high + at), b0, b1, b2, b3);
-                    mma_bf16_16816(carried[2 * q], a0, a1, a2, a3, b0, b1);
-                    mma_bf16_16816(carried[2 * q + 1], a0, a1, a2, a3, b2, b3);
-                    ldmatrix_x4_trans(smem_u32(state_low + at), b0, b1, b2, b3);
-                    mma_bf16_16816(carried[2 * q], a0, a1, a2, a3, b0, b1);
-                    mma_bf16_16816(carried[2 * q + 1], a0, a1, a2, a3, b2, b3);
-                }
-            }
-            const uint32_t t[2] = {tile_row * 16 + row0, tile_row * 16 + row0 + 8};
-            const float log_high[2] = {factors[t[0]].log_high, factors[t[1]].log_high};
-            const float log_low[2] = {factors[t[0]].log_low, factors[t[1]].log_low};
-            float sum[4][4] = {};
-#pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) {
-                if (j > tile_row) {
-                    continue;
-                }
+            for (uint32_t q = 0; q < kTiles / 2; ++q) {
+                if (!FULL && q * 16 >= padded) continue;
+                if (q + 1 < kTiles / 2 && (FULL || (q + 1) * 16 < padded)) load_tokens(q + 1);
                 uint32_t high[4], low[4];
 #pragma unroll
-                for (uint32_t part = 0; part < 2; ++part) {            // 8 tokens s each
-                    const uint32_t s = j * 16 + part * 8 + pair;
-                    const TokenFactors from[2] = {factors[s], factors[s + 1]};
+                for (uint32_t half = 0; half < 2; ++half) {        // of the columns
+                    split_pair(held[2 * q][2 * half], held[2 * q][2 * half + 1], high[2 * half], low[2 * half]);
+                    split_pair(held[2 * q + 1][2 * half], held[2 * q + 1][2 * half + 1], high[2 * half + 1],
+                               low[2 * half + 1]);
+                }
 #pragma unroll
-                    for (uint32_t half = 0; half < 2; ++half) {
-                        const float first_weight =
-                            fast_exp2((log_high[half] - from[0].log_high) + (log_low[half] - from[0].log_low)) * from[0].step;
-                        const float second_weight =
-                            fast_exp2((log_high[half] - from[1].log_high) + (log_low[half] - from[1].log_low)) * from[1].step;
-                        const float first_value = s <= t[half] ? products[2 * j + part][2 * half] * first_weight : 0.0f;
-                        const float second_value =
-                            s + 1 <= t[half] ? products[2 * j + part][2 * half + 1] * second_weight : 0.0f;
-                        split_pair(first_value, second_value, high[2 * part + half], low[2 * part + half]);
+                for (uint32_t part = 0; part < 2; ++part) {
+                    const uint32_t(&state_part)[4] = part == 0 ? high : low;
+#pragma unroll
+                    for (uint32_t row_tile = 0; row_tile < 4; ++row_tile) {
+                        const uint32_t(&a)[4] = tokens[q % 2][row_tile];
+                        mma_bf16_16816(carried[row_tile][0], a[0], a[1], a[2], a[3], state_part[0], state_part[1]);
+                        mma_bf16_16816(carried[row_tile][1], a[0], a[1], a[2], a[3], state_part[2], state_part[3]);
+                    }
+                }
+            }
+            // ---- from the chunk's own inputs
+            const uint32_t rows_left = end - first > row0 ? end - first - row0 : 0;
+            float carries[8];
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) {
+                const TokenFactors& token = factors[i * 8 + row0];
+                carries[i] = fast_exp2(token.log_high + token.log_low);
+            }
+            uint32_t inputs[4][4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                ldmatrix_x4_trans(smem_u32(x + (j * 16 + (lane >> 3 & 1) * 8 + (lane & 7)) * kColumnPitch + (lane >> 4) * 8),
+                                  inputs[j][0], inputs[j][1], inputs[j][2], inputs[j][3]);
+            }
+#pragma unroll
+            for (uint32_t first_tile = 0; first_tile < 4; first_tile += 2) {
+                float sum[2][2][4] = {};
+#pragma unroll
+                for (uint32_t j = 0; j < first_tile + 2; ++j) {
+                    uint4 part[2][2];
+#pragma unroll
+                    for (uint32_t r = 0; r < 2; ++r) {
+                        const uint32_t row_tile = first_tile + r;
+                        if (j > row_tile) continue;
+                        const uint4* source =
+                            weights + ((buffer * kBlocks + row_tile * (row_tile + 1) / 2 + j) * 2) * 32 + lane;
+                        part[r][0] = source[0];
+                        part[r][1] = source[32];
+                    }
+#pragma unroll
+                    for (uint32_t p = 0; p < 2; ++p) {
+#pragma unroll
+                        for (uint32_t r = 0; r < 2; ++r) {
+                            if (j > first_tile + r) continue;
+                            const uint4& a = part[r][p];
+                            mma_bf16_16816(sum[r][0], a.x, a.y, a.z, a.w, inputs[j][0], inputs[j][1]);
+                            mma_bf16_16816(sum[r][1], a.x, a.y, a.z, a.w, inputs[j][2], inputs[j][3]);
+                        }
                     }
                 }
 #pragma unroll
-                for (uint32_t q = 0; q < 2; ++q) {
-                    uint32_t b0, b1, b2, b3;
-                    ldmatrix_x4_trans(smem_u32(x + (j * 16 + (lane >> 3 & 1) * 8 + (lane & 7)) * kColumnPitch + half_column +
-                                               q * 16 + (lane >> 4) * 8),
-                                      b0, b1, b2, b3);
-                    mma_bf16_16816(sum[2 * q], high[0], high[1], high[2], high[3], b0, b1);
-                    mma_bf16_16816(sum[2 * q + 1], high[0], high[1], high[2], high[3], b2, b3);
-                    mma_bf16_16816(sum[2 * q], low[0], low[1], low[2], low[3], b0, b1);
-                    mma_bf16_16816(sum[2 * q + 1], low[0], low[1], low[2], low[3], b2, b3);
-                }
-            }
+                for (uint32_t r = 0; r < 2; ++r) {
+                    const uint32_t row_tile = first_tile + r;
 #pragma unroll
-            for (uint32_t half = 0; half < 2; ++half) {
-                const uint32_t token = first + t[half];
-                const float carry = fast_exp2(log_high[half] + log_low[half]);
-                if (token < end) {
+                    for (uint32_t half = 0; half < 2; ++half) {
+                        const uint32_t t = row_tile * 16 + half * 8;
+                        const float carry = carries[2 * row_tile + half];
 #pragma unroll
-                    for (uint32_t tile = 0; tile < 4; ++tile) {
-                        const uint32_t local = half_column + tile * 8 + pair;
-                        if (column0 + local < args.vdim) {
+                        for (uint32_t tile = 0; tile < 2; ++tile) {
                             const float2 input = __bfloat1622float2(
-                                *reinterpret_cast<const __nv_bfloat162*>(x + t[half] * kColumnPitch + local));
-                            const float low = fmaf(skip, input.x, fmaf(carry, carried[tile][2 * half], sum[tile][2 * half]));
-                            const float high =
-                                fmaf(skip, input.y, fmaf(carry, carried[tile][2 * half + 1], sum[tile][2 * half + 1]));
-                            *reinterpret_cast<uint32_t*>(args.out + token * inner + head * args.vdim + column0 + local) =
-                                pack_bf16x2(low, high);
+                                *reinterpret_cast<const __nv_bfloat162*>(x + (t + row0) * kColumnPitch + tile * 8 + pair));
+                            const float even = fmaf(
+                                skip, input.x, fmaf(carry, carried[row_tile][tile][2 * half], sum[r][tile][2 * half]));
+                            const float odd = fmaf(
+                                skip, input.y, fmaf(carry, carried[row_tile][tile][2 * half + 1], sum[r][tile][2 * half + 1]));
+                            if (t < rows_left && tile * 8 < columns_left) {
+                                *reinterpret_cast<uint32_t*>(target + t * inner + tile * 8) = pack_bf16x2(even, odd);
+                            }
                         }
                     }
                 }
             }
+            target += kTokens * inner;
         }
 
         // ---- the state behind the chunk
@@ -401,47 +485,60 @@ state_space_chunk_kernel(const StateSpaceArgs<__nv_bfloat16> args, const PieceAr
         const float decay = fast_exp2(chunk_log);
         total_log += chunk_log;
 #pragma unroll
-        for (int unit = 0; unit < UNITS; ++unit) {
-            const uint32_t part = warp + 8 * unit;
-            const uint32_t n0 = part / 2 * 16;
-            if (n0 >= padded) {
-                continue;
+        for (uint32_t tile = 0; tile < kTiles; ++tile) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) held[tile][i] *= decay;
+        }
+        uint32_t rows[2][2][4];                        // B of 16 tokens and 32 state rows, and of the next ones
+        constexpr uint32_t kGroups = kTiles / 4;
+        const auto load_rows = [&](uint32_t step) {
+            const uint32_t k = step / kGroups * 16;
+#pragma unroll
+            for (uint32_t i = 0; i < 2; ++i) {
+                const uint32_t q = step % kGroups * 2 + i;
+                if (!FULL && q * 16 >= padded) continue;
+                uint32_t(&out)[4] = rows[step % 2][i];
+                ldmatrix_x4_trans(smem_u32(b + (k + (lane >> 3 & 1) * 8 + (lane & 7)) * pitch + q * 16 + (lane >> 4) * 8),
+                                  out[0], out[1], out[2], out[3]);
+            }
+        };
+        load_rows(0);
+        uint32_t high[4], low[4];
+#pragma unroll
+        for (uint32_t step = 0; step < kTokens / 16 * kGroups; ++step) {
+            if (step + 1 < kTokens / 16 * kGroups) load_rows(step + 1);
+            if (step % kGroups == 0) {
+                const uint32_t k = step / kGroups * 16;
+                uint32_t raw[4];
+                ldmatrix_x4_trans(smem_u32(x + (k + (lane >> 4) * 8 + (lane & 7)) * kColumnPitch + (lane >> 3 & 1) * 8),
+                                  raw[0], raw[1], raw[2], raw[3]);
+#pragma unroll
+                for (uint32_t i = 0; i < 4; ++i) {
+                    const uint32_t t = k + (i >> 1) * 8 + pair;
+                    const float2 value = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[i]));
+                    split_pair(value.x * factors[t].into_state, value.y * factors[t + 1].into_state, high[i], low[i]);
+                }
             }
 #pragma unroll
-            for (uint32_t tile = 0; tile < 4; ++tile) {
+            for (uint32_t part = 0; part < 2; ++part) {
+                const uint32_t(&a)[4] = part == 0 ? high : low;
 #pragma unroll
-                for (uint32_t i = 0; i < 4; ++i) held[unit][tile][i] *= decay;
-            }
-#pragma unroll
-            for (uint32_t k = 0; k < kTokens; k += 16) {
-                uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
-                ldmatrix_x4_trans(smem_u32(b + (k + (lane >> 4) * 8 + (lane & 7)) * pitch + n0 + (lane >> 3 & 1) * 8), a0, a1,
-                                  a2, a3);
-#pragma unroll
-                for (uint32_t q = 0; q < 2; ++q) {
-                    const uint32_t at = (k + (lane >> 3 & 1) * 8 + (lane & 7)) * kColumnPitch + part % 2 * 32 + q * 16 +
-                                        (lane >> 4) * 8;
-                    ldmatrix_x4_trans(smem_u32(input_high + at), b0, b1, b2, b3);
-                    mma_bf16_16816(held[unit][2 * q], a0, a1, a2, a3, b0, b1);
-                    mma_bf16_16816(held[unit][2 * q + 1], a0, a1, a2, a3, b2, b3);
-                    ldmatrix_x4_trans(smem_u32(input_low + at), b0, b1, b2, b3);
-                    mma_bf16_16816(held[unit][2 * q], a0, a1, a2, a3, b0, b1);
-                    mma_bf16_16816(held[unit][2 * q + 1], a0, a1, a2, a3, b2, b3);
+                for (uint32_t i = 0; i < 2; ++i) {
+                    const uint32_t q = step % kGroups * 2 + i;
+                    if (!FULL && q * 16 >= padded) continue;
+                    const uint32_t(&row)[4] = rows[step % 2][i];
+                    mma_bf16_16816(held[2 * q], a[0], a[1], a[2], a[3], row[0], row[1]);
+                    mma_bf16_16816(held[2 * q + 1], a[0], a[1], a[2], a[3], row[2], row[3]);
                 }
             }
         }
-        __syncthreads();
-        if (buffers == 2) {
-            buffer ^= 1;
-        } else if (first + kTokens < end) {
-            load_chunk(first + kTokens, 0);
-        }
+        if (end - first > 2 * kTokens) barrier_arrive(kFreeBarrier + buffer, kThreads);
     }
     if (PASS == Pass::kContribute) {
-        each_pair(state_between(piece), kColumns, write);
+        each_between(piece, write_between);
         if (threadIdx.x == 0 && block == 0) decay_between(piece) = total_log;
     } else if (piece == last_piece) {
-        each_pair(state + column0, args.vdim, write);
+        each_value(write);
     }
 }
 
@@ -498,21 +595,18 @@ cudaError_t launch_state_space_chunk(cudaStream_t stream, const StateSpaceLaunch
         const size_t state_floats = bound * per_segment * launch.size * kColumns;
         pieces.states = launch.pieces;
         pieces.decays = launch.pieces + state_floats;
-        split = launch.pieces != nullptr && (state_floats + bound * launch.heads) * sizeof(float) <= launch.piece_bytes;
+        split = launch.pieces != nullptr && aligned_to(launch.pieces, 16) &&
+                (state_floats + bound * launch.heads) * sizeof(float) <= launch.piece_bytes;
         if (!split) bound = segments;
     }
     const size_t blocks = bound * per_segment;
     const auto go = [&](auto kernel, bool outputs) {
-        // two CTAs per SM hide each other's loads; a second buffer does where it fits beside that or there are not enough CTAs
-        const bool alone = blocks <= 148 || shared_bytes(padded, 1, outputs) > kSharedLimit / 2 - 1024;
-        const uint32_t buffers =
-            shared_bytes(padded, 2, outputs) <= (alone ? kSharedLimit : kSharedLimit / 2 - 1024) ? 2 : 1;
-        const size_t shared = shared_bytes(padded, buffers, outputs);
+        const size_t shared = shared_bytes(padded, outputs);
         const cudaError_t set = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared));
         if (set != cudaSuccess) return set;
         return launch_kernel(kernel, static_cast<unsigned int>(blocks), kThreads, shared, stream, 1, args, pieces, column_blocks,
-                             padded, buffers);
+                             padded);
     };
     const auto sized = [&](auto units) {
         constexpr int kUnits = decltype(units)::value;
