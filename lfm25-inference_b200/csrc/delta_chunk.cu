@@ -27,7 +27,7 @@
 //   * the elements' own layout (tokens x channels) is that of A and B fragments too, so the triangles' products start from
 //     registers.
 // The elements take eight warps, the others four each; the matrices' warps get the registers that copies and triangles leave
-// (in 96 they spill: 4296 instead of 3900 cycles a step and all others wait).  One head of one segment, 4096 tokens: 770 us
+// (in 96 they spill: 5136 instead of 3900 cycles a step and all others wait).  One head of one segment, 4096 tokens: 770 us
 // with operands in plain rows and four equal groups, 663 us now; 7 segments of 300 to 700 tokens, 32 heads: 274 us in the order
 // of the step, 245 us with the longest segments first, 180 us with both.
 #include <type_traits>
