@@ -917,8 +917,10 @@ bool prompt_kernel_takes(const DeltaArgs<__nv_bfloat16>& args) {
 // twice the arithmetic and takes three launches, so it pays while the carrying CTAs leave most SMs idle and a prompt is
 // long.  The lengths are on the device, so the line is drawn for segments of equal length, where the longest one does not
 // help.  Inside steps of whole models, segments x heads (of 64 dimensions): what a layer gains in us at tokens a segment
-//     16: 256 1, 320 10, 1000 114, 4000 495        32: 320 0, 400 9 to 11, 600 8, 1000 70, 4096 292
-//     48: 400 -29, 512 -13, 720 21, 2000 67        64: 400 -25, 1000 -20 to 1, 2000 -36 to 38
+//     16: 320 -4, 400 1, 512 18, 1000 86, 4000 384     32: 400 -2, 600 -9, 1000 42, 4096 209
+//     48: 720 0, 1000 -3, 2000 9                       64: 1000 -80, 2000 -138
+// (The lines were drawn where the carrying kernel of an earlier form, up to 35 % slower, broke even; they lie within 9 us a
+// layer of that still.)
 constexpr size_t kSplitMostHeads = 48;             // of all segments
 constexpr size_t split_shortest(size_t heads) { return heads <= 16 ? 320 : (heads <= 32 ? 400 : 720); }
 
