@@ -917,10 +917,9 @@ bool prompt_kernel_takes(const DeltaArgs<__nv_bfloat16>& args) {
 // twice the arithmetic and takes three launches, so it pays while the carrying CTAs leave most SMs idle and a prompt is
 // long.  The lengths are on the device, so the line is drawn for segments of equal length, where the longest one does not
 // help.  Inside steps of whole models, segments x heads (of 64 dimensions): what a layer gains in us at tokens a segment
-//     16: 320 -4, 400 1, 512 18, 1000 86, 4000 384     32: 400 -2, 600 -9, 1000 42, 4096 209
-//     48: 720 0, 1000 -3, 2000 9                       64: 1000 -80, 2000 -138
-// (The lines were drawn where the carrying kernel of an earlier form, up to 35 % slower, broke even; they lie within 9 us a
-// layer of that still.)
+//     16: 320 -1, 400 8, 512 22, 1000 90, 4000 392     32: 400 2, 600 -5, 1000 49, 4096 187
+//     48: 720 7, 1000 3, 2000 26                       64: 1000 -70, 2000 -114
+// (The lines were drawn between earlier forms of both; these meet within 5 us a layer of them.)
 constexpr size_t kSplitMostHeads = 48;             // of all segments
 constexpr size_t split_shortest(size_t heads) { return heads <= 16 ? 320 : (heads <= 32 ? 400 : 720); }
 

@@ -13,8 +13,8 @@
 //     form     P, A, D, R', O' of every chunk of every head                     all chunks side by side
 //     carry    S through each segment's chunks, S_0 in the place of D           one product of 64 x 64 x 16 per chunk
 //     finish   O = R' S_0 + O', norm, gate                                      all chunks side by side
-// so only `carry` is serial, in steps of 64 tokens of a single small product.  4096 tokens of 32 heads: 418 us for the three
-// (one CTA per head, tile after tile of 16 tokens: 769 us on 32 SMs).
+// so only `carry` is serial, in steps of 64 tokens of a single small product.  4096 tokens of 32 heads: 395 us for the three
+// (one CTA per head, tile after tile of 16 tokens: 663 us on 32 SMs).
 //
 // Decays are multiplied up by a scan, never summed as logarithms: P_t and the 1 / P_s that meets it come from the same
 // factors, and both carry a handful of roundings.  A decay is at least exp(-exp(-1/2)), so 1 / P_t stays below 1e17 and a
@@ -25,10 +25,11 @@
 // added up outside the tensor cores, decays rounded without a direction (decay_of), the state's own part diag(P) S_0 as f32
 // multiply-adds.  State against float64 (2-norm; 300 to 4096 tokens, heads of 64, decay logits around 0, spread around -2,
 // around -6): 1.5e-7, 2.2e-7, 2.9e-7; the carrying kernel 4.1e-7, 7.4e-7, 1.7e-6.  With plain parts and sums inside the tensor
-// cores it was 9e-7, 1.6e-6, 2.0e-6 in 338 us instead of 418.  The outputs' own product ends in their bf16 rounding and needs
+// cores it was 9e-7, 1.6e-6, 2.0e-6 in 338 us instead of the 418 of that time.  The outputs' own product ends in their bf16 rounding and needs
 // none of this.  Not for f32 activations: the decays' products, their reciprocals and the parts each round once more than the
 // token-by-token recurrence does (250 tokens of 16 heads: 1.44e-7 at best, 0.76e-7 token by token).
 #include <algorithm>
+#include <cstddef>
 
 #include "delta_rule.h"
 #include "launch.h"
@@ -136,8 +137,22 @@ __device__ __forceinline__ float2 load_pair(const __nv_bfloat16* source) {
 }
 
 // 1 - (1 - exp(x)): close to 1, where a rounding to the same side in every token would add up over a long memory, the sum is
-// rounded to nearest
-__device__ __forceinline__ float decay_of(float logit) { return 1.0f + expm1f(-kDecayScale * sigmoidf(logit)); }
+// rounded to nearest.  x lies between -exp(-1/2) and 0, where ten terms of the exponential's power series leave 2e-10: errors of
+// the state as with expm1f (4096 tokens; decay logits around 0, -2, -6, -10: 1.39e-7, 1.83e-7, 2.97e-7, 4.70e-7 with either), 9 us
+// of 404 for the three kernels.
+__device__ __forceinline__ float decay_of(float logit) {
+    const float x = -kDecayScale * sigmoidf(logit);
+    float sum = 1.0f / 3628800.0f;
+    sum = fmaf(sum, x, 1.0f / 362880.0f);
+    sum = fmaf(sum, x, 1.0f / 40320.0f);
+    sum = fmaf(sum, x, 1.0f / 5040.0f);
+    sum = fmaf(sum, x, 1.0f / 720.0f);
+    sum = fmaf(sum, x, 1.0f / 120.0f);
+    sum = fmaf(sum, x, 1.0f / 24.0f);
+    sum = fmaf(sum, x, 1.0f / 6.0f);
+    sum = fmaf(sum, x, 0.5f);
+    return 1.0f + fmaf(sum * x, x, x);
+}
 
 struct FormShared {
     float u[kTokens * kPitch];                     // U, then W
@@ -153,7 +168,9 @@ struct FormShared {
 
 // About 6500 m16n8k8 products per chunk, eight cycles each per SM quarter, beside cutting their operands and adding up their
 // sums; the rest is the latency of the five stages between barriers, which two CTAs per SM hide in part.  Longer loops are
-// not unrolled further: the code then outgrows the instruction cache.
+// not unrolled further: the code then outgrows the instruction cache.  r, k and the removal's logit come by asynchronous copies
+// during the decay product; as 24 loads of four bytes a thread ahead of it they took 14 us more of 418 for the three kernels
+// (4096 tokens of 32 heads).
 __global__ void __launch_bounds__(kFormThreads, 2)
 delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t head_count, float* chunks) {
     constexpr uint32_t kParts = 3;                 // bf16 parts of tanh(z)
@@ -172,35 +189,27 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
     const __nv_bfloat16* projected = args.projected + static_cast<size_t>(tile.first) * args.pitch;
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 
-    // ---- V
+    // ---- V, and r, k and the removal's logit as they are, where K and B will lie: on their way during the decay product
     constexpr uint32_t kPiece = 8;                 // elements of 16 bytes
+    constexpr uint32_t kRaw = kTokens * kPitch;
+    __nv_bfloat16* raw = reinterpret_cast<__nv_bfloat16*>(shared.k);
+    static_assert(3 * kRaw * 2 <= 2 * kTokens * kPitch * 4 && offsetof(FormShared, b) == offsetof(FormShared, k) + kRaw * 4,
+                  "inside K and B");
     for (uint32_t item = threadIdx.x; item < kTokens * kDim / kPiece; item += kFormThreads) {
         const uint32_t token = item / (kDim / kPiece), column = item % (kDim / kPiece) * kPiece;
         const bool inside = token < tile.count && column < dim;
-        copy_async_16(shared.v + token * kPitch + column,
-                      inside ? projected + token * args.pitch + 2 * width + head_base + column : projected, inside);
+        const __nv_bfloat16* source = inside ? projected + token * args.pitch + head_base + column : projected;
+        const uint32_t at = token * kPitch + column;
+        copy_async_16(raw + at, source, inside);
+        copy_async_16(raw + kRaw + at, source + (inside ? width : 0), inside);
+        copy_async_16(raw + 2 * kRaw + at, source + (inside ? 4 * width : 0), inside);
+        copy_async_16(shared.v + at, source + (inside ? 2 * width : 0), inside);
     }
     copy_async_commit();
 
-    // ---- r, k and the removal's logit: 16 tokens x 32 channels per warp, in the layout of the decay product below
+    // 16 tokens x 32 channels per warp, in the layout of the decay product below
     const uint32_t block = warp % 4, half = warp / 4;
     const uint32_t row0 = block * 16 + (lane >> 2), pair = (lane & 3) * 2;
-    float2 r[4][2], k[4][2], removal[4][2];
-#pragma unroll
-    for (uint32_t n = 0; n < 4; ++n) {
-        const uint32_t channel = half * 32 + n * 8 + pair;
-#pragma unroll
-        for (uint32_t i = 0; i < 2; ++i) {
-            const uint32_t token = row0 + i * 8;
-            r[n][i] = k[n][i] = removal[n][i] = make_float2(0.0f, 0.0f);
-            if (token < tile.count && channel < dim) {
-                const __nv_bfloat16* source = projected + token * args.pitch + head_base + channel;
-                r[n][i] = load_pair(source);
-                k[n][i] = load_pair(source + width);
-                removal[n][i] = load_pair(source + 4 * width);
-            }
-        }
-    }
     // ---- decay logits W2 tanh(z), 64 columns of z at a time; their operands lie where U and R will
     float logits[4][4] = {};
     {
@@ -266,6 +275,19 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
                     }
                 }
             }
+        }
+    }
+    copy_async_wait<0>();
+    __syncthreads();
+    float2 r[4][2], k[4][2], removal[4][2];
+#pragma unroll
+    for (uint32_t n = 0; n < 4; ++n) {
+#pragma unroll
+        for (uint32_t i = 0; i < 2; ++i) {
+            const __nv_bfloat16* source = raw + (row0 + i * 8) * kPitch + half * 32 + n * 8 + pair;
+            r[n][i] = load_pair(source);
+            k[n][i] = load_pair(source + kRaw);
+            removal[n][i] = load_pair(source + 2 * kRaw);
         }
     }
     // ---- products of the decays up to each token: of its block of 16 here, of the blocks before it below
@@ -341,7 +363,6 @@ delta_form_kernel(const DeltaArgs<__nv_bfloat16> args, uint32_t head0, uint32_t 
                                                                     -fast_sigmoid(removal[n][i].y + bias.y) * uy * iy);
         }
     }
-    copy_async_wait<0>();
     __syncthreads();
 
     float* chunk = chunks + static_cast<size_t>(blockIdx.x) * kChunkFloats;
