@@ -30,11 +30,12 @@
 //     here                      19.1            24.6           10.6           12.1           13.8               610
 //
 // Every mbarrier wait is bounded; a wait that runs out sets the CTA's abort flag, is recorded in the device status words, and
-// the CTA (in a cluster: all its CTAs) leaves without storing.
+// the CTA (in a cluster: all its CTAs) leaves without storing, once its copies and MMAs are through (drain()).
 #include <cooperative_groups.h>
 
 #include <algorithm>
 #include <atomic>
+#include <cstddef>
 
 #include "kernels.h"
 #include "launch.h"
@@ -130,6 +131,39 @@ __device__ __forceinline__ void umma(uint32_t accumulator, uint64_t a, uint64_t 
         : "memory");
 }
 
+__device__ __forceinline__ void store_shared(uint32_t address, uint32_t value) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(address), "r"(value) : "memory");
+}
+
+// What each role has got through when it leaves: blocks of weights requested, blocks of MMAs issued, blocks converted by each warp.
+struct Progress {
+    uint32_t requested, multiplied, converted[kConverters];
+};
+constexpr uint32_t kProgressAt = 16 * kMaxStages + 24;   // in the control bytes, behind the barriers and two words
+static_assert(kProgressAt + sizeof(Progress) <= 256, "the control bytes end");
+
+// Nobody leaves with a copy or an MMA in flight: only once all roles are through is it known that a wait of the CTA has run out.
+// By itself, so that it takes no registers from the roles.
+template <uint32_t N>
+__device__ __noinline__ void drain(uint8_t* control, uint64_t wait_limit) {
+    constexpr uint32_t kStages = Shape<N>::kStages;
+    const volatile Progress& progress = *reinterpret_cast<volatile Progress*>(control + kProgressAt);
+    if (threadIdx.x == 0) {
+        // The last copy of every slot.  Its barrier also counts the converting warps: what those have left out is made good.
+        const uint32_t requested = progress.requested;
+        for (uint32_t block = requested > kStages ? requested - kStages : 0; block < requested; ++block) {
+            const uint32_t bar = smem_u32(control) + 8 * (block % kStages);
+            for (uint32_t i = 0; i < kConverters; ++i) {
+                if (progress.converted[i] <= block) mbar_arrive(bar);
+            }
+            (void)mbar_wait_bounded(bar, block / kStages & 1, wait_limit);
+        }
+    } else if (threadIdx.x / 32 == 1 && progress.multiplied > 0) {
+        const uint32_t block = progress.multiplied - 1;
+        (void)mbar_wait_bounded(smem_u32(control) + 8 * kMaxStages + 8 * (block % kStages), block / kStages & 1, wait_limit);
+    }
+}
+
 template <uint32_t N>
 __global__ void __launch_bounds__(kThreads, Shape<N>::kCtas)
 linear_f32_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const LinearParams p) {
@@ -143,6 +177,7 @@ linear_f32_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const Lin
     const uint32_t bar_taken = bar_read + 8 * kMaxStages;                  // [2] a short sum has been added up
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(control + 16 * kMaxStages + 16);
     volatile uint32_t* abort_flag = tmem_slot + 1;
+    const uint32_t progress = bar_ready + kProgressAt;
     const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t split = blockIdx.x % p.splits;
@@ -168,6 +203,7 @@ linear_f32_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const Lin
         }
         mbar_init(bar_taken, kAdders);
         mbar_init(bar_taken + 8, kAdders);
+        for (uint32_t i = 0; i < kConverters; ++i) store_shared(progress + offsetof(Progress, converted) + 4 * i, 0);
         *abort_flag = 0;
         fence_barrier_init();
         fence_proxy_async_smem();
@@ -202,10 +238,7 @@ linear_f32_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const Lin
                     parity ^= 1;
                 }
             }
-            // nobody leaves with a copy in flight: the last one of every slot
-            for (uint32_t block = issued > S::kStages ? issued - S::kStages : 0; *abort_flag && block < issued; ++block) {
-                (void)mbar_wait_bounded(bar_ready + 8 * (block % S::kStages), block / S::kStages & 1, p.wait_limit);
-            }
+            store_shared(progress + offsetof(Progress, requested), issued);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -216,8 +249,8 @@ linear_f32_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const Lin
                                                  (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
             constexpr uint32_t kPart = S::kPartBytes >> 4;
             const uint32_t rest = tmem + 4 * N;
-            uint32_t stage = 0, parity = 0, slot = ring, accumulate = 0;
-            for (uint32_t block = 0; block < blocks; ++block) {
+            uint32_t stage = 0, parity = 0, slot = ring, accumulate = 0, block = 0;
+            for (; block < blocks; ++block) {
                 const uint32_t pair = block / 2;
                 if (!mbar_wait_bounded(bar_ready + 8 * stage, parity, p.wait_limit) ||
                     (block % 2 == 0 && pair > 1 && !mbar_wait_bounded(bar_taken + 8 * (pair & 1), (pair / 2 - 1) & 1, p.wait_limit))) {
@@ -246,6 +279,7 @@ linear_f32_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const Lin
                     parity ^= 1;
                 }
             }
+            store_shared(progress + offsetof(Progress, multiplied), block);
         }
         __syncwarp();
     } else if (warp < kFirstAdder) {
@@ -288,7 +322,10 @@ linear_f32_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const Lin
             }
             fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_ready + 8 * stage);
+            if (lane == 0) {
+                mbar_arrive(bar_ready + 8 * stage);
+                store_shared(progress + offsetof(Progress, converted) + 4 * (warp - kFirstConverter), block + 1);
+            }
             if (++stage == S::kStages) {
                 stage = 0;
                 parity ^= 1;
@@ -346,7 +383,9 @@ linear_f32_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const Lin
     pdl_launch_dependents();
     pdl_wait();                  // y may still be read by an earlier kernel
     __syncthreads();
+    if (*abort_flag) drain<N>(control, p.wait_limit);
     if (warp == 1) {
+        __syncwarp();
         tcgen05_fence_after();
         tmem_free(tmem, S::kColumns);
     }

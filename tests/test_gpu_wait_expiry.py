@@ -12,10 +12,11 @@ import cases
 from conftest import assert_within_oracle, bits_of, to_bf16, to_u32
 from lfm25_inference_b200 import _abi, ops, workloads
 from oracle import oracle
+from test_gpu_linear_f32 import product as f32_product, sum_bound
 
 pytestmark = pytest.mark.gpu
 
-TAG_ATTENTION, TAG_GEMM_UMMA, TAG_GEMM_ROWS = 1, 3, 5
+TAG_ATTENTION, TAG_GEMM_UMMA, TAG_GEMM_ROWS, TAG_LINEAR_F32 = 1, 3, 5, 9
 LIMIT_NS = 3_000_000
 
 
@@ -80,6 +81,29 @@ def test_attention_wait_runs_out_and_the_next_launch_is_clean(device, library_op
                                              case["block_tables"], case["request_slots"], case["position_ids"],
                                              want_exact=True)
     assert_within_oracle(bits_of(output), exact)
+    assert ops.device_status()[0] == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(40, 300, 64),          # one block of k
+                                   (250, 6144, 1024),      # all of k in a CTA, more blocks than slots in the ring
+                                   (16, 128, 512),         # k over a cluster, fewer blocks than slots
+                                   (16, 128, 4104),        # k over a cluster, more of them, the last one cut
+                                   (97, 130, 7168)])
+def test_f32_linear_wait_runs_out_and_the_next_launch_is_clean(device, library_option, m, n, k):
+    rng = np.random.default_rng(m + n + k)
+    x, weight = rng.standard_normal((m, k)).astype(np.float32), rng.choice([-1.5, 0.75, 2.0], size=(n, k))
+    assert ops.device_status()[0] == 0
+    library_option("wait_limit_ns", LIMIT_NS)
+    library_option("wait_selftest_drop", 1)
+    out = f32_product(device, x, weight)
+    count, last_tag, _, _ = ops.device_status()
+    assert count >= 1 and last_tag == TAG_LINEAR_F32
+    assert np.all(out == 7.0)                     # as f32_product fills it
+    library_option("wait_selftest_drop", 0)
+    library_option("wait_limit_ns", 1_000_000_000)
+    out = f32_product(device, x, weight)
+    error = np.abs(out - x.astype(np.float64) @ weight.T)
+    assert (error <= sum_bound(k) * (np.abs(x).astype(np.float64) @ np.abs(weight).T)).all()
     assert ops.device_status()[0] == 0
 
 
