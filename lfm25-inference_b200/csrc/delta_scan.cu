@@ -26,6 +26,10 @@ namespace {
 
 constexpr uint32_t kElementTokens = 16;      // tokens per CTA of the elements kernel
 constexpr uint32_t kElementThreads = 256;
+// Values of tanh(z) per token that a launch of the elements kernel holds in shared memory, beside a word per token: as many as
+// every kernel may have without asking.  Larger ranks take several launches, which leave the logits in the place of w.
+constexpr uint32_t kRankBlock = 760;
+static_assert(kRankBlock % 8 == 0 && kElementTokens * (1 + kRankBlock) * sizeof(float) <= 48 * 1024, "whole pieces of W2's rows");
 constexpr uint32_t kVectors = 6;             // r, w, -(a * u), u, k, v
 constexpr uint32_t kValues = 5;              // place of v, and of the result after the scan
 
@@ -39,12 +43,12 @@ struct ScanVectors {
 };
 
 template <typename T, uint32_t DP>
-__global__ void __launch_bounds__(kElementThreads)
-delta_scan_elements_kernel(const DeltaArgs<T> args, const ScanVectors vectors) {
+__global__ void __launch_bounds__(kElementThreads, 2)
+delta_scan_elements_kernel(const DeltaArgs<T> args, const ScanVectors vectors, uint32_t first_z, uint32_t z_count) {
     extern __shared__ __align__(16) float element_shared[];
-    __shared__ float unit_scale[kElementTokens];
-    const uint32_t padded_z = (args.rank + 3) / 4 * 4;
-    float* z_values = element_shared;                                  // [token][padded_z], tanh applied
+    const uint32_t padded_z = (z_count + 3) / 4 * 4;
+    float* unit_scale = element_shared;                                // [token]
+    float* z_values = element_shared + kElementTokens;                 // [token][padded_z], tanh applied
     const uint32_t head = blockIdx.x % vectors.heads;
     const size_t first = static_cast<size_t>(blockIdx.x / vectors.heads) * kElementTokens;
     const uint32_t tokens = static_cast<uint32_t>(min(args.segments.num_tokens - first, size_t(kElementTokens)));
@@ -58,13 +62,13 @@ delta_scan_elements_kernel(const DeltaArgs<T> args, const ScanVectors vectors) {
     const uint32_t channel = threadIdx.x % DP;
     const bool live = channel < dim;
     const size_t index = head_base + (live ? channel : 0);
-    const __nv_bfloat16* decay_row = args.decay_up + index * args.rank;
+    const __nv_bfloat16* decay_row = args.decay_up + index * args.rank + first_z;
     const bool vector_rank = args.rank % 8 == 0 && (reinterpret_cast<uintptr_t>(args.decay_up) & 15) == 0;
     uint4 early[kEarly / 8] = {};
     if (vector_rank) {
 #pragma unroll
         for (uint32_t i = 0; i < kEarly / 8; ++i) {
-            if (i * 8 < args.rank) early[i] = *reinterpret_cast<const uint4*>(decay_row + i * 8);
+            if (i * 8 < z_count) early[i] = *reinterpret_cast<const uint4*>(decay_row + i * 8);
         }
     }
     const float bias = __bfloat162float(args.removal_bias[index]), base = __bfloat162float(args.decay_base[index]);
@@ -85,8 +89,8 @@ delta_scan_elements_kernel(const DeltaArgs<T> args, const ScanVectors vectors) {
     }
     for (uint32_t item = threadIdx.x; item < kElementTokens * padded_z; item += kElementThreads) {
         const uint32_t t = item / padded_z, z = item % padded_z;
-        z_values[item] = t < tokens && z < args.rank
-                             ? tanhf(to_float<T>(args.projected[(first + t) * args.pitch + 5 * width + z]))
+        z_values[item] = t < tokens && z < z_count
+                             ? tanhf(to_float<T>(args.projected[(first + t) * args.pitch + 5 * width + first_z + z]))
                              : 0.0f;
     }
     __syncthreads();
@@ -123,16 +127,22 @@ delta_scan_elements_kernel(const DeltaArgs<T> args, const ScanVectors vectors) {
             }
         }
         float logit[4] = {};
+        if (first_z > 0) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                if (t0 + i < tokens) logit[i] = vectors.at(first + t0 + i, head)[vectors.pitch + channel];
+            }
+        }
         if (vector_rank) {
 #pragma unroll
             for (uint32_t i = 0; i < kEarly / 8; ++i) {
-                if (i * 8 < args.rank) add_products(early[i], t0, i * 8, logit);
+                if (i * 8 < z_count) add_products(early[i], t0, i * 8, logit);
             }
-            for (uint32_t z = kEarly; z < args.rank; z += 8) {
+            for (uint32_t z = kEarly; z < z_count; z += 8) {
                 add_products(*reinterpret_cast<const uint4*>(decay_row + z), t0, z, logit);
             }
         } else {
-            for (uint32_t z = 0; z < args.rank; ++z) {
+            for (uint32_t z = 0; z < z_count; ++z) {
                 const float weight = __bfloat162float(decay_row[z]);
 #pragma unroll
                 for (uint32_t i = 0; i < 4; ++i) logit[i] = fmaf(weight, z_values[(t0 + i) * padded_z + z], logit[i]);
@@ -143,6 +153,10 @@ delta_scan_elements_kernel(const DeltaArgs<T> args, const ScanVectors vectors) {
             const uint32_t t = t0 + i;
             if (t >= tokens) break;
             float* target = vectors.at(first + t, head) + channel;
+            if (first_z + z_count < args.rank) {
+                target[1 * vectors.pitch] = logit[i];
+                continue;
+            }
             float w = 0.0f, removal = 0.0f, u = 0.0f;
             if (live) {
                 w = expf(-kDecayScale * sigmoidf(logit[i] + base));
@@ -170,6 +184,7 @@ struct ScanShape {
     static constexpr uint32_t kPieces = (kTokenFloats / 4 + 31) / 32;       // 16-byte pieces of a token per lane of a warp
     static constexpr size_t kShared = (2 * kTokens + 1) * kTokenFloats * sizeof(float);
     static_assert(kRows % 4 == 0, "four consecutive key channels per access");
+    static_assert(kShared <= 227 * 1024, "shared memory");
 };
 
 template <uint32_t GROUPS>
@@ -385,14 +400,6 @@ delta_scan_output_kernel(const DeltaArgs<T> args, const ScanVectors vectors) {
 
 size_t head_bytes(size_t tokens, uint32_t dim) { return tokens * kVectors * ((dim + 3) / 4 * 4) * sizeof(float); }
 
-template <typename Kernel>
-cudaError_t allow_shared(Kernel kernel, size_t bytes) {
-    if (bytes > 227 * 1024) return cudaErrorInvalidValue;
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(bytes));
-}
-
 template <typename T, uint32_t DP, uint32_t LANES, uint32_t COLUMNS>
 cudaError_t launch_sized(cudaStream_t stream, DeltaArgs<T> args, ScanVectors vectors, uint32_t heads_at_once) {
     using Shape = ScanShape<DP, LANES, COLUMNS>;
@@ -400,15 +407,21 @@ cudaError_t launch_sized(cudaStream_t stream, DeltaArgs<T> args, ScanVectors vec
     args.splits = (args.dim + COLUMNS - 1) / COLUMNS;
     const auto elements = delta_scan_elements_kernel<T, DP>;
     const auto scan = delta_scan_kernel<T, DP, LANES, COLUMNS>;
-    const size_t element_shared = static_cast<size_t>(kElementTokens) * ((args.rank + 3) / 4 * 4) * sizeof(float);
-    cudaError_t status = allow_shared(elements, element_shared);
-    if (status == cudaSuccess) status = allow_shared(scan, Shape::kShared);
+    cudaError_t status = cudaSuccess;
+    if (Shape::kShared > 48 * 1024) {
+        status = cudaFuncSetAttribute(reinterpret_cast<const void*>(scan), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(Shape::kShared));
+    }
     for (uint32_t first = 0; first < args.heads && status == cudaSuccess; first += heads_at_once) {
         vectors.first_head = first;
         vectors.heads = std::min(heads_at_once, args.heads - first);
         const size_t tiles = (tokens + kElementTokens - 1) / kElementTokens;
-        status = launch_kernel(elements, static_cast<unsigned int>(tiles * vectors.heads), kElementThreads, element_shared,
-                               stream, 1, args, vectors);
+        for (uint32_t first_z = 0; first_z < args.rank && status == cudaSuccess; first_z += kRankBlock) {
+            const uint32_t z_count = std::min(args.rank - first_z, kRankBlock);
+            const size_t shared = static_cast<size_t>(kElementTokens) * (1 + (z_count + 3) / 4 * 4) * sizeof(float);
+            status = launch_kernel(elements, static_cast<unsigned int>(tiles * vectors.heads), kElementThreads, shared, stream, 1,
+                                   args, vectors, first_z, z_count);
+        }
         if (status != cudaSuccess) break;
         status = launch_kernel(scan, static_cast<unsigned int>(args.segments.num_segments * vectors.heads * args.splits),
                                Shape::kThreads, Shape::kShared, stream, 1, args, vectors);

@@ -116,10 +116,12 @@ def test_delta_rule_layer(device, dtype, heads, dim, rank):
 
 
 @pytest.mark.parametrize("dtype", TYPES)
-@pytest.mark.parametrize("heads,dim,rank", [(1, 8, 3), (2, 64, 72), (3, 36, 64), (1, 72, 8), (2, 136, 65)])
+@pytest.mark.parametrize("heads,dim,rank", [(1, 8, 3), (2, 64, 72), (3, 36, 64), (1, 72, 8), (2, 136, 65), (2, 64, 760), (1, 20, 765),
+                                            (1, 64, 768), (1, 200, 1528), (1, 8, 4100)])
 def test_delta_rule_token_by_token(device, library_option, dtype, heads, dim, rank):
-    """The f32 kernels for prompts at the edges of their tiles of 16 and 8 tokens and of 8 and 16 value columns; bf16 models take
-    them by the option, with scratch for one head at a time."""
+    """The f32 kernels for prompts at the edges of their tiles of 16 and 8 tokens and of 8 and 16 value columns, with ranks of the
+    decays around multiples of 760, what one launch takes; bf16 models take them by the option, with scratch for one head at a
+    time."""
     library_option("delta_prompt", 2)
     config = cases.config_of([cases.delta_layer(heads, dim, ff=0)])
     check_layer(config, 19, device, dtype, [1, 1, 15, 16, 17, 2, 7, 8, 9, 33], rank)
