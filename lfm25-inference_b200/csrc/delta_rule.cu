@@ -905,12 +905,17 @@ cudaError_t launch_prompt(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& a
                          DP / COLUMNS * 8 + HELPERS, shared, stream, 1, args);
 }
 
-bool prompt_kernel_takes(const DeltaArgs<__nv_bfloat16>& args) {
-    const size_t shared = args.dim <= 64 ? PromptLayout<64>(args.rank).total : PromptLayout<128>(args.rank).total;
-    return args.dim % 8 == 0 && args.dim <= 128 && args.rank <= kPromptMaxRank && args.pitch % 8 == 0 &&
-           args.out_pitch % 2 == 0 && aligned_to(args.projected, 16) && aligned_to(args.out, 4) &&
-           aligned_to(args.decay_up, 16) &&
-           shared <= 227 * 1024;
+// Whether bf16 prompts of these sizes have kernels of their own.  Asked before a launch and where scratch is sized, so that
+// whatever they do not take finds room for all its heads.
+bool prompt_kernels_take(uint32_t dim, uint32_t rank, size_t pitch, size_t out_pitch, const void* decay_up) {
+    const size_t shared = dim <= 64 ? PromptLayout<64>(rank).total : PromptLayout<128>(rank).total;
+    return dim % 8 == 0 && dim <= 128 && rank <= kPromptMaxRank && pitch % 8 == 0 && out_pitch % 2 == 0 &&
+           aligned_to(decay_up, 16) && shared <= 227 * 1024;
+}
+
+bool prompt_kernels_take(const DeltaArgs<__nv_bfloat16>& args) {
+    return prompt_kernels_take(args.dim, args.rank, args.pitch, args.out_pitch, args.decay_up) &&
+           aligned_to(args.projected, 16) && aligned_to(args.out, 4);
 }
 
 // Where prompts are split along the sequence (delta_split.cu) instead of carried by one CTA per segment and head: it does about
@@ -987,7 +992,7 @@ cudaError_t launch_typed(cudaStream_t stream, const DeltaRuleLaunch& launch) {
         return launch_decode<T, 128>(stream, args);
     }
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-        if (launch.segments.offsets != nullptr && option(kOptDeltaPrompt) != 2 && prompt_kernel_takes(args)) {
+        if (launch.segments.offsets != nullptr && option(kOptDeltaPrompt) != 2 && prompt_kernels_take(args)) {
             if (delta_chunk_takes(launch.dim, launch.rank) && option(kOptDeltaPrompt) != 1) {
                 // the kernels for larger ranks keep more bits than the split ones
                 if (split_takes(args, launch)) return launch_delta_split(stream, args, launch.chunks, launch.chunk_bytes);
@@ -1010,9 +1015,8 @@ cudaError_t launch_typed(cudaStream_t stream, const DeltaRuleLaunch& launch) {
 bool delta_rule_needs_scratch(uint32_t dim) { return dim > 128; }
 
 size_t delta_rule_vector_bytes(Activation type, uint32_t heads, uint32_t dim, uint32_t rank, size_t pitch, size_t out_pitch,
-                               size_t tokens) {
-    const bool others = type == Activation::kBf16 && dim % 8 == 0 && dim <= 128 && rank <= kPromptMaxRank && pitch % 8 == 0 &&
-                        out_pitch % 2 == 0;      // kernels of their own, see prompt_kernel_takes()
+                               const void* decay_up, size_t tokens) {
+    const bool others = type == Activation::kBf16 && prompt_kernels_take(dim, rank, pitch, out_pitch, decay_up);
     return delta_scan_bytes(others ? 1 : heads, dim, tokens);
 }
 

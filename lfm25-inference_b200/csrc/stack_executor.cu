@@ -807,7 +807,7 @@ int32_t lfm25_stack_executor_create(lfm25_blaslt* blaslt, const lfm25_stack_mode
                                                                               maximum_rows));
             vector_bytes = std::max(vector_bytes, lfm25::delta_rule_vector_bytes(type, layer.heads, layer.dim, layer.rank,
                                                                                  layer.projection.n, layer.output.k,
-                                                                                 maximum_tokens));
+                                                                                 layer.decay_up, maximum_tokens));
         }
         if (layer.mixer == LFM25_MIXER_LATENT_ATTENTION) {
             const lfm25::LatentAttentionShape shape = {layer.heads, layer.dim, layer.rot_dim, layer.vdim, layer.kv_rank,

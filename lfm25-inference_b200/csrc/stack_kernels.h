@@ -386,7 +386,7 @@ size_t delta_rule_chunk_bytes(Activation type, uint32_t heads, uint32_t dim, siz
 // Scratch for prompts that run token by token in f32, in steps of up to `tokens` tokens: every head of the shapes that always
 // do, one head (heads are taken in turns) of those with faster kernels.
 size_t delta_rule_vector_bytes(Activation type, uint32_t heads, uint32_t dim, uint32_t rank, size_t pitch, size_t out_pitch,
-                               size_t tokens);
+                               const void* decay_up, size_t tokens);
 cudaError_t launch_delta_rule(cudaStream_t stream, const DeltaRuleLaunch& launch);
 
 }  // namespace lfm25

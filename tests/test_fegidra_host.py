@@ -236,3 +236,23 @@ def test_stack_executor_rejects_bad_models_before_touching_the_device():
     assert create(tokens=4, rows=8)[0] == _abi.ERR_INVALID_ARGUMENT
     model.head = _abi.StackLinear(fake, 8, 64)
     assert create() == (_abi.ERR_INVALID_ARGUMENT, "stack model sizes are inconsistent")
+
+
+@pytest.mark.parametrize("dim,rank,decay_up,heads", [
+    (128, 192, 0x1000, 1),        # the last rank whose prompt kernel fits shared memory with heads of 128
+    (128, 193, 0x1000, 16),
+    (72, 256, 0x1000, 16),
+    (64, 256, 0x1000, 1),
+    (64, 257, 0x1000, 16),
+    (64, 64, 0x1008, 16),         # rows of W2 that are not read in whole pieces
+    (60, 64, 0x1000, 16)])
+def test_scratch_of_the_token_by_token_delta_rule(dim, rank, decay_up, heads):
+    """Room for every head of the bf16 shapes that no other kernel takes, so that a step of as many tokens as the executor takes
+    runs its heads side by side."""
+    # lfm25::delta_rule_vector_bytes(Activation, heads, dim, rank, pitch, out_pitch, decay_up, tokens)
+    scratch = getattr(_abi.library(), "_ZN5lfm2523delta_rule_vector_bytesENS_10ActivationEjjjmmPKvm")
+    scratch.argtypes = [ctypes.c_int] + [ctypes.c_uint32] * 3 + [ctypes.c_size_t] * 2 + [ctypes.c_void_p, ctypes.c_size_t]
+    scratch.restype = ctypes.c_size_t
+    pitch = (5 * 16 * dim + rank + 7) // 8 * 8
+    vectors = 100 * 6 * dim * 4   # r, w, the removal, u, k, v of 100 tokens of a head
+    assert scratch(0, 16, dim, rank, pitch, 16 * dim, decay_up, 100) == heads * vectors

@@ -109,7 +109,7 @@ def test_decode_attention_groups(device, library_option, heads, kv_heads, dim, c
 
 @pytest.mark.parametrize("dtype", TYPES)
 @pytest.mark.parametrize("heads,dim,rank", [(3, 16, 5), (2, 64, 16), (1, 24, 1), (2, 128, 33), (1, 80, 3), (2, 160, 8),
-                                            (1, 256, 64), (1, 10, 7), (2, 128, 700)])
+                                            (1, 256, 64), (1, 10, 7), (2, 128, 700), (3, 128, 224), (2, 72, 256)])
 def test_delta_rule_layer(device, dtype, heads, dim, rank):
     config = cases.config_of([cases.delta_layer(heads, dim, ff=0)])
     check_layer(config, 13, device, dtype, [37, 2, 1, 16, 1, 5], rank)
