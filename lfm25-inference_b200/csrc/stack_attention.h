@@ -75,7 +75,6 @@ bool stack_attention_umma_supports(const StackAttentionLaunch& launch);
 cudaError_t launch_stack_attention_umma(cudaStream_t stream, const StackAttentionLaunch& launch);
 
 // The first decode_tokens tokens (every one a segment of its own).
-uint32_t stack_attention_splits(const StackAttentionShape& shape, size_t tokens, size_t context);
 bool stack_attention_decode_supports(const StackAttentionLaunch& launch);
 cudaError_t launch_stack_attention_decode(cudaStream_t stream, const StackAttentionLaunch& launch);
 

@@ -9,13 +9,19 @@
 // bits); maximum, sum and accumulators are f32.  The warps merge through shared memory, the splits of a token through the
 // distributed shared memory of their cluster.
 //
-// Bound by the latency of a page in a warp until the memory's rate is reached.  32 tokens, 32 query heads on 8 key/value heads of
-// 64, us with four warps and the heads as rows, and now: contexts of 128 to 4096 48.4 / 31.3 (the longest decides), all 4096
-// 57.1 / 46.2 (5.8 TB/s), all 1100 19.0 / 11.7; 24 tokens of 100 to 4000 on 2 heads of 128 21.5 / 16.8.
+// Bound by the latency of a page in a warp until the memory's rate is reached.  us with four warps and the heads as rows, with
+// twelve warps two pages at a time and splits of eight pages, and now (eight warps, one page at a time, splits and shared memory
+// chosen so that the CTAs spread over the SMs); launches back to back, caches beyond the L2:
+//     32 tokens, 32 heads on 8 of 64: contexts of 128 to 4096     46.7 / 29.8 / 29.2      all 4096 (6.4 TB/s)  55.8 / 44.8 / 42.2
+//     the same, all 1100    19.6 / 15.5 / 14.3                    24 tokens of 100 to 4000 on 2 of 128         21.2 / 18.3 / 18.6
+//     groups of 16 heads of 64: 32 tokens of 4096 on 1    19.5 / 36.2 / 13.9     64 of 1024 on 4     20.6 / 24.7 / 16.6
+//     8 tokens of 256 on 8 of 64    6.0 / 6.3 / 3.7               64 of 1024 on 8 of 64                        34.5 / 27.3 / 23.5
+// Over 552 shapes and contexts 0.82 of the first and 0.76 of the second.
 #include <cooperative_groups.h>
 #include <math.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "launch.h"
 #include "options.h"
@@ -30,27 +36,38 @@ namespace cg = cooperative_groups;
 
 constexpr uint32_t kBoxBytes = kPageSize * 128;   // 16 keys x 64 dimensions
 constexpr uint32_t kGroupRows = 16;
+constexpr uint32_t kMostSplits = 8;
+// Of shared memory, so that no second CTA of the kernel is put on the SM while others are empty: 128 CTAs in clusters of 4 (32
+// tokens of 4096 keys, 16 heads on 1 with values of 128) 18.6 us, 27.0 with what they need.
+constexpr uint32_t kAloneBytes = 116 * 1024;
 
-template <uint32_t KC, uint32_t VC>
+// WIDE: eight warps with short rings, where all CTAs are resident at once and there is a page for more than half of them.
+// Otherwise four, so that more CTAs share an SM: 64 tokens of 1024 keys on 8 heads of 64 23.4 us, with eight warps 25.3.
+// Of 14 combinations of 4 to 12 warps, 2 to 4 stages and 1 or 2 pages at a time, (8, 2, 1) or its neighbours (8, 3, 1) and
+// (8, 2, 2) were fastest wherever all CTAs are resident.
+template <uint32_t KC, uint32_t VC, uint32_t TILES, bool WIDE>
 struct Layout {
-    // Many warps with short rings, taken two pages at a time: 96 KiB of ring, two CTAs per SM.  32 tokens of 128 to 4096 keys,
-    // 8 key/value heads of 64, by (warps, stages, pages at a time): (4, 4, 1) 53 us, (4, 6, 3) 42, (6, 4, 2) 37, (8, 3, 3) 34,
-    // (12, 2, 2) 31.
-    static constexpr uint32_t kWarps = KC + VC <= 2 ? 12 : (KC + VC <= 4 ? 6 : 4);
+    static constexpr uint32_t kWarps = WIDE ? 8 : 4;
     static constexpr uint32_t kThreads = kWarps * 32;
     static constexpr uint32_t kStageBytes = (KC + VC) * kBoxBytes;
-    static constexpr uint32_t kStages = 2;
-    static constexpr uint32_t kPages = KC + VC <= 4 ? 2 : 1;        // that a warp takes at a time
+    static constexpr uint32_t kStages = !WIDE && (KC + VC == 3 || KC + VC == 4) ? 3 : 2;
+    static constexpr uint32_t kPages = kStages == 3 ? 2 : 1;        // that a warp takes at a time
+    // per SM that the registers must allow: beside small rings the compiler takes more than 128 where nothing is said
+    static constexpr uint32_t kCtas = WIDE && KC + VC <= 3 ? 2 : 1;
     static constexpr uint32_t kRingBytes = kWarps * kStages * kStageBytes;
     static constexpr uint32_t kColumns = 64 * VC;
     // the warps' partial results reuse the ring once every page has been consumed
-    static constexpr uint32_t kPartialBytes = kWarps * kGroupRows * kColumns * 4;
+    static constexpr uint32_t kPartialPitch = kColumns + 4;          // rows 2 apart lie 8 banks apart
+    static constexpr uint32_t kPartialBytes = kWarps * kGroupRows * kPartialPitch * 4;
     static constexpr uint32_t kBodyBytes = kRingBytes > kPartialBytes ? kRingBytes : kPartialBytes;
     // behind it: the CTA's result, maxima and sums per warp, maxima and sums per CTA, barriers, abort flag
     static constexpr uint32_t kResultBytes = kGroupRows * kColumns * 4;
     static constexpr uint32_t kSharedBytes = kBodyBytes + kResultBytes + (kWarps + 1) * kGroupRows * 8 +
                                              kWarps * kStages * 8 + 16 + 1024;
     static_assert(kSharedBytes <= 227 * 1024, "shared memory");
+    static constexpr uint32_t shared_bytes(bool alone) {
+        return alone && kSharedBytes < kAloneBytes ? kAloneBytes : kSharedBytes;
+    }
 };
 
 struct Params {
@@ -76,11 +93,11 @@ __device__ __forceinline__ uint32_t transposed_8x8(uint32_t pair) {
     return out;
 }
 
-template <uint32_t KC, uint32_t VC, uint32_t TILES>
-__global__ void __launch_bounds__(Layout<KC, VC>::kThreads)
+template <uint32_t KC, uint32_t VC, uint32_t TILES, bool WIDE>
+__global__ void __launch_bounds__(Layout<KC, VC, TILES, WIDE>::kThreads, Layout<KC, VC, TILES, WIDE>::kCtas)
 stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const __grid_constant__ CUtensorMap value_map,
                               const Params p) {
-    using L = Layout<KC, VC>;
+    using L = Layout<KC, VC, TILES, WIDE>;
     constexpr uint32_t kWarps = L::kWarps, kThreads = L::kThreads;
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31;
@@ -372,7 +389,7 @@ stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const
                     warp_top[warp * kGroupRows + row] = top[tile][h];
                     warp_sums[warp * kGroupRows + row] = sum[tile][h];
                 }
-                float* target = partial + (warp * kGroupRows + row) * L::kColumns + g;
+                float* target = partial + (warp * kGroupRows + row) * L::kPartialPitch + g;
 #pragma unroll
                 for (uint32_t m = 0; m < VC * 4; ++m) {
                     target[m * 16] = out[m][tile][h];
@@ -397,7 +414,7 @@ stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const
         for (uint32_t w = 0; w < kWarps; ++w) {
             const float factor = fast_exp2((warp_top[w * kGroupRows + row] - base) * scale_log2);
             total = fmaf(warp_sums[w * kGroupRows + row], factor, total);
-            value = fmaf(partial[(w * kGroupRows + row) * L::kColumns + column], factor, value);
+            value = fmaf(partial[(w * kGroupRows + row) * L::kPartialPitch + column], factor, value);
         }
         if (p.splits == 1) {
             if (!aborted) target[item] = __float2bfloat16_rn(total > 0.0f ? value / total : 0.0f);
@@ -438,18 +455,50 @@ stack_attention_decode_kernel(const __grid_constant__ CUtensorMap key_map, const
     cluster.sync();           // nobody leaves while its results are being read
 }
 
+// Clusters of `size` CTAs of the wide form that the device holds at once, asked once per kernel, size and spread.
 template <uint32_t KC, uint32_t VC, uint32_t TILES>
-cudaError_t launch_tiles(cudaStream_t stream, const StackAttentionLaunch& launch, uint32_t splits) {
-    using L = Layout<KC, VC>;
+size_t resident_clusters(uint32_t size, bool alone) {
+    using L = Layout<KC, VC, TILES, true>;
+    static std::atomic<int> answers[2][kMostSplits + 1];
+    std::atomic<int>& known = answers[alone ? 1 : 0][size];
+    int clusters = known.load(std::memory_order_relaxed);
+    if (clusters == 0) {
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(size, 1, 1);
+        config.blockDim = dim3(L::kThreads, 1, 1);
+        config.dynamicSmemBytes = L::shared_bytes(alone);
+        cudaLaunchAttribute attribute;
+        attribute.id = cudaLaunchAttributeClusterDimension;
+        attribute.val.clusterDim.x = size;
+        attribute.val.clusterDim.y = 1;
+        attribute.val.clusterDim.z = 1;
+        config.attrs = &attribute;
+        config.numAttrs = 1;
+        int count = 0;
+        if (cudaOccupancyMaxActiveClusters(&count, stack_attention_decode_kernel<KC, VC, TILES, true>, &config) != cudaSuccess) {
+            (void)cudaGetLastError();
+            count = 0;
+        }
+        clusters = count + 1;
+        known.store(clusters, std::memory_order_relaxed);
+    }
+    return static_cast<size_t>(clusters - 1);
+}
+
+template <uint32_t KC, uint32_t VC, uint32_t TILES, bool WIDE>
+cudaError_t allow_shared() {
+    return cudaFuncSetAttribute(reinterpret_cast<const void*>(stack_attention_decode_kernel<KC, VC, TILES, WIDE>),
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(Layout<KC, VC, TILES, WIDE>::shared_bytes(true)));
+}
+
+template <uint32_t KC, uint32_t VC, uint32_t TILES, bool WIDE>
+cudaError_t launch_form(cudaStream_t stream, const StackAttentionLaunch& launch, uint32_t splits, bool alone) {
+    using L = Layout<KC, VC, TILES, WIDE>;
     CUtensorMap key_map, value_map;
     if (!make_page_map(&key_map, launch, false) || !make_page_map(&value_map, launch, true)) {
         return cudaErrorInvalidValue;
     }
-    const auto kernel = stack_attention_decode_kernel<KC, VC, TILES>;
-    const cudaError_t status = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
-                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                    static_cast<int>(L::kSharedBytes));
-    if (status != cudaSuccess) return status;
     Params params;
     params.shape = launch.shape;
     params.query = static_cast<const __nv_bfloat16*>(launch.query);
@@ -465,35 +514,59 @@ cudaError_t launch_tiles(cudaStream_t stream, const StackAttentionLaunch& launch
     params.splits = splits;
     params.wait_limit = wait_limit_ns();
     const size_t blocks = launch.decode_tokens * launch.shape.kv_heads * splits;
-    return launch_kernel(kernel, static_cast<unsigned int>(blocks), L::kThreads, L::kSharedBytes, stream, splits, key_map,
-                         value_map, params);
+    return launch_kernel(stack_attention_decode_kernel<KC, VC, TILES, WIDE>, static_cast<unsigned int>(blocks), L::kThreads,
+                         L::shared_bytes(alone), stream, splits, key_map, value_map, params);
+}
+
+template <uint32_t KC, uint32_t VC, uint32_t TILES>
+cudaError_t launch_tiles(cudaStream_t stream, const StackAttentionLaunch& launch) {
+    cudaError_t status = allow_shared<KC, VC, TILES, true>();
+    if (status == cudaSuccess) status = allow_shared<KC, VC, TILES, false>();
+    if (status != cudaSuccess) return status;
+    const size_t clusters = launch.decode_tokens * launch.shape.kv_heads;
+    const size_t visible = launch.shape.chunk != 0 ? std::min<size_t>(launch.decode_context, launch.shape.chunk)
+                                                   : launch.decode_context;
+    const size_t pages = (visible + kPageSize - 1) / kPageSize;
+    constexpr size_t kWarps = Layout<KC, VC, TILES, true>::kWarps;
+    // Measured, in rounds of a page per warp (0.6 to 0.75 us; 1024 keys of one token and head 8 rounds, 10.4 us in one CTA and 9.4,
+    // 8.0, 8.2 in 2, 4, 8; 4096 keys 28.5 and 18.7, 12.7, 10.6): a cluster's merge costs 2.9 (2 or 4 CTAs) or 4.5 of them (8), a
+    // round half as much again where two CTAs share an SM and a group is one tile of columns, twice as much where it is two.
+    uint32_t splits = 0;
+    bool alone = false;
+    double best = 0.0;
+    for (uint32_t size = 1; size <= kMostSplits; size *= 2) {
+        const bool spread = clusters <= resident_clusters<KC, VC, TILES>(size, true);
+        const size_t resident = resident_clusters<KC, VC, TILES>(size, false);
+        if (!spread && (clusters > resident || (size > 1 && clusters * size > 2 * 148))) continue;
+        const double rounds = static_cast<double>((pages + kWarps * size - 1) / (kWarps * size));
+        const double cost = rounds * (spread ? 1.0 : (TILES == 1 ? 1.5 : 2.0)) + (size == 1 ? 0.0 : (size < 8 ? 2.9 : 4.5)) *
+                                                                                    (spread || TILES == 1 ? 1.0 : 2.0);
+        if (splits == 0 || cost < best) {
+            splits = size;
+            alone = spread;
+            best = cost;
+        }
+    }
+    if (splits > 0 && pages > kWarps / 2) return launch_form<KC, VC, TILES, true>(stream, launch, splits, alone);
+    return launch_form<KC, VC, TILES, false>(stream, launch, 1, clusters <= 148);
 }
 
 template <uint32_t KC, uint32_t VC>
-cudaError_t launch_sized(cudaStream_t stream, const StackAttentionLaunch& launch, uint32_t splits) {
-    return launch.shape.heads / launch.shape.kv_heads <= 8 ? launch_tiles<KC, VC, 1>(stream, launch, splits)
-                                                           : launch_tiles<KC, VC, 2>(stream, launch, splits);
+cudaError_t launch_sized(cudaStream_t stream, const StackAttentionLaunch& launch) {
+    return launch.shape.heads / launch.shape.kv_heads <= 8 ? launch_tiles<KC, VC, 1>(stream, launch)
+                                                           : launch_tiles<KC, VC, 2>(stream, launch);
 }
 
 template <uint32_t KC>
-cudaError_t launch_keys(cudaStream_t stream, const StackAttentionLaunch& launch, uint32_t splits) {
+cudaError_t launch_keys(cudaStream_t stream, const StackAttentionLaunch& launch) {
     switch ((launch.shape.vdim + 63) / 64) {
-        case 1: return launch_sized<KC, 1>(stream, launch, splits);
-        case 2: return launch_sized<KC, 2>(stream, launch, splits);
+        case 1: return launch_sized<KC, 1>(stream, launch);
+        case 2: return launch_sized<KC, 2>(stream, launch);
         default: return cudaErrorInvalidValue;
     }
 }
 
 }  // namespace
-
-// CTAs per token and head over the key axis: enough to fill the machine twice while a CTA keeps eight pages.
-uint32_t stack_attention_splits(const StackAttentionShape& shape, size_t tokens, size_t context) {
-    const size_t visible = shape.chunk != 0 ? std::min<size_t>(context, shape.chunk) : context;
-    const size_t pages = (visible + kPageSize - 1) / kPageSize;
-    uint32_t splits = 1;
-    while (splits < 8 && tokens * shape.kv_heads * splits * 2 <= 2 * 148 && pages >= 16 * splits) splits *= 2;
-    return splits;
-}
 
 bool stack_attention_decode_supports(const StackAttentionLaunch& launch) {
     const StackAttentionShape& shape = launch.shape;
@@ -502,12 +575,11 @@ bool stack_attention_decode_supports(const StackAttentionLaunch& launch) {
 }
 
 cudaError_t launch_stack_attention_decode(cudaStream_t stream, const StackAttentionLaunch& launch) {
-    const uint32_t splits = stack_attention_splits(launch.shape, launch.decode_tokens, launch.decode_context);
     switch ((launch.shape.dim + 63) / 64) {
-        case 1: return launch_keys<1>(stream, launch, splits);
-        case 2: return launch_keys<2>(stream, launch, splits);
-        case 3: return launch_keys<3>(stream, launch, splits);
-        case 4: return launch_keys<4>(stream, launch, splits);
+        case 1: return launch_keys<1>(stream, launch);
+        case 2: return launch_keys<2>(stream, launch);
+        case 3: return launch_keys<3>(stream, launch);
+        case 4: return launch_keys<4>(stream, launch);
         default: return cudaErrorInvalidValue;
     }
 }

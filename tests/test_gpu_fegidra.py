@@ -68,17 +68,22 @@ def test_attention_layer(device, dtype, shape):
 @pytest.mark.parametrize("heads,kv_heads,dim,copies", [(8, 2, 64, 1), (3, 3, 128, 1), (16, 16, 16, 1), (32, 8, 64, 1),
                                                        (32, 8, 64, 2), (16, 8, 128, 3)])
 def test_decode_attention_long_contexts(device, library_option, heads, kv_heads, dim, copies):
-    """Single tokens behind long and short contexts side by side, around borders of pages and of 1024 keys, in clusters of
-    8, 8, 2, 4, 2 and 1 CTAs per token and head (9 tokens times `copies`), against the general kernel: the weights keep 16
+    """Single tokens behind long and short contexts side by side, around borders of pages and of 1024 keys (9 tokens times
+    `copies`), with all keys of a token and head in one CTA and in clusters, against the general kernel: the weights keep 16
     bits in one and 32 in the other."""
+    check_decode_attention(device, library_option, heads, kv_heads, dim, [3, 1022, 1023, 1024, 40, 2047, 2048, 4100, 0] * copies)
+
+
+def check_decode_attention(device, library_option, heads, kv_heads, dim, prefixes):
     import torch
 
     from lfm25_inference_b200 import model as lfm_model
     from lfm25_inference_b200 import ops, stack, workloads
-    config = cases.config_of([cases.attention_layer(heads, kv_heads, dim, dim, 1 << 20, 8, ff=0)])
+    # values of more than 128 are no longer the decode kernel's
+    config = cases.config_of([cases.attention_layer(heads, kv_heads, dim, min(dim, 128), 1 << 20, 8, ff=0)])
     tensors = cases.random_tensors(config, 31)
-    prefixes = np.array([3, 1022, 1023, 1024, 40, 2047, 2048, 4100, 0] * copies)
-    pages = 800 * copies
+    prefixes = np.array(prefixes)
+    pages = int((prefixes // 16 + 1).sum()) + 5
     tokens = np.random.default_rng(5).integers(0, config["vocab"], size=len(prefixes)).astype(np.uint32)
     layout = workloads.mixed_step_batch(1, prefixes, np.ones(len(prefixes), np.int64), pages)
     results = []
@@ -100,11 +105,20 @@ def test_decode_attention_long_contexts(device, library_option, heads, kv_heads,
 
 
 @pytest.mark.parametrize("heads,kv_heads,dim,copies", [(8, 1, 64, 1), (9, 1, 64, 1), (16, 1, 64, 2), (24, 2, 128, 1), (16, 1, 72, 1),
-                                                       (6, 2, 136, 1), (13, 1, 256, 1)])
+                                                       (6, 2, 136, 1), (13, 1, 256, 1), (8, 8, 64, 5), (72, 8, 64, 5),
+                                                       (20, 2, 128, 9)])
 def test_decode_attention_groups(device, library_option, heads, kv_heads, dim, copies):
     """The same with groups of eight heads and less, which are one tile of columns, and beyond, with heads of one to four
-    pieces of 64: every number of warps, pages at a time and tiles of the decode kernel."""
+    pieces of 64, and with more CTAs than are resident at once: every form, number of pages at a time and tiles of the
+    decode kernel."""
     test_decode_attention_long_contexts(device, library_option, heads, kv_heads, dim, copies)
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim", [(8, 1, 64), (18, 2, 64), (6, 2, 128), (11, 1, 104), (2, 2, 256), (9, 1, 136)])
+@pytest.mark.parametrize("longest", [63, 64])
+def test_decode_attention_short_contexts(device, library_option, heads, kv_heads, dim, longest):
+    """Up to four pages, which four warps take, and the first page beyond."""
+    check_decode_attention(device, library_option, heads, kv_heads, dim, [0, 15, 16, 40, 47, longest])
 
 
 @pytest.mark.parametrize("dtype", TYPES)
