@@ -67,12 +67,24 @@ struct Params {
     uint64_t wait_limit;
 };
 
-// Weights of a stage as the second operand of O^T: a line of 128 bytes per key holds 64 columns, the high parts of all heads and
+// Weights of a stage as the second operand of O^T: a line per key holds 64 columns (128 bytes), the high parts of all heads and
 // then their low parts, so that a softmax thread stores what it has of a key in pieces of 16 bytes.  With a line per head, in
 // pieces of two bytes, 32 tokens of 128 to 4096 keys took 49.3 instead of 46.1 us, 32 of 4096 keys 52.7 instead of 49.7 us, 128
-// of 1024 keys 64.6 instead of 60.7 us (32 heads, latents of 512 dimensions).
-constexpr uint32_t kWeightBlock = kKeys * 128;
-constexpr __host__ __device__ uint32_t weight_bytes(uint32_t heads) { return (2 * heads + 63) / 64 * kWeightBlock; }
+// of 1024 keys 64.6 instead of 60.7 us (32 heads, latents of 512 dimensions).  16 heads have 32 columns: lines of 64 bytes, so that
+// the ring keeps its slots (in lines of 128 bytes keys of 8 chunks were left two of three: three layers of 32 tokens of 4096 keys
+// 270 instead of 227 us a step, and 229 with a line per head).
+template <uint32_t N>
+struct Weights {
+    static constexpr uint32_t kLine = 2 * N < 64 ? 4 * N : 128;               // bytes, and the width of the swizzle
+    static constexpr uint32_t kBlock = kKeys * kLine;
+    static constexpr uint32_t kBytes = (4 * N + kLine - 1) / kLine * kBlock;
+    static_assert(kLine == 64 || kLine == 128, "widths that the swizzle has");
+    // where 16 bytes of `key` from `column` on lie: pieces of a line change places with bits 7 and up of the address
+    static __device__ __forceinline__ uint32_t at(uint32_t key, uint32_t column) {
+        const uint32_t piece = column % (kLine / 2) / 8, turn = kLine == 128 ? key % 8 : key / 2 % 4;
+        return column / (kLine / 2) * kBlock + key * kLine + ((piece ^ turn) << 4);
+    }
+};
 
 // Floats and barriers behind the ring
 template <uint32_t N>
@@ -96,7 +108,7 @@ struct Control {
 
 template <uint32_t N>
 constexpr size_t shared_bytes(uint32_t chunks, uint32_t stages) {
-    return 1024 + static_cast<size_t>(chunks) * N * 128 + 2 * weight_bytes(N) +
+    return 1024 + static_cast<size_t>(chunks) * N * 128 + 2 * Weights<N>::kBytes +
            static_cast<size_t>(stages) * chunks * kGroups * kChunkBytes + sizeof(Control<N>);
 }
 
@@ -129,14 +141,15 @@ __device__ __forceinline__ void load_4d(uint32_t dst, const void* tensor_map, ui
         : "memory");
 }
 
-// Operand with 128-byte swizzle whose 8-line groups are `group_bytes` apart.  K-major (lines are rows): `leading_bytes` is
-// not used.  MN-major (a line holds 64 rows at one k): the next 64 rows lie `leading_bytes` further on.
+// Operand with 128-byte (LINE: or 64-byte) swizzle whose 8-line groups are `group_bytes` apart.  K-major (lines are rows):
+// `leading_bytes` is not used.  MN-major (a line holds 64 rows at one k): the next 64 rows lie `leading_bytes` further on.
+template <uint32_t LINE = 128>
 __device__ __forceinline__ uint64_t descriptor(uint32_t address, uint32_t group_bytes, uint32_t leading_bytes) {
     uint64_t value = static_cast<uint64_t>((address & 0x3ffff) >> 4);
     value |= static_cast<uint64_t>(leading_bytes >> 4) << 16;
     value |= static_cast<uint64_t>(group_bytes >> 4) << 32;
     value |= static_cast<uint64_t>(1) << 46;
-    value |= static_cast<uint64_t>(2) << 61;
+    value |= static_cast<uint64_t>(LINE == 128 ? 2 : 4) << 61;
     return value;
 }
 
@@ -185,8 +198,8 @@ latent_attention_umma_kernel(const __grid_constant__ CUtensorMap absorbed_map,
     const uint32_t stage_bytes = kGroups * p.chunks * kChunkBytes;
     const uint32_t q_base = smem_u32(smem);
     const uint32_t p_base = q_base + p.chunks * N * 128;         // two buffers of weights
-    const uint32_t ring = p_base + 2 * weight_bytes(N);
-    uint8_t* ring_bytes = smem + p.chunks * N * 128 + 2 * weight_bytes(N);
+    const uint32_t ring = p_base + 2 * Weights<N>::kBytes;
+    uint8_t* ring_bytes = smem + p.chunks * N * 128 + 2 * Weights<N>::kBytes;
     Control<N>& control = *reinterpret_cast<Control<N>*>(ring_bytes + p.stages * stage_bytes);
     const uint32_t bar_full = smem_u32(control.full);
     const uint32_t bar_empty = smem_u32(control.empty);
@@ -377,7 +390,8 @@ latent_attention_umma_kernel(const __grid_constant__ CUtensorMap absorbed_map,
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tcgen05_fence_after();
-                const uint64_t weights = descriptor(p_base + buffer * weight_bytes(N), 1024, kWeightBlock);
+                const uint64_t weights = descriptor<Weights<N>::kLine>(p_base + buffer * Weights<N>::kBytes, 8 * Weights<N>::kLine,
+                                                                           Weights<N>::kBlock);
                 uint64_t v_desc = descriptor(ring + stage * stage_bytes, group_bytes, kChunkBytes);
                 if (issuer) {
 #pragma unroll
@@ -385,7 +399,7 @@ latent_attention_umma_kernel(const __grid_constant__ CUtensorMap absorbed_map,
                         if (step < present) {
                             for (uint32_t block = 0; block < p.blocks; ++block) {
                                 mma_shared(tmem_out + block * 2 * N, v_desc + block * (2 * kChunkBytes >> 4),
-                                           weights + step * (kPageSize * 128 >> 4), idesc_out, index + step);
+                                           weights + step * (kPageSize * Weights<N>::kLine >> 4), idesc_out, index + step);
                             }
                         }
                         v_desc += 2 * group_bytes >> 4;
@@ -494,7 +508,7 @@ latent_attention_umma_kernel(const __grid_constant__ CUtensorMap absorbed_map,
             if (index >= 2) {
                 ok = mbar_wait_bounded(bar_product + 8 * buffer, ((index >> 1) - 1) & 1, p.wait_limit) && ok;
             }
-            uint8_t* line = smem + p.chunks * N * 128 + buffer * weight_bytes(N) + key * 128;
+            uint8_t* weights = smem + p.chunks * N * 128 + buffer * Weights<N>::kBytes;
 #pragma unroll
             for (uint32_t part = 0; part < kShare / 8; ++part) {
                 uint32_t high[4], low[4];
@@ -511,11 +525,9 @@ latent_attention_umma_kernel(const __grid_constant__ CUtensorMap absorbed_map,
                     low[pair] = pack_bf16x2(first - rounded.x, second - rounded.y);
                 }
                 if (lane < 16) {
-                    const auto columns = [&](uint32_t column) {
-                        return reinterpret_cast<uint4*>(line + column / 64 * kWeightBlock + ((column % 64 / 8 ^ key % 8) << 4));
-                    };
-                    *columns(first_head + part * 8) = make_uint4(high[0], high[1], high[2], high[3]);
-                    *columns(N + first_head + part * 8) = make_uint4(low[0], low[1], low[2], low[3]);
+                    const uint32_t column = first_head + part * 8;
+                    *reinterpret_cast<uint4*>(weights + Weights<N>::at(key, column)) = make_uint4(high[0], high[1], high[2], high[3]);
+                    *reinterpret_cast<uint4*>(weights + Weights<N>::at(key, N + column)) = make_uint4(low[0], low[1], low[2], low[3]);
                 }
             }
             // latents behind the last key may hold anything: clear them (a zero weight times a NaN pattern is NaN)

@@ -44,6 +44,7 @@ LATENT_SHAPES = [   # heads, dim, rot_dim, vdim, q_rank, kv_rank
     (20, 48, 16, 40, 40, 192),         # more heads than one block of columns, an odd number of latent chunks
     (70, 16, 32, 24, 24, 64),          # several blocks of 64 heads
     (40, 32, 128, 32, 56, 448),        # a rotated part of two chunks
+    (9, 32, 64, 32, 24, 448),          # keys of eight chunks for one block of 16 columns
     (2, 192, 64, 128, 48, 96),
     (3, 200, 64, 72, 32, 64),          # keys beyond the prompt kernel
     (2, 64, 32, 136, 32, 64),          # values beyond it
