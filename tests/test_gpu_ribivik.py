@@ -76,6 +76,7 @@ STATE_SHAPES = [    # heads, vdim, state, groups, norm_groups, conv
     (4, 64, 128, 1, 1, 4),
     (8, 64, 64, 2, 8, 4),
     (2, 128, 256, 2, 1, 4),
+    (2, 64, 192, 1, 1, 4),
     (3, 48, 80, 1, 3, 4),
     (5, 40, 24, 5, 4, 2),
     (2, 16, 512, 1, 1, 4),
@@ -93,7 +94,7 @@ def test_state_space_layer(device, dtype, shape):
     check_layers(config, 13, device, dtype, [70, 2, 1, 16, 1, 5, 133])
 
 
-@pytest.mark.parametrize("shape", STATE_SHAPES[:5] + [(4, 64, 96, 2, 1, 4), (2, 24, 200, 1, 1, 4)],
+@pytest.mark.parametrize("shape", STATE_SHAPES[:6] + [(4, 64, 96, 2, 1, 4), (2, 24, 136, 1, 1, 4), (2, 24, 200, 1, 1, 4)],
                          ids=lambda shape: "x".join(map(str, shape)))
 def test_state_space_prompt_kernels_agree(device, library_option, shape):
     """Chunks on the tensor cores and the token-by-token kernel on the same bf16 inputs: both keep the recurrence in 32
@@ -108,7 +109,8 @@ def test_state_space_prompt_kernels_agree(device, library_option, shape):
     assert cases.relative_error(results[1], results[0]).max() < 4e-3
 
 
-@pytest.mark.parametrize("shape", [(4, 64, 128, 1, 1, 4), (8, 64, 64, 2, 8, 4), (2, 128, 256, 2, 1, 4), (5, 40, 24, 5, 4, 2)],
+@pytest.mark.parametrize("shape", [(4, 64, 128, 1, 1, 4), (8, 64, 64, 2, 8, 4), (2, 128, 256, 2, 1, 4), (5, 40, 24, 5, 4, 2),
+                                   (3, 64, 192, 1, 1, 4)],
                          ids=lambda shape: "x".join(map(str, shape)))
 def test_state_space_in_pieces(device, library_option, shape):
     """Sequences long enough to be cut into pieces, behind single tokens and beside short ones, against the token-by-token
