@@ -9,12 +9,12 @@
 //     output     norm and gate                                                   one warp per token and head
 // What bounds them: `scan` the latency of the chain (about 290 cycles a token in heads of 64), so a head's columns are spread
 // over as many CTAs as there are groups of eight or sixteen, operands arrive through cp.async a tile ahead and, for heads up to
-// 64, in registers a token ahead, and the result of a token is reduced beside the dot product of the next one.  Eight lanes a
+// 128, in registers a token ahead, and the result of a token is reduced beside the dot product of the next one.  Eight lanes a
 // column: with four a thread's reads of its operands outweigh the shorter sum, with sixteen nothing is left to win (48, 60 and
-// 48 us below).  `elements` and `scan` let their successors in at their end only: CTAs of `scan` that start early are put on the
-// SMs that `elements` has left free, several on one, and share its issue slots and shared memory for the whole scan (81 -> 116).
-// 250 tokens, 16 heads of 64: 49 us for the three; preparation and recurrence in turns in one CTA per head: 219 us.  Eight
-// segments of 200 tokens: 154 and 234 us.
+// 48 us below).  `elements` lets its successor in at its end only: CTAs of `scan` that start early are put on the SMs that
+// `elements` has left free, several on one, and share its issue slots and shared memory for the whole scan (81 -> 116).
+// 250 tokens, 16 heads of 64 with ranks of 64: 47 us for the three; preparation and recurrence in turns in one CTA per head:
+// 219 us.  Eight segments of 200 tokens: 143 and 234 us; 16 heads of 128 with ranks of 224, bf16: 425 and 451 us.
 #include <algorithm>
 
 #include "delta_rule.h"
@@ -25,11 +25,11 @@ namespace lfm25 {
 namespace {
 
 constexpr uint32_t kElementTokens = 16;      // tokens per CTA of the elements kernel
-constexpr uint32_t kElementThreads = 256;
-// Values of tanh(z) per token that a launch of the elements kernel holds in shared memory, beside a word per token: as many as
-// every kernel may have without asking.  Larger ranks take several launches, which leave the logits in the place of w.
+// Values of tanh(z) per token that a launch of the elements kernel holds in shared memory; larger ranks take several launches,
+// which leave the logits in the place of w.
 constexpr uint32_t kRankBlock = 760;
-static_assert(kRankBlock % 8 == 0 && kElementTokens * (1 + kRankBlock) * sizeof(float) <= 48 * 1024, "whole pieces of W2's rows");
+// 128 threads are as many as 16 tokens of 32 channels need
+constexpr __host__ __device__ uint32_t element_threads(uint32_t dim) { return dim <= 32 ? 128 : 256; }
 constexpr uint32_t kVectors = 6;             // r, w, -(a * u), u, k, v
 constexpr uint32_t kValues = 5;              // place of v, and of the result after the scan
 
@@ -42,61 +42,123 @@ struct ScanVectors {
     }
 };
 
+__host__ __device__ constexpr uint32_t padded_rank(uint32_t count) { return (count + 7) / 8 * 8; }
+// Columns of W2 in shared memory at a time, and elements between its rows: an odd number of 16-byte pieces, so that the rows'
+// pieces lie in different banks.
+template <uint32_t DP>
+constexpr uint32_t kTileRank = DP <= 64 ? 512 : (DP <= 128 ? 320 : 160);
+template <uint32_t DP>
+__host__ __device__ constexpr uint32_t tile_pitch(uint32_t z_count) {
+    return ((z_count < kTileRank<DP> ? padded_rank(z_count) : kTileRank<DP>) / 8 | 1) * 8;
+}
+template <uint32_t DP>
+constexpr size_t element_bytes(uint32_t z_count) {
+    return kElementTokens * (1 + static_cast<size_t>(padded_rank(z_count))) * sizeof(float) +
+           static_cast<size_t>(DP) * tile_pitch<DP>(z_count) * 2;
+}
+static_assert(kRankBlock % 8 == 0 && element_bytes<128>(kRankBlock) <= 227 * 1024 && element_bytes<256>(kRankBlock) <= 227 * 1024,
+              "whole pieces, in shared memory");
+
+// One channel and groups of four tokens per thread, so that a value of W2 serves four tokens.  W2 is constant and on its way to
+// shared memory before the dependency wait; from global memory a thread's row would fetch 32 bytes for every 16 that are used.
+// Bound by the latency of its loads, so registers are kept for four CTAs of 256 threads per SM, and a round trip to memory serves
+// keys, z and the first tokens' values.  1600 tokens of 32 heads of 64 with ranks of 64, f32: 67 us, and 120 with W2 from global
+// memory and 64 values of a row in registers; 16 heads of 128 with ranks of 256, bf16: 144 and 419 us.
 template <typename T, uint32_t DP>
-__global__ void __launch_bounds__(kElementThreads, 2)
+__global__ void __launch_bounds__(element_threads(DP), 1024 / element_threads(DP))
 delta_scan_elements_kernel(const DeltaArgs<T> args, const ScanVectors vectors, uint32_t first_z, uint32_t z_count) {
+    constexpr uint32_t kThreads = element_threads(DP), kWarps = kThreads / 32;
     extern __shared__ __align__(16) float element_shared[];
-    const uint32_t padded_z = (z_count + 3) / 4 * 4;
+    const uint32_t padded_z = padded_rank(z_count);
     float* unit_scale = element_shared;                                // [token]
-    float* z_values = element_shared + kElementTokens;                 // [token][padded_z], tanh applied
+    float* z_values = element_shared + kElementTokens;                 // [token][padded_z], tanh applied, zeros behind z_count
+    auto* tile = reinterpret_cast<__nv_bfloat16*>(z_values + kElementTokens * padded_z);      // of W2, [channel][pitch]
+    const uint32_t pitch = tile_pitch<DP>(z_count);
     const uint32_t head = blockIdx.x % vectors.heads;
     const size_t first = static_cast<size_t>(blockIdx.x / vectors.heads) * kElementTokens;
     const uint32_t tokens = static_cast<uint32_t>(min(args.segments.num_tokens - first, size_t(kElementTokens)));
     const uint32_t dim = args.dim;
     const size_t width = static_cast<size_t>(args.heads) * dim;
     const size_t head_base = static_cast<size_t>(vectors.first_head + head) * dim;
-    // One channel and groups of four tokens per thread, so that a value of W2 serves four tokens.  The first kEarly values of
-    // the channel's row of W2 are constants and on their way before the dependency wait.
-    constexpr uint32_t kGroups = kElementThreads / DP;
-    constexpr uint32_t kEarly = 64;
+    constexpr uint32_t kGroups = kThreads / DP;
     const uint32_t channel = threadIdx.x % DP;
     const bool live = channel < dim;
     const size_t index = head_base + (live ? channel : 0);
-    const __nv_bfloat16* decay_row = args.decay_up + index * args.rank + first_z;
-    const bool vector_rank = args.rank % 8 == 0 && (reinterpret_cast<uintptr_t>(args.decay_up) & 15) == 0;
-    uint4 early[kEarly / 8] = {};
-    if (vector_rank) {
-#pragma unroll
-        for (uint32_t i = 0; i < kEarly / 8; ++i) {
-            if (i * 8 < z_count) early[i] = *reinterpret_cast<const uint4*>(decay_row + i * 8);
+    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+
+    // W2 from z on, zeros behind z_count and the head's channels, in the largest pieces that every row can be read in
+    const __nv_bfloat16* decay_rows = args.decay_up + head_base * args.rank + first_z;
+    const uint32_t alignment = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(args.decay_up) | args.rank * 2);
+    auto load_tile = [&](uint32_t z) {
+        const uint32_t count = min(z_count - z, kTileRank<DP>), columns = padded_rank(count);
+        for (uint32_t row = warp; row < DP; row += kWarps) {
+            const __nv_bfloat16* source = decay_rows + static_cast<size_t>(row) * args.rank + z;
+            __nv_bfloat16* target = tile + row * pitch;
+            if (alignment % 16 == 0) {
+                for (uint32_t column = lane * 8; column < columns; column += 256) {
+                    copy_async_16(target + column, row < dim ? source + column : args.decay_up, row < dim);
+                }
+            } else if (alignment % 4 == 0) {
+                for (uint32_t column = lane * 2; column < columns; column += 64) {
+                    const bool inside = row < dim && column < count;   // the rank is even
+                    copy_async_4(target + column, inside ? source + column : args.decay_up, inside);
+                }
+            } else {
+                for (uint32_t column = lane; column < columns; column += 32) {
+                    target[column] = row < dim && column < count ? source[column] : __float2bfloat16_rn(0.0f);
+                }
+            }
         }
-    }
+        copy_async_commit();
+    };
+    load_tile(0);
     const float bias = __bfloat162float(args.removal_bias[index]), base = __bfloat162float(args.decay_base[index]);
     pdl_wait();
     if (first + tokens <= args.segments.offsets[0]) {
+        copy_async_wait<0>();
         return;                                                        // single tokens in front of the prompts
     }
-    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    for (uint32_t t = warp; t < tokens; t += kElementThreads / 32) {
-        const T* row = args.projected + (first + t) * args.pitch;
-        float sum = 0.0f;
-        for (uint32_t channel = lane; channel < dim; channel += 32) {
-            const float value = to_float<T>(row[width + head_base + channel]);
-            sum = fmaf(value, value, sum);
+    float r[4], k[4], v[4], rate[4];
+    auto load_tokens = [&](uint32_t t0) {
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            r[i] = k[i] = v[i] = rate[i] = 0.0f;
+            if (live && t0 + i < tokens) {
+                const T* row = args.projected + (first + t0 + i) * args.pitch + index;
+                r[i] = to_float<T>(row[0]);
+                k[i] = to_float<T>(row[width]);
+                v[i] = to_float<T>(row[2 * width]);
+                rate[i] = to_float<T>(row[4 * width]);
+            }
         }
+    };
+    load_tokens(threadIdx.x / DP * 4);                                 // on their way while norms and tanh(z) are formed
+    for (uint32_t t = warp; t < kElementTokens; t += kWarps) {
+        const T* row = args.projected + (first + t) * args.pitch;
+        float keys[DP / 32], sum = 0.0f;
+#pragma unroll
+        for (uint32_t i = 0; i < DP / 32; ++i) {
+            keys[i] = t < tokens && lane + i * 32 < dim ? to_float<T>(row[width + head_base + lane + i * 32]) : 0.0f;
+        }
+        for (uint32_t z0 = lane; z0 < padded_z; z0 += 128) {           // four loads at a time
+            float raw[4];
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                const uint32_t z = z0 + i * 32;
+                raw[i] = t < tokens && z < z_count ? to_float<T>(row[5 * width + first_z + z]) : 0.0f;
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                if (z0 + i * 32 < padded_z) z_values[t * padded_z + z0 + i * 32] = tanhf(raw[i]);
+            }
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < DP / 32; ++i) sum = fmaf(keys[i], keys[i], sum);
         sum = warp_sum(sum);
         if (lane == 0) unit_scale[t] = 1.0f / sqrtf(sum + kUnitEps);
     }
-    for (uint32_t item = threadIdx.x; item < kElementTokens * padded_z; item += kElementThreads) {
-        const uint32_t t = item / padded_z, z = item % padded_z;
-        z_values[item] = t < tokens && z < z_count
-                             ? tanhf(to_float<T>(args.projected[(first + t) * args.pitch + 5 * width + first_z + z]))
-                             : 0.0f;
-    }
+    copy_async_wait<0>();
     __syncthreads();
-    if (channel >= vectors.pitch) {
-        return;
-    }
     // products of eight values of W2 with those of four tokens, in the order of the values
     auto add_products = [&](const uint4& raw, uint32_t t0, uint32_t z, float (&logit)[4]) {
         const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -114,40 +176,32 @@ delta_scan_elements_kernel(const DeltaArgs<T> args, const ScanVectors vectors, u
             }
         }
     };
-    for (uint32_t t0 = threadIdx.x / DP * 4; t0 < tokens; t0 += kGroups * 4) {
-        float r[4] = {}, k[4] = {}, v[4] = {}, rate[4] = {};
-#pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-            if (live && t0 + i < tokens) {
-                const T* row = args.projected + (first + t0 + i) * args.pitch + index;
-                r[i] = to_float<T>(row[0]);
-                k[i] = to_float<T>(row[width]);
-                v[i] = to_float<T>(row[2 * width]);
-                rate[i] = to_float<T>(row[4 * width]);
-            }
-        }
+    uint32_t held = 0;                                                 // where the tile in shared memory begins
+    for (uint32_t turn = 0; turn < tokens; turn += kGroups * 4) {
+        const uint32_t t0 = threadIdx.x / DP * 4 + turn;
+        if (turn > 0) load_tokens(t0);
         float logit[4] = {};
-        if (first_z > 0) {
+        if (first_z > 0 && channel < vectors.pitch) {
 #pragma unroll
             for (uint32_t i = 0; i < 4; ++i) {
                 if (t0 + i < tokens) logit[i] = vectors.at(first + t0 + i, head)[vectors.pitch + channel];
             }
         }
-        if (vector_rank) {
-#pragma unroll
-            for (uint32_t i = 0; i < kEarly / 8; ++i) {
-                if (i * 8 < z_count) add_products(early[i], t0, i * 8, logit);
+        const uint32_t row0 = min(t0, kElementTokens - 4);             // threads without tokens stay for the barriers
+        for (uint32_t z = 0; z < z_count; z += kTileRank<DP>) {
+            if (z != held) {
+                __syncthreads();
+                load_tile(z);
+                copy_async_wait<0>();
+                __syncthreads();
+                held = z;
             }
-            for (uint32_t z = kEarly; z < z_count; z += 8) {
-                add_products(*reinterpret_cast<const uint4*>(decay_row + z), t0, z, logit);
-            }
-        } else {
-            for (uint32_t z = 0; z < z_count; ++z) {
-                const float weight = __bfloat162float(decay_row[z]);
-#pragma unroll
-                for (uint32_t i = 0; i < 4; ++i) logit[i] = fmaf(weight, z_values[(t0 + i) * padded_z + z], logit[i]);
+            const uint32_t count = min(z_count - z, kTileRank<DP>);
+            for (uint32_t at = 0; at < count; at += 8) {
+                add_products(*reinterpret_cast<const uint4*>(tile + channel * pitch + at), row0, z + at, logit);
             }
         }
+        if (channel >= vectors.pitch) continue;
 #pragma unroll
         for (uint32_t i = 0; i < 4; ++i) {
             const uint32_t t = t0 + i;
@@ -179,11 +233,13 @@ struct ScanShape {
     static constexpr uint32_t kThreads = LANES * COLUMNS;
     static constexpr uint32_t kRows = DP / LANES;
     static constexpr uint32_t kGroups = kRows / 4;
-    static constexpr uint32_t kTokens = DP <= 64 ? 16 : 8;                  // per stage
+    // Per stage.  Heads beyond 128: with 8 two CTAs fit an SM instead of four (bf16, 4 heads of 160, 8 x 200 tokens 369 -> 281 us
+    // a layer; one prompt of 4096 tokens pays 3 %).
+    static constexpr uint32_t kTokens = DP <= 64 ? 16 : (DP <= 128 ? 8 : 4);
     static constexpr uint32_t kTokenFloats = 5 * DP + COLUMNS;         // r, w, removal, u, k over DP channels, v
     static constexpr uint32_t kPieces = (kTokenFloats / 4 + 31) / 32;       // 16-byte pieces of a token per lane of a warp
     static constexpr size_t kShared = (2 * kTokens + 1) * kTokenFloats * sizeof(float);
-    static_assert(kRows % 4 == 0, "four consecutive key channels per access");
+    static_assert(kRows % 4 == 0 && kTokenFloats % 4 == 0, "four consecutive key channels per access");
     static_assert(kShared <= 227 * 1024, "shared memory");
 };
 
@@ -239,8 +295,12 @@ delta_scan_kernel(const DeltaArgs<T> args, const ScanVectors vectors) {
         state[2 * g + 1] = pair_of(value.z, value.w);
     }
     // channels behind the pitch are never copied and stay zero
-    for (uint32_t item = threadIdx.x; item < (2 * kTokens + 1) * Shape::kTokenFloats; item += kThreads) scan_shared[item] = 0.0f;
-    __syncthreads();
+    if (pitch < DP) {
+        for (uint32_t item = threadIdx.x; item < (2 * kTokens + 1) * Shape::kTokenFloats / 4; item += kThreads) {
+            reinterpret_cast<float4*>(scan_shared)[item] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        __syncthreads();
+    }
 
     // 16-byte pieces of a token: r, w, removal, u, k and this CTA's part of v.  A warp moves a token; where its lanes' pieces
     // lie does not change.
@@ -351,6 +411,7 @@ delta_scan_kernel(const DeltaArgs<T> args, const ScanVectors vectors) {
         }
         __syncthreads();
     }
+    pdl_launch_dependents();
 #pragma unroll
     for (uint32_t delta = 1; delta < LANES; delta <<= 1) pending += __shfl_xor_sync(0xffffffffu, pending, delta);
     store(pending);
@@ -400,6 +461,14 @@ delta_scan_output_kernel(const DeltaArgs<T> args, const ScanVectors vectors) {
 
 size_t head_bytes(size_t tokens, uint32_t dim) { return tokens * kVectors * ((dim + 3) / 4 * 4) * sizeof(float); }
 
+// of kernels without static shared memory
+template <typename Kernel>
+cudaError_t allow_shared(Kernel kernel, size_t bytes) {
+    if (bytes <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(bytes));
+}
+
 template <typename T, uint32_t DP, uint32_t LANES, uint32_t COLUMNS>
 cudaError_t launch_sized(cudaStream_t stream, DeltaArgs<T> args, ScanVectors vectors, uint32_t heads_at_once) {
     using Shape = ScanShape<DP, LANES, COLUMNS>;
@@ -407,20 +476,16 @@ cudaError_t launch_sized(cudaStream_t stream, DeltaArgs<T> args, ScanVectors vec
     args.splits = (args.dim + COLUMNS - 1) / COLUMNS;
     const auto elements = delta_scan_elements_kernel<T, DP>;
     const auto scan = delta_scan_kernel<T, DP, LANES, COLUMNS>;
-    cudaError_t status = cudaSuccess;
-    if (Shape::kShared > 48 * 1024) {
-        status = cudaFuncSetAttribute(reinterpret_cast<const void*>(scan), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(Shape::kShared));
-    }
+    cudaError_t status = allow_shared(scan, Shape::kShared);
+    if (status == cudaSuccess) status = allow_shared(elements, element_bytes<DP>(std::min(args.rank, kRankBlock)));
     for (uint32_t first = 0; first < args.heads && status == cudaSuccess; first += heads_at_once) {
         vectors.first_head = first;
         vectors.heads = std::min(heads_at_once, args.heads - first);
         const size_t tiles = (tokens + kElementTokens - 1) / kElementTokens;
         for (uint32_t first_z = 0; first_z < args.rank && status == cudaSuccess; first_z += kRankBlock) {
             const uint32_t z_count = std::min(args.rank - first_z, kRankBlock);
-            const size_t shared = static_cast<size_t>(kElementTokens) * (1 + (z_count + 3) / 4 * 4) * sizeof(float);
-            status = launch_kernel(elements, static_cast<unsigned int>(tiles * vectors.heads), kElementThreads, shared, stream, 1,
-                                   args, vectors, first_z, z_count);
+            status = launch_kernel(elements, static_cast<unsigned int>(tiles * vectors.heads), element_threads(DP),
+                                   element_bytes<DP>(z_count), stream, 1, args, vectors, first_z, z_count);
         }
         if (status != cudaSuccess) break;
         status = launch_kernel(scan, static_cast<unsigned int>(args.segments.num_segments * vectors.heads * args.splits),

@@ -84,6 +84,10 @@ __device__ __forceinline__ void copy_async_16(void* target, const void* source, 
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(target)), "l"(source), "r"(inside ? 16 : 0)
                  : "memory");
 }
+__device__ __forceinline__ void copy_async_4(void* target, const void* source, bool inside) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(target)), "l"(source), "r"(inside ? 4 : 0)
+                 : "memory");
+}
 __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <uint32_t NEWER>
 __device__ __forceinline__ void copy_async_wait() {
