@@ -12,8 +12,8 @@
 // Short sums of 32, 64, 128 and 256 products: 1.17, 1.07, 1.37 and 2.38e-7 from float64 (2-norm, k = 1024, not in pairs), all of
 // k in one: 1.0e-6.
 //
-// A tile is 128 weight rows (the M operand, from TMA) times N rows of x (the N operand).  Per 64 of k a slot of the ring holds
-// the weights and the three parts of x.  Warps:
+// A tile is 128 weight rows (the M operand, from TMA) times N rows of x (the N operand), 16, 32, 64 or 96.  Per 64
+// of k a slot of the ring holds the weights and the three parts of x.  Warps:
 //     0         TMA loads of the weights; the first ring is requested before the dependency wait (they are constants)
 //     1         issues the MMAs: four for the high parts into one of four accumulators that take turns, eight for the others,
 //               and allocates tensor memory.  One commit and two waits a slot: with a barrier for each purpose and short sums of
@@ -24,10 +24,13 @@
 // 100 + 16 N cycles, the MMAs' arithmetic 6 N.  Where the tiles do not fill the device, the CTAs of a cluster share a tile's
 // k range and add their f32 parts in rank order through distributed shared memory.
 //
-// Against the same products through mma.sync (three 16x8x16 per block, 64 x 128 outputs per CTA), us:
+// Against the same products through mma.sync (three 16x8x16 per block, 64 x 128 outputs per CTA), us, launches back to back and
+// weights beyond the L2:
 //     rows x n x k     250x6144x1024   250x1024x7168   64x6144x1024   16x1024x7168   1x32768x1024   2500x2048x12288
-//     mma.sync                  49.7            46.1           17.4           14.8           20.2              1553
-//     here                      19.1            24.6           10.6           12.1           13.8               610
+//     mma.sync                  49.1            45.3           16.7           18.4           22.4              1553
+//     here                      19.1            24.9            9.9           10.2           13.1               615
+// Up to 16 rows take tiles of 16: 1 x 6144 x 1024 7.9 / 7.2, 16 x 1024 x 2048 6.7 / 6.1 (in tiles of 32 8.2 and 7.0, 16 x 64 x 64
+// 2.3 / 2.6 instead of 2.1); 16 x 2048 x 2048, four blocks of k in 128 CTAs, stays behind with 7.4 / 7.9.
 //
 // Every mbarrier wait is bounded; a wait that runs out sets the CTA's abort flag, is recorded in the device status words, and
 // the CTA (in a cluster: all its CTAs) leaves without storing, once its copies and MMAs are through (drain()).
@@ -64,9 +67,12 @@ struct Shape {
     static constexpr uint32_t kStages = (kBudget - kControlBytes) / kStageBytes < kMaxStages
                                             ? (kBudget - kControlBytes) / kStageBytes : kMaxStages;
     static constexpr uint32_t kShared = kStages * kStageBytes + kControlBytes;
-    static constexpr uint32_t kColumns = 5 * N <= 256 ? 256 : 512;       // of tensor memory: four short sums, the rest
+    // of tensor memory: four short sums, the rest
+    static constexpr uint32_t kColumns = N == 16 ? 128 : (5 * N <= 256 ? 256 : 512);
+    static constexpr uint32_t kPiece = N == 16 ? 8 : 16;                   // columns that an adding thread reads at a time
     static constexpr uint32_t kLoads = N / (2 * kConverters);              // float4 of x per converting thread and slot
-    static_assert(N % 32 == 0 && N * kTileM * 4 <= kStages * kStageBytes, "whole loads; a parked tile fits the ring");
+    static_assert(N % 16 == 0 && N / 2 % kPiece == 0, "whole loads");
+    static_assert(N * kTileM * 4 <= kStages * kStageBytes, "a parked tile fits the ring");
 };
 
 struct LinearParams {
@@ -130,6 +136,9 @@ __device__ __forceinline__ void umma(uint32_t accumulator, uint64_t a, uint64_t 
         "l"(a), "l"(b), "r"(descriptor), "r"(accumulate)
         : "memory");
 }
+
+__device__ __forceinline__ void load_columns(uint32_t address, uint32_t (&raw)[8]) { tmem_load8_nowait(address, raw); }
+__device__ __forceinline__ void load_columns(uint32_t address, uint32_t (&raw)[16]) { tmem_load16_nowait(address, raw); }
 
 __device__ __forceinline__ void store_shared(uint32_t address, uint32_t value) {
     asm volatile("st.shared.u32 [%0], %1;" ::"r"(address), "r"(value) : "memory");
@@ -349,14 +358,14 @@ linear_f32_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const Lin
             tcgen05_fence_after();
             const uint32_t source = address + (pair & 1) * 2 * N;
 #pragma unroll
-            for (uint32_t j = 0; j < N / 2; j += 16) {
-                uint32_t raw[2][16];
-                tmem_load16_nowait(source + j, raw[0]);
-                tmem_load16_nowait(source + N + j, raw[1]);
+            for (uint32_t j = 0; j < N / 2; j += S::kPiece) {
+                uint32_t raw[2][S::kPiece];
+                load_columns(source + j, raw[0]);
+                load_columns(source + N + j, raw[1]);
                 tmem_load_wait();
                 // without a second block the other short sum is an old one
 #pragma unroll
-                for (uint32_t i = 0; i < 16; ++i) {
+                for (uint32_t i = 0; i < S::kPiece; ++i) {
                     sums[j + i] += __uint_as_float(raw[0][i]) + (both ? __uint_as_float(raw[1][i]) : 0.0f);
                 }
             }
@@ -367,11 +376,12 @@ linear_f32_umma_kernel(const __grid_constant__ CUtensorMap weight_map, const Lin
         if (!ok && lane == 0) give_up(4);
         tcgen05_fence_after();
 #pragma unroll
-        for (uint32_t j = 0; j < N / 2; j += 16) {
-            uint32_t raw[16];
-            tmem_load16(address + 4 * N + j, raw);
+        for (uint32_t j = 0; j < N / 2; j += S::kPiece) {
+            uint32_t raw[S::kPiece];
+            load_columns(address + 4 * N + j, raw);
+            tmem_load_wait();
 #pragma unroll
-            for (uint32_t i = 0; i < 16; ++i) {
+            for (uint32_t i = 0; i < S::kPiece; ++i) {
                 // a weight that is no finite number meets parts that are zero: the high part alone has the right answer
                 const float rest = __uint_as_float(raw[i]);
                 sums[j + i] += isfinite(rest) ? rest : 0.0f;
@@ -480,8 +490,8 @@ Choice choose(size_t m, size_t column_tiles, size_t k_blocks) {
         const size_t resident = splits == 1 ? 148 * Shape<N>::kCtas : resident_clusters<N>(splits);
         if (resident == 0) continue;
         const size_t waves = (tiles + resident - 1) / resident;
-        // Measured: a K block takes a CTA 100 + 16 N cycles (1000, 1650 and 2230 for N = 64, 96 and 128; the MMAs alone 6 N to
-        // 12 N), 1.6 times as long where two share an SM, and 11000 pass before the first and behind the last.
+        // Measured: a K block takes a CTA 100 + 16 N cycles (1000 and 1650 for N = 64 and 96; the MMAs alone 6 N to 12 N), 1.6
+        // times as long where two share an SM, and 11000 pass before the first and behind the last.
         const double block = (100.0 + 16.0 * N) * (Shape<N>::kCtas > 1 && tiles * splits > 148 ? 1.6 : 1.0);
         const double cycles = static_cast<double>(waves) * (block * static_cast<double>((k_blocks + splits - 1) / splits) + 11000.0) +
                               (splits > 1 ? 2000.0 : 0.0);
@@ -509,9 +519,9 @@ bool linear_f32_supports(const void* x, const void* weight, size_t m, size_t n, 
 
 cudaError_t launch_linear_f32(cudaStream_t stream, const void* x, const void* weight, void* y, size_t m, size_t n, size_t k) {
     if (m == 0 || n == 0) return cudaErrorInvalidValue;
-    cudaError_t status = allow_shared<32>();
-    if (status == cudaSuccess) status = allow_shared<64>();
-    if (status == cudaSuccess) status = allow_shared<96>();
+    cudaError_t status = m <= 16 ? allow_shared<16>() : allow_shared<32>();
+    if (status == cudaSuccess && m > 16) status = allow_shared<64>();
+    if (status == cudaSuccess && m > 16) status = allow_shared<96>();
     if (status != cudaSuccess) return status;
     CUtensorMap weight_map;
     if (!make_swizzled_2d_map(&weight_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, weight, n, k * 2, kTileM)) {
@@ -528,6 +538,7 @@ cudaError_t launch_linear_f32(cudaStream_t stream, const void* x, const void* we
     params.column_tiles = static_cast<uint32_t>((n + kTileM - 1) / kTileM);
     params.k_blocks = static_cast<uint32_t>((k + kBlockK - 1) / kBlockK);
     params.drop_block = wait_selftest_drop() ? 0u : 0xffffffffu;
+    if (m <= 16) return launch<16>(stream, params, weight_map, choose<16>(m, params.column_tiles, params.k_blocks));
     // the tile height that is through first: few rows waste less of a low one, 250 rows of 48 column tiles fill the device
     // with three of 96
     const Choice low = choose<32>(m, params.column_tiles, params.k_blocks), middle = choose<64>(m, params.column_tiles, params.k_blocks),

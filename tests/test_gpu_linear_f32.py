@@ -93,9 +93,9 @@ def test_values_that_are_no_finite_numbers(device, m, k, n):
 
 
 @pytest.mark.parametrize("m,k,n", [(31, 64, 127), (32, 72, 128), (64, 192, 129), (65, 128, 1), (96, 328, 300), (97, 520, 24),
-                                   (400, 2056, 700), (3, 2048, 1100)])
+                                   (400, 2056, 700), (3, 2048, 1100), (16, 2056, 300)])
 def test_edges_of_tiles(device, m, k, n):
-    """Tiles of 32, 64 and 96 rows by 128 columns, whole and cut; odd and even numbers of 64-wide blocks of k, the last one cut;
+    """Tiles of 16, 32, 64 and 96 rows by 128 columns, whole and cut; odd and even numbers of 64-wide blocks of k, the last one cut;
     sums in one CTA and in clusters."""
     rng = np.random.default_rng(m * k + n)
     weight = rng.standard_normal((n, k)).astype(np.float32).view(np.uint32) & 0xFFFF0000
