@@ -535,12 +535,14 @@ cudaError_t launch_tiles(cudaStream_t stream, const StackAttentionLaunch& launch
     bool alone = false;
     double best = 0.0;
     for (uint32_t size = 1; size <= kMostSplits; size *= 2) {
+        const double merge = size == 1 ? 0.0 : (size < 8 ? 2.9 : 4.5);
+        if (splits > 0 && best <= merge + 1.0) break;
         const bool spread = clusters <= resident_clusters<KC, VC, TILES>(size, true);
-        const size_t resident = resident_clusters<KC, VC, TILES>(size, false);
-        if (!spread && (clusters > resident || (size > 1 && clusters * size > 2 * 148))) continue;
+        const bool shares = !spread && (size == 1 || clusters * size <= 2 * 148) &&
+                            clusters <= resident_clusters<KC, VC, TILES>(size, false);
+        if (!spread && !shares) continue;
         const double rounds = static_cast<double>((pages + kWarps * size - 1) / (kWarps * size));
-        const double cost = rounds * (spread ? 1.0 : (TILES == 1 ? 1.5 : 2.0)) + (size == 1 ? 0.0 : (size < 8 ? 2.9 : 4.5)) *
-                                                                                    (spread || TILES == 1 ? 1.0 : 2.0);
+        const double cost = rounds * (spread ? 1.0 : (TILES == 1 ? 1.5 : 2.0)) + merge * (spread || TILES == 1 ? 1.0 : 2.0);
         if (splits == 0 || cost < best) {
             splits = size;
             alone = spread;
