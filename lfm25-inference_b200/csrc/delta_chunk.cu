@@ -23,7 +23,8 @@
 //   * the matrices' products are transposed (value columns are the rows of the MMA), and the contracted index of a fragment is
 //     numbered so that places j and j + 4 hold neighbours 2 j and 2 j + 1.  An accumulator is then the A operand of the next
 //     product as it stands: the state, the right-hand side and Y never leave their registers.
-//   * U, R, K, B and the triangles lie in shared memory as B fragments, already in two parts: 16 bytes per lane, one load.
+//   * U, R, K, B and the triangles lie in shared memory as B fragments, already in two parts: 16 bytes per lane, one load (K and B
+//     for ranks up to 64, beyond which there is no room).
 //   * the elements' own layout (tokens x channels) is that of A and B fragments too, so the triangles' products start from
 //     registers.
 // The elements take eight warps, the others four each; the matrices' warps get the registers that copies and triangles leave
@@ -53,9 +54,10 @@ constexpr uint32_t kThreads = 32 * (12 + kElementWarps);
 
 template <bool SPLIT>
 struct Layout {
-    uint32_t rank_pad, z_stride, early_row;
-    size_t early, late, rows, columns, partials, triangles, lower, decay_end, tanh_parts, w2, constants, scale, produced, total;
-    __host__ __device__ explicit Layout(uint32_t rank) {
+    uint32_t rank_pad = 0, z_stride = 0, early_row = 0;
+    size_t early = 0, late = 0, rows = 0, columns = 0, partials = 0, triangles = 0, lower = 0, decay_end = 0, tanh_parts = 0,
+           w2 = 0, constants = 0, scale = 0, produced = 0, total = 0;
+    __host__ __device__ constexpr explicit Layout(uint32_t rank) {
         rank_pad = (rank + 31) / 32 * 32;
         z_stride = rank_pad + 8;
         early_row = 3 * kDim + rank_pad + 8;
@@ -767,14 +769,16 @@ cudaError_t launch(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& args) {
 
 constexpr size_t kSharedLimit = 226 * 1024;            // beside the static word; holds Layout<false> of kMostRank
 constexpr uint32_t kMostRank = 128;                    // larger ones keep the plain f32 arithmetic of the prompt kernel
+constexpr uint32_t kMostTwoPartRank = 64;                // K and B in two parts where shared memory holds them
+static_assert(Layout<true>(kMostTwoPartRank).total <= kSharedLimit && Layout<true>(kMostTwoPartRank + 1).total > kSharedLimit &&
+                  Layout<false>(kMostRank).total <= kSharedLimit, "what shared memory holds");
 
 }  // namespace
 
 bool delta_chunk_takes(uint32_t dim, uint32_t rank) { return dim <= kDim && rank <= kMostRank; }
 
 cudaError_t launch_delta_chunk(cudaStream_t stream, const DeltaArgs<__nv_bfloat16>& args) {
-    // K and B in two parts where shared memory holds them (ranks up to 96)
-    return Layout<true>(args.rank).total <= kSharedLimit ? launch<true>(stream, args) : launch<false>(stream, args);
+    return args.rank <= kMostTwoPartRank ? launch<true>(stream, args) : launch<false>(stream, args);
 }
 
 }  // namespace lfm25

@@ -157,14 +157,14 @@ def test_delta_rule_prompt_kernels_agree(device, library_option, heads, dim, ran
         assert cases.relative_error(other, results[0]).max() < 4e-3
 
 
-@pytest.mark.parametrize("rank,chunks", [(64, [3, 200, 16, 33, 2, 65]), (96, [17, 15, 129]), (97, [31, 16, 47]), (128, [2, 64, 250]),
-                                         (120, [2 + index * 7 % 23 for index in range(64)]),
+@pytest.mark.parametrize("rank,chunks", [(64, [3, 200, 16, 33, 2, 65]), (65, [3, 16, 33, 140]), (96, [17, 15, 129]), (97, [31, 16, 47]),
+                                         (128, [2, 64, 250]), (120, [2 + index * 7 % 23 for index in range(64)]),
                                          (32, [2 + index * 11 % 37 for index in range(65)])],
                          ids=lambda value: str(value) if isinstance(value, int) else str(len(value)))
 def test_delta_rule_chunks(device, library_option, rank, chunks):
-    """Tensor-core chunks against the token-by-token prompt kernel where the ranks of the decays change the pipeline (96, 128) and
-    where segments are no longer taken longest first (64).  Both keep 32-bit accuracy, so that they differ by rounding of the
-    bf16 output only."""
+    """Tensor-core chunks against the token-by-token prompt kernel at the ranks of the decays where operands lie in one part
+    instead of two (65) and where the rows of z grow (97, 128), and where segments are no longer taken longest first (64).
+    Both keep 32-bit accuracy, so that they differ by rounding of the bf16 output only."""
     config = cases.config_of([cases.delta_layer(2, 64, ff=0)])
     tensors = cases.random_tensors(config, 41, rank)
     tensors["l0.mix.w0"][::2] = 9.0
