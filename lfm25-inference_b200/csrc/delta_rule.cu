@@ -6,13 +6,16 @@
 //
 // A column of S (one value channel) never meets another one, so a CTA takes the columns of one head of one sequence and
 // keeps them in registers over the whole segment: the state is read from and written to memory once per step however
-// long the segment is.  Few long bf16 segments are split along the sequence instead (delta_split.cu).  Four kernels:
+// long the segment is.  Few long bf16 segments are split along the sequence instead (delta_split.cu).  Kernels for single tokens:
 //   decode    one token per sequence: every load is issued up front, then three barriers
-//   chunk     bf16 segments, heads up to 64: tiles of 16 tokens as matrix products on the tensor cores (delta_chunk.cu)
-//   prompt    bf16 segments, larger heads: half of the warps prepare a tile of 16 tokens (decays with one small tensor-core
-//             product, removal rates, unit scales) and finish the previous one (norm, gate), the others run the recurrence
-//             over the tile between them; projections arrive through cp.async two tiles ahead
 //   general   one token per sequence, head sizes and ranks beyond the decode kernel
+// and for prompts:
+//   chunk     bf16 segments, heads up to 64, ranks up to 128: tiles of 16 tokens as matrix products on the tensor cores
+//             (delta_chunk.cu), or split along the sequence (delta_split.cu)
+//   prompt    bf16 segments, heads up to 128, ranks up to 256: half of the warps prepare a tile of 16 tokens (decays with one
+//             small tensor-core product, removal rates, unit scales) and finish the previous one (norm, gate), the others run
+//             the recurrence over the tile between them; projections arrive through cp.async two tiles ahead
+//   scan      every other segment, f32 ones among them, token by token in three kernels (delta_scan.cu)
 // Outside delta_chunk.cu and delta_split.cu all arithmetic on the state is f32 multiply-adds, two-wide where the
 // sm_100 packed instructions take it (each half rounds like the scalar one).
 #include <math.h>
@@ -921,10 +924,13 @@ bool prompt_kernels_take(const DeltaArgs<__nv_bfloat16>& args) {
 // Where prompts are split along the sequence (delta_split.cu) instead of carried by one CTA per segment and head: it does about
 // twice the arithmetic and takes three launches, so it pays while the carrying CTAs leave most SMs idle and a prompt is
 // long.  The lengths are on the device, so the line is drawn for segments of equal length, where the longest one does not
-// help.  Inside steps of whole models, segments x heads (of 64 dimensions): what a layer gains in us at tokens a segment
-//     16: 320 -1, 400 8, 512 22, 1000 90, 4000 392     32: 400 2, 600 -5, 1000 49, 4096 187
-//     48: 720 7, 1000 3, 2000 26                       64: 1000 -70, 2000 -114
-// (The lines were drawn between earlier forms of both; these meet within 5 us a layer of them.)
+// help.  Inside steps of four layers, segments x heads (of 64 dimensions): what a layer gains in us at tokens a segment (two
+// runs, one to eight segments)
+//     16: 320 6, 400 16, 500 33, 600 40, 1000 91          32: 320 -1, 400 5 to 7, 500 23, 600 4 to 8, 700 14 to 19, 1000 43 to 49
+//     48: 320 -4, 400 -24, 600 -5 to -9, 720 1 to 5, 800 -10 to -16, 1000 1 to 2, 1500 27
+//     64 (whole models): 1000 -70, 2000 -114
+// The steps in between are waves of CTAs.  (The lines were drawn between earlier forms of both.  Today's form beside them gains at
+// 16 and 32 heads wherever it is taken; at 48 it loses around 800 tokens.)
 constexpr size_t kSplitMostHeads = 48;             // of all segments
 constexpr size_t split_shortest(size_t heads) { return heads <= 16 ? 320 : (heads <= 32 ? 400 : 720); }
 

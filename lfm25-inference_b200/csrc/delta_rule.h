@@ -119,14 +119,6 @@ __device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA<NEAR
     const FragmentB<NEAREST> both[2] = {b0, b1};
     mma_split<NEAREST, 2>(d, a, both);
 }
-// B is exact in TF32
-__device__ __forceinline__ void mma_split(float (&d)[2][4], const FragmentA<>& a, const float (&b0)[2], const float (&b1)[2]) {
-    mma_tf32(d[0], a.low, b0);
-    mma_tf32(d[1], a.low, b1);
-    mma_tf32(d[0], a.high, b0);
-    mma_tf32(d[1], a.high, b1);
-}
-
 // rows `source[row * stride + column]` of a 16 x 8 operand
 template <bool NEAREST = false>
 __device__ __forceinline__ FragmentA<NEAREST> load_a(const float* source, uint32_t stride, uint32_t lane) {
@@ -149,21 +141,13 @@ __device__ __forceinline__ FragmentA<NEAREST> load_a_transposed(const float* sou
     out.set(3, at[4 * stride + 8]);
     return out;
 }
-// an 8 x 8 operand B[k][n] stored as `source[k * stride + n]`, or transposed as `source[n * stride + k]`
+// an 8 x 8 operand B[k][n] stored as `source[k * stride + n]`
 template <bool NEAREST = false>
 __device__ __forceinline__ FragmentB<NEAREST> load_b(const float* source, uint32_t stride, uint32_t lane) {
     FragmentB<NEAREST> out;
     const float* at = source + (lane & 3) * stride + (lane >> 2);
     out.set(0, at[0]);
     out.set(1, at[4 * stride]);
-    return out;
-}
-template <bool NEAREST = false>
-__device__ __forceinline__ FragmentB<NEAREST> load_b_transposed(const float* source, uint32_t stride, uint32_t lane) {
-    FragmentB<NEAREST> out;
-    const float* at = source + (lane >> 2) * stride + (lane & 3);
-    out.set(0, at[0]);
-    out.set(1, at[4]);
     return out;
 }
 // a 16 x 8 result to `target[row * stride + column]`
