@@ -241,6 +241,14 @@ int32_t project_qkv(lfm25_decode_executor* self, const lfm25_layer& layer, size_
 int32_t append_qkv(lfm25_decode_executor* self, const lfm25_qk_postprocess_launch& post, bool packed) {
     RegionTimer timer(self, LFM25_REGION_APPEND);
     if (!packed) return lfm25_qk_norm_rope_kv_write_decode(self->blaslt->stream, &post);
+    // what that call refuses of a model
+    if (post.num_pages == 0) {
+        return lfm25::report_error(LFM25_ERR_INVALID_ARGUMENT, "fused QK postprocess requires cache pages");
+    }
+    if (!post.query_norm.ptr || !post.key_norm.ptr || !post.inv_freq.ptr || !post.position_ids.ptr || !post.slot_mapping.ptr ||
+        !post.key_cache.ptr || !post.value_cache.ptr) {
+        return lfm25::report_error(LFM25_ERR_NULL_POINTER, "fused QK postprocess received a null device pointer");
+    }
     const uint16_t* packed_rows = static_cast<const uint16_t*>(self->wide);
     lfm25::QkPostprocessArgs strided;
     strided.query = packed_rows;

@@ -7,6 +7,7 @@ import torch
 
 from oracle import step_oracle
 from conftest import bits_of
+from lfm25_inference_b200 import Lfm25Error, _abi
 from lfm25_inference_b200 import model as lfm_model
 from lfm25_inference_b200 import ops, workloads
 from oracle import oracle
@@ -60,6 +61,30 @@ def test_mixed_step_against_the_oracle(device, use_fp8, prefixes, chunks):
         want = oracle.bf16_to_f32(host.layers[index]["conv_state"]).astype(np.float64)
         assert np.abs(got - want).max() <= (0.15 if use_fp8 else 0.05) * max(1.0, np.abs(want).max())
     assert ops.device_status()[0] == 0
+    executor.close()
+    blaslt.close()
+
+
+@pytest.mark.parametrize("pack_qkv", [True, False])
+@pytest.mark.parametrize("missing", ["query_norm", "key_norm", "key_cache", "value_cache"])
+def test_a_layer_without_its_tensors_is_refused(device, pack_qkv, missing):
+    """Before the kernel that would read or write them, whether or not the projections share one matrix."""
+    batch = workloads.mixed_step_batch(3, [0], [5], 4)
+    model = lfm_model.RandomModel(3, device, 4, 1, pack_qkv=pack_qkv)
+    blaslt = ops.BlasLt()
+    executor = lfm_model.DecodeExecutor(blaslt, 16, maximum_segments=2)
+    step = lfm_model.RaggedBatch(device, batch, np.arange(5, dtype=np.uint32))
+    layer = model.struct.layers[lfm_model.ATTENTION_LAYERS[0]]
+    pointer = getattr(layer, missing)
+    assert pointer
+    setattr(layer, missing, None)
+    with pytest.raises(Lfm25Error) as raised:
+        executor.forward_ragged(model, step, use_fp8=False)
+    assert raised.value.code == _abi.ERR_NULL_POINTER
+    torch.cuda.synchronize()
+    setattr(layer, missing, pointer)
+    executor.forward_ragged(model, step, use_fp8=False)
+    assert np.isfinite(oracle.bf16_to_f32(executor.logits(1))).all()
     executor.close()
     blaslt.close()
 
