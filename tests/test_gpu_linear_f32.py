@@ -11,8 +11,8 @@ pytestmark = pytest.mark.gpu
 
 # lfm25::launch_linear_f32(cudaStream_t, const void* x, const void* weight, void* y, size_t m, size_t n, size_t k)
 SYMBOL = "_ZN5lfm2517launch_linear_f32EP11CUstream_stPKvS3_Pvmmm"
-# row counts of every tile size (16, 32, three times 32, 64), sums in one CTA and shared by a cluster, sizes that end inside
-# a round of 32 and inside a tile of 128 columns
+# row counts of every tile size (16, 32, 64, 96), whole and cut, sums in one CTA and shared by a cluster, sizes that end inside a
+# block of 64 of k and inside a tile of 128 columns
 SHAPES = [(1, 8, 5), (16, 40, 128), (17, 1000, 130), (33, 1024, 64), (70, 1024, 260), (97, 136, 40), (250, 7168, 129)]
 
 
@@ -32,11 +32,11 @@ def product(device, x, weight):
 
 def sum_bound(k):
     """Part of the sum of the products' sizes that an error may be, with 64 products in a short sum: a rounding (2^-24) for each
-    of them, for every pair of them and in a cluster's sum; 2^-20 for what the tensor core cuts on the way: it adds four times
-    16 products, each time cutting less than 2^-22 of the largest term or partial sum for each of up to 17 terms' alignment
-    and the result, so less than 4 * 2^-22 of the products' sizes where it cuts terms that are aligned to their largest; and
-    2^-23 per 16 products for the two lower parts, which are at most 2^-7 of the first."""
-    return (k / 64 + k / 128 + 10) * 2.0 ** -24 + 2.0 ** -20 + k / 8 * 2.0 ** -30
+    of them, for every pair of them and in a cluster's sum; 2^-21 for what the tensor core cuts on the way (four steps of 16
+    products, each of which leaves off less than 2^-23 of the sizes that it adds up: one bit of f32 for the largest of them); and
+    2^-23 per 16 products for the two lower parts, which are at most 2^-7 of the first.  Errors measured over these tests' shapes
+    and seeds are at most a third of it."""
+    return (k / 64 + k / 128 + 8) * 2.0 ** -24 + 2.0 ** -21 + k / 8 * 2.0 ** -30
 
 
 def spread(rng, shape):
@@ -58,16 +58,13 @@ def test_nothing_of_x_is_lost(device, m, k, n):
 
 @pytest.mark.parametrize("m,k,n", SHAPES)
 def test_sums(device, m, k, n):
-    """Against float64, as part of the sum of the products' sizes: a rounding (2^-24) per 32 products and in the sums of a
-    cluster; inside the tensor cores, which cut, 2^-21 for the 32 products' own sum and 2^-23 per 16 for the two lower
-    parts, which are at most 2^-7 of the first."""
+    """Against float64, as part of the sum of the products' sizes."""
     rng = np.random.default_rng(k + m)
     weight = rng.standard_normal((n, k)).astype(np.float32).view(np.uint32) & 0xFFFF0000
     weight = weight.view(np.float32).astype(np.float64)
     for x in (spread(rng, (m, k)), rng.standard_normal((m, k)).astype(np.float32)):
         error = np.abs(product(device, x, weight) - x.astype(np.float64) @ weight.T)
-        bound = (k / 32 + 8) * 2.0 ** -24 + 2.0 ** -21 + k / 8 * 2.0 ** -30
-        assert (error <= bound * (np.abs(x).astype(np.float64) @ np.abs(weight).T)).all()
+        assert (error <= sum_bound(k) * (np.abs(x).astype(np.float64) @ np.abs(weight).T)).all()
 
 
 @pytest.mark.parametrize("m,k,n", SHAPES)
