@@ -336,33 +336,33 @@ int32_t feed_forward(lfm25_decode_executor* self, const lfm25_layer& layer, size
                                                kFfn));
         }
     } else {
-    LFM25_TRY(linear_decode(self, layer.gate_up, self->normalized, self->wide, tokens, use_fp8, gate_up_fp8));
-    if (use_fp8 && layer.down.fp8.data != nullptr) {
-        RegionTimer timer(self, LFM25_REGION_FP8_LINEAR);
-        LFM25_TRY(lfm25_silu_mul_packed_bf16_to_e4m3(stream, slice_of(self->wide, tokens * 2 * kFfn),
-                                                     slice_of(self->fp8_input, self->maximum_tokens * kFfn),
-                                                     tokens, kFfn, layer.down.fp8.activation_quantize));
-        lfm25_fp8_linear_config config;
-        config.m = tokens;
-        config.n = kHidden;
-        config.k = kFfn;
-        config.scale_mode = LFM25_FP8_SCALE_TENSORWIDE;
-        config.output_scale = layer.down.fp8.activation_dequantize * layer.down.fp8.weight_dequantize;
-        LFM25_TRY(lfm25_blaslt_linear_fp8_scaled(self->blaslt, slice_of(self->fp8_input, tokens * kFfn),
-                                                 slice_of(layer.down.fp8.data, kHidden * kFfn),
-                                                 slice_of(self->operator_output, tokens * kHidden), &config));
-    } else {
-        RegionTimer timer(self, LFM25_REGION_BF16_LINEAR);
-        LFM25_TRY(lfm25_silu_mul_packed_bf16(stream, slice_of(self->wide, tokens * 2 * kFfn),
-                                             slice_of(self->activated, tokens * kFfn), tokens, kFfn));
-        if (layer.down.bf16 == nullptr) {
-            return lfm25::report_error(LFM25_ERR_NULL_POINTER, "Down site has no BF16 weights resident");
+        LFM25_TRY(linear_decode(self, layer.gate_up, self->normalized, self->wide, tokens, use_fp8, gate_up_fp8));
+        if (use_fp8 && layer.down.fp8.data != nullptr) {
+            RegionTimer timer(self, LFM25_REGION_FP8_LINEAR);
+            LFM25_TRY(lfm25_silu_mul_packed_bf16_to_e4m3(stream, slice_of(self->wide, tokens * 2 * kFfn),
+                                                         slice_of(self->fp8_input, self->maximum_tokens * kFfn),
+                                                         tokens, kFfn, layer.down.fp8.activation_quantize));
+            lfm25_fp8_linear_config config;
+            config.m = tokens;
+            config.n = kHidden;
+            config.k = kFfn;
+            config.scale_mode = LFM25_FP8_SCALE_TENSORWIDE;
+            config.output_scale = layer.down.fp8.activation_dequantize * layer.down.fp8.weight_dequantize;
+            LFM25_TRY(lfm25_blaslt_linear_fp8_scaled(self->blaslt, slice_of(self->fp8_input, tokens * kFfn),
+                                                     slice_of(layer.down.fp8.data, kHidden * kFfn),
+                                                     slice_of(self->operator_output, tokens * kHidden), &config));
+        } else {
+            RegionTimer timer(self, LFM25_REGION_BF16_LINEAR);
+            LFM25_TRY(lfm25_silu_mul_packed_bf16(stream, slice_of(self->wide, tokens * 2 * kFfn),
+                                                 slice_of(self->activated, tokens * kFfn), tokens, kFfn));
+            if (layer.down.bf16 == nullptr) {
+                return lfm25::report_error(LFM25_ERR_NULL_POINTER, "Down site has no BF16 weights resident");
+            }
+            LFM25_TRY(lfm25_blaslt_linear_bf16(self->blaslt, slice_of(self->activated, tokens * kFfn),
+                                               slice_of(layer.down.bf16, kHidden * kFfn),
+                                               slice_of(self->operator_output, tokens * kHidden), tokens, kHidden,
+                                               kFfn));
         }
-        LFM25_TRY(lfm25_blaslt_linear_bf16(self->blaslt, slice_of(self->activated, tokens * kFfn),
-                                           slice_of(layer.down.bf16, kHidden * kFfn),
-                                           slice_of(self->operator_output, tokens * kHidden), tokens, kHidden,
-                                           kFfn));
-    }
     }
     return LFM25_OK;
 }
