@@ -280,15 +280,16 @@ state_space_chunk_kernel(const StateSpaceArgs<__nv_bfloat16> args, const PieceAr
                 const std::integral_constant<uint32_t, 1> one;
                 const std::integral_constant<uint32_t, 2> two;
                 const std::integral_constant<uint32_t, 3> three;
+                const uint32_t left = end - first;             // rows behind the end have no outputs
                 if (weigher == 0) {
                     weigh(zero, zero, zero);
-                    weigh(three, zero, zero);
+                    if (left > 48) weigh(three, zero, zero);
                 } else if (weigher == 1) {
-                    weigh(one, zero, one);
+                    if (left > 16) weigh(one, zero, one);
                 } else if (weigher == 2) {
-                    weigh(two, zero, two);
+                    if (left > 32) weigh(two, zero, two);
                 } else {
-                    weigh(three, one, three);
+                    if (left > 48) weigh(three, one, three);
                 }
             }
             barrier_arrive(kFullBarrier + buffer, kThreads);
@@ -308,13 +309,17 @@ state_space_chunk_kernel(const StateSpaceArgs<__nv_bfloat16> args, const PieceAr
     const uint32_t own = warp * 16;                    // first column
     // calls `visit` with the address in the record and the value
     const auto each_value = [&](auto&& visit) {
+        const uint32_t column = column0 + own + row0;
+        const bool inside[2] = {column < args.vdim, column + 8 < args.vdim};
+        float* at = state + static_cast<size_t>(pair) * args.vdim + column;
 #pragma unroll
         for (uint32_t tile = 0; tile < kTiles; ++tile) {
 #pragma unroll
             for (uint32_t i = 0; i < 4; ++i) {
-                const uint32_t n = tile * 8 + pair + (i & 1), v = column0 + own + row0 + (i >> 1) * 8;
-                if (n < args.size && v < args.vdim) visit(state + static_cast<size_t>(n) * args.vdim + v, held[tile][i]);
+                const uint32_t n = tile * 8 + pair + (i & 1);
+                if ((FULL || n < args.size) && inside[i >> 1]) visit(at + (i & 1) * args.vdim + (i >> 1) * 8, held[tile][i]);
             }
+            at += 8 * args.vdim;
         }
     };
     const auto read = [](const float* at, float& x) { x = *at; };
