@@ -16,7 +16,8 @@
 //     the same, all 1100    19.6 / 15.5 / 14.3                    24 tokens of 100 to 4000 on 2 of 128         21.2 / 18.3 / 18.6
 //     groups of 16 heads of 64: 32 tokens of 4096 on 1    19.5 / 36.2 / 13.9     64 of 1024 on 4     20.6 / 24.7 / 16.6
 //     8 tokens of 256 on 8 of 64    6.0 / 6.3 / 3.7               64 of 1024 on 8 of 64                        34.5 / 27.3 / 23.5
-// Over 552 shapes and contexts 0.82 of the first and 0.76 of the second.
+// Over 847 shapes and contexts, one to 192 tokens, 0.88 of the first and 0.86 of the second.  Equal long contexts in a few CTAs
+// more than are resident are what is slower than in either (40 tokens of 4096 keys on 8 heads of 64 57.2 / 66.2 / 67.7).
 #include <cooperative_groups.h>
 #include <math.h>
 
@@ -37,14 +38,14 @@ namespace cg = cooperative_groups;
 constexpr uint32_t kBoxBytes = kPageSize * 128;   // 16 keys x 64 dimensions
 constexpr uint32_t kGroupRows = 16;
 constexpr uint32_t kMostSplits = 8;
+constexpr size_t kLongPages = 128;
 // Of shared memory, so that no second CTA of the kernel is put on the SM while others are empty: 128 CTAs in clusters of 4 (32
 // tokens of 4096 keys, 16 heads on 1 with values of 128) 18.6 us, 27.0 with what they need.
 constexpr uint32_t kAloneBytes = 116 * 1024;
 
-// WIDE: eight warps with short rings, where all CTAs are resident at once and there is a page for more than half of them.
-// Otherwise four, so that more CTAs share an SM: 64 tokens of 1024 keys on 8 heads of 64 23.4 us, with eight warps 25.3.
-// Of 14 combinations of 4 to 12 warps, 2 to 4 stages and 1 or 2 pages at a time, (8, 2, 1) or its neighbours (8, 3, 1) and
-// (8, 2, 2) were fastest wherever all CTAs are resident.
+// WIDE: eight warps with short rings; otherwise four, so that more CTAs share an SM.  Of 14 combinations of 4 to 12 warps, 2 to 4
+// stages and 1 or 2 pages at a time, (8, 2, 1) or its neighbours (8, 3, 1) and (8, 2, 2) were fastest wherever all CTAs are
+// resident.
 template <uint32_t KC, uint32_t VC, uint32_t TILES, bool WIDE>
 struct Layout {
     static constexpr uint32_t kWarps = WIDE ? 8 : 4;
@@ -549,7 +550,13 @@ cudaError_t launch_tiles(cudaStream_t stream, const StackAttentionLaunch& launch
             best = cost;
         }
     }
-    if (splits > 0 && pages > kWarps / 2) return launch_form<KC, VC, TILES, true>(stream, launch, splits, alone);
+    // More CTAs than are resident: eight warps where contexts may be long, since of unequal ones the longest decides (80 tokens of
+    // 128 to 4096 keys, 8 heads of 64 59.5 us, with four warps 64.4; 96 of 4096 118 and 137), or where rings of three boxes leave
+    // room for two such CTAs anyway (keys of 128, values of 64: 128 tokens of 1024 keys 63 and 71; not with two tiles of columns);
+    // four for the others (64 of 256 keys 8.5, with eight 11.3).  All resident: four only where each has at most one page and no two CTAs share an SM.
+    const bool wide = splits == 0 ? (KC + VC == 3 && TILES == 1) || pages >= kLongPages
+                                  : pages > kWarps / 2 || clusters > 148;
+    if (wide) return launch_form<KC, VC, TILES, true>(stream, launch, std::max(splits, 1u), alone);
     return launch_form<KC, VC, TILES, false>(stream, launch, 1, clusters <= 148);
 }
 

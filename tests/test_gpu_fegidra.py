@@ -109,9 +109,15 @@ def check_decode_attention(device, library_option, heads, kv_heads, dim, prefixe
                                                        (20, 2, 128, 9)])
 def test_decode_attention_groups(device, library_option, heads, kv_heads, dim, copies):
     """The same with groups of eight heads and less, which are one tile of columns, and beyond, with heads of one to four
-    pieces of 64, and with more CTAs than are resident at once: every form, number of pages at a time and tiles of the
-    decode kernel."""
+    pieces of 64, and with more CTAs than are resident at once: every number of pieces and tiles of the decode kernel."""
     test_decode_attention_long_contexts(device, library_option, heads, kv_heads, dim, copies)
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,copies", [(8, 8, 64, 8), (72, 8, 64, 8), (20, 2, 128, 16), (6, 2, 136, 16), (24, 8, 104, 8),
+                                                       (36, 2, 72, 30)])
+def test_decode_attention_many_contexts(device, library_option, heads, kv_heads, dim, copies):
+    """More CTAs than are resident behind contexts that are not long, which four warps take."""
+    check_decode_attention(device, library_option, heads, kv_heads, dim, [3, 1022, 1023, 1024, 40, 200] * copies)
 
 
 @pytest.mark.parametrize("heads,kv_heads,dim", [(8, 1, 64), (18, 2, 64), (6, 2, 128), (11, 1, 104), (2, 2, 256), (9, 1, 136)])
