@@ -553,7 +553,8 @@ cudaError_t launch_tiles(cudaStream_t stream, const StackAttentionLaunch& launch
     // More CTAs than are resident: eight warps where contexts may be long, since of unequal ones the longest decides (80 tokens of
     // 128 to 4096 keys, 8 heads of 64 59.5 us, with four warps 64.4; 96 of 4096 118 and 137), or where rings of three boxes leave
     // room for two such CTAs anyway (keys of 128, values of 64: 128 tokens of 1024 keys 63 and 71; not with two tiles of columns);
-    // four for the others (64 of 256 keys 8.5, with eight 11.3).  All resident: four only where each has at most one page and no two CTAs share an SM.
+    // four for the others (64 of 256 keys 8.5, with eight 11.3).  All resident: four only where each has at most one page and no
+    // two CTAs share an SM.
     const bool wide = splits == 0 ? (KC + VC == 3 && TILES == 1) || pages >= kLongPages
                                   : pages > kWarps / 2 || clusters > 148;
     if (wide) return launch_form<KC, VC, TILES, true>(stream, launch, std::max(splits, 1u), alone);
